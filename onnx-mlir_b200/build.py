@@ -27,6 +27,7 @@ SOURCES = [
     "model/encoder.cpp",
     "kernels/dql.cu",
     "kernels/gemm_simt.cu",
+    "kernels/gemm_batched.cu",
     "kernels/gemm_tc.cu",
     "kernels/encoder_ops.cu",
     "kernels/attention_mma.cu",

@@ -292,6 +292,8 @@ struct MatDims {
   int64_t batch, M, K, N;
   bool b_batched;
   std::vector<int64_t> a_off, b_off;
+  // the same offsets as strides over the batch dimensions
+  std::vector<int64_t> size, a_stride, b_stride;
 };
 
 int matmul_dims(const OMTensor *A, const OMTensor *B, MatDims *d) {
@@ -338,6 +340,9 @@ int matmul_dims(const OMTensor *A, const OMTensor *B, MatDims *d) {
   }
   d->batch = batch;
   d->b_batched = true;
+  d->size = dims;
+  d->a_stride = astr;
+  d->b_stride = bstr;
   d->a_off.assign((size_t)batch, 0);
   d->b_off.assign((size_t)batch, 0);
   for (int64_t i = 0; i < batch; ++i) {
@@ -352,6 +357,34 @@ int matmul_dims(const OMTensor *A, const OMTensor *B, MatDims *d) {
     d->b_off[(size_t)i] = bo;
   }
   return OMCUDA_OK;
+}
+
+// The batch dimensions of a product for the one-launch kernel: dimensions of
+// size 1 dropped, neighbours that advance as one merged.  False when more
+// remain than its argument block holds.
+bool batched_dims(const MatDims &d, BatchedGemm *g) {
+  g->dims = 0;
+  for (size_t i = 0; i < d.size.size(); ++i) {
+    if (d.size[i] == 1)
+      continue;
+    if (g->dims > 0) {
+      const int p = g->dims - 1;
+      if (g->a_stride[p] == d.size[i] * d.a_stride[i] &&
+          g->b_stride[p] == d.size[i] * d.b_stride[i]) {
+        g->size[p] *= d.size[i];
+        g->a_stride[p] = d.a_stride[i];
+        g->b_stride[p] = d.b_stride[i];
+        continue;
+      }
+    }
+    if (g->dims == BatchedGemm::kMaxDims)
+      return false;
+    g->size[g->dims] = d.size[i];
+    g->a_stride[g->dims] = d.a_stride[i];
+    g->b_stride[g->dims] = d.b_stride[i];
+    ++g->dims;
+  }
+  return true;
 }
 
 bool is_8bit(OM_DATA_TYPE t) { return t == ONNX_TYPE_UINT8 || t == ONNX_TYPE_INT8; }
@@ -629,6 +662,23 @@ void omcudaMatMulInteger(OMTensor *Y, const OMTensor *A, const OMTensor *B,
   int32_t *dY = (int32_t *)sg.out(Y);
   if (!sg.ok())
     return;
+  // B is an activation: all products in one launch, nothing prepared.
+  BatchedGemm bg;
+  memset(&bg, 0, sizeof(bg));
+  if (azn <= 1 && gemm_batched_wanted(d.batch, d.M, d.N, d.K) && batched_dims(d, &bg) &&
+      !is_registered_constant(omTensorGetDataPtr(B))) {
+    bg.M = (int)d.M;
+    bg.N = (int)d.N;
+    bg.K = (int)d.K;
+    bg.a_zp = dAz;
+    bg.a_zp_len = (int)azn;
+    bg.b_zp = dBz;
+    bg.b_zp_len = (int)bzn;
+    sg.set(launch_gemm_batched(dA, at == ONNX_TYPE_INT8, dB, bt == ONNX_TYPE_INT8, dY,
+        d.batch, bg, st));
+    sg.finish(false);
+    return;
+  }
   // A B slice that several products share (a broadcast batch dimension) is
   // prepared once.
   std::map<int64_t, omcudaPreparedB> prepared;

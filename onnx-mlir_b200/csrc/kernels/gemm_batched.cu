@@ -1,0 +1,376 @@
+// int8 x int8 -> int32 products whose B operand is an activation: MatMulInteger
+// with a batched B (attention scores and contexts of a quantized model) or
+// with a small B that is no registered constant.  Replaces, like the other
+// GEMM kernels, the CPU loops of src/Conversion/ONNXToKrnl/Math/MatMulInteger.cpp:59-90.
+//
+// Preparing such a B as if it were a weight (a K-major copy and a column-sum
+// pass, two launches, then a GEMM launch per product) costs three launches for
+// each of the batch * heads products: 384 products of 128 x 64 x 128 took
+// 9.0 ms, all of it launches and launch gaps; 14.4 us with this kernel (256
+// products of 512 x 64 x 512: 7.0 ms -> 101 us, 2.7 TB/s of results).  One
+// launch covers every product and reads both operands as they lie:
+//
+//  * what bounds it is the i32 result (4 bytes per output against
+//    (M + N) K / (M N) bytes of operands: 25 of 31 MB for that shape), so the
+//    arithmetic runs on mma.sync (m16n8k32) from plain shared-memory tiles,
+//    which take any K, N and alignment -- a TMA tile would need 16-byte row
+//    pitches that a sequence length does not give;
+//  * a block of four warps makes a 64 x 64 tile (each warp 32 x 32) with 16 KiB
+//    of shared memory, so that several blocks per SM overlap one's loads with
+//    another's stores; the K loop is short (head size or sequence length);
+//  * B is transposed on its way into shared memory, four K rows by four
+//    columns at a time in registers; row sums of A and column sums of B for
+//    the zero points are taken there as well, where each byte passes once.
+#include "../runtime/internal.h"
+#include "gemm_epilogue.cuh"
+
+namespace omcuda {
+
+namespace {
+
+constexpr int kTile = 64;     // rows and columns of a block's tile
+constexpr int kRowBytes = 128; // of K in a shared-memory row
+constexpr int kBatThreads = 128;
+
+template <bool kASigned, bool kBSigned>
+__device__ __forceinline__ void mma_i8(int32_t (&c)[4], uint32_t a0, uint32_t a1,
+    uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+#define OMCUDA_MMA_I8(types)                                                   \
+  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32." types ".s32 "          \
+               "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"         \
+               : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])                \
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1))
+  if (kASigned && kBSigned)
+    OMCUDA_MMA_I8("s8.s8");
+  else if (kASigned)
+    OMCUDA_MMA_I8("s8.u8");
+  else if (kBSigned)
+    OMCUDA_MMA_I8("u8.s8");
+  else
+    OMCUDA_MMA_I8("u8.u8");
+#undef OMCUDA_MMA_I8
+}
+
+// Sum of the four bytes of w, added to c.
+template <bool kSigned>
+__device__ __forceinline__ int32_t add_bytes(uint32_t w, int32_t c) {
+  return kSigned ? __dp4a((int)w, 0x01010101, c)
+                 : (int32_t)__dp4a(w, 0x01010101u, (uint32_t)c);
+}
+
+// kWords words starting at any byte address, of which the first `len` bytes
+// (0..4 * kWords) exist; the rest reads as zero.  Only aligned words that hold
+// an existing byte are touched.
+template <int kWords>
+__device__ __forceinline__ void load_bytes(
+    const uint8_t *p, int len, uint32_t (&w)[kWords]) {
+  const int off = (int)((uintptr_t)p & 3u);
+  const uint32_t *q = reinterpret_cast<const uint32_t *>(p - off);
+  uint32_t raw[kWords + 1];
+#pragma unroll
+  for (int i = 0; i <= kWords; ++i)
+    raw[i] = (4 * i < len + off && len > 0) ? __ldg(q + i) : 0u;
+#pragma unroll
+  for (int i = 0; i < kWords; ++i) {
+    uint32_t v = __funnelshift_r(raw[i], raw[i + 1], 8 * off);
+    const int have = len - 4 * i;
+    w[i] = have >= 4 ? v : (have <= 0 ? 0u : v & ((1u << (8 * have)) - 1u));
+  }
+}
+
+// Shared-memory tiles are rows of 128 bytes of K in eight 16-byte chunks.  The
+// chunk index is XORed so that a fragment read (lanes of rows n, n + 1, four
+// chunks each) and the transposing write (lanes four rows apart, one word
+// each) both spread over the banks.
+__device__ __forceinline__ uint32_t chunk_at(int row, int chunk) {
+  return (uint32_t)(chunk ^ ((row >> 2) & 7) ^ ((row & 1) << 2)) * 16u;
+}
+
+} // namespace
+
+// kVecA / kVecB: every chunk of A is a whole aligned 16-byte one (K % 16 == 0),
+// every word of B an aligned one (N % 4 == 0).  kStep: bytes of K staged per step, 64
+// when K has no more (a head size), so that every thread has a chunk to load.
+template <bool kASigned, bool kBSigned, bool kVecA, bool kVecB, int kStep>
+__global__ void __launch_bounds__(kBatThreads, 5)
+    gemm_i8_batched_kernel(const uint8_t *__restrict__ A, const uint8_t *__restrict__ B,
+        int32_t *__restrict__ Y, BatchedGemm g) {
+  __shared__ __align__(16) uint8_t sA[kTile * kRowBytes];
+  __shared__ __align__(16) uint8_t sB[kTile * kRowBytes];
+  __shared__ int32_t s_row[kTile], s_col[kTile];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+  // Blocks of one product are neighbours: its operands stay in L1 / L2.
+  const uint32_t per = (uint32_t)g.tiles_m * (uint32_t)g.tiles_n;
+  const uint32_t prod = blockIdx.x / per, rest = blockIdx.x - prod * per;
+  const int tile_m = (int)(rest / (uint32_t)g.tiles_n);
+  const int m0 = tile_m * kTile, n0 = (int)(rest - (uint32_t)tile_m * g.tiles_n) * kTile;
+  {
+    uint32_t rem = prod;
+    for (int d = g.dims - 1; d >= 0; --d) {
+      const uint32_t size = (uint32_t)g.size[d], next = rem / size, i = rem - next * size;
+      rem = next;
+      A += (int64_t)i * g.a_stride[d];
+      B += (int64_t)i * g.b_stride[d];
+    }
+    Y += (int64_t)prod * ((int64_t)g.M * g.N);
+  }
+  const bool want_row = g.b_zp_len != 0, want_col = g.a_zp_len != 0;
+
+  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+  const int gq = lane >> 2, q = lane & 3;
+  int32_t acc[2][4][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        acc[i][j][e] = 0;
+
+  // A: thread -> one chunk of kARows rows.  B: thread -> four columns of
+  // kBBlocks groups of four K rows.
+  constexpr int kChunks = kStep / 16, kARowStep = kBatThreads / kChunks;
+  constexpr int kARows = kTile / kARowStep, kBBlocks = kStep / 32;
+  const int ac = tid % kChunks, ar = tid / kChunks;
+  const int bn = (tid & 15) * 4, bk = (tid >> 4) * 4;
+  const int ncols = g.N - (n0 + bn) < 4 ? g.N - (n0 + bn) : 4;
+  const uint8_t *pa = A + (m0 + ar) * g.K + 16 * ac; // (M K and K N are below 2^31)
+  const uint8_t *pb = B + bk * g.N + n0 + bn;
+  int32_t rsum[kARows], csum[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int i = 0; i < kARows; ++i)
+    rsum[i] = 0;
+
+  for (int k0 = 0; k0 < g.K; k0 += kStep) {
+    const int kk = g.K - k0 < kStep ? g.K - k0 : kStep;
+    uint32_t wa[kARows][4], wb[kBBlocks][4];
+    const int len = kk - 16 * ac > 16 ? 16 : kk - 16 * ac;
+#pragma unroll
+    for (int i = 0; i < kARows; ++i) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        wa[i][j] = 0;
+      if (m0 + ar + kARowStep * i < g.M && len > 0) {
+        const uint8_t *p = pa + kARowStep * i * g.K + k0;
+        if (kVecA) {
+          const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p));
+          wa[i][0] = v.x, wa[i][1] = v.y, wa[i][2] = v.z, wa[i][3] = v.w;
+        } else {
+          load_bytes(p, len, wa[i]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kBBlocks; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        wb[i][j] = 0;
+        if (bk + 32 * i + j < kk && ncols > 0) {
+          const uint8_t *p = pb + (k0 + 32 * i + j) * g.N;
+          if (kVecB) {
+            wb[i][j] = __ldg(reinterpret_cast<const uint32_t *>(p));
+          } else {
+            uint32_t w[1];
+            load_bytes(p, ncols, w);
+            wb[i][j] = w[0];
+          }
+        }
+      }
+    if (k0)
+      __syncthreads(); // the fragments of the step before have been read
+#pragma unroll
+    for (int i = 0; i < kARows; ++i) {
+      const int r = ar + kARowStep * i;
+      if (want_row)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          rsum[i] = add_bytes<kASigned>(wa[i][j], rsum[i]);
+      *reinterpret_cast<uint4 *>(sA + r * kRowBytes + chunk_at(r, ac)) =
+          make_uint4(wa[i][0], wa[i][1], wa[i][2], wa[i][3]);
+    }
+#pragma unroll
+    for (int i = 0; i < kBBlocks; ++i) {
+      const int k = bk + 32 * i;
+      // 4 x 4 bytes: word j of the result holds column j's four K values
+      const uint32_t(&r)[4] = wb[i];
+      const uint32_t t0 = __byte_perm(r[0], r[1], 0x5140), t1 = __byte_perm(r[2], r[3], 0x5140);
+      const uint32_t t2 = __byte_perm(r[0], r[1], 0x7362), t3 = __byte_perm(r[2], r[3], 0x7362);
+      const uint32_t c[4] = {__byte_perm(t0, t1, 0x5410), __byte_perm(t0, t1, 0x7632),
+          __byte_perm(t2, t3, 0x5410), __byte_perm(t2, t3, 0x7632)};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        *reinterpret_cast<uint32_t *>(
+            sB + (bn + j) * kRowBytes + chunk_at(bn + j, k >> 4) + (k & 15)) = c[j];
+        if (want_col)
+          csum[j] = add_bytes<kBSigned>(c[j], csum[j]);
+      }
+    }
+    __syncthreads();
+    // A lane's fragments are the 16 bytes at offset 16 q of its rows: the
+    // instruction orders K differently, but the same order for A and B gives
+    // the same sum, and one 16-byte read feeds two MMAs.
+#pragma unroll
+    for (int h = 0; h < kStep / 64; ++h) {
+      if (h * 64 >= kk)
+        break;
+      uint4 a[2][2], b[4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int r = wm + 16 * i + 8 * e + gq;
+          a[i][e] = *reinterpret_cast<const uint4 *>(sA + r * kRowBytes + chunk_at(r, 4 * h + q));
+        }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int n = wn + 8 * j + gq;
+        b[j] = *reinterpret_cast<const uint4 *>(sB + n * kRowBytes + chunk_at(n, 4 * h + q));
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          mma_i8<kASigned, kBSigned>(
+              acc[i][j], a[i][0].x, a[i][1].x, a[i][0].y, a[i][1].y, b[j].x, b[j].y);
+          mma_i8<kASigned, kBSigned>(
+              acc[i][j], a[i][0].z, a[i][1].z, a[i][0].w, a[i][1].w, b[j].z, b[j].w);
+        }
+    }
+  }
+
+  if (want_row) { // kChunks neighbouring lanes share a row
+#pragma unroll
+    for (int i = 0; i < kARows; ++i) {
+#pragma unroll
+      for (int o = 1; o < kChunks; o <<= 1)
+        rsum[i] += __shfl_xor_sync(0xffffffffu, rsum[i], o);
+      if (ac == 0)
+        s_row[ar + kARowStep * i] = rsum[i];
+    }
+  }
+  if (want_col) { // threads tid % 16 share four columns: two lanes of each warp
+    if (tid < kTile)
+      s_col[tid] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int32_t s = csum[j] + __shfl_xor_sync(0xffffffffu, csum[j], 16);
+      if (lane < 16)
+        atomicAdd(&s_col[bn + j], s);
+    }
+  }
+  if (want_row || want_col)
+    __syncthreads();
+
+  const int32_t az = want_col ? load_zp8(g.a_zp, 0, kASigned) : 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int nl = wn + 8 * j + 2 * q, n = n0 + nl;
+    if (n >= g.N)
+      continue;
+    // - az colsum[n] - bz[n] rowsum[m] + K az bz[n], wrapping
+    uint32_t bz[2] = {0, 0}, base[2] = {0, 0};
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      if (want_row && n + e < g.N)
+        bz[e] = (uint32_t)load_zp8(g.b_zp, g.b_zp_len == 1 ? 0 : n + e, kBSigned);
+      if (want_col)
+        base[e] = (uint32_t)az * ((uint32_t)g.K * bz[e] - (uint32_t)s_col[nl + e]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int ml = wm + 16 * i + 8 * e + gq, m = m0 + ml;
+        if (m >= g.M)
+          continue;
+        const uint32_t rs = want_row ? (uint32_t)s_row[ml] : 0u;
+        const uint32_t v0 = (uint32_t)acc[i][j][2 * e] + base[0] - bz[0] * rs;
+        const uint32_t v1 = (uint32_t)acc[i][j][2 * e + 1] + base[1] - bz[1] * rs;
+        int32_t *dst = Y + (int64_t)m * g.N + n;
+        if (g.y_vec) { // N even and Y 8-byte aligned: n + 1 < N
+          *reinterpret_cast<int2 *>(dst) = make_int2((int)v0, (int)v1);
+        } else {
+          dst[0] = (int32_t)v0;
+          if (n + 1 < g.N)
+            dst[1] = (int32_t)v1;
+        }
+      }
+  }
+}
+
+// A product of this many operations is worth preparing B for and running on
+// tcgen05: mma.sync makes the same tile several times slower, while the three
+// launches of the prepared path cost some 20 us.
+constexpr int64_t kBatchedMaxOps = int64_t(1) << 31;
+// One product alone has to fill the machine with 64 x 64 tiles and a K loop
+// that no other product overlaps: only small ones gain.
+constexpr int64_t kSingleMaxOps = int64_t(1) << 26;
+
+bool gemm_batched_wanted(int64_t batch, int64_t M, int64_t N, int64_t K) {
+  if (K <= 0 || M >= (int64_t(1) << 30) || N >= (int64_t(1) << 30) || K >= (int64_t(1) << 30))
+    return false;
+  const int64_t blocks = batch * ceil_div(M, kTile) * ceil_div(N, kTile);
+  if (blocks <= 0 || blocks >= (int64_t(1) << 31))
+    return false;
+  const double ops = 2.0 * (double)M * (double)N * (double)K;
+  return ops <= (double)(batch > 1 ? kBatchedMaxOps : kSingleMaxOps);
+}
+
+template <bool kASigned, bool kBSigned, bool kVecA, bool kVecB>
+static void launch_step(unsigned grid, const uint8_t *a, const uint8_t *b, int32_t *Y,
+    const BatchedGemm &g, cudaStream_t st) {
+  if (g.K <= 64)
+    gemm_i8_batched_kernel<kASigned, kBSigned, kVecA, kVecB, 64>
+        <<<grid, kBatThreads, 0, st>>>(a, b, Y, g);
+  else
+    gemm_i8_batched_kernel<kASigned, kBSigned, kVecA, kVecB, 128>
+        <<<grid, kBatThreads, 0, st>>>(a, b, Y, g);
+}
+
+template <bool kASigned, bool kBSigned>
+static void launch_variant(unsigned grid, bool vec_a, bool vec_b, const uint8_t *a,
+    const uint8_t *b, int32_t *Y, const BatchedGemm &g, cudaStream_t st) {
+  if (vec_a && vec_b)
+    launch_step<kASigned, kBSigned, true, true>(grid, a, b, Y, g, st);
+  else if (vec_a)
+    launch_step<kASigned, kBSigned, true, false>(grid, a, b, Y, g, st);
+  else if (vec_b)
+    launch_step<kASigned, kBSigned, false, true>(grid, a, b, Y, g, st);
+  else
+    launch_step<kASigned, kBSigned, false, false>(grid, a, b, Y, g, st);
+}
+
+int launch_gemm_batched(const void *A, int a_signed, const void *B, int b_signed,
+    int32_t *Y, int64_t batch, BatchedGemm g, cudaStream_t st) {
+  g.tiles_m = (int)ceil_div(g.M, kTile);
+  g.tiles_n = (int)ceil_div(g.N, kTile);
+  uintptr_t a_low = (uintptr_t)A | (uintptr_t)g.K, b_low = (uintptr_t)B | (uintptr_t)g.N;
+  for (int d = 0; d < g.dims; ++d) {
+    a_low |= (uintptr_t)g.a_stride[d];
+    b_low |= (uintptr_t)g.b_stride[d];
+  }
+  const bool vec_a = (a_low & 15u) == 0, vec_b = (b_low & 3u) == 0;
+  g.y_vec = (((uintptr_t)Y & 7u) == 0) && (g.N & 1) == 0;
+  const unsigned grid = (unsigned)(batch * g.tiles_m * g.tiles_n);
+  const uint8_t *a = (const uint8_t *)A, *b = (const uint8_t *)B;
+  switch ((a_signed ? 2 : 0) | (b_signed ? 1 : 0)) {
+  case 0:
+    launch_variant<false, false>(grid, vec_a, vec_b, a, b, Y, g, st);
+    break;
+  case 1:
+    launch_variant<false, true>(grid, vec_a, vec_b, a, b, Y, g, st);
+    break;
+  case 2:
+    launch_variant<true, false>(grid, vec_a, vec_b, a, b, Y, g, st);
+    break;
+  default:
+    launch_variant<true, true>(grid, vec_a, vec_b, a, b, Y, g, st);
+    break;
+  }
+  OMCUDA_CHECK_LAUNCH("gemm_i8_batched_kernel");
+  return OMCUDA_OK;
+}
+
+} // namespace omcuda

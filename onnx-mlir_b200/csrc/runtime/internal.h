@@ -48,6 +48,26 @@ bool gemm_tc_supported(const omcudaGemmArgs &a);
 int launch_gemm_tc(const omcudaGemmArgs &a, cudaStream_t st);
 int launch_gemm_simt(const omcudaGemmArgs &a, cudaStream_t st);
 
+// gemm_batched.cu: every product of a MatMulInteger whose B is an activation in
+// one launch, operands read as they lie.  Product i (row-major over size[])
+// reads A and B at the element offsets its strides give (0 along a broadcast
+// dimension) and writes Y at i * M * N.
+struct BatchedGemm {
+  static constexpr int kMaxDims = 6;
+  int M, N, K;
+  int dims;
+  int64_t size[kMaxDims], a_stride[kMaxDims], b_stride[kMaxDims];
+  const void *a_zp; // one value
+  int a_zp_len;     // 0 or 1
+  const void *b_zp;
+  int b_zp_len;     // 0, 1 or N
+  // set by the launcher
+  int tiles_m, tiles_n, y_vec;
+};
+bool gemm_batched_wanted(int64_t batch, int64_t M, int64_t N, int64_t K);
+int launch_gemm_batched(const void *A, int a_signed, const void *B, int b_signed,
+    int32_t *Y, int64_t batch, BatchedGemm g, cudaStream_t st);
+
 // attention_mma.cu
 bool attention_mma_supported(const float *Q, const float *K, const float *V,
     const float *out, int64_t dh, int64_t ld_in, int64_t ld_out);

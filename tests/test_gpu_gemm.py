@@ -511,3 +511,35 @@ def test_random_few_rows_long_k_auto_dispatch(gpu, seed):
     Y = dg.matmul_integer(A, B, za, None, 0)
     want = (A.astype(np.float64) - za.astype(np.float64).reshape(-1, 1)) @ B.astype(np.float64)
     assert np.array_equal(Y.astype(np.float64), want), (M, N, K, a_signed, b_signed)
+
+
+@pytest.mark.parametrize("lead,M,K,N,adt,bdt", [
+    ((1,), 1, 1, 1, np.uint8, np.int8),            # one byte each way
+    ((2, 3), 64, 64, 64, np.uint8, np.uint8),      # whole tiles, whole K blocks
+    ((2, 3), 61, 61, 64, np.uint8, np.uint8),      # odd K and row pitch
+    ((5,), 65, 129, 63, np.int8, np.uint8),        # one past the tile and the K step
+    ((3,), 128, 192, 130, np.int8, np.int8),       # N even, not a multiple of 4
+    ((2,), 17, 500, 77, np.uint8, np.int8),        # several K steps, ragged last one
+    ((), 33, 100, 45, np.uint8, np.uint8),         # one small product, B not a constant
+])
+def test_batched_b_operand(gpu, orc, lead, M, K, N, adt, bdt):
+    # Products whose B is an activation run as one launch on operands as they
+    # lie; also with A and B starting at an odd address (views of device
+    # buffers), which the word-wise loads have to shift.
+    rng = np.random.default_rng(31)
+    A, B = rand8(rng, lead + (M, K), adt), rand8(rng, lead + (K, N), bdt)
+    az, bz = rand8(rng, (), adt), rand8(rng, (), bdt)
+    bzn = rand8(rng, N, bdt)
+    for a_zp, b_zp in ((None, None), (az, None), (az, bz), (None, bzn), (az, bzn)):
+        want = orc.matmul_integer(A, B, a_zp, b_zp)
+        assert np.array_equal(gpu.matmul_integer(A, B, a_zp, b_zp), want), (a_zp, b_zp)
+    import torch
+    at, bt = (torch.empty(x.size + 3, dtype=torch.uint8, device="cuda") for x in (A, B))
+    at[3:] = torch.from_numpy(A.view(np.uint8).reshape(-1)).cuda()
+    bt[1:1 + B.size] = torch.from_numpy(B.view(np.uint8).reshape(-1)).cuda()
+    av = at[3:].view(torch.int8 if adt == np.int8 else torch.uint8).view(A.shape)
+    bv = bt[1:1 + B.size].view(torch.int8 if bdt == np.int8 else torch.uint8).view(B.shape)
+    torch.cuda.synchronize()
+    got = gpu.matmul_integer(gpu.Tensor.from_cuda_array(av), gpu.Tensor.from_cuda_array(bv), az, bz,
+                             device=True)
+    assert np.array_equal(got.numpy(), orc.matmul_integer(A, B, az, bz))
