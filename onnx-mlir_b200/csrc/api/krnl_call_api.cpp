@@ -280,6 +280,30 @@ int prepared_b(Stage &sg, const void *key_ptr, const void *b_dev, int b_signed,
   return OMCUDA_OK;
 }
 
+// Gives the GEMM g its A operand ([M,K], any alignment) and, when b_zp is
+// given, A's row sums.  The tensor-core kernels need rows that start 16-byte
+// aligned: an A that does not have them is copied into rows that do, in the
+// pass that makes the row sums.
+void set_a_operand(Stage &sg, GemmCall *g, const void *A, cudaStream_t st) {
+  g->A = A;
+  g->lda = g->K;
+  const bool aligned = (g->K % 16 == 0) && (((uintptr_t)A & 15u) == 0);
+  const bool sums = g->b_zp_len != 0;
+  if (aligned ? !sums : (!sums && g->M <= 16))
+    return; // (a few rows: the GEMV-shaped kernels read them as they are)
+  int32_t *rs = sums ? (int32_t *)sg.scratch((size_t)g->M * sizeof(int32_t)) : nullptr;
+  uint8_t *rows = nullptr;
+  if (!aligned) {
+    g->lda = (g->K + 15) & ~int64_t(15);
+    rows = (uint8_t *)sg.scratch((size_t)(g->M * g->lda));
+    g->A = rows;
+  }
+  if (!sg.ok())
+    return;
+  sg.set(launch_repitch(A, g->a_signed, g->M, g->K, g->lda, rows, rs, st));
+  g->a_rowsum = rs;
+}
+
 bool begin_call() { return !sticky_error() && ensure_init() == OMCUDA_OK; }
 
 // numpy-style matmul shapes (src/Dialect/ONNX/ONNXOps/Math/MatMul.cpp:46-166):
@@ -683,12 +707,10 @@ void omcudaMatMulInteger(OMTensor *Y, const OMTensor *A, const OMTensor *B,
   // prepared once.
   std::map<int64_t, omcudaPreparedB> prepared;
   for (int64_t b = 0; b < d.batch && sg.ok(); ++b) {
-    omcudaGemmArgs g;
-    memset(&g, 0, sizeof(g));
+    GemmCall g;
     g.M = d.M;
     g.N = d.N;
     g.K = d.K;
-    g.A = dA + d.a_off[(size_t)b];
     g.a_signed = at == ONNX_TYPE_INT8;
     const int64_t bo = d.b_off[(size_t)b];
     auto hit = prepared.find(bo);
@@ -705,16 +727,12 @@ void omcudaMatMulInteger(OMTensor *Y, const OMTensor *A, const OMTensor *B,
     g.a_zp_len = azn;
     g.b_zp = dBz;
     g.b_zp_len = bzn;
-    if (bzn) {
-      int32_t *rs = (int32_t *)sg.scratch((size_t)d.M * sizeof(int32_t));
-      if (!rs)
-        break;
-      sg.set(omcudaDevRowSum(g.A, g.a_signed, d.M, d.K, rs, st));
-      g.a_rowsum = rs;
-    }
+    set_a_operand(sg, &g, dA + d.a_off[(size_t)b], st);
+    if (!sg.ok())
+      break;
     g.epilogue = OMCUDA_EPI_I32;
     g.Y = dY + b * d.M * d.N;
-    sg.set(omcudaDevGemmI8(&g, st));
+    sg.set(gemm_i8(g, st));
   }
   sg.finish(true);
 }
@@ -794,12 +812,10 @@ void omcudaQLinearMatMul(OMTensor *y, const OMTensor *a, const OMTensor *aScale,
   }
   if (!sg.ok())
     return;
-  omcudaGemmArgs g;
-  memset(&g, 0, sizeof(g));
+  GemmCall g;
   g.M = d.M;
   g.N = d.N;
   g.K = d.K;
-  g.A = dA;
   g.a_signed = at == ONNX_TYPE_INT8;
   sg.set(prepared_b(sg, omTensorGetDataPtr(b), dB, bt == ONNX_TYPE_INT8, d.K, d.N,
       st, &g.B));
@@ -811,11 +827,7 @@ void omcudaQLinearMatMul(OMTensor *y, const OMTensor *a, const OMTensor *aScale,
   g.a_zp_len = 1;
   g.b_zp = dBz;
   g.b_zp_len = bzn;
-  int32_t *rs = (int32_t *)sg.scratch((size_t)d.M * sizeof(int32_t));
-  if (!rs)
-    return;
-  sg.set(omcudaDevRowSum(dA, g.a_signed, d.M, d.K, rs, st));
-  g.a_rowsum = rs;
+  set_a_operand(sg, &g, dA, st);
   g.epilogue = OMCUDA_EPI_REQUANT;
   g.Y = dY;
   g.sb = S;
@@ -823,7 +835,7 @@ void omcudaQLinearMatMul(OMTensor *y, const OMTensor *a, const OMTensor *aScale,
   g.y_zp = yzp;
   g.y_signed = yt == ONNX_TYPE_INT8;
   if (sg.ok())
-    sg.set(omcudaDevGemmI8(&g, st));
+    sg.set(gemm_i8(g, st));
   sg.finish(true);
 }
 
@@ -873,18 +885,38 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
   const void *dWz = sg.in(wZp);
   const float *dBias = (const float *)sg.in(bias);
   float *dY = (float *)sg.out(Y);
-  uint8_t *xq = (uint8_t *)sg.scratch((size_t)(d.M * d.K));
+  // The quantized activations get rows of a multiple of 16 bytes whatever K is,
+  // which is what the tensor-core kernels take (777 x 1001 x 1537: 686 us with the
+  // dp4a kernel, 27.7 us with them).
+  GemmCall g;
+  g.M = d.M;
+  g.N = d.N;
+  g.K = d.K;
+  g.lda = (d.K + 15) & ~int64_t(15);
+  uint8_t *xq = (uint8_t *)sg.scratch((size_t)(d.M * g.lda));
   float *xs = (float *)sg.scratch(16);
   void *scr = dql_scratch_for(sg, st);
   if (!sg.ok() || !scr)
     return;
   uint8_t *xz = (uint8_t *)(xs + 1);
-  sg.set(omcudaDevDynamicQuantizeLinear(dX, d.M * d.K, xq, xs, xz, scr, st));
-  omcudaGemmArgs g;
-  memset(&g, 0, sizeof(g));
-  g.M = d.M;
-  g.N = d.N;
-  g.K = d.K;
+  if (wzn) {
+    g.b_zp = dWz;
+    g.b_zp_len = wzn;
+    g.a_rowsum = (int32_t *)sg.scratch((size_t)d.M * sizeof(int32_t));
+    if (!sg.ok())
+      return;
+  }
+  if (g.lda == d.K) {
+    sg.set(omcudaDevDynamicQuantizeLinear(dX, d.M * d.K, xq, xs, xz, scr, st));
+    if (wzn && sg.ok())
+      sg.set(omcudaDevRowSum(xq, 0, d.M, d.K, (int32_t *)g.a_rowsum, st));
+  } else {
+    const float *params = nullptr;
+    sg.set(launch_dql_range(dX, d.M * d.K, scr, xs, xz, &params, st));
+    if (sg.ok())
+      sg.set(launch_quantize_rows(
+          dX, d.M, d.K, g.lda, xq, (int32_t *)g.a_rowsum, params, st));
+  }
   g.A = xq;
   g.a_signed = 0;
   if (sg.ok())
@@ -892,16 +924,6 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
         d.N, st, &g.B));
   g.a_zp = xz;
   g.a_zp_len = 1;
-  if (wzn) {
-    g.b_zp = dWz;
-    g.b_zp_len = wzn;
-    int32_t *rs = (int32_t *)sg.scratch((size_t)d.M * sizeof(int32_t));
-    if (!rs)
-      return;
-    if (sg.ok())
-      sg.set(omcudaDevRowSum(xq, 0, d.M, d.K, rs, st));
-    g.a_rowsum = rs;
-  }
   g.epilogue = OMCUDA_EPI_DEQUANT;
   g.Y = dY;
   g.sa = xs;
@@ -910,7 +932,7 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
   g.scale_form = (int)scaleForm;
   g.bias = dBias;
   if (sg.ok())
-    sg.set(omcudaDevGemmI8(&g, st));
+    sg.set(gemm_i8(g, st));
   sg.finish(true);
 }
 

@@ -238,6 +238,53 @@ __global__ void __launch_bounds__(kDqlThreads)
   }
 }
 
+// The quantize pass for rows whose length is no multiple of 16, written in the
+// aligned rows the GEMM kernels take (zero from cols up to pitch), with the sums
+// of the quantized rows where the weight has a zero point.  One block per row
+// at a time: a thread makes one output word from four neighbouring values.
+__global__ void __launch_bounds__(kDqlThreads)
+    quantize_rows_kernel(const float *__restrict__ x, int64_t rows, int cols, int pitch,
+        uint8_t *__restrict__ y, int32_t *__restrict__ rowsum,
+        const float *__restrict__ params, int mode) {
+  __shared__ int32_t part[kDqlThreads / 32];
+  const QuantConsts qc = make_quant_consts(__ldg(params), __ldg(params + 1), mode);
+  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+    const float *xr = x + r * cols;
+    uint32_t *yr = reinterpret_cast<uint32_t *>(y + r * pitch);
+    int32_t sum = 0;
+    for (int j = threadIdx.x; 4 * j < pitch; j += kDqlThreads) {
+      const int have = cols - 4 * j;
+      float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (e < have)
+          v[e] = __ldg(xr + 4 * j + e);
+      uint32_t w = 0;
+      if (have > 0)
+        w = quantize_four<false>(make_float4(v[0], v[1], v[2], v[3]), qc);
+      if (have > 0 && have < 4)
+        w &= (1u << (8 * have)) - 1u;
+      yr[j] = w;
+      sum = add_bytes<false>(w, sum);
+    }
+    if (rowsum) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      __syncthreads(); // part[] of the row before has been read
+      if ((threadIdx.x & 31) == 0)
+        part[threadIdx.x >> 5] = sum;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        int32_t s = 0;
+        for (int w = 0; w < kDqlThreads / 32; ++w)
+          s += part[w];
+        rowsum[r] = s;
+      }
+    }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
     dequantize_kernel(const T *__restrict__ x, int64_t n,
@@ -273,6 +320,25 @@ int launch_quantize_with_params(const float *x, int64_t n, uint8_t *y,
   return OMCUDA_OK;
 }
 
+int launch_quantize_rows(const float *x, int64_t rows, int64_t cols, int64_t pitch,
+    uint8_t *y, int32_t *rowsum, const float *params, cudaStream_t st) {
+  const int64_t cap = (int64_t)sm_count() * 8;
+  quantize_rows_kernel<<<(unsigned)(rows < cap ? rows : cap), kDqlThreads, 0, st>>>(
+      x, rows, (int)cols, (int)pitch, y, rowsum, params, quant_mode());
+  OMCUDA_CHECK_LAUNCH("quantize_rows_kernel");
+  return OMCUDA_OK;
+}
+
+int launch_dql_range(const float *x, int64_t n, void *scratch, float *y_scale,
+    uint8_t *y_zp, const float **params, cudaStream_t st) {
+  DqlScratch *scr = (DqlScratch *)scratch;
+  dql_minmax_kernel<<<grid_for(n, kDqlThreads * 16), kDqlThreads, 0, st>>>(
+      x, n, scr, y_scale, y_zp, quant_mode());
+  OMCUDA_CHECK_LAUNCH("dql_minmax_kernel");
+  *params = scr->params;
+  return OMCUDA_OK;
+}
+
 } // namespace omcuda
 
 using namespace omcuda;
@@ -286,12 +352,12 @@ extern "C" int omcudaDevDynamicQuantizeLinear(const float *x, int64_t n,
   if (n < 0 || (n > 0 && (!x || !y)) || !scratch)
     return fail(OMCUDA_EINVAL, "DynamicQuantizeLinear: bad argument");
   cudaStream_t st = (cudaStream_t)stream;
-  DqlScratch *scr = (DqlScratch *)scratch;
-  int grid = grid_for(n, kDqlThreads * 16);
-  dql_minmax_kernel<<<grid, kDqlThreads, 0, st>>>(x, n, scr, y_scale, y_zp, quant_mode());
-  OMCUDA_CHECK_LAUNCH("dql_minmax_kernel");
+  const float *params = nullptr;
+  int rc = launch_dql_range(x, n, scratch, y_scale, y_zp, &params, st);
+  if (rc != OMCUDA_OK)
+    return rc;
   if (n > 0)
-    return launch_quantize_with_params(x, n, y, scr->params, st);
+    return launch_quantize_with_params(x, n, y, params, st);
   return OMCUDA_OK;
 }
 

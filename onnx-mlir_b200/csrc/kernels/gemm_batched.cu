@@ -51,33 +51,6 @@ __device__ __forceinline__ void mma_i8(int32_t (&c)[4], uint32_t a0, uint32_t a1
 #undef OMCUDA_MMA_I8
 }
 
-// Sum of the four bytes of w, added to c.
-template <bool kSigned>
-__device__ __forceinline__ int32_t add_bytes(uint32_t w, int32_t c) {
-  return kSigned ? __dp4a((int)w, 0x01010101, c)
-                 : (int32_t)__dp4a(w, 0x01010101u, (uint32_t)c);
-}
-
-// kWords words starting at any byte address, of which the first `len` bytes
-// (0..4 * kWords) exist; the rest reads as zero.  Only aligned words that hold
-// an existing byte are touched.
-template <int kWords>
-__device__ __forceinline__ void load_bytes(
-    const uint8_t *p, int len, uint32_t (&w)[kWords]) {
-  const int off = (int)((uintptr_t)p & 3u);
-  const uint32_t *q = reinterpret_cast<const uint32_t *>(p - off);
-  uint32_t raw[kWords + 1];
-#pragma unroll
-  for (int i = 0; i <= kWords; ++i)
-    raw[i] = (4 * i < len + off && len > 0) ? __ldg(q + i) : 0u;
-#pragma unroll
-  for (int i = 0; i < kWords; ++i) {
-    uint32_t v = __funnelshift_r(raw[i], raw[i + 1], 8 * off);
-    const int have = len - 4 * i;
-    w[i] = have >= 4 ? v : (have <= 0 ? 0u : v & ((1u << (8 * have)) - 1u));
-  }
-}
-
 // Shared-memory tiles are rows of 128 bytes of K in eight 16-byte chunks.  The
 // chunk index is XORed so that a fragment read (lanes of rows n, n + 1, four
 // chunks each) and the transposing write (lanes four rows apart, one word

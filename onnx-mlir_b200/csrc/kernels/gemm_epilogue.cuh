@@ -28,11 +28,13 @@
 #pragma once
 
 #include "../common.cuh"
+#include "../runtime/internal.h"
 
 namespace omcuda {
 
 struct EpiParams {
   int64_t M, N, K;
+  int64_t lda; // row pitch of A in bytes
   const void *a_zp;
   int a_zp_len; // 0, 1, or M
   int a_signed;
@@ -72,7 +74,7 @@ struct EpiParams {
 };
 
 // Host: flattens the public argument block (gemm_simt.cu).
-EpiParams make_epi_params(const omcudaGemmArgs &a);
+EpiParams make_epi_params(const GemmCall &a);
 
 // The tails that start with the DEQUANT arithmetic.
 __host__ __device__ constexpr bool epi_is_dequant(int kind) {

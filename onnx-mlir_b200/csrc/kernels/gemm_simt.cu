@@ -63,20 +63,36 @@ __global__ void __launch_bounds__(256)
                 part[2][threadIdx.x] + part[3][threadIdx.x];
 }
 
+// One warp per row, a 16-byte chunk per lane and trip; with dst, the row is also
+// copied into an aligned row of `pitch` bytes whose tail is zero.
 template <bool kSigned>
 __global__ void __launch_bounds__(256)
     rowsum_kernel(const uint8_t *__restrict__ A, int64_t M, int64_t K,
-        int32_t *__restrict__ rowsum) {
-  // One warp per row.
+        int32_t *__restrict__ rowsum, uint8_t *__restrict__ dst, int64_t pitch) {
   const int64_t m = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (m >= M)
     return;
   const int lane = threadIdx.x & 31;
+  const uint8_t *row = A + m * K;
+  const bool vec = (((uintptr_t)row) & 15u) == 0;
   int32_t s = 0;
-  for (int64_t k = lane; k < K; k += 32) {
-    uint8_t a = A[m * K + k];
-    s += kSigned ? (int32_t)(int8_t)a : (int32_t)a;
+#pragma unroll 4
+  for (int64_t k = 16 * lane; k < K; k += 512) {
+    uint32_t w[4];
+    if (vec && k + 16 <= K) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row + k));
+      w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+    } else {
+      load_bytes(row + k, (int)(K - k < 16 ? K - k : 16), w);
+    }
+    if (dst)
+      *reinterpret_cast<uint4 *>(dst + m * pitch + k) = make_uint4(w[0], w[1], w[2], w[3]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      s = add_bytes<kSigned>(w[j], s);
   }
+  if (!rowsum)
+    return;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
     s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -108,19 +124,17 @@ __device__ __forceinline__ int32_t dp4a_mixed(uint32_t a, uint32_t b, int32_t c)
   return d;
 }
 
+// 16 bytes of row m of A from K offset k0 on, zeros beyond the matrix.  vec_ok:
+// rows are 16-byte aligned and, where K ends inside a chunk, zero up to its end.
 __device__ __forceinline__ uint4 load_a_chunk(const uint8_t *__restrict__ A,
-    int64_t m, int64_t M, int64_t K, int64_t k0, bool vec_ok) {
-  uint4 v = make_uint4(0, 0, 0, 0);
-  if (m >= M)
-    return v;
-  if (vec_ok && k0 + 16 <= K)
-    return __ldg(reinterpret_cast<const uint4 *>(A + m * K + k0));
-  uint32_t w[4] = {0, 0, 0, 0};
-  for (int j = 0; j < 16; ++j) {
-    int64_t k = k0 + j;
-    if (k < K)
-      w[j >> 2] |= (uint32_t)A[m * K + k] << (8 * (j & 3));
-  }
+    int64_t m, const EpiParams &p, int64_t k0, bool vec_ok) {
+  if (m >= p.M || k0 >= p.K)
+    return make_uint4(0, 0, 0, 0);
+  const uint8_t *src = A + m * p.lda + k0;
+  if (vec_ok)
+    return __ldg(reinterpret_cast<const uint4 *>(src));
+  uint32_t w[4];
+  load_bytes(src, (int)(p.K - k0 < 16 ? p.K - k0 : 16), w);
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
@@ -133,7 +147,7 @@ __global__ void __launch_bounds__(256)
   const int64_t m0 = (int64_t)blockIdx.y * MT;
   if (n >= p.N)
     return; // whole warp leaves together
-  const bool vec_ok = ((p.K & 15) == 0) && (((uintptr_t)A & 15u) == 0);
+  const bool vec_ok = ((p.lda & 15) == 0) && (((uintptr_t)A & 15u) == 0);
   int32_t acc[MT];
 #pragma unroll
   for (int i = 0; i < MT; ++i)
@@ -144,7 +158,7 @@ __global__ void __launch_bounds__(256)
     uint4 b = __ldg(brow + c);
 #pragma unroll
     for (int i = 0; i < MT; ++i) {
-      uint4 a = load_a_chunk(A, m0 + i, p.M, p.K, c << 4, vec_ok);
+      uint4 a = load_a_chunk(A, m0 + i, p, c << 4, vec_ok);
       int32_t s = acc[i];
       s = dp4a_mixed<kASigned, kBSigned>(a.x, b.x, s);
       s = dp4a_mixed<kASigned, kBSigned>(a.y, b.y, s);
@@ -212,7 +226,7 @@ __global__ void __launch_bounds__(32 * kGemvWarps)
         const uint8_t *__restrict__ Bt, int64_t kp, EpiParams p) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t m0 = (int64_t)blockIdx.y * MT;
-  const bool vec_ok = ((p.K & 15) == 0) && (((uintptr_t)A & 15u) == 0);
+  const bool vec_ok = ((p.lda & 15) == 0) && (((uintptr_t)A & 15u) == 0);
   const int64_t chunks = kp >> 4;
   constexpr int kStep = 32 * kGemvWarps;
   __shared__ int32_t part[kGemvWarps][MT * CB];
@@ -238,7 +252,7 @@ __global__ void __launch_bounds__(32 * kGemvWarps)
     auto consume = [&](int64_t c, const uint4 (&b)[CB]) {
 #pragma unroll
       for (int i = 0; i < MT; ++i) {
-        const uint4 a = load_a_chunk(A, m0 + i, p.M, p.K, c << 4, vec_ok);
+        const uint4 a = load_a_chunk(A, m0 + i, p, c << 4, vec_ok);
 #pragma unroll
         for (int j = 0; j < CB; ++j) {
           int32_t s = acc[i][j];
@@ -364,7 +378,7 @@ __global__ void __launch_bounds__(32 * kGemvMmaWarps)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, q = lane & 3;
   const int64_t m0 = (int64_t)blockIdx.y * 16;
-  const bool vec_ok = ((p.K & 15) == 0) && (((uintptr_t)A & 15u) == 0);
+  const bool vec_ok = ((p.lda & 15) == 0) && (((uintptr_t)A & 15u) == 0);
   const int64_t blocks64 = (kp + 63) >> 6;
   __shared__ int32_t part[kGemvMmaWarps][16][kCols + 1];
   const EpiScalars sc = epi_scalars(p);
@@ -401,8 +415,8 @@ __global__ void __launch_bounds__(32 * kGemvMmaWarps)
 #pragma unroll
       for (int u = 0; u < kGemvMmaUnroll; ++u) {
         const int64_t koff = ((b0 + u) << 6) + 16 * q;
-        const uint4 a_lo = load_a_chunk(A, m0 + g, p.M, p.K, koff, vec_ok);
-        const uint4 a_hi = load_a_chunk(A, m0 + g + 8, p.M, p.K, koff, vec_ok);
+        const uint4 a_lo = load_a_chunk(A, m0 + g, p, koff, vec_ok);
+        const uint4 a_hi = load_a_chunk(A, m0 + g + 8, p, koff, vec_ok);
 #pragma unroll
         for (int j = 0; j < CG; ++j) {
           mma_m16n8k32<kASigned, kBSigned>(
@@ -451,11 +465,12 @@ __global__ void __launch_bounds__(32 * kGemvMmaWarps)
     epi_range_commit(p.out_range, lo, hi);
 }
 
-EpiParams make_epi_params(const omcudaGemmArgs &a) {
+EpiParams make_epi_params(const GemmCall &a) {
   EpiParams p;
   p.M = a.M;
   p.N = a.N;
   p.K = a.K;
+  p.lda = a.lda;
   p.a_zp = a.a_zp;
   p.a_zp_len = a.a_zp ? (int)(a.a_zp_len > 1 ? 2 : a.a_zp_len) : 0;
   p.a_signed = a.a_signed;
@@ -493,7 +508,7 @@ EpiParams make_epi_params(const omcudaGemmArgs &a) {
 }
 
 template <int MT>
-static void launch_warp_gemm(const omcudaGemmArgs &a, cudaStream_t st) {
+static void launch_warp_gemm(const GemmCall &a, cudaStream_t st) {
   EpiParams p = make_epi_params(a);
   dim3 grid((unsigned)ceil_div(a.N, 8), (unsigned)ceil_div(a.M, MT));
   const uint8_t *A = (const uint8_t *)a.A;
@@ -516,7 +531,7 @@ static void launch_warp_gemm(const omcudaGemmArgs &a, cudaStream_t st) {
 }
 
 template <int MT, int CB>
-static void launch_gemv(const omcudaGemmArgs &a, cudaStream_t st) {
+static void launch_gemv(const GemmCall &a, cudaStream_t st) {
   EpiParams p = make_epi_params(a);
   // Up to 12 resident blocks of 128 threads per SM (1536 threads, 8 x 16-byte
   // loads in flight each with CB = 4).
@@ -543,7 +558,7 @@ static void launch_gemv(const omcudaGemmArgs &a, cudaStream_t st) {
 }
 
 template <int CG>
-static void launch_gemv_mma(const omcudaGemmArgs &a, cudaStream_t st) {
+static void launch_gemv_mma(const GemmCall &a, cudaStream_t st) {
   EpiParams p = make_epi_params(a);
   // One block per 8 * CG columns (it reads 8 * CG * K bytes of the weight); very
   // wide weights wrap around a grid of 16 blocks per SM.
@@ -595,7 +610,7 @@ static int64_t gemv_max_m() {
   return gemv_mma_max_m() > 4 ? gemv_mma_max_m() : 4;
 }
 
-int launch_gemm_simt(const omcudaGemmArgs &a, cudaStream_t st) {
+int launch_gemm_simt(const GemmCall &a, cudaStream_t st) {
   // The GEMV-shaped kernels: dp4a up to 4 rows, mma.sync above (with more
   // rows the dp4a work per weight byte outgrows the weight read).
   // (OMCUDA_GEMV_MMA_MIN_M moves the hand-over from the dp4a kernel, for
@@ -631,6 +646,17 @@ int launch_gemm_simt(const omcudaGemmArgs &a, cudaStream_t st) {
   else
     launch_warp_gemm<16>(a, st);
   OMCUDA_CHECK_LAUNCH("gemm_i8_warp_kernel");
+  return OMCUDA_OK;
+}
+
+int launch_repitch(const void *A, int a_signed, int64_t M, int64_t K, int64_t pitch,
+    uint8_t *dst, int32_t *rowsum, cudaStream_t st) {
+  const unsigned grid = (unsigned)ceil_div(M, 8);
+  if (a_signed)
+    rowsum_kernel<true><<<grid, 256, 0, st>>>((const uint8_t *)A, M, K, rowsum, dst, pitch);
+  else
+    rowsum_kernel<false><<<grid, 256, 0, st>>>((const uint8_t *)A, M, K, rowsum, dst, pitch);
+  OMCUDA_CHECK_LAUNCH("rowsum_kernel");
   return OMCUDA_OK;
 }
 
@@ -677,13 +703,7 @@ extern "C" int omcudaDevRowSum(const void *A, int a_signed, int64_t M,
   if (!A || !rowsum || M <= 0 || K <= 0)
     return fail(OMCUDA_EINVAL, "RowSum: bad argument");
   cudaStream_t st = (cudaStream_t)stream;
-  unsigned grid = (unsigned)ceil_div(M, 8);
-  if (a_signed)
-    rowsum_kernel<true><<<grid, 256, 0, st>>>((const uint8_t *)A, M, K, rowsum);
-  else
-    rowsum_kernel<false><<<grid, 256, 0, st>>>((const uint8_t *)A, M, K, rowsum);
-  OMCUDA_CHECK_LAUNCH("rowsum_kernel");
-  return OMCUDA_OK;
+  return launch_repitch(A, a_signed, M, K, 0, nullptr, rowsum, st);
 }
 
 extern "C" int omcudaDevRequantScale(const float *a_scale, const float *b_scale,
@@ -699,7 +719,10 @@ extern "C" int omcudaDevRequantScale(const float *a_scale, const float *b_scale,
 extern "C" int omcudaDevGemmI8(const omcudaGemmArgs *args, void *stream) {
   if (!args)
     return fail(OMCUDA_EINVAL, "GemmI8: null args");
-  const omcudaGemmArgs &a = *args;
+  return gemm_i8(GemmCall(*args), (cudaStream_t)stream);
+}
+
+int omcuda::gemm_i8(const GemmCall &a, cudaStream_t st) {
   if (a.M < 0 || a.N <= 0 || a.K <= 0 || !a.A || !a.B.bt ||
       (!a.Y && a.epilogue != OMCUDA_EPI_DEQUANT_RANGE))
     return fail(OMCUDA_EINVAL, "GemmI8: bad shape or null operand");
@@ -729,7 +752,6 @@ extern "C" int omcudaDevGemmI8(const omcudaGemmArgs *args, void *stream) {
     return fail(OMCUDA_EINVAL, "GemmI8: requant epilogue needs S");
   if (a.epilogue != OMCUDA_EPI_I32 && a.sb_len != 1 && a.sb_len != a.N)
     return fail(OMCUDA_EINVAL, "GemmI8: scale length must be 1 or N");
-  cudaStream_t st = (cudaStream_t)stream;
   bool tc_ok = gemm_tc_supported(a);
   if (a.kernel_choice == 1 && !tc_ok)
     return fail(OMCUDA_ENOTSUP,

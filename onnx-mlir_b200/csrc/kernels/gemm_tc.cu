@@ -92,6 +92,12 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a,
                : "memory");
 }
 
+__device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+
 // ---- epilogue arithmetic on one 32-column chunk ---------------------------------------
 
 // Loads 32 consecutive per-column values with 16-byte loads when allowed.
@@ -337,7 +343,6 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
   constexpr int kSlabsPerHalf = kHalfCols / kSlabCols;
   static_assert(kHalfCols % 32 == 0 && kHalfCols % kSlabCols == 0, "tile shape");
   const int64_t m = m_warp + lane;
-  const bool y4_ok = ((p.N & 3) == 0) && (((uintptr_t)p.Y & 15u) == 0);
   const bool row_ok = m < p.M;
   EpiRow row;
   row.az = 0;
@@ -429,8 +434,11 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
       }
     }
   } else {
-    // Fallback when the row pitch of Y is not a multiple of 16 bytes:
-    // direct stores, one row per thread.
+    // The row pitch of Y is not a multiple of 16 bytes (a ragged N), so no TMA
+    // store: a 32 x 32 block passes through the slab and every row leaves as
+    // one coalesced warp-wide store, instead of 32 rows in 32 sectors each
+    // (777 x 1001 x 1537, f32: the whole call 687 -> 27.7 us with padded rows
+    // on these kernels instead of the dp4a one).
 #pragma unroll 1
     for (int c = 0; c < kHalfCols; c += 32) {
       uint32_t v[32];
@@ -441,12 +449,15 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
         release();
       const int64_t nc = n0 + c;
       const int valid = (int)((p.N - nc) < 32 ? (p.N - nc) : 32);
-      if (!row_ok || valid <= 0)
+      if (valid <= 0)
         continue;
-      epilogue_chunk<EPI>(p, sc, qc, row, res_row, nc, valid, v, lo, hi);
+      if (row_ok)
+        epilogue_chunk<EPI>(p, sc, qc, row, res_row, nc, valid, v, lo, hi);
       if (kNoStore)
         continue;
       if (kSplit) {
+        if (!row_ok)
+          continue;
         split_words_bf16(v);
         uint16_t *dhi = reinterpret_cast<uint16_t *>(p.Y) + m * p.N + nc;
         uint16_t *dlo = dhi + p.M * p.N;
@@ -456,25 +467,32 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
             dhi[j] = (uint16_t)(v[j >> 1] >> (16 * (j & 1)));
             dlo[j] = (uint16_t)(v[16 + (j >> 1)] >> (16 * (j & 1)));
           }
-      } else if (kOutBytes == 4) {
-        uint32_t *dst = reinterpret_cast<uint32_t *>(p.Y) + m * p.N + nc;
-        if (y4_ok && valid == 32) {
+        continue;
+      }
+      // slab word (r, j) sits at piece (j / 4) ^ (r % 8) of row r
+      const int rows = (int)(p.M - m_warp < 32 ? p.M - m_warp : 32);
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            reinterpret_cast<uint4 *>(dst)[j] = make_uint4(
-                v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (j < valid)
-              dst[j] = v[j];
+      for (int j = 0; j < 8; ++j)
+        if (!kPacked)
+          st_shared_v4(slab0 + (uint32_t)lane * 128u + (uint32_t)((j ^ (lane & 7)) * 16),
+              v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        else if (j < 2)
+          st_shared_v4(slab0 + (uint32_t)lane * 128u + (uint32_t)((j ^ (lane & 7)) * 16),
+              v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      __syncwarp();
+      const int piece = kPacked ? lane >> 4 : lane >> 2;
+      const uint32_t in_piece = kPacked ? (uint32_t)(lane & 15) & ~3u : (uint32_t)(lane & 3) * 4u;
+      for (int r = 0; r < rows; ++r) {
+        const uint32_t w = ld_shared_u32(
+            slab0 + (uint32_t)r * 128u + (uint32_t)((piece ^ (r & 7)) * 16) + in_piece);
+        if (lane < valid) {
+          const int64_t at = (m_warp + r) * p.N + nc + lane;
+          if (kOutBytes == 4)
+            reinterpret_cast<uint32_t *>(p.Y)[at] = w;
+          else
+            reinterpret_cast<uint8_t *>(p.Y)[at] =
+                (uint8_t)(kPacked ? w >> (8 * (lane & 3)) : w);
         }
-      } else {
-        uint8_t *dst = reinterpret_cast<uint8_t *>(p.Y) + m * p.N + nc;
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (j < valid)
-            dst[j] = kPacked ? (uint8_t)(v[j >> 2] >> (8 * (j & 3))) : (uint8_t)v[j];
       }
     }
   }
@@ -1096,7 +1114,7 @@ uint32_t make_idesc(int a_signed, int b_signed, int n) {
 // 16-byte stores of whole lines need an aligned base and row pitch (the
 // range-only tail stores nothing and walks the tile the same way).
 template <int EPI>
-bool y_takes_line_stores(const omcudaGemmArgs &a) {
+bool y_takes_line_stores(const GemmCall &a) {
   if (EPI == OMCUDA_EPI_DEQUANT_RANGE)
     return true;
   const int esize = (EPI == OMCUDA_EPI_REQUANT || EPI == OMCUDA_EPI_DEQUANT_QUANT)
@@ -1111,7 +1129,7 @@ bool y_takes_line_stores(const omcudaGemmArgs &a) {
 // them (16-byte aligned base and row pitch); otherwise the kernel stores
 // directly and never reads the maps.
 template <int EPI>
-int make_y_maps(const omcudaGemmArgs &a, int half_cols, bool line_store,
+int make_y_maps(const GemmCall &a, int half_cols, bool line_store,
     CUtensorMap *map_y, CUtensorMap *map_y2) {
   memset(map_y, 0, sizeof(*map_y));
   memset(map_y2, 0, sizeof(*map_y2));
@@ -1224,8 +1242,8 @@ __global__ void __launch_bounds__(256)
 }
 
 // The arguments of the pass that produces the raw partial sums.
-omcudaGemmArgs split_pass_args(const omcudaGemmArgs &a, const SplitPlan &plan) {
-  omcudaGemmArgs r = a;
+GemmCall split_pass_args(const GemmCall &a, const SplitPlan &plan) {
+  GemmCall r = a;
   r.epilogue = OMCUDA_EPI_I32;
   r.a_zp = nullptr;
   r.a_zp_len = 0;
@@ -1239,7 +1257,7 @@ omcudaGemmArgs split_pass_args(const omcudaGemmArgs &a, const SplitPlan &plan) {
 }
 
 template <int BN, int EPI, int EW>
-int launch_bn_epi_ew(const omcudaGemmArgs &a, cudaStream_t st, const SplitPlan &plan = SplitPlan()) {
+int launch_bn_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan = SplitPlan()) {
   using Cfg = TcConfig<BN, EW>;
   static PerDeviceInt attr_set;
   if (!attr_set.get()) {
@@ -1248,7 +1266,7 @@ int launch_bn_epi_ew(const omcudaGemmArgs &a, cudaStream_t st, const SplitPlan &
     attr_set.set(1);
   }
   CUtensorMap map_a, map_b;
-  int rc = make_map(&map_a, a.A, a.M, a.K, a.K, kBM);
+  int rc = make_map(&map_a, a.A, a.M, a.K, a.lda, kBM);
   if (rc != OMCUDA_OK)
     return rc;
   rc = make_map(&map_b, a.B.bt, a.N, a.B.kp, a.B.kp, BN);
@@ -1263,7 +1281,7 @@ int launch_bn_epi_ew(const omcudaGemmArgs &a, cudaStream_t st, const SplitPlan &
   if (!status)
     return fail(OMCUDA_ENOMEM, "GemmI8: cannot allocate the status word");
   CUtensorMap map_y, map_y2;
-  omcudaGemmArgs ya = a; // the matrix the stores see: all slices of the workspace
+  GemmCall ya = a; // the matrix the stores see: all slices of the workspace
   if (plan.split > 1)
     ya.M = plan.split * plan.ws_rows;
   rc = make_y_maps<EPI>(ya, epi_cols_per_warp(BN, EW), p.line_store != 0, &map_y, &map_y2);
@@ -1281,7 +1299,7 @@ int launch_bn_epi_ew(const omcudaGemmArgs &a, cudaStream_t st, const SplitPlan &
 // A long K loop hides the epilogue behind the MMAs and wants pipeline depth;
 // a short one is bounded by the epilogue and wants more warps on it.
 // (OMCUDA_GEMM_EW=8|16 overrides the choice, for experiments.)
-inline bool want_wide_epilogue(const omcudaGemmArgs &a) {
+inline bool want_wide_epilogue(const GemmCall &a) {
   static const int forced = [] {
     const char *s = getenv("OMCUDA_GEMM_EW");
     return s ? atoi(s) : 0;
@@ -1292,13 +1310,13 @@ inline bool want_wide_epilogue(const omcudaGemmArgs &a) {
 }
 
 template <int BN, int EPI>
-int launch_bn_epi(const omcudaGemmArgs &a, cudaStream_t st) {
+int launch_bn_epi(const GemmCall &a, cudaStream_t st) {
   return want_wide_epilogue(a) ? launch_bn_epi_ew<BN, EPI, 16>(a, st)
                                : launch_bn_epi_ew<BN, EPI, 8>(a, st);
 }
 
 template <int BN>
-int launch_bn(const omcudaGemmArgs &a, cudaStream_t st) {
+int launch_bn(const GemmCall &a, cudaStream_t st) {
   switch (a.epilogue) {
   case OMCUDA_EPI_I32:
     return launch_bn_epi<BN, OMCUDA_EPI_I32>(a, st);
@@ -1329,7 +1347,7 @@ inline bool pair_half_tiles_wanted() {
 
 // The 2-CTA kernel: 256 x 256 tiles on clusters of two CTAs.
 template <int EPI, int EW>
-int launch_pair_epi_ew(const omcudaGemmArgs &a, cudaStream_t st, const SplitPlan &plan = SplitPlan()) {
+int launch_pair_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan = SplitPlan()) {
   constexpr int kThreads = tc_threads(EW);
   constexpr int kPairSmemBytes =
       tc_stages(kBM * kBK + 128 * kBK, EW) * (kBM * kBK + 128 * kBK) +
@@ -1356,7 +1374,7 @@ int launch_pair_epi_ew(const omcudaGemmArgs &a, cudaStream_t st, const SplitPlan
     max_clusters_dev.set(max_clusters);
   }
   CUtensorMap map_a, map_b;
-  int rc = make_map(&map_a, a.A, a.M, a.K, a.K, kBM);
+  int rc = make_map(&map_a, a.A, a.M, a.K, a.lda, kBM);
   if (rc != OMCUDA_OK)
     return rc;
   rc = make_map(&map_b, a.B.bt, a.N, a.B.kp, a.B.kp, 128);
@@ -1403,7 +1421,7 @@ int launch_pair_epi_ew(const omcudaGemmArgs &a, cudaStream_t st, const SplitPlan
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   CUtensorMap map_y, map_y2;
-  omcudaGemmArgs ya = a; // the matrix the stores see: all slices of the workspace
+  GemmCall ya = a; // the matrix the stores see: all slices of the workspace
   if (plan.split > 1)
     ya.M = plan.split * plan.ws_rows;
   rc = make_y_maps<EPI>(ya, epi_cols_per_warp(256, EW), p.line_store != 0, &map_y, &map_y2);
@@ -1417,12 +1435,12 @@ int launch_pair_epi_ew(const omcudaGemmArgs &a, cudaStream_t st, const SplitPlan
 }
 
 template <int EPI>
-int launch_pair_epi(const omcudaGemmArgs &a, cudaStream_t st) {
+int launch_pair_epi(const GemmCall &a, cudaStream_t st) {
   return want_wide_epilogue(a) ? launch_pair_epi_ew<EPI, 16>(a, st)
                                : launch_pair_epi_ew<EPI, 8>(a, st);
 }
 
-int launch_pair(const omcudaGemmArgs &a, cudaStream_t st) {
+int launch_pair(const GemmCall &a, cudaStream_t st) {
   switch (a.epilogue) {
   case OMCUDA_EPI_I32:
     return launch_pair_epi<OMCUDA_EPI_I32>(a, st);
@@ -1458,7 +1476,7 @@ inline int split_k_forced() {
 // would occupy at most half of the machine and the K loop is long (measured
 // with 32..512 rows: K = 14336, N = 4096 29-36 us against 43-45 us unsplit;
 // K = 4096 20-37 us against 19-27 us, so K below 8192 stays unsplit).
-int split_k_for(const omcudaGemmArgs &a, cudaStream_t st) {
+int split_k_for(const GemmCall &a, cudaStream_t st) {
   if (split_k_forced() == 0 || a.M > 512 || a.N < 256 || (a.N & 3) != 0)
     return 1;
   if (a.epilogue != OMCUDA_EPI_I32 && a.epilogue != OMCUDA_EPI_DEQUANT &&
@@ -1489,7 +1507,7 @@ int split_k_for(const omcudaGemmArgs &a, cudaStream_t st) {
   return (int)split;
 }
 
-int launch_split_k(const omcudaGemmArgs &a, cudaStream_t st, int split) {
+int launch_split_k(const GemmCall &a, cudaStream_t st, int split) {
   SplitPlan plan;
   plan.split = split;
   plan.ws_rows = (a.M + 31) & ~int64_t(31);
@@ -1497,7 +1515,7 @@ int launch_split_k(const omcudaGemmArgs &a, cudaStream_t st, int split) {
   plan.ws = static_cast<int32_t *>(pool_alloc_on(ws_bytes, st));
   if (!plan.ws)
     return fail(OMCUDA_ENOMEM, "GemmI8: cannot allocate the split-K workspace");
-  const omcudaGemmArgs part = split_pass_args(a, plan);
+  const GemmCall part = split_pass_args(a, plan);
   int rc;
   if (a.M > kBM)
     rc = want_wide_epilogue(a) ? launch_pair_epi_ew<OMCUDA_EPI_I32, 16>(part, st, plan)
@@ -1524,13 +1542,13 @@ int launch_split_k(const omcudaGemmArgs &a, cudaStream_t st, int split) {
 
 } // namespace
 
-bool gemm_tc_supported(const omcudaGemmArgs &a) {
-  return (a.K % 16 == 0) && (((uintptr_t)a.A & 15u) == 0) &&
+bool gemm_tc_supported(const GemmCall &a) {
+  return (a.lda % 16 == 0) && (((uintptr_t)a.A & 15u) == 0) &&
          (((uintptr_t)a.B.bt & 15u) == 0) && a.M < (int64_t(1) << 31) &&
          a.N < (int64_t(1) << 31);
 }
 
-int launch_gemm_tc(const omcudaGemmArgs &a, cudaStream_t st) {
+int launch_gemm_tc(const GemmCall &a, cudaStream_t st) {
   // Tile width: the widest tile that still gives every SM work
   // (OMCUDA_GEMM_BN=64|128|256 overrides the choice, 512 selects the 2-CTA
   // kernel, for experiments).

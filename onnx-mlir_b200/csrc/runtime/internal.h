@@ -43,10 +43,35 @@ uint64_t tc_wait_limit_ns();
 int launch_quantize_with_params(const float *x, int64_t n, uint8_t *y,
     const float *params, cudaStream_t st);
 
+// DynamicQuantizeLinear's reduction alone: scale and zero point of x.  *params
+// (in scratch, see omcudaDevDynamicQuantizeLinear) is what the quantize passes take.
+int launch_dql_range(const float *x, int64_t n, void *scratch, float *y_scale,
+    uint8_t *y_zp, const float **params, cudaStream_t st);
+// The quantize pass of a [rows, cols] matrix into rows of
+// `pitch` bytes (a multiple of 16, y 16-byte aligned), the tail of a row zero:
+// the form the GEMM kernels take when cols is no multiple of 16.  rowsum (i32
+// [rows], sums of a row's bytes) may be null.
+int launch_quantize_rows(const float *x, int64_t rows, int64_t cols, int64_t pitch,
+    uint8_t *y, int32_t *rowsum, const float *params, cudaStream_t st);
+
 // gemm_tc.cu / gemm_simt.cu
-bool gemm_tc_supported(const omcudaGemmArgs &a);
-int launch_gemm_tc(const omcudaGemmArgs &a, cudaStream_t st);
-int launch_gemm_simt(const omcudaGemmArgs &a, cudaStream_t st);
+//
+// What the library itself can say about a GEMM beyond the public argument block.
+struct GemmCall : omcudaGemmArgs {
+  // Row pitch of A in bytes.  More than K only with rows that start 16-byte
+  // aligned and hold zeros from K up to the next multiple of 16.
+  int64_t lda;
+  GemmCall() : omcudaGemmArgs(), lda(0) {}
+  explicit GemmCall(const omcudaGemmArgs &a) : omcudaGemmArgs(a), lda(a.K) {}
+};
+int gemm_i8(const GemmCall &a, cudaStream_t st);
+bool gemm_tc_supported(const GemmCall &a);
+int launch_gemm_tc(const GemmCall &a, cudaStream_t st);
+int launch_gemm_simt(const GemmCall &a, cudaStream_t st);
+// Copies an 8-bit [M,K] matrix of any alignment into rows of `pitch` bytes (a
+// multiple of 16, dst 16-byte aligned), zero from K on; rowsum may be null.
+int launch_repitch(const void *A, int a_signed, int64_t M, int64_t K, int64_t pitch,
+    uint8_t *dst, int32_t *rowsum, cudaStream_t st);
 
 // gemm_batched.cu: every product of a MatMulInteger whose B is an activation in
 // one launch, operands read as they lie.  Product i (row-major over size[])

@@ -543,3 +543,33 @@ def test_batched_b_operand(gpu, orc, lead, M, K, N, adt, bdt):
     got = gpu.matmul_integer(gpu.Tensor.from_cuda_array(av), gpu.Tensor.from_cuda_array(bv), az, bz,
                              device=True)
     assert np.array_equal(got.numpy(), orc.matmul_integer(A, B, az, bz))
+
+
+@pytest.mark.parametrize("M,K,N,wdt", [
+    (1, 17, 5, np.uint8), (16, 257, 33, np.int8),   # GEMV-shaped kernels, padded rows
+    (17, 15, 64, np.uint8),                         # less than one 16-byte chunk of K
+    (33, 129, 63, np.int8),                         # one past a K step, ragged store
+    (300, 1001, 257, np.uint8),                     # several tiles each way
+    (2100, 143, 300, np.int8),                      # CTA pairs
+])
+def test_ragged_k_and_n(gpu, orc, M, K, N, wdt):
+    # K that is no multiple of 16: the quantized rows (and an 8-bit A) are laid
+    # out with a padded pitch for the tensor-core kernels.  N that is none:
+    # results leave row by row instead of through TMA stores.
+    rng = np.random.default_rng(32)
+    X = rng.normal(size=(M, K)).astype(np.float32)
+    W, wz, bias = rand8(rng, (K, N), wdt), rand8(rng, (), wdt), rng.normal(size=N).astype(np.float32)
+    ref = orc.dyn_quant_linear(X, W, 0.01, bias) if wdt == np.int8 else None
+    if ref is not None:
+        assert gpu.dyn_quant_linear(X, W, np.float32(0.01), None, bias).tobytes() == ref["Y"].tobytes()
+    xq, xs, xz = orc.dynamic_quantize_linear(X)
+    acc = orc.matmul_integer(xq, W, xz, wz)
+    want = orc.dequant_tail(acc, xs * np.float32(0.01), 0.0, 0, bias)
+    assert gpu.dyn_quant_linear(X, W, np.float32(0.01), wz, bias).tobytes() == want.tobytes()
+    # per-row A zero points take the prepared path whatever the size
+    azn, bzn = rand8(rng, M, np.uint8), rand8(rng, N, wdt)
+    assert np.array_equal(gpu.matmul_integer(xq, W, azn, bzn), orc.matmul_integer_2d(xq, W, azn, bzn))
+    if wdt == np.int8:
+        bs = rng.uniform(0.001, 0.01, N).astype(np.float32)
+        args = (xq, np.float32(0.02), np.uint8(128), W, bs, bzn, np.float32(0.5), np.uint8(7))
+        assert np.array_equal(gpu.qlinear_matmul(*args), orc.qlinear_matmul(*args))
