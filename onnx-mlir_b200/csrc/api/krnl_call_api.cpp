@@ -552,11 +552,17 @@ void omcudaDynamicQuantizeLinear(
   uint8_t *dy = (uint8_t *)sg.out(y);
   float *ds = (float *)sg.out(yScale);
   uint8_t *dz = (uint8_t *)sg.out(yZp);
+  const int64_t n = omTensorGetNumElems(x);
+  if (dql_small_wanted(1, n)) {
+    if (sg.ok())
+      sg.set(launch_dql_small(dx, 1, n, n, dy, nullptr, ds, dz, st));
+    sg.finish(false);
+    return;
+  }
   void *scr = dql_scratch_for(sg, st);
   if (!sg.ok() || !scr)
     return;
-  sg.set(omcudaDevDynamicQuantizeLinear(
-      dx, omTensorGetNumElems(x), dy, ds, dz, scr, st));
+  sg.set(omcudaDevDynamicQuantizeLinear(dx, n, dy, ds, dz, scr, st));
   sg.finish(false);
 }
 
@@ -895,8 +901,9 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
   g.lda = (d.K + 15) & ~int64_t(15);
   uint8_t *xq = (uint8_t *)sg.scratch((size_t)(d.M * g.lda));
   float *xs = (float *)sg.scratch(16);
-  void *scr = dql_scratch_for(sg, st);
-  if (!sg.ok() || !scr)
+  const bool small = dql_small_wanted(d.M, g.lda);
+  void *scr = small ? nullptr : dql_scratch_for(sg, st);
+  if (!sg.ok() || (!small && !scr))
     return;
   uint8_t *xz = (uint8_t *)(xs + 1);
   if (wzn) {
@@ -906,7 +913,10 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
     if (!sg.ok())
       return;
   }
-  if (g.lda == d.K) {
+  if (small) {
+    sg.set(launch_dql_small(
+        dX, d.M, d.K, g.lda, xq, (int32_t *)g.a_rowsum, xs, xz, st));
+  } else if (g.lda == d.K) {
     sg.set(omcudaDevDynamicQuantizeLinear(dX, d.M * d.K, xq, xs, xz, scr, st));
     if (wzn && sg.ok())
       sg.set(omcudaDevRowSum(xq, 0, d.M, d.K, (int32_t *)g.a_rowsum, st));

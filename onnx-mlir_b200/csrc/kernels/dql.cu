@@ -14,9 +14,13 @@
 // another.  The quantize pass is a second launch that reads the two scalars
 // from device memory; for tensors that fit in L2 its read of x is served from
 // there.
+#include <cooperative_groups.h>
+
 #include "../common.cuh"
 #include "../runtime/internal.h"
 #include "quantize.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace omcuda {
 
@@ -285,6 +289,149 @@ __global__ void __launch_bounds__(kDqlThreads)
   }
 }
 
+// DynamicQuantizeLinear of a tensor that one cluster can hold in registers: up
+// to 16 CTAs x 1024 threads x 4 words of four values.  What bounds small
+// tensors is launches (scratch memset, reduction, quantize pass: three, each
+// with its own way through memory); here every thread loads its values once,
+// the CTAs exchange their {min,max} through distributed shared memory, every
+// thread derives the two scalars and quantizes what it still holds.  The same
+// minima, maxima and per-element arithmetic as the passes above, so the same
+// bytes.  The operator on 1000 values 10.3 -> 5.2 us, on 98304 12.6 -> 8.2, on
+// 262144 13.3 -> 10.3; the linear 128 x 768 x 768 22.5 -> 16.9.
+//
+// The tensor is [rows, cols], written in rows of `pitch` bytes (zero from cols
+// on); a flat tensor is one row of pitch == cols.  rowsum (may be null) gets
+// the sums of the quantized rows.
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallMaxWords = 4; // per thread
+constexpr int kSmallMaxCluster = 16;
+
+struct SmallDql {
+  const float *x;
+  uint8_t *y;
+  int32_t *rowsum;
+  float *y_scale;
+  uint8_t *y_zp;
+  int rows, cols, pitch;
+  int row_words; // words per row: ceil(pitch / 4)
+  int words;     // rows * row_words
+  int vec_in;    // every whole word of x takes a 16-byte load
+  int vec_out;   // every whole word of y takes a 4-byte store
+  int mode;
+};
+
+template <int kWords>
+__global__ void __launch_bounds__(kSmallThreads) dql_small_kernel(SmallDql p) {
+  __shared__ float s_lo[kSmallThreads / 32], s_hi[kSmallThreads / 32];
+  __shared__ float c_lo[kSmallMaxCluster], c_hi[kSmallMaxCluster];
+  cg::cluster_group cluster = cg::this_cluster();
+  const unsigned ctas = cluster.num_blocks(), rank = cluster.block_rank();
+  cluster.barrier_arrive(); // "has started": waited for before the first remote store
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tid = (int)(rank * kSmallThreads + threadIdx.x);
+  const int nthreads = (int)(ctas * kSmallThreads);
+  if (p.rowsum)
+    for (int r = tid; r < p.rows; r += nthreads)
+      p.rowsum[r] = 0;
+  float4 v[kWords];
+  float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+  for (int u = 0; u < kWords; ++u) {
+    const int w = tid + u * nthreads;
+    v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (w >= p.words)
+      continue;
+    const int r = w / p.row_words, c = 4 * (w - r * p.row_words);
+    const float *src = p.x + (int64_t)r * p.cols + c;
+    const int have = p.cols - c;
+    if (have >= 4 && p.vec_in) {
+      v[u] = __ldg(reinterpret_cast<const float4 *>(src));
+    } else {
+      if (have > 0)
+        v[u].x = __ldg(src);
+      if (have > 1)
+        v[u].y = __ldg(src + 1);
+      if (have > 2)
+        v[u].z = __ldg(src + 2);
+      if (have > 3)
+        v[u].w = __ldg(src + 3);
+    }
+  }
+  // Zeros that stand for no element change neither scalar: the range is
+  // widened to hold 0 before anything is derived from it.
+#pragma unroll
+  for (int u = 0; u < kWords; ++u) {
+    lo = fminf(lo, fminf(fminf(v[u].x, v[u].y), fminf(v[u].z, v[u].w)));
+    hi = fmaxf(hi, fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w)));
+  }
+  lo = warp_min(lo);
+  hi = warp_max(hi);
+  if (lane == 0) {
+    s_lo[warp] = lo;
+    s_hi[warp] = hi;
+  }
+  __syncthreads();
+  cluster.barrier_wait();
+  if (warp == 0) {
+    static_assert(kSmallThreads / 32 == 32, "one value per lane");
+    lo = warp_min(s_lo[lane]);
+    hi = warp_max(s_hi[lane]);
+    if (lane < (int)ctas) { // lane i tells CTA i
+      *cluster.map_shared_rank(&c_lo[rank], lane) = lo;
+      *cluster.map_shared_rank(&c_hi[rank], lane) = hi;
+    }
+  }
+  cluster.sync(); // orders the remote stores, and the zeroes in rowsum
+  lo = c_lo[0];
+  hi = c_hi[0];
+  for (unsigned i = 1; i < ctas; ++i) {
+    lo = fminf(lo, c_lo[i]);
+    hi = fmaxf(hi, c_hi[i]);
+  }
+  float scale, zp_f;
+  dql_params_from_range(lo, hi, &scale, &zp_f, p.mode);
+  if (tid == 0) {
+    if (p.y_scale)
+      *p.y_scale = scale;
+    if (p.y_zp)
+      *p.y_zp = (uint8_t)(unsigned int)zp_f; // fptoui; zp_f is in [0,255]
+  }
+  const QuantConsts qc = make_quant_consts(scale, zp_f, p.mode);
+#pragma unroll
+  for (int u = 0; u < kWords; ++u) {
+    const int w = tid + u * nthreads;
+    if (w - lane >= p.words)
+      break; // the whole warp is past the end
+    const bool in = w < p.words;
+    const int r = in ? w / p.row_words : p.rows - 1;
+    const int c = 4 * (w - r * p.row_words);
+    const int have = in ? p.cols - c : 0;
+    uint32_t q = have > 0 ? quantize_four<false>(v[u], qc) : 0u;
+    if (have < 4)
+      q = have > 0 ? q & ((1u << (8 * have)) - 1u) : 0u;
+    if (in) {
+      uint8_t *dst = p.y + (int64_t)r * p.pitch + c;
+      if (p.vec_out && c + 4 <= p.pitch) {
+        *reinterpret_cast<uint32_t *>(dst) = q;
+      } else {
+        for (int e = 0; e < 4 && c + e < p.pitch; ++e)
+          dst[e] = (uint8_t)(q >> (8 * e));
+      }
+    }
+    if (p.rowsum) {
+      int32_t sum = add_bytes<false>(q, 0);
+      // rows grow with the lane: first and last alike means one row
+      if (__shfl_sync(0xffffffffu, r, 0) == __shfl_sync(0xffffffffu, r, 31)) {
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (lane == 0)
+          atomicAdd(p.rowsum + r, sum);
+      } else if (in) {
+        atomicAdd(p.rowsum + r, sum);
+      }
+    }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
     dequantize_kernel(const T *__restrict__ x, int64_t n,
@@ -329,6 +476,90 @@ int launch_quantize_rows(const float *x, int64_t rows, int64_t cols, int64_t pit
   return OMCUDA_OK;
 }
 
+namespace {
+
+// The largest cluster of dql_small_kernel the device can place.
+int small_cluster_limit() {
+  static PerDeviceInt limit;
+  int n = limit.get();
+  if (n == 0) {
+    n = 8; // always placeable
+    cudaLaunchConfig_t q = {};
+    q.gridDim = dim3(kSmallMaxCluster, 1, 1);
+    q.blockDim = dim3(kSmallThreads, 1, 1);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kSmallMaxCluster;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    q.attrs = at;
+    q.numAttrs = 1;
+    int a = 0, b = 0;
+    if (cudaFuncSetAttribute(dql_small_kernel<2>,
+            cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaFuncSetAttribute(dql_small_kernel<kSmallMaxWords>,
+            cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&a, dql_small_kernel<2>, &q) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&b, dql_small_kernel<kSmallMaxWords>, &q) ==
+            cudaSuccess &&
+        a > 0 && b > 0)
+      n = kSmallMaxCluster;
+    (void)cudaGetLastError();
+    limit.set(n);
+  }
+  return n;
+}
+
+} // namespace
+
+bool dql_small_wanted(int64_t rows, int64_t pitch) {
+  // Four words per thread: 262144 values take 10.3 us this way and 13.3 in three
+  // launches.  With sixteen (524288 values, 512 threads) the few SMs of one
+  // cluster were slower than the whole machine in three, 18.1 against 14.7 us.
+  return rows <= (1 << 20) && pitch <= (1 << 20) &&
+         rows * ceil_div(pitch, 4) <=
+             (int64_t)small_cluster_limit() * kSmallThreads * kSmallMaxWords;
+}
+
+int launch_dql_small(const float *x, int64_t rows, int64_t cols, int64_t pitch,
+    uint8_t *y, int32_t *rowsum, float *y_scale, uint8_t *y_zp, cudaStream_t st) {
+  SmallDql p;
+  p.x = x;
+  p.y = y;
+  p.rowsum = rowsum;
+  p.y_scale = y_scale;
+  p.y_zp = y_zp;
+  p.rows = (int)rows;
+  p.cols = (int)cols;
+  p.pitch = (int)pitch;
+  p.row_words = (int)ceil_div(pitch, 4);
+  p.words = (int)(rows * p.row_words);
+  p.vec_in = ((uintptr_t)x & 15u) == 0 && (rows == 1 || cols % 4 == 0);
+  p.vec_out = ((uintptr_t)y & 3u) == 0 && (rows == 1 || pitch % 4 == 0);
+  p.mode = quant_mode();
+  // Two words per thread while the cluster can still grow.
+  int ctas = 1;
+  while (ctas < small_cluster_limit() && ctas * kSmallThreads * 2 < p.words)
+    ctas *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas, 1, 1);
+  cfg.blockDim = dim3(kSmallThreads, 1, 1);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)ctas;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  OMCUDA_CHECK(cudaLaunchKernelEx(&cfg,
+      p.words <= ctas * kSmallThreads * 2 ? dql_small_kernel<2>
+                                          : dql_small_kernel<kSmallMaxWords>,
+      p));
+  count_launch();
+  return OMCUDA_OK;
+}
+
 int launch_dql_range(const float *x, int64_t n, void *scratch, float *y_scale,
     uint8_t *y_zp, const float **params, cudaStream_t st) {
   DqlScratch *scr = (DqlScratch *)scratch;
@@ -352,6 +583,8 @@ extern "C" int omcudaDevDynamicQuantizeLinear(const float *x, int64_t n,
   if (n < 0 || (n > 0 && (!x || !y)) || !scratch)
     return fail(OMCUDA_EINVAL, "DynamicQuantizeLinear: bad argument");
   cudaStream_t st = (cudaStream_t)stream;
+  if (dql_small_wanted(1, n))
+    return launch_dql_small(x, 1, n, n, y, nullptr, y_scale, y_zp, st);
   const float *params = nullptr;
   int rc = launch_dql_range(x, n, scratch, y_scale, y_zp, &params, st);
   if (rc != OMCUDA_OK)

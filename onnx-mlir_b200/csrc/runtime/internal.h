@@ -54,6 +54,13 @@ int launch_dql_range(const float *x, int64_t n, void *scratch, float *y_scale,
 int launch_quantize_rows(const float *x, int64_t rows, int64_t cols, int64_t pitch,
     uint8_t *y, int32_t *rowsum, const float *params, cudaStream_t st);
 
+// Both in one launch, without scratch, for a tensor that one cluster holds in
+// its registers.  [rows, cols] into rows of `pitch` bytes as above, or one row
+// of pitch == cols of any alignment.
+bool dql_small_wanted(int64_t rows, int64_t pitch);
+int launch_dql_small(const float *x, int64_t rows, int64_t cols, int64_t pitch,
+    uint8_t *y, int32_t *rowsum, float *y_scale, uint8_t *y_zp, cudaStream_t st);
+
 // gemm_tc.cu / gemm_simt.cu
 //
 // What the library itself can say about a GEMM beyond the public argument block.

@@ -130,3 +130,28 @@ def test_argument_errors(gpu):
     with pytest.raises(gpu.OmcudaError) as ei:
         gpu.check()
     assert ei.value.code == gpu.EINVAL
+
+
+@pytest.mark.parametrize("n", [4, 4095, 8191, 8192, 8193, 65537, 131071, 131073, 262143, 262144,
+                               262145])
+def test_one_cluster_sizes(gpu, orc, n):
+    # Up to 262144 values are reduced and quantized by one cluster that holds
+    # them in registers: the sizes at which it grows, the last it takes and the
+    # first it does not, on aligned data and on data that starts at an odd element
+    # (and is written at an odd byte).
+    import torch
+    x = np.random.default_rng(n).normal(1, 3, size=n).astype(np.float32)
+    check_dql(gpu, orc, x, device=True)
+    xt = torch.zeros(n + 1, device="cuda")
+    xt[1:] = torch.from_numpy(x).cuda()
+    yt = torch.zeros(n + 2, dtype=torch.uint8, device="cuda")
+    s, z = torch.zeros((), device="cuda"), torch.zeros((), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    t = [gpu.Tensor.from_cuda_array(a) for a in (yt[1:n + 1], s, z, xt[1:])]
+    gpu.lib().omcudaDynamicQuantizeLinear(*[a.handle for a in t])
+    gpu.check()
+    torch.cuda.synchronize()
+    want_y, want_s, want_z = orc.dynamic_quantize_linear(x)
+    y = yt.cpu().numpy()
+    assert np.array_equal(y[1:n + 1], want_y) and y[0] == 0 and y[n + 1] == 0
+    assert s.item() == want_s and z.item() == want_z
