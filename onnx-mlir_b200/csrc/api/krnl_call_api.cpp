@@ -283,8 +283,9 @@ int prepared_b(Stage &sg, const void *key_ptr, const void *b_dev, int b_signed,
 // Gives the GEMM g its A operand ([M,K], any alignment) and, when b_zp is
 // given, A's row sums.  The tensor-core kernels need rows that start 16-byte
 // aligned: an A that does not have them is copied into rows that do, in the
-// pass that makes the row sums.
-void set_a_operand(Stage &sg, GemmCall *g, const void *A, cudaStream_t st) {
+// pass that makes the row sums.  rq (needs b_zp): the scales made in that pass.
+void set_a_operand(Stage &sg, GemmCall *g, const void *A, cudaStream_t st,
+    const RequantScale &rq = RequantScale()) {
   g->A = A;
   g->lda = g->K;
   const bool aligned = (g->K % 16 == 0) && (((uintptr_t)A & 15u) == 0);
@@ -300,7 +301,7 @@ void set_a_operand(Stage &sg, GemmCall *g, const void *A, cudaStream_t st) {
   }
   if (!sg.ok())
     return;
-  sg.set(launch_repitch(A, g->a_signed, g->M, g->K, g->lda, rows, rs, st));
+  sg.set(launch_repitch(A, g->a_signed, g->M, g->K, g->lda, rows, rs, rq, st));
   g->a_rowsum = rs;
 }
 
@@ -803,18 +804,17 @@ void omcudaQLinearMatMul(OMTensor *y, const OMTensor *a, const OMTensor *aScale,
   const void *dAz = sg.in(aZp);
   const void *dBz = sg.in(bZp);
   void *dY = sg.out(y);
-  // The output zero point enters the epilogue as an immediate.
+  // The output zero point: an immediate of the epilogue, or read there when it
+  // lies on the device (copying it back first stalled the host behind all work
+  // queued on the stream: 64 x 768 x 768 33.5 us a call, 14.4 us without).
   int32_t yzp = 0;
+  const uint8_t *yzp_dev = nullptr;
   {
-    uint8_t raw = 0;
-    const void *p = omTensorGetDataPtr(yZp);
+    const uint8_t *p = (const uint8_t *)omTensorGetDataPtr(yZp);
     if (is_device_ptr(p))
-      sg.set(check_cuda(cudaMemcpyAsync(&raw, p, 1, cudaMemcpyDeviceToHost, st),
-          "read y_zero_point")),
-          sg.set(check_cuda(cudaStreamSynchronize(st), "sync"));
+      yzp_dev = p;
     else
-      raw = *(const uint8_t *)p;
-    yzp = (yt == ONNX_TYPE_INT8) ? (int32_t)(int8_t)raw : (int32_t)raw;
+      yzp = (yt == ONNX_TYPE_INT8) ? (int32_t)(int8_t)*p : (int32_t)*p;
   }
   if (!sg.ok())
     return;
@@ -828,17 +828,17 @@ void omcudaQLinearMatMul(OMTensor *y, const OMTensor *a, const OMTensor *aScale,
   float *S = (float *)sg.scratch((size_t)bsn * sizeof(float));
   if (!sg.ok() || !S)
     return;
-  sg.set(omcudaDevRequantScale(dAs, dBs, bsn, dYs, S, st));
   g.a_zp = dAz;
   g.a_zp_len = 1;
   g.b_zp = dBz;
   g.b_zp_len = bzn;
-  set_a_operand(sg, &g, dA, st);
+  set_a_operand(sg, &g, dA, st, RequantScale{dAs, dBs, dYs, bsn, S});
   g.epilogue = OMCUDA_EPI_REQUANT;
   g.Y = dY;
   g.sb = S;
   g.sb_len = bsn;
   g.y_zp = yzp;
+  g.y_zp_dev = yzp_dev;
   g.y_signed = yt == ONNX_TYPE_INT8;
   if (sg.ok())
     sg.set(gemm_i8(g, st));

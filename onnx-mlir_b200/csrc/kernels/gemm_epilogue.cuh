@@ -52,6 +52,7 @@ struct EpiParams {
   const float *bias;
   int gelu;
   int32_t y_zp;
+  const uint8_t *y_zp_dev; // y zero point in device memory, in place of y_zp
   const float *residual; // f32 [M,N] added after the DEQUANT tail, or nullptr
   int res_vec_ok;        // residual rows take 16-byte loads
   uint32_t *out_range; // ordered-uint {min,max} or nullptr
@@ -112,12 +113,14 @@ __device__ __forceinline__ EpiRow epi_row(const EpiParams &p, int64_t m) {
 struct EpiScalars {
   float sa;
   float s0;
+  uint32_t yz; // y zero point, modulo 2^8 (the result is truncated to 8 bits)
 };
 
 __device__ __forceinline__ EpiScalars epi_scalars(const EpiParams &p) {
   EpiScalars s;
   s.sa = 1.0f;
   s.s0 = 1.0f;
+  s.yz = (uint32_t)p.y_zp;
   if (epi_is_dequant(p.kind)) {
     s.sa = __ldg(p.sa);
     if (p.sb_len == 1)
@@ -125,6 +128,8 @@ __device__ __forceinline__ EpiScalars epi_scalars(const EpiParams &p) {
   } else if (p.kind == OMCUDA_EPI_REQUANT) {
     if (p.sb_len == 1)
       s.s0 = __ldg(p.sb);
+    if (p.y_zp_dev)
+      s.yz = __ldg(p.y_zp_dev);
   }
   return s;
 }
@@ -165,7 +170,7 @@ __device__ __forceinline__ uint32_t epi_requant(const EpiParams &p,
   float f = __int2float_rn(v);
   float sc = (p.sb_len == 1) ? s.s0 : __ldg(p.sb + n);
   float r = round_even(__fmul_rn(f, sc));
-  uint32_t t = (uint32_t)__float2int_rz(r) + (uint32_t)p.y_zp;
+  uint32_t t = (uint32_t)__float2int_rz(r) + s.yz;
   return t & 0xffu; // arith.trunci to 8 bits: wraps, does not saturate
 }
 

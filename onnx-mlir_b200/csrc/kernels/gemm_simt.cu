@@ -63,12 +63,23 @@ __global__ void __launch_bounds__(256)
                 part[2][threadIdx.x] + part[3][threadIdx.x];
 }
 
+// QLinearMatMul's column scales (src/Conversion/ONNXToKrnl/Math/QLinearMatMul.cpp:123-138).
+__device__ __forceinline__ float requant_scale(const RequantScale &rq, int64_t i) {
+  return __fdiv_rn(__fmul_rn(*rq.a_scale, rq.b_scale[i]), *rq.y_scale);
+}
+
 // One warp per row, a 16-byte chunk per lane and trip; with dst, the row is also
-// copied into an aligned row of `pitch` bytes whose tail is zero.
+// copied into an aligned row of `pitch` bytes whose tail is zero.  The column
+// scales of a QLinearMatMul ride along (rq.len != 0): a launch of their own was
+// 2.1 us for a few thousand divides.
 template <bool kSigned>
 __global__ void __launch_bounds__(256)
     rowsum_kernel(const uint8_t *__restrict__ A, int64_t M, int64_t K,
-        int32_t *__restrict__ rowsum, uint8_t *__restrict__ dst, int64_t pitch) {
+        int32_t *__restrict__ rowsum, uint8_t *__restrict__ dst, int64_t pitch,
+        RequantScale rq) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rq.len;
+       i += (int64_t)gridDim.x * blockDim.x)
+    rq.S[i] = requant_scale(rq, i);
   const int64_t m = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (m >= M)
     return;
@@ -100,12 +111,10 @@ __global__ void __launch_bounds__(256)
     rowsum[m] = s;
 }
 
-__global__ void requant_scale_kernel(const float *__restrict__ a_scale,
-    const float *__restrict__ b_scale, int64_t len,
-    const float *__restrict__ y_scale, float *__restrict__ S) {
+__global__ void requant_scale_kernel(RequantScale rq) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < len)
-    S[i] = __fdiv_rn(__fmul_rn(*a_scale, b_scale[i]), *y_scale);
+  if (i < rq.len)
+    rq.S[i] = requant_scale(rq, i);
 }
 
 // ---- SIMT GEMM ----------------------------------------------------------------
@@ -488,6 +497,7 @@ EpiParams make_epi_params(const GemmCall &a) {
   p.bias = a.bias;
   p.gelu = a.gelu;
   p.y_zp = a.y_zp;
+  p.y_zp_dev = a.y_zp_dev;
   p.residual = (a.epilogue == OMCUDA_EPI_DEQUANT) ? a.residual : nullptr;
   p.res_vec_ok = ((((uintptr_t)a.residual) & 15u) == 0) && (a.N % 4 == 0);
   p.out_range = reinterpret_cast<uint32_t *>(a.out_minmax);
@@ -650,12 +660,12 @@ int launch_gemm_simt(const GemmCall &a, cudaStream_t st) {
 }
 
 int launch_repitch(const void *A, int a_signed, int64_t M, int64_t K, int64_t pitch,
-    uint8_t *dst, int32_t *rowsum, cudaStream_t st) {
+    uint8_t *dst, int32_t *rowsum, const RequantScale &rq, cudaStream_t st) {
   const unsigned grid = (unsigned)ceil_div(M, 8);
   if (a_signed)
-    rowsum_kernel<true><<<grid, 256, 0, st>>>((const uint8_t *)A, M, K, rowsum, dst, pitch);
+    rowsum_kernel<true><<<grid, 256, 0, st>>>((const uint8_t *)A, M, K, rowsum, dst, pitch, rq);
   else
-    rowsum_kernel<false><<<grid, 256, 0, st>>>((const uint8_t *)A, M, K, rowsum, dst, pitch);
+    rowsum_kernel<false><<<grid, 256, 0, st>>>((const uint8_t *)A, M, K, rowsum, dst, pitch, rq);
   OMCUDA_CHECK_LAUNCH("rowsum_kernel");
   return OMCUDA_OK;
 }
@@ -703,7 +713,7 @@ extern "C" int omcudaDevRowSum(const void *A, int a_signed, int64_t M,
   if (!A || !rowsum || M <= 0 || K <= 0)
     return fail(OMCUDA_EINVAL, "RowSum: bad argument");
   cudaStream_t st = (cudaStream_t)stream;
-  return launch_repitch(A, a_signed, M, K, 0, nullptr, rowsum, st);
+  return launch_repitch(A, a_signed, M, K, 0, nullptr, rowsum, RequantScale(), st);
 }
 
 extern "C" int omcudaDevRequantScale(const float *a_scale, const float *b_scale,
@@ -711,7 +721,7 @@ extern "C" int omcudaDevRequantScale(const float *a_scale, const float *b_scale,
   if (!a_scale || !b_scale || !y_scale || !S || len <= 0)
     return fail(OMCUDA_EINVAL, "RequantScale: bad argument");
   requant_scale_kernel<<<(unsigned)ceil_div(len, 256), 256, 0,
-      (cudaStream_t)stream>>>(a_scale, b_scale, len, y_scale, S);
+      (cudaStream_t)stream>>>(RequantScale{a_scale, b_scale, y_scale, len, S});
   OMCUDA_CHECK_LAUNCH("requant_scale_kernel");
   return OMCUDA_OK;
 }

@@ -247,7 +247,7 @@ __device__ __forceinline__ void epilogue_chunk(const EpiParams &p,
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
       float r = round_even(__fmul_rn(__int2float_rn((int32_t)v[j]), sc.s0));
-      v[j] = ((uint32_t)__float2int_rz(r) + (uint32_t)p.y_zp) & 0xffu;
+      v[j] = ((uint32_t)__float2int_rz(r) + sc.yz) & 0xffu;
     }
   } else {
     float S[32];
@@ -255,7 +255,7 @@ __device__ __forceinline__ void epilogue_chunk(const EpiParams &p,
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
       float r = round_even(__fmul_rn(__int2float_rn((int32_t)v[j]), S[j]));
-      v[j] = ((uint32_t)__float2int_rz(r) + (uint32_t)p.y_zp) & 0xffu;
+      v[j] = ((uint32_t)__float2int_rz(r) + sc.yz) & 0xffu;
     }
   }
 }

@@ -68,17 +68,29 @@ struct GemmCall : omcudaGemmArgs {
   // Row pitch of A in bytes.  More than K only with rows that start 16-byte
   // aligned and hold zeros from K up to the next multiple of 16.
   int64_t lda;
-  GemmCall() : omcudaGemmArgs(), lda(0) {}
-  explicit GemmCall(const omcudaGemmArgs &a) : omcudaGemmArgs(a), lda(a.K) {}
+  // The output zero point of the REQUANT tail (one byte of device memory, the
+  // output's type); null: y_zp.  Read by the kernel, so that the host never
+  // waits for it.
+  const uint8_t *y_zp_dev;
+  GemmCall() : omcudaGemmArgs(), lda(0), y_zp_dev(nullptr) {}
+  explicit GemmCall(const omcudaGemmArgs &a)
+      : omcudaGemmArgs(a), lda(a.K), y_zp_dev(nullptr) {}
 };
 int gemm_i8(const GemmCall &a, cudaStream_t st);
 bool gemm_tc_supported(const GemmCall &a);
 int launch_gemm_tc(const GemmCall &a, cudaStream_t st);
 int launch_gemm_simt(const GemmCall &a, cudaStream_t st);
+// S[i] = a_scale * b_scale[i] / y_scale, the column scales of a QLinearMatMul.
+struct RequantScale {
+  const float *a_scale, *b_scale, *y_scale;
+  int64_t len; // 0: none
+  float *S;
+};
 // Copies an 8-bit [M,K] matrix of any alignment into rows of `pitch` bytes (a
-// multiple of 16, dst 16-byte aligned), zero from K on; rowsum may be null.
+// multiple of 16, dst 16-byte aligned), zero from K on; dst or rowsum may be
+// null.  Makes the scales of rq in the same launch.
 int launch_repitch(const void *A, int a_signed, int64_t M, int64_t K, int64_t pitch,
-    uint8_t *dst, int32_t *rowsum, cudaStream_t st);
+    uint8_t *dst, int32_t *rowsum, const RequantScale &rq, cudaStream_t st);
 
 // gemm_batched.cu: every product of a MatMulInteger whose B is an activation in
 // one launch, operands read as they lie.  Product i (row-major over size[])

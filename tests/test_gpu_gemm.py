@@ -573,3 +573,21 @@ def test_ragged_k_and_n(gpu, orc, M, K, N, wdt):
         bs = rng.uniform(0.001, 0.01, N).astype(np.float32)
         args = (xq, np.float32(0.02), np.uint8(128), W, bs, bzn, np.float32(0.5), np.uint8(7))
         assert np.array_equal(gpu.qlinear_matmul(*args), orc.qlinear_matmul(*args))
+
+
+@pytest.mark.parametrize("ydt", [np.uint8, np.int8])
+@pytest.mark.parametrize("M,K,N,per_column", [(1, 64, 40, False), (9, 48, 33, True),
+                                              (40, 100, 300, True), (300, 64, 512, False)])
+def test_qlinear_parameters_on_the_device(gpu, orc, ydt, M, K, N, per_column):
+    # y_zero_point is read by the kernels' tails and the column scales are made
+    # in the row-sum pass; every kernel family, both output types, host and
+    # device parameters alike.
+    rng = np.random.default_rng(33)
+    A, B = rand8(rng, (M, K), np.uint8), rand8(rng, (K, N), np.int8)
+    bs = rng.uniform(0.001, 0.01, N if per_column else ()).astype(np.float32)
+    bz = rand8(rng, N if per_column else (), np.int8)
+    yz = np.asarray(-77 if ydt == np.int8 else 200, ydt)
+    args = (A, np.float32(0.02), np.uint8(128), B, bs, bz, np.float32(0.5), yz)
+    want = orc.qlinear_matmul(*args)
+    assert np.array_equal(gpu.qlinear_matmul(*args), want)
+    assert np.array_equal(gpu.qlinear_matmul(*args, device=True).numpy(), want)
