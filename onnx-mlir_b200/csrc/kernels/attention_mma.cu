@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(128)
   constexpr int NT_S = kKeys / 8;
 
   extern __shared__ __align__(16) __nv_bfloat16 att_smem[];
+  pdl_sync();
   // [hi|lo][key][dh] for K, then the same for V
   __nv_bfloat16 (*sK)[kKeys * LD] =
       reinterpret_cast<__nv_bfloat16 (*)[kKeys * LD]>(att_smem);
@@ -293,11 +294,11 @@ int launch_attention_mma(const float *Q, const float *K, const float *V,
   uint32_t *rng = (uint32_t *)out_range;
   const size_t smem = (size_t)4 * kKeys * (dh + kPad) * sizeof(__nv_bfloat16);
   if (dh == 64) {
-    attention_mma_kernel<64><<<grid, 128, smem, st>>>(
-        Q, K, V, S, heads, scale, out, ld_in, ld_out, rng);
+    OMCUDA_CHECK(launch_pdl(attention_mma_kernel<64>, grid, 128, smem, st, 0,
+        pdl_pays(B * S * heads * dh), Q, K, V, S, heads, scale, out, ld_in, ld_out, rng));
   } else if (dh == 32) {
-    attention_mma_kernel<32><<<grid, 128, smem, st>>>(
-        Q, K, V, S, heads, scale, out, ld_in, ld_out, rng);
+    OMCUDA_CHECK(launch_pdl(attention_mma_kernel<32>, grid, 128, smem, st, 0,
+        pdl_pays(B * S * heads * dh), Q, K, V, S, heads, scale, out, ld_in, ld_out, rng));
   } else {
     static PerDeviceInt attr_set;
     if (!attr_set.get()) {
@@ -305,8 +306,8 @@ int launch_attention_mma(const float *Q, const float *K, const float *V,
           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       attr_set.set(1);
     }
-    attention_mma_kernel<128><<<grid, 128, smem, st>>>(
-        Q, K, V, S, heads, scale, out, ld_in, ld_out, rng);
+    OMCUDA_CHECK(launch_pdl(attention_mma_kernel<128>, grid, 128, smem, st, 0,
+        pdl_pays(B * S * heads * dh), Q, K, V, S, heads, scale, out, ld_in, ld_out, rng));
   }
   OMCUDA_CHECK_LAUNCH("attention_mma_kernel");
   return OMCUDA_OK;

@@ -242,6 +242,7 @@ __global__ void __launch_bounds__(kTcAttThreads, 2)
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem = tmem_slot;
+  pdl_sync();
   const uint32_t t_s = tmem;          // scores, then P, columns 0..127
   const uint32_t t_o = tmem + 128u;   // P V of the current key block
   const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
@@ -605,9 +606,9 @@ int launch_attention_tc(const void *hi, const void *lo, int64_t ld_planes,
   // (batch, head, 128-query-row) items.
   const int64_t resident = (int64_t)sm_count() * 2;
   const unsigned grid = (unsigned)(n_items < resident ? n_items : resident);
-  attention_tc_kernel<<<grid, kTcAttThreads, kTcAttSmem, st>>>(map_hi, map_lo, map_out,
-      (int32_t)q_col, (int32_t)k_col, (int32_t)v_col, S, heads, n_items, scale_log2e,
-      (uint32_t *)out_range, status, tc_wait_limit_ns());
+  OMCUDA_CHECK(launch_pdl(attention_tc_kernel, grid, kTcAttThreads, kTcAttSmem, st, 0,
+      pdl_pays(B * S * heads * kTDh), map_hi, map_lo, map_out, (int32_t)q_col, (int32_t)k_col, (int32_t)v_col, S, heads, n_items, scale_log2e,
+      (uint32_t *)out_range, status, tc_wait_limit_ns()));
   OMCUDA_CHECK_LAUNCH("attention_tc_kernel");
   return OMCUDA_OK;
 }

@@ -40,6 +40,7 @@ __global__ void __launch_bounds__(kDqlThreads)
     dql_minmax_kernel(const float *__restrict__ x, int64_t n,
         DqlScratch *__restrict__ scr, float *__restrict__ y_scale,
         uint8_t *__restrict__ y_zp, int mode) {
+  pdl_sync();
   float lo = INFINITY, hi = -INFINITY;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
@@ -185,6 +186,11 @@ __global__ void __launch_bounds__(kDqlThreads)
         uint8_t *__restrict__ y, const float *__restrict__ params,
         const float *__restrict__ scale_ptr, const void *__restrict__ zp8,
         int has_zp, const uint32_t *__restrict__ range, QuantOutputs outs, int mode) {
+  pdl_sync();
+  params = after_pdl(params);
+  scale_ptr = after_pdl(scale_ptr);
+  zp8 = after_pdl(zp8);
+  range = after_pdl(range);
   float scale, zp_f;
   if (range) {
     // Scale and zero point straight from a producer's running range (every
@@ -250,6 +256,8 @@ __global__ void __launch_bounds__(kDqlThreads)
     quantize_rows_kernel(const float *__restrict__ x, int64_t rows, int cols, int pitch,
         uint8_t *__restrict__ y, int32_t *__restrict__ rowsum,
         const float *__restrict__ params, int mode) {
+  pdl_sync();
+  params = after_pdl(params);
   __shared__ int32_t part[kDqlThreads / 32];
   const QuantConsts qc = make_quant_consts(__ldg(params), __ldg(params + 1), mode);
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
@@ -326,6 +334,7 @@ __global__ void __launch_bounds__(kSmallThreads) dql_small_kernel(SmallDql p) {
   __shared__ float c_lo[kSmallMaxCluster], c_hi[kSmallMaxCluster];
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned ctas = cluster.num_blocks(), rank = cluster.block_rank();
+  pdl_sync();
   cluster.barrier_arrive(); // "has started": waited for before the first remote store
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tid = (int)(rank * kSmallThreads + threadIdx.x);
@@ -461,8 +470,9 @@ static int grid_for(int64_t work_items, int per_block) {
 int launch_quantize_with_params(const float *x, int64_t n, uint8_t *y,
     const float *params, cudaStream_t st) {
   int grid = grid_for(n, kDqlThreads * 16);
-  quantize_kernel<false><<<grid, kDqlThreads, 0, st>>>(
-      x, n, y, params, nullptr, nullptr, 1, nullptr, QuantOutputs{}, quant_mode());
+  OMCUDA_CHECK(launch_pdl(quantize_kernel<false>, grid, kDqlThreads, 0, st, 0,
+      pdl_pays(n), x, n, y, params, nullptr, nullptr, 1, nullptr, QuantOutputs{},
+      quant_mode()));
   OMCUDA_CHECK_LAUNCH("quantize_kernel");
   return OMCUDA_OK;
 }
@@ -470,8 +480,9 @@ int launch_quantize_with_params(const float *x, int64_t n, uint8_t *y,
 int launch_quantize_rows(const float *x, int64_t rows, int64_t cols, int64_t pitch,
     uint8_t *y, int32_t *rowsum, const float *params, cudaStream_t st) {
   const int64_t cap = (int64_t)sm_count() * 8;
-  quantize_rows_kernel<<<(unsigned)(rows < cap ? rows : cap), kDqlThreads, 0, st>>>(
-      x, rows, (int)cols, (int)pitch, y, rowsum, params, quant_mode());
+  OMCUDA_CHECK(launch_pdl(quantize_rows_kernel, (unsigned)(rows < cap ? rows : cap),
+      kDqlThreads, 0, st, 0, pdl_pays(rows * cols), x, rows, (int)cols, (int)pitch, y,
+      rowsum, params, quant_mode()));
   OMCUDA_CHECK_LAUNCH("quantize_rows_kernel");
   return OMCUDA_OK;
 }
@@ -541,21 +552,10 @@ int launch_dql_small(const float *x, int64_t rows, int64_t cols, int64_t pitch,
   int ctas = 1;
   while (ctas < small_cluster_limit() && ctas * kSmallThreads * 2 < p.words)
     ctas *= 2;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)ctas, 1, 1);
-  cfg.blockDim = dim3(kSmallThreads, 1, 1);
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)ctas;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  OMCUDA_CHECK(cudaLaunchKernelEx(&cfg,
-      p.words <= ctas * kSmallThreads * 2 ? dql_small_kernel<2>
-                                          : dql_small_kernel<kSmallMaxWords>,
-      p));
+  OMCUDA_CHECK(launch_pdl(p.words <= ctas * kSmallThreads * 2
+                              ? dql_small_kernel<2>
+                              : dql_small_kernel<kSmallMaxWords>,
+      (unsigned)ctas, kSmallThreads, 0, st, (unsigned)ctas, true, p));
   count_launch();
   return OMCUDA_OK;
 }
@@ -563,8 +563,8 @@ int launch_dql_small(const float *x, int64_t rows, int64_t cols, int64_t pitch,
 int launch_dql_range(const float *x, int64_t n, void *scratch, float *y_scale,
     uint8_t *y_zp, const float **params, cudaStream_t st) {
   DqlScratch *scr = (DqlScratch *)scratch;
-  dql_minmax_kernel<<<grid_for(n, kDqlThreads * 16), kDqlThreads, 0, st>>>(
-      x, n, scr, y_scale, y_zp, quant_mode());
+  OMCUDA_CHECK(launch_pdl(dql_minmax_kernel, grid_for(n, kDqlThreads * 16), kDqlThreads,
+      0, st, 0, pdl_pays(n), x, n, scr, y_scale, y_zp, quant_mode()));
   OMCUDA_CHECK_LAUNCH("dql_minmax_kernel");
   *params = scr->params;
   return OMCUDA_OK;
@@ -614,8 +614,9 @@ extern "C" int omcudaDevQuantizeFromRange(const float *x, int64_t n, void *range
   // block of its own when there is nothing to quantize).
   int grid = grid_for(n, kDqlThreads * 16);
   QuantOutputs outs{params, y_scale, y_zp};
-  quantize_kernel<false><<<grid, kDqlThreads, 0, st>>>(
-      x, n, y, nullptr, nullptr, nullptr, 1, (const uint32_t *)range, outs, quant_mode());
+  OMCUDA_CHECK(launch_pdl(quantize_kernel<false>, grid, kDqlThreads, 0, st, 0,
+      pdl_pays(n), x, n, y, nullptr, nullptr, nullptr, 1, (const uint32_t *)range, outs,
+      quant_mode()));
   OMCUDA_CHECK_LAUNCH("quantize_kernel");
   return OMCUDA_OK;
 }
@@ -629,13 +630,13 @@ extern "C" int omcudaDevQuantizeLinear(const float *x, int64_t n, void *y,
   cudaStream_t st = (cudaStream_t)stream;
   int grid = grid_for(n, kDqlThreads * 16);
   if (y_signed)
-    quantize_kernel<true><<<grid, kDqlThreads, 0, st>>>(
-        x, n, (uint8_t *)y, nullptr, scale, zp, zp != nullptr, nullptr, QuantOutputs{},
-        quant_mode());
+    OMCUDA_CHECK(launch_pdl(quantize_kernel<true>, grid, kDqlThreads, 0, st, 0,
+        pdl_pays(n), x, n, (uint8_t *)y, nullptr, scale, zp, zp != nullptr, nullptr,
+        QuantOutputs{}, quant_mode()));
   else
-    quantize_kernel<false><<<grid, kDqlThreads, 0, st>>>(
-        x, n, (uint8_t *)y, nullptr, scale, zp, zp != nullptr, nullptr, QuantOutputs{},
-        quant_mode());
+    OMCUDA_CHECK(launch_pdl(quantize_kernel<false>, grid, kDqlThreads, 0, st, 0,
+        pdl_pays(n), x, n, (uint8_t *)y, nullptr, scale, zp, zp != nullptr, nullptr,
+        QuantOutputs{}, quant_mode()));
   OMCUDA_CHECK_LAUNCH("quantize_kernel");
   return OMCUDA_OK;
 }

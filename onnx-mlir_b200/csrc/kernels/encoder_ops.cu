@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(256)
         const float *__restrict__ gamma, const float *__restrict__ beta,
         float eps, float *__restrict__ y, uint32_t *__restrict__ out_range) {
   constexpr int64_t cols = (int64_t)NV * 128;
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   float lo = INFINITY, hi = -INFINITY;
@@ -397,6 +398,7 @@ __global__ void __launch_bounds__(kAttWarps * 32)
 // Arms running {min,max} ranges (ordered-uint encoding): min side all ones,
 // max side zero, so that the first value folded in replaces both.
 __global__ void range_init_kernel(uint32_t *ranges, int count) {
+  pdl_sync();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) {
     ranges[2 * i] = 0xffffffffu;
@@ -441,11 +443,11 @@ extern "C" int omcudaDevLayerNorm(const float *x, const float *residual,
   cudaStream_t st = (cudaStream_t)stream;
   uint32_t *rng = reinterpret_cast<uint32_t *>(out_minmax);
   if (vec_ok && cols == 768)
-    layernorm_rows_vec_kernel<6><<<grid, 256, 0, st>>>(
-        x, residual, rows, gamma, beta, eps, y, rng);
+    OMCUDA_CHECK(launch_pdl(layernorm_rows_vec_kernel<6>, grid, 256, 0, st, 0,
+        pdl_pays(rows * cols), x, residual, rows, gamma, beta, eps, y, rng));
   else if (vec_ok && cols == 1024)
-    layernorm_rows_vec_kernel<8><<<grid, 256, 0, st>>>(
-        x, residual, rows, gamma, beta, eps, y, rng);
+    OMCUDA_CHECK(launch_pdl(layernorm_rows_vec_kernel<8>, grid, 256, 0, st, 0,
+        pdl_pays(rows * cols), x, residual, rows, gamma, beta, eps, y, rng));
   else
     layernorm_rows_kernel<<<grid, 256, 0, st>>>(
         x, residual, rows, cols, gamma, beta, eps, y, rng);
@@ -504,8 +506,8 @@ extern "C" int omcudaDevMatMulF32(const float *A, const float *B, int64_t batch,
 extern "C" int omcudaDevRangeInit(void *ranges, int64_t count, void *stream) {
   if (!ranges || count <= 0)
     return fail(OMCUDA_EINVAL, "RangeInit: bad argument");
-  range_init_kernel<<<(unsigned)ceil_div(count, 128), 128, 0,
-      (cudaStream_t)stream>>>((uint32_t *)ranges, (int)count);
+  OMCUDA_CHECK(launch_pdl(range_init_kernel, (unsigned)ceil_div(count, 128), 128, 0,
+      (cudaStream_t)stream, 0, true, (uint32_t *)ranges, (int)count));
   OMCUDA_CHECK_LAUNCH("range_init_kernel");
   return OMCUDA_OK;
 }

@@ -564,6 +564,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   tcgen05_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
   volatile int *abortp = &abort_flag;
+  pdl_sync(); // (every load below is guarded by a branch on the warp)
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -839,6 +840,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   tcgen05_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
   volatile int *abortp = &abort_flag;
+  pdl_sync(); // (every load below is guarded by a branch on the warp)
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
@@ -1290,8 +1292,9 @@ int launch_bn_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan =
   int64_t tiles = ceil_div(a.M, kBM) * ceil_div(a.N, BN) * plan.split;
   int grid = (int)(tiles < sm_count() ? tiles : sm_count());
   uint32_t idesc = make_idesc(a.a_signed, a.B.b_signed, BN);
-  gemm_i8_tc_kernel<BN, EPI, EW><<<grid, tc_threads(EW), Cfg::kSmemBytes, st>>>(
-      map_a, map_b, map_y, map_y2, p, idesc, status, tc_wait_limit_ns());
+  OMCUDA_CHECK(launch_pdl(gemm_i8_tc_kernel<BN, EPI, EW>, (unsigned)grid, tc_threads(EW),
+      Cfg::kSmemBytes, st, 0, pdl_pays(a.M * a.N), map_a, map_b, map_y, map_y2, p, idesc, status,
+      tc_wait_limit_ns()));
   OMCUDA_CHECK_LAUNCH("gemm_i8_tc_kernel");
   return OMCUDA_OK;
 }
@@ -1408,18 +1411,6 @@ int launch_pair_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan
   idesc = (idesc & ~(0x1fu << 24)) | ((uint32_t)(256 >> 4) << 24);
   uint32_t idesc_half = make_idesc(a.a_signed, a.B.b_signed, 128);
   idesc_half = (idesc_half & ~(0x1fu << 24)) | ((uint32_t)(256 >> 4) << 24);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(2 * clusters), 1, 1);
-  cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = kPairSmemBytes;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   CUtensorMap map_y, map_y2;
   GemmCall ya = a; // the matrix the stores see: all slices of the workspace
   if (plan.split > 1)
@@ -1427,9 +1418,9 @@ int launch_pair_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan
   rc = make_y_maps<EPI>(ya, epi_cols_per_warp(256, EW), p.line_store != 0, &map_y, &map_y2);
   if (rc != OMCUDA_OK)
     return rc;
-  OMCUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_i8_tc2_kernel<EPI, EW>, map_a, map_b,
-      map_b_half, map_y, map_y2, p, idesc, idesc_half, full_units, num_units, status,
-      tc_wait_limit_ns()));
+  OMCUDA_CHECK(launch_pdl(gemm_i8_tc2_kernel<EPI, EW>, (unsigned)(2 * clusters), kThreads,
+      kPairSmemBytes, st, 2, pdl_pays(a.M * a.N), map_a, map_b, map_b_half, map_y, map_y2, p, idesc, idesc_half,
+      full_units, num_units, status, tc_wait_limit_ns()));
   count_launch();
   return OMCUDA_OK;
 }
