@@ -38,13 +38,7 @@ __host__ __device__
 static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 #ifdef __CUDACC__
-// Launches a kernel that may be set up while the kernel before it on the stream
-// is still running (programmatic dependent launch).  Such a kernel calls
-// pdl_sync() before its first access to global memory; what comes before that
-// (barriers, tensor memory, descriptor fetches) and the launch itself are then
-// hidden behind its predecessor.  cluster: CTAs per cluster, 0 for none; overlap:
-// see pdl_pays().
-// Whether a kernel that makes this many values is launched that way.  Kernels of
+// Whether a kernel that makes this many values is launched with launch_pdl's overlap.  Kernels of
 // a few tens of microseconds gain what their launch takes (linear 128 x 768 x 768 16.9
 // -> 12.3 us, an encoder run of 32 x 128 tokens 2.03 -> 1.97 ms); in long ones
 // the early blocks only hold registers and shared memory of the SMs that
@@ -52,6 +46,12 @@ static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 // took 119.7 ms instead of 113.2.
 inline bool pdl_pays(int64_t values) { return values <= ((int64_t)16 << 20); }
 
+// Launches a kernel that may be set up while the kernel before it on the stream
+// is still running (programmatic dependent launch).  Such a kernel calls
+// pdl_sync() before its first access to global memory; what comes before that
+// (barriers, tensor memory, descriptor fetches) and the launch itself are then
+// hidden behind its predecessor.  cluster: CTAs per cluster, 0 for none; overlap:
+// see pdl_pays().
 template <typename... P, typename... A>
 inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, unsigned block,
     size_t smem, cudaStream_t st, unsigned cluster, bool overlap, A &&...args) {

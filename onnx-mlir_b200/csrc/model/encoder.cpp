@@ -552,6 +552,11 @@ int run_launches(omcudaEncoder *e, const float *x, int64_t batch, int64_t seq, f
   // attention kernel, which reads Q, K, V as bf16 hi/lo planes.
   const bool use_tc_attention =
       omcudaDevAttentionBf16Supported(batch, seq, heads, dh, 3 * H, H) != 0;
+  // Other sequence lengths: the mma.sync kernel reads the same planes.  (Up to
+  // 16 tokens the projection runs on the GEMV-shaped kernels, which write fp32.)
+  const bool use_mma_planes = !use_tc_attention && T > 16 &&
+      attention_mma_planes_supported(batch, seq, heads, dh, 3 * H, H, e->qkv.p,
+          (const uint8_t *)e->qkv.p + (size_t)(T * 3 * H) * 2, (const float *)e->ctx.p);
   // (the f32 [T,3H] buffer holds the two bf16 [T,3H] planes instead)
   const bool fuse_residual = (size_t)(T * H) * 4 >= ((size_t)64 << 20);
   // Gelu(Linear(h1)) feeds nothing but a DynamicQuantizeLinear, so the f32
@@ -618,14 +623,18 @@ int run_launches(omcudaEncoder *e, const float *x, int64_t batch, int64_t seq, f
     const int64_t tb = l * tl.layer_stride;
     RUN(tap_copy(e, tb + tl.x, cur, T * H * 4, st));
     RUN(tap_copy(e, tb + tl.xq_x, xq, T * H, st));
-    if (use_tc_attention) {
+    if (use_tc_attention || use_mma_planes) {
       // The projection writes q | k | v straight into the bf16 hi/lo planes
       // the attention kernel reads; the f32 values never reach HBM.
       RUN(gemm(e, xq, (const uint8_t *)(p_x + 3), p_x + 2, L.wqkv, T,
           (const float *)L.qkv_scale.p, 3 * H, (const float *)L.bqkv.p, 0,
           planes_hi, nullptr, st, OMCUDA_EPI_DEQUANT_SPLIT));
-      RUN(omcudaDevAttentionBf16(planes_hi, planes_lo, 3 * H, 0, H, 2 * H, batch,
-          seq, heads, dh, att_scale, (float *)e->ctx.p, H, r_ctx, st));
+      if (use_tc_attention)
+        RUN(omcudaDevAttentionBf16(planes_hi, planes_lo, 3 * H, 0, H, 2 * H, batch,
+            seq, heads, dh, att_scale, (float *)e->ctx.p, H, r_ctx, st));
+      else
+        RUN(launch_attention_mma_planes(planes_hi, planes_lo, 3 * H, 0, H, 2 * H, batch, seq,
+            heads, att_scale, (float *)e->ctx.p, H, r_ctx, st));
     } else {
       RUN(gemm(e, xq, (const uint8_t *)(p_x + 3), p_x + 2, L.wqkv, T,
           (const float *)L.qkv_scale.p, 3 * H, (const float *)L.bqkv.p, 0,

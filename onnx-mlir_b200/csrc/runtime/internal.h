@@ -118,6 +118,13 @@ bool attention_mma_supported(const float *Q, const float *K, const float *V,
 int launch_attention_mma(const float *Q, const float *K, const float *V,
     int64_t B, int64_t S, int64_t heads, int64_t dh, float scale, float *out,
     int64_t ld_in, int64_t ld_out, void *out_range, cudaStream_t st);
+// The same kernel on bf16 hi/lo planes (columns of Q, K and V in one row): bit for
+// bit what it gives for the fp32 values they were split from.
+bool attention_mma_planes_supported(int64_t B, int64_t S, int64_t heads, int64_t dh,
+    int64_t ld_planes, int64_t ld_out, const void *hi, const void *lo, const float *out);
+int launch_attention_mma_planes(const void *hi, const void *lo, int64_t ld_planes,
+    int64_t q_col, int64_t k_col, int64_t v_col, int64_t B, int64_t S, int64_t heads,
+    float scale, float *out, int64_t ld_out, void *out_range, cudaStream_t st);
 
 // attention_tc.cu: tcgen05 attention over bf16 hi/lo planes [T, ld_planes]
 // (head size 64, sequence a multiple of 128), and the fp32 -> planes split.

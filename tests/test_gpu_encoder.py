@@ -204,3 +204,20 @@ def test_bert_large_size_batch_permutation(gpu):
     # and the run is repeatable
     assert np.array_equal(enc.run(x), y)
     enc.close()
+
+
+@pytest.mark.parametrize("B,S,layers", [(1, 17, 1), (2, 63, 1), (3, 65, 1), (2, 129, 2), (1, 200, 1)])
+def test_ragged_sequences_equal_unfused_chain(gpu, B, S, layers):
+    # Sequences that are no multiple of 128 go from the projection's bf16 planes
+    # through the mma.sync kernel (masked last block, one or several key blocks, two
+    # sets of buffers); the separate calls hand it fp32 operands.  Same bits.
+    H, heads, F = 128, 2, 256
+    ws = make_encoder(25, H, F, layers)
+    x = np.random.default_rng(26).normal(size=(B, S, H)).astype(np.float32)
+    enc = gpu.Encoder(H, heads, F, ws)
+    got = enc.run(x)
+    cur = x
+    for w in ws:
+        cur = unfused_layer_on_gpu(gpu, cur, B, S, H, heads, w)
+    assert got.tobytes() == cur.reshape(B, S, H).tobytes()
+    enc.close()
