@@ -155,3 +155,43 @@ def test_one_cluster_sizes(gpu, orc, n):
     y = yt.cpu().numpy()
     assert np.array_equal(y[1:n + 1], want_y) and y[0] == 0 and y[n + 1] == 0
     assert s.item() == want_s and z.item() == want_z
+
+
+@pytest.mark.parametrize("n", [3, 4096, 4099, 262147, 1048575, 9 << 20])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_pass_run_edges(gpu, orc, n, shift):
+    # QuantizeLinear and DequantizeLinear take runs of 4096 values per block: part
+    # of a run, whole runs, several runs per block, and addresses that allow no
+    # vector access.
+    import torch
+    rng = np.random.default_rng(n)
+    x = rng.normal(0, 20, size=n).astype(np.float32)
+    xt = torch.zeros(n + 1, device="cuda")
+    xt[shift:shift + n] = torch.from_numpy(x).cuda()
+    qt = torch.zeros(n + 1, dtype=torch.uint8, device="cuda")
+    q, xd = (gpu.Tensor.from_cuda_array(a[shift:shift + n]) for a in (qt, xt))
+    zp = np.array(131, np.uint8)
+    L = gpu.lib()
+    s, z = gpu.Tensor.from_numpy(np.array(0.37, np.float32)), gpu.Tensor.from_numpy(zp)
+    torch.cuda.synchronize()
+    L.omcudaQuantizeLinear(q.handle, xd.handle, s.handle, z.handle)
+    gpu.check()
+    torch.cuda.synchronize()
+    want = orc.quantize(x, 0.37, 131.0, False)
+    got = qt.cpu().numpy()
+    assert np.array_equal(got[shift:shift + n], want)
+    assert not got[:shift].any() and not got[shift + n:].any()
+    for dt in (np.uint8, np.int8, np.int32):
+        src = torch.zeros(n + 1, dtype=getattr(torch, np.dtype(dt).name), device="cuda")
+        vals = want.view(np.int8).astype(dt) if dt != np.uint8 else want
+        src[shift:shift + n] = torch.from_numpy(vals).cuda()
+        y = torch.full((n + 1,), -1.0, device="cuda")
+        zpd = gpu.Tensor.from_numpy(np.array(5, dt))
+        torch.cuda.synchronize()
+        yd, sd = (gpu.Tensor.from_cuda_array(a[shift:shift + n]) for a in (y, src))
+        L.omcudaDequantizeLinear(yd.handle, sd.handle, s.handle, zpd.handle)
+        gpu.check()
+        torch.cuda.synchronize()
+        out = y.cpu().numpy()
+        assert out[shift:shift + n].tobytes() == orc.dequantize_linear(vals, 0.37, 5).tobytes()
+        assert (out[:shift] == -1).all() and (out[shift + n:] == -1).all()
