@@ -229,6 +229,22 @@ __global__ void __launch_bounds__(256)
 // exact in any order, so the result equals the other kernels' bit for bit.
 constexpr int kGemvWarps = 4;
 
+// Asks for `cols` columns of the weight (rows of Bt, kp bytes each) in L2.  The
+// GEMV-shaped kernels do this before pdl_sync(): their blocks are resident while
+// the activation is still being quantized, and the weight, which is all they
+// have to wait for, is on its way by then.  A prefetch reads nothing, so it does
+// not matter whether the weight has been written yet.  Weights of more than
+// half of L2 would be evicted before they are read: those are left alone.
+// Linear 16 x 14336 x 4096 28.7 -> 24.6 us, 1 x 4096 x 14336 18.4 -> 17.7.
+__device__ __forceinline__ void prefetch_weight(
+    const uint8_t *Bt, int64_t kp, int64_t n0, int cols, int64_t N) {
+  const int j = threadIdx.x;
+  if (j < cols && n0 + j < N && N * kp <= ((int64_t)64 << 20))
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(Bt + (n0 + j) * kp),
+                 "r"((uint32_t)kp)
+                 : "memory");
+}
+
 template <int MT, int CB, bool kASigned, bool kBSigned>
 __global__ void __launch_bounds__(32 * kGemvWarps)
     gemm_i8_gemv_kernel(const uint8_t *__restrict__ A,
@@ -240,12 +256,18 @@ __global__ void __launch_bounds__(32 * kGemvWarps)
   constexpr int kStep = 32 * kGemvWarps;
   __shared__ int32_t part[kGemvWarps][MT * CB];
   static_assert(MT * CB <= 32, "the epilogue runs in the first warp");
-  const EpiScalars sc = epi_scalars(p);
   float lo = INFINITY, hi = -INFINITY;
   // A block walks column groups (grid-stride), so that a launch is a few
   // resident blocks per SM streaming the weight rather than thousands of
   // short-lived ones.
   const int64_t groups = ceil_div(p.N, CB);
+  for (int64_t g = blockIdx.x; g < groups; g += gridDim.x)
+    prefetch_weight(Bt, kp, g * CB, CB, p.N);
+  pdl_sync();
+  A = after_pdl(A);
+  p.sa = after_pdl(p.sa);
+  p.sb = after_pdl(p.sb);
+  const EpiScalars sc = epi_scalars(p);
   for (int64_t g = blockIdx.x; g < groups; g += gridDim.x) {
     const int64_t n0 = g * CB;
     int32_t acc[MT][CB];
@@ -390,9 +412,16 @@ __global__ void __launch_bounds__(32 * kGemvMmaWarps)
   const bool vec_ok = ((p.lda & 15) == 0) && (((uintptr_t)A & 15u) == 0);
   const int64_t blocks64 = (kp + 63) >> 6;
   __shared__ int32_t part[kGemvMmaWarps][16][kCols + 1];
-  const EpiScalars sc = epi_scalars(p);
   float lo = INFINITY, hi = -INFINITY;
   const int64_t groups = ceil_div(p.N, kCols);
+  if (blockIdx.y == 0)
+    for (int64_t grp = blockIdx.x; grp < groups; grp += gridDim.x)
+      prefetch_weight(Bt, kp, grp * kCols, kCols, p.N);
+  pdl_sync();
+  A = after_pdl(A);
+  p.sa = after_pdl(p.sa);
+  p.sb = after_pdl(p.sb);
+  const EpiScalars sc = epi_scalars(p);
   for (int64_t grp = blockIdx.x; grp < groups; grp += gridDim.x) {
     const int64_t n0 = grp * kCols;
     int32_t acc[CG][4];
@@ -545,24 +574,26 @@ static void launch_gemv(const GemmCall &a, cudaStream_t st) {
   EpiParams p = make_epi_params(a);
   // Up to 12 resident blocks of 128 threads per SM (1536 threads, 8 x 16-byte
   // loads in flight each with CB = 4).
+  // Every block takes the same number of column groups, give or take one.
   const int64_t groups = ceil_div(a.N, CB), resident = (int64_t)sm_count() * 12;
-  dim3 grid((unsigned)(groups < resident ? groups : resident), (unsigned)ceil_div(a.M, MT));
+  const int64_t rounds = ceil_div(groups, resident);
+  dim3 grid((unsigned)ceil_div(groups, rounds), (unsigned)ceil_div(a.M, MT));
   const uint8_t *A = (const uint8_t *)a.A;
   const uint8_t *Bt = (const uint8_t *)a.B.bt;
   const int threads = 32 * kGemvWarps;
   int sel = (a.a_signed ? 2 : 0) | (a.B.b_signed ? 1 : 0);
   switch (sel) {
   case 0:
-    gemm_i8_gemv_kernel<MT, CB, false, false><<<grid, threads, 0, st>>>(A, Bt, a.B.kp, p);
+    (void)launch_pdl(gemm_i8_gemv_kernel<MT, CB, false, false>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   case 1:
-    gemm_i8_gemv_kernel<MT, CB, false, true><<<grid, threads, 0, st>>>(A, Bt, a.B.kp, p);
+    (void)launch_pdl(gemm_i8_gemv_kernel<MT, CB, false, true>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   case 2:
-    gemm_i8_gemv_kernel<MT, CB, true, false><<<grid, threads, 0, st>>>(A, Bt, a.B.kp, p);
+    (void)launch_pdl(gemm_i8_gemv_kernel<MT, CB, true, false>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   default:
-    gemm_i8_gemv_kernel<MT, CB, true, true><<<grid, threads, 0, st>>>(A, Bt, a.B.kp, p);
+    (void)launch_pdl(gemm_i8_gemv_kernel<MT, CB, true, true>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   }
 }
@@ -580,16 +611,16 @@ static void launch_gemv_mma(const GemmCall &a, cudaStream_t st) {
   int sel = (a.a_signed ? 2 : 0) | (a.B.b_signed ? 1 : 0);
   switch (sel) {
   case 0:
-    gemm_i8_gemv_mma_kernel<CG, false, false><<<grid, threads, 0, st>>>(A, Bt, a.B.kp, p);
+    (void)launch_pdl(gemm_i8_gemv_mma_kernel<CG, false, false>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   case 1:
-    gemm_i8_gemv_mma_kernel<CG, false, true><<<grid, threads, 0, st>>>(A, Bt, a.B.kp, p);
+    (void)launch_pdl(gemm_i8_gemv_mma_kernel<CG, false, true>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   case 2:
-    gemm_i8_gemv_mma_kernel<CG, true, false><<<grid, threads, 0, st>>>(A, Bt, a.B.kp, p);
+    (void)launch_pdl(gemm_i8_gemv_mma_kernel<CG, true, false>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   default:
-    gemm_i8_gemv_mma_kernel<CG, true, true><<<grid, threads, 0, st>>>(A, Bt, a.B.kp, p);
+    (void)launch_pdl(gemm_i8_gemv_mma_kernel<CG, true, true>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   }
 }
