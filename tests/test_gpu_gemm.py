@@ -591,3 +591,19 @@ def test_qlinear_parameters_on_the_device(gpu, orc, ydt, M, K, N, per_column):
     want = orc.qlinear_matmul(*args)
     assert np.array_equal(gpu.qlinear_matmul(*args), want)
     assert np.array_equal(gpu.qlinear_matmul(*args, device=True).numpy(), want)
+
+
+@pytest.mark.parametrize("scale", [0.9, 70.0, 3e7])
+def test_qlinear_large_results(gpu, orc, scale):
+    # Results around and beyond 2^22 (and 2^31, where the conversion saturates):
+    # the tail's one-addition rounding hands those to the separate instructions.
+    rng = np.random.default_rng(34)
+    A, B = rand8(rng, (200, 512), np.uint8), rand8(rng, (512, 320), np.int8)
+    bs = (rng.uniform(0.5, 1.5, 320) * scale).astype(np.float32)
+    args = (A, np.float32(1.0), np.uint8(128), B, bs, np.zeros(320, np.int8), np.float32(1.0),
+            np.uint8(9))
+    x = np.abs((A.astype(np.int64) - 128) @ B.astype(np.int64)) * bs[None, :].astype(np.float64)
+    inside = x < 2**31 - 256     # beyond it the C conversion of the oracle is undefined
+    got, want = gpu.qlinear_matmul(*args), orc.qlinear_matmul(*args)
+    assert np.array_equal(got[inside], want[inside]) and inside.any()
+    assert (x > 2**22).any() or scale < 1
