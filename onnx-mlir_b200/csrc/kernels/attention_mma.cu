@@ -213,7 +213,11 @@ __global__ void __launch_bounds__(128)
         asm volatile("cp.async.wait_group 0;" ::: "memory");
       }
     } else {
-      // Stage K and V rows j0..j0+63 as bf16 hi/lo.
+      // Stage K and V rows j0..j0+63 as bf16 hi/lo, the loads of four trips
+      // together.  64 x 500 tokens, 12 heads of 64: 1009 us with ldmatrix
+      // below and one trip at a time, 831 with plain loads below, 688 with
+      // both; 8 x 512, 8 heads of 128: 131, 132, 121.
+#pragma unroll 4
       for (int i = threadIdx.x; i < kKeys * (DH / 4); i += 128) {
         const int key = i / (DH / 4), c4 = (i % (DH / 4)) * 4;
         float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
@@ -243,12 +247,22 @@ __global__ void __launch_bounds__(128)
     for (int ks = 0; ks < KS; ++ks) {
 #pragma unroll
       for (int nt = 0; nt < NT_S; ++nt) {
-        // 8x8 blocks: hi of k 0..7 and 8..15, then lo; a lane supplies one key row
         uint32_t bh0, bh1, bl0, bl1;
-        ldmatrix_x4((uint32_t)__cvta_generic_to_shared(
-                        &sK[lane >> 4][(nt * 8 + (lane & 7)) * LD + ks * 16 +
-                                       ((lane >> 3) & 1) * 8]),
-            bh0, bh1, bl0, bl1);
+        if (kPlanes) {
+          // 8x8 blocks: hi of k 0..7 and 8..15, then lo; a lane supplies one key row
+          ldmatrix_x4((uint32_t)__cvta_generic_to_shared(
+                          &sK[lane >> 4][(nt * 8 + (lane & 7)) * LD + ks * 16 +
+                                         ((lane >> 3) & 1) * 8]),
+              bh0, bh1, bl0, bl1);
+        } else {
+          // Plain loads here: these the compiler may move ahead among the MMAs,
+          // which the fp32 form needs, with the conversions between its barriers.
+          const int off = (nt * 8 + g) * LD + ks * 16 + 2 * t;
+          bh0 = *reinterpret_cast<const uint32_t *>(&sK[0][off]);
+          bh1 = *reinterpret_cast<const uint32_t *>(&sK[0][off + 8]);
+          bl0 = *reinterpret_cast<const uint32_t *>(&sK[1][off]);
+          bl1 = *reinterpret_cast<const uint32_t *>(&sK[1][off + 8]);
+        }
         mma_bf16(s[nt], ql[ks], bh0, bh1); // small terms first
         mma_bf16(s[nt], qh[ks], bl0, bl1);
         mma_bf16(s[nt], qh[ks], bh0, bh1);

@@ -87,6 +87,17 @@ def test_attention(gpu, orc, B, S, heads, dh):
     close(gpu.attention(q, k, v, heads, scale), orc.attention(q, k, v, heads, scale), 1e-3, 1e-5)
 
 
+@pytest.mark.parametrize("S", [1, 63, 65, 130, 333])
+@pytest.mark.parametrize("dh", [32, 64, 128])
+def test_attention_of_fp32_operands(gpu, orc, S, dh):
+    # The kernel that splits K and V into bf16 itself, 64 keys at a time: one
+    # ragged block, a whole one and a ragged one, several.
+    rng = np.random.default_rng(S + dh)
+    q, k, v = (rng.normal(size=(2, S, 3 * dh)).astype(np.float32) for _ in range(3))
+    scale = 1.0 / np.sqrt(dh)
+    close(gpu.attention(q, k, v, 3, scale), orc.attention(q, k, v, 3, scale), 1e-3, 1e-5)
+
+
 def test_attention_non_positive_scale(gpu, orc):
     # The graph's Mul constant may be any float.  The tensor-core kernel folds
     # the scale into the row maximum, which is only valid for a positive scale;
