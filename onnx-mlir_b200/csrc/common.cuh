@@ -90,11 +90,27 @@ __device__ __forceinline__ void pdl_sync() {
 
 // The pointer, for use after pdl_sync().  Read-only loads (__ldg, const
 // __restrict__) may legally be moved across a memory clobber; through the
-// pointer this returns they depend on what follows the wait.  Not needed where
-// a branch that is decided after the wait guards the load.
+// pointer this returns they depend on what follows the wait.  Every pointer
+// that such a kernel reads through passes through here, since any of a caller's
+// tensors may be its predecessor's output.  Not needed for copies issued by volatile asm
+// (TMA, cp.async), nor where a branch that is decided after the wait guards the
+// load: a bounds check on thread and block indices is not one, the wait for an
+// mbarrier that those copies complete is.
 template <typename T>
 __device__ __forceinline__ T *after_pdl(T *p) {
-  asm volatile("" : "+l"(p)::"memory");
+  // an offset of zero that the compiler cannot know: the pointer keeps what
+  // __restrict__ says about it
+  int64_t zero = 0;
+  asm volatile("" : "+l"(zero));
+  return (T *)((char *)p + zero);
+}
+
+// The same for a pointer of which the compiler shall forget what it knows, for
+// kernels that measured better so: all their loads are explicit (__ldg, __ldcs)
+// and the rest only moves registers.
+template <typename T>
+__device__ __forceinline__ T *after_pdl_opaque(T *p) {
+  asm volatile("" : "+l"(p));
   return p;
 }
 

@@ -117,6 +117,14 @@ __global__ void __launch_bounds__(128)
 
   extern __shared__ __align__(16) __nv_bfloat16 att_smem[];
   pdl_sync();
+  if (kPlanes) {
+    in.hi = after_pdl(in.hi);
+    in.lo = after_pdl(in.lo);
+  } else {
+    in.q = after_pdl(in.q);
+    in.k = after_pdl(in.k);
+    in.v = after_pdl(in.v);
+  }
   // [hi|lo][key][dh] for K, then the same for V; two such sets with kPlanes
   constexpr int kSet = 4 * kKeys * LD;
 

@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(kDqlThreads)
         DqlScratch *__restrict__ scr, float *__restrict__ y_scale,
         uint8_t *__restrict__ y_zp, int mode) {
   pdl_sync();
+  x = after_pdl(x);
   float lo = INFINITY, hi = -INFINITY;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
@@ -69,13 +70,13 @@ __global__ void __launch_bounds__(kDqlThreads)
       hi = fmaxf(hi, fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)));
     }
     for (int64_t j = (n4 << 2) + tid; j < n; j += nthreads) {
-      float v = x[j];
+      float v = __ldg(x + j);
       lo = fminf(lo, v);
       hi = fmaxf(hi, v);
     }
   } else {
     for (int64_t j = tid; j < n; j += nthreads) {
-      float v = x[j];
+      float v = __ldg(x + j);
       lo = fminf(lo, v);
       hi = fmaxf(hi, v);
     }
@@ -188,6 +189,7 @@ __global__ void __launch_bounds__(kDqlThreads)
         int has_zp, const uint32_t *__restrict__ range, QuantOutputs outs, int mode,
         int unroll) {
   pdl_sync();
+  x = after_pdl(x);
   params = after_pdl(params);
   scale_ptr = after_pdl(scale_ptr);
   zp8 = after_pdl(zp8);
@@ -252,7 +254,7 @@ __global__ void __launch_bounds__(kDqlThreads)
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
   for (int64_t j = (n4 << 2) + tid; j < n; j += nthreads)
-    y[j] = (uint8_t)quantize_one<kSigned>(x[j], qc);
+    y[j] = (uint8_t)quantize_one<kSigned>(__ldg(x + j), qc);
 }
 
 // The quantize pass for rows whose length is no multiple of 16, written in the
@@ -264,6 +266,7 @@ __global__ void __launch_bounds__(kDqlThreads)
         uint8_t *__restrict__ y, int32_t *__restrict__ rowsum,
         const float *__restrict__ params, int mode) {
   pdl_sync();
+  x = after_pdl(x);
   params = after_pdl(params);
   __shared__ int32_t part[kDqlThreads / 32];
   const QuantConsts qc = make_quant_consts(__ldg(params), __ldg(params + 1), mode);
@@ -342,6 +345,7 @@ __global__ void __launch_bounds__(kSmallThreads) dql_small_kernel(SmallDql p) {
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned ctas = cluster.num_blocks(), rank = cluster.block_rank();
   pdl_sync();
+  const float *x = after_pdl(p.x);
   cluster.barrier_arrive(); // "has started": waited for before the first remote store
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tid = (int)(rank * kSmallThreads + threadIdx.x);
@@ -358,7 +362,7 @@ __global__ void __launch_bounds__(kSmallThreads) dql_small_kernel(SmallDql p) {
     if (w >= p.words)
       continue;
     const int r = w / p.row_words, c = 4 * (w - r * p.row_words);
-    const float *src = p.x + (int64_t)r * p.cols + c;
+    const float *src = x + (int64_t)r * p.cols + c;
     const int have = p.cols - c;
     if (have >= 4 && p.vec_in) {
       v[u] = __ldg(reinterpret_cast<const float4 *>(src));

@@ -98,6 +98,11 @@ __global__ void __launch_bounds__(256)
         float eps, float *__restrict__ y, uint32_t *__restrict__ out_range) {
   constexpr int64_t cols = (int64_t)NV * 128;
   pdl_sync();
+  // (opaque: an encoder run of 1 x 61 tokens 667 us, 673 with after_pdl)
+  x = after_pdl_opaque(x);
+  residual = after_pdl_opaque(residual);
+  gamma = after_pdl_opaque(gamma);
+  beta = after_pdl_opaque(beta);
   const int lane = threadIdx.x & 31;
   const int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   float lo = INFINITY, hi = -INFINITY;

@@ -90,6 +90,22 @@ __device__ __forceinline__ int32_t load_zp8(
                    : (int32_t) reinterpret_cast<const uint8_t *>(p)[i];
 }
 
+// The parameters for a kernel that pdl_sync() precedes (see after_pdl).  The
+// tensor-core kernels do without: per tile they read behind the mbarrier wait
+// for its accumulators, and what they read before is wrapped where it is read.
+__device__ __forceinline__ EpiParams epi_after_pdl(EpiParams p) {
+  p.a_zp = after_pdl(p.a_zp);
+  p.b_zp = after_pdl(p.b_zp);
+  p.colsum = after_pdl(p.colsum);
+  p.rowsum = after_pdl(p.rowsum);
+  p.sa = after_pdl(p.sa);
+  p.sb = after_pdl(p.sb);
+  p.bias = after_pdl(p.bias);
+  p.y_zp_dev = after_pdl(p.y_zp_dev);
+  p.residual = after_pdl(p.residual);
+  return p;
+}
+
 // Values that are fixed for one output row.
 struct EpiRow {
   int32_t az;
@@ -122,14 +138,14 @@ __device__ __forceinline__ EpiScalars epi_scalars(const EpiParams &p) {
   s.s0 = 1.0f;
   s.yz = (uint32_t)p.y_zp;
   if (epi_is_dequant(p.kind)) {
-    s.sa = __ldg(p.sa);
+    s.sa = __ldg(after_pdl(p.sa));
     if (p.sb_len == 1)
-      s.s0 = __fmul_rn(s.sa, __ldg(p.sb)); // onnx.Mul of the two scalars
+      s.s0 = __fmul_rn(s.sa, __ldg(after_pdl(p.sb))); // onnx.Mul of the two scalars
   } else if (p.kind == OMCUDA_EPI_REQUANT) {
     if (p.sb_len == 1)
-      s.s0 = __ldg(p.sb);
+      s.s0 = __ldg(after_pdl(p.sb));
     if (p.y_zp_dev)
-      s.yz = __ldg(p.y_zp_dev);
+      s.yz = __ldg(after_pdl(p.y_zp_dev));
   }
   return s;
 }

@@ -316,8 +316,9 @@ __device__ __forceinline__ QuantConsts epi_quant_consts(const EpiParams &p, bool
   if (EPI != OMCUDA_EPI_DEQUANT_QUANT)
     return QuantConsts{1.0f, 1.0f, 0.0f, true};
   float scale, zp_f;
-  dql_params_from_range(ordered_to_f32(__ldg(p.q_range)),
-      ordered_to_f32(__ldg(p.q_range + 1)), &scale, &zp_f, p.quant_mode);
+  const uint32_t *range = after_pdl(p.q_range);
+  dql_params_from_range(ordered_to_f32(__ldg(range)), ordered_to_f32(__ldg(range + 1)),
+      &scale, &zp_f, p.quant_mode);
   if (publish) {
     p.q_params[0] = scale;
     p.q_params[1] = zp_f;
@@ -582,7 +583,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   tcgen05_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
   volatile int *abortp = &abort_flag;
-  pdl_sync(); // (every load below is guarded by a branch on the warp)
+  pdl_sync(); // (loads below: see epi_after_pdl)
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -858,7 +859,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   tcgen05_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
   volatile int *abortp = &abort_flag;
-  pdl_sync(); // (every load below is guarded by a branch on the warp)
+  pdl_sync(); // (loads below: see epi_after_pdl)
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------

@@ -1,0 +1,99 @@
+"""Kernels that may be set up while their predecessor still runs, checked in
+their sources (no GPU): each waits for it, and each pointer it reads through
+passes through after_pdl() behind that wait, so that the order of a read-only
+load does not rest on what the compiler happens not to move."""
+import glob
+import os
+import re
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "onnx-mlir_b200", "csrc")
+
+
+def sources():
+    text = ""
+    for path in sorted(glob.glob(os.path.join(CSRC, "**", "*.cu*"), recursive=True)):
+        text += re.sub(r"//[^\n]*", "", open(path).read()) + "\n"
+    return text
+
+
+def block(text, start, opening, closing):
+    """text[start] is `opening`; the text up to its partner, and the index behind it."""
+    depth = 0
+    for i in range(start, len(text)):
+        depth += (text[i] == opening) - (text[i] == closing)
+        if depth == 0:
+            return text[start + 1:i], i + 1
+    raise AssertionError("unbalanced")
+
+
+def kernels(text):
+    """name -> (parameter list, body)"""
+    out = {}
+    for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\s*(?P<b>\())?", text):
+        at = m.end()
+        if m.group("b"):
+            _, at = block(text, m.end() - 1, "(", ")")
+        name = re.compile(r"\s*(\w+)\s*").match(text, at)
+        params, at = block(text, name.end(), "(", ")")
+        brace = text.index("{", at)
+        if text[at:brace].strip():
+            continue  # a declaration
+        body, _ = block(text, brace, "{", "}")
+        out[name.group(1)] = (params, body)
+    return out
+
+
+def const_pointer_members(text, struct):
+    m = re.search(r"\bstruct %s\s*\{" % struct, text)
+    body, _ = block(text, m.end() - 1, "{", "}")
+    return [name for decl in re.findall(r"\bconst\s+\w+\s*(\*[^;(]*);", body)
+            for name in re.findall(r"\*\s*(\w+)", decl)]
+
+
+def test_every_overlapped_kernel_waits():
+    text = sources()
+    launched = set(re.findall(r"launch_pdl\(\s*(\w+_kernel)\b", text))
+    launched |= set(re.findall(r"\?\s*(\w+_kernel)<", text))  # chosen inside the call
+    ks = kernels(text)
+    assert len(launched) >= 9
+    for name in launched:
+        assert len(re.findall(r"\bpdl_sync\(\)", ks[name][1])) == 1, name
+
+
+def test_loads_depend_on_the_wait():
+    text = sources()
+    epilogue = re.search(r"EpiParams epi_after_pdl\(EpiParams p\)\s*\{", text)
+    wrapped_by_epilogue = block(text, epilogue.end() - 1, "{", "}")[0] if epilogue else ""
+    missing = []
+    for name, (params, body) in kernels(text).items():
+        if "pdl_sync()" not in body:
+            continue
+        behind = body[body.index("pdl_sync()"):]
+        for ptr in re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", params):
+            if not re.search(r"\b%s = after_pdl(?:_opaque)?\(%s\);" % (ptr, ptr), behind):
+                missing.append((name, ptr))
+        for struct, arg in re.findall(r"\b([A-Z]\w+)\s+(\w+)\s*(?:,|$)", params):
+            if struct not in ("EpiParams", "SmallDql", "AttOperands"):
+                continue
+            for member in const_pointer_members(text, struct):
+                if struct == "EpiParams":
+                    # The tensor-core kernels read it per tile, behind the
+                    # mbarrier wait for the tile's accumulators, and the
+                    # scalars (below) before that; the range is theirs alone.
+                    if "mbar_wait(" in behind or member == "q_range":
+                        continue
+                    done = ("epi_after_pdl(%s)" % arg in behind and
+                            "p.%s = after_pdl(p.%s);" % (member, member) in wrapped_by_epilogue)
+                else:
+                    done = "after_pdl(%s.%s)" % (arg, member) in behind
+                if not done:
+                    missing.append((name, "%s.%s" % (arg, member)))
+    assert not missing, missing
+    for name, members in (("epi_scalars", ("sa", "sb", "y_zp_dev")),
+                          ("epi_quant_consts", ("q_range",))):
+        m = re.search(r"%s\(const EpiParams &p[^)]*\)\s*\{" % name, text)
+        body, _ = block(text, m.end() - 1, "{", "}")
+        for member in members:
+            assert not re.search(r"__ldg\(p\.%s\b" % member, body), (name, member)
+            assert "after_pdl(p.%s)" % member in body, (name, member)
