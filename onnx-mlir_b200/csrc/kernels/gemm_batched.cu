@@ -108,8 +108,11 @@ __global__ void __launch_bounds__(kBatThreads, 5)
   const int ac = tid % kChunks, ar = tid / kChunks;
   const int bn = (tid & 15) * 4, bk = (tid >> 4) * 4;
   const int ncols = g.N - (n0 + bn) < 4 ? g.N - (n0 + bn) : 4;
-  const uint8_t *pa = A + (m0 + ar) * g.K + 16 * ac; // (M K and K N are below 2^31)
-  const uint8_t *pb = B + bk * g.N + n0 + bn;
+  // Offsets of rows that exist fit 31 bits, M K and K N being at most 2^30.  A thread
+  // past M or K forms some other offset, without overflow in the unsigned, and never
+  // reads there.  (64 bits here take registers the loop needs: spills.)
+  const uint8_t *pa = A + (uint32_t)(m0 + ar) * (uint32_t)g.K + 16 * ac;
+  const uint8_t *pb = B + (uint32_t)bk * (uint32_t)g.N + n0 + bn;
   int32_t rsum[kARows], csum[4] = {0, 0, 0, 0};
 #pragma unroll
   for (int i = 0; i < kARows; ++i)

@@ -545,6 +545,25 @@ def test_batched_b_operand(gpu, orc, lead, M, K, N, adt, bdt):
     assert np.array_equal(got.numpy(), orc.matmul_integer(A, B, az, bz))
 
 
+@pytest.mark.parametrize("M,K,N", [(1, 2, (1 << 27) + 4),  # 28 rows of B are beyond 2^31
+                                   (1, 17 << 21, 1)])       # 63 rows of A are
+def test_batched_b_operand_offsets(gpu, M, K, N):
+    # The offsets of a tile's rows that do not exist would not fit 32 bits.
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(35)
+    a = torch.randint(0, 256, (3, M, K), device="cuda", generator=g, dtype=torch.uint8)
+    b = torch.randint(0, 256, (3, K, N), device="cuda", generator=g, dtype=torch.uint8)
+    torch.cuda.synchronize()
+    y = gpu.matmul_integer(gpu.Tensor.from_cuda_array(a), gpu.Tensor.from_cuda_array(b), device=True)
+    got = torch.as_tensor(y, device="cuda")
+    for i in range(3):
+        if N == 1:
+            want = (a[i, 0].int() * b[i, :, 0].int()).sum(dtype=torch.int64).to(torch.int32)
+            assert got[i].item() == want.item()
+        else:
+            assert torch.equal(got[i, 0], (a[i].reshape(K, 1).int() * b[i].int()).sum(0, dtype=torch.int32))
+
+
 @pytest.mark.parametrize("M,K,N,wdt", [
     (1, 17, 5, np.uint8), (16, 257, 33, np.int8),   # GEMV-shaped kernels, padded rows
     (17, 15, 64, np.uint8),                         # less than one 16-byte chunk of K
