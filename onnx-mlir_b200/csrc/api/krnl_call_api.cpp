@@ -696,11 +696,9 @@ void omcudaMatMulInteger(OMTensor *Y, const OMTensor *A, const OMTensor *B,
   // B is an activation: all products in one launch, nothing prepared.
   BatchedGemm bg;
   memset(&bg, 0, sizeof(bg));
-  if (azn <= 1 && gemm_batched_wanted(d.batch, d.M, d.N, d.K) && batched_dims(d, &bg) &&
+  if (azn <= 1 && batched_dims(d, &bg) &&
+      gemm_batched_wanted(dA, dB, d.batch, d.M, d.N, d.K, &bg) &&
       !is_registered_constant(omTensorGetDataPtr(B))) {
-    bg.M = (int)d.M;
-    bg.N = (int)d.N;
-    bg.K = (int)d.K;
     bg.a_zp = dAz;
     bg.a_zp_len = (int)azn;
     bg.b_zp = dBz;

@@ -280,18 +280,51 @@ __global__ void __launch_bounds__(kBatThreads, 5)
 // tcgen05: mma.sync makes the same tile several times slower, while the three
 // launches of the prepared path cost some 20 us.
 constexpr int64_t kBatchedMaxOps = int64_t(1) << 31;
-// One product alone has to fill the machine with 64 x 64 tiles and a K loop
-// that no other product overlaps: only small ones gain.
 constexpr int64_t kSingleMaxOps = int64_t(1) << 26;
+// Preparing B goes along K with one block row per 64 bytes, of which a grid
+// holds this many: beyond, this kernel is the only one that takes the product.
+constexpr int64_t kPreparedMaxK = int64_t(65535) * 64;
 
-bool gemm_batched_wanted(int64_t batch, int64_t M, int64_t N, int64_t K) {
+// A block walks K by itself, a step of 128 bytes after another: 11 ns per byte of
+// K where A and B take whole words, 16 where only B does, 19 to 36 where B does
+// not (us for K bytes, here / prepared):
+//   one product, whole words   64 x 4096 x 64     52 /  70   1 x 16384 x 64  191 / 193
+//                              1 x 65536 x 64    750 / 732   (N > 64: 970 / 4269 for two
+//                              of 1 x 65536 x 1024; one of 1 x 32768 x 1024 361 / 439)
+//   A in single bytes          64 x 2047 x 64     40 /  45   64 x 4095 x 64   75 /  70
+//   B in single bytes          1 x 255 x 63       14 /  18   1 x 511 x 63     22 /  20
+//   two products, B so         16 x 2047 x 255    76 /  78   16 x 4095 x 255 146 / 124
+// The prepared path takes products one after another, so that from three on
+// this kernel was never slower (three of 1 x 65536 x 63 2190 / 2217), and two in
+// whole words of B never either.
+bool gemm_batched_wanted(const void *A, const void *B, int64_t batch, int64_t M, int64_t N,
+    int64_t K, BatchedGemm *g) {
   if (K <= 0 || M >= (int64_t(1) << 30) || N >= (int64_t(1) << 30) || K >= (int64_t(1) << 30))
     return false;
   const int64_t blocks = batch * ceil_div(M, kTile) * ceil_div(N, kTile);
   if (blocks <= 0 || blocks >= (int64_t(1) << 31))
     return false;
   const double ops = 2.0 * (double)M * (double)N * (double)K;
-  return ops <= (double)(batch > 1 ? kBatchedMaxOps : kSingleMaxOps);
+  if (ops > (double)(batch > 1 ? kBatchedMaxOps : kSingleMaxOps))
+    return false;
+  g->M = (int)M;
+  g->N = (int)N;
+  g->K = (int)K;
+  uintptr_t a_low = (uintptr_t)A | (uintptr_t)K, b_low = (uintptr_t)B | (uintptr_t)N;
+  for (int d = 0; d < g->dims; ++d) {
+    a_low |= (uintptr_t)g->a_stride[d];
+    b_low |= (uintptr_t)g->b_stride[d];
+  }
+  g->vec_a = (a_low & 15u) == 0;
+  g->vec_b = (b_low & 3u) == 0;
+  if (batch > 2 || K > kPreparedMaxK)
+    return true;
+  if (batch == 2)
+    return g->vec_b || K <= 2048;
+  if (!g->vec_b)
+    return K <= 384;
+  // (up to 16 rows a thread reads one of them, in single bytes as fast)
+  return g->vec_a || M <= 16 ? K <= 16384 || N > kTile : K <= 2048;
 }
 
 template <bool kASigned, bool kBSigned, bool kVecA, bool kVecB>
@@ -322,12 +355,7 @@ int launch_gemm_batched(const void *A, int a_signed, const void *B, int b_signed
     int32_t *Y, int64_t batch, BatchedGemm g, cudaStream_t st) {
   g.tiles_m = (int)ceil_div(g.M, kTile);
   g.tiles_n = (int)ceil_div(g.N, kTile);
-  uintptr_t a_low = (uintptr_t)A | (uintptr_t)g.K, b_low = (uintptr_t)B | (uintptr_t)g.N;
-  for (int d = 0; d < g.dims; ++d) {
-    a_low |= (uintptr_t)g.a_stride[d];
-    b_low |= (uintptr_t)g.b_stride[d];
-  }
-  const bool vec_a = (a_low & 15u) == 0, vec_b = (b_low & 3u) == 0;
+  const bool vec_a = g.vec_a != 0, vec_b = g.vec_b != 0;
   g.y_vec = (((uintptr_t)Y & 7u) == 0) && (g.N & 1) == 0;
   const unsigned grid = (unsigned)(batch * g.tiles_m * g.tiles_n);
   const uint8_t *a = (const uint8_t *)A, *b = (const uint8_t *)B;

@@ -105,10 +105,15 @@ struct BatchedGemm {
   int a_zp_len;     // 0 or 1
   const void *b_zp;
   int b_zp_len;     // 0, 1 or N
+  // set by gemm_batched_wanted: A takes 16-byte loads everywhere, B 4-byte ones
+  int vec_a, vec_b;
   // set by the launcher
   int tiles_m, tiles_n, y_vec;
 };
-bool gemm_batched_wanted(int64_t batch, int64_t M, int64_t N, int64_t K);
+// Whether this kernel is the one for these products; g has its batch dimensions
+// and gets its sizes and alignment.
+bool gemm_batched_wanted(const void *A, const void *B, int64_t batch, int64_t M, int64_t N,
+    int64_t K, BatchedGemm *g);
 int launch_gemm_batched(const void *A, int a_signed, const void *B, int b_signed,
     int32_t *Y, int64_t batch, BatchedGemm g, cudaStream_t st);
 

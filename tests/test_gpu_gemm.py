@@ -545,6 +545,29 @@ def test_batched_b_operand(gpu, orc, lead, M, K, N, adt, bdt):
     assert np.array_equal(got.numpy(), orc.matmul_integer(A, B, az, bz))
 
 
+@pytest.mark.parametrize("batch,M,K,N,one", [
+    (1, 1, 16384, 64, True), (1, 1, 16400, 64, False), (1, 1, 16400, 68, True),  # whole words
+    (1, 17, 2047, 64, True), (1, 17, 2049, 64, False),      # A in single bytes
+    (1, 16, 2049, 64, True),                                # ... of which there are few
+    (1, 1, 384, 63, True), (1, 1, 385, 63, False),          # B in single bytes
+    (2, 1, 2048, 63, True), (2, 1, 2049, 63, False), (2, 1, 4099, 64, True),
+    (3, 1, 16401, 63, True),                                # from three products on
+    (1, 1, 65535 * 64 + 1, 1, True),                        # B cannot be prepared
+])
+def test_which_products_run_in_one_launch(gpu, orc, batch, M, K, N, one):
+    # A product whose B is no constant goes to the one-launch kernel where that
+    # is the faster way: both sides of each line of the rule.
+    rng = np.random.default_rng(K + N)
+    lead = (batch,) if batch > 1 else ()
+    A, B = rand8(rng, lead + (M, K), np.uint8), rand8(rng, lead + (K, N), np.int8)
+    az, bz = rand8(rng, (), np.uint8), rand8(rng, (), np.int8)
+    t = [gpu.Tensor.from_numpy(x).to_device() for x in (A, B, az, bz)]
+    before = gpu.launch_count()
+    got = gpu.matmul_integer(*t, device=True)
+    assert (gpu.launch_count() - before == 1) == one
+    assert np.array_equal(got.numpy(), orc.matmul_integer(A, B, az, bz))
+
+
 @pytest.mark.parametrize("M,K,N", [(1, 2, (1 << 27) + 4),  # 28 rows of B are beyond 2^31
                                    (1, 17 << 21, 1)])       # 63 rows of A are
 def test_batched_b_operand_offsets(gpu, M, K, N):
