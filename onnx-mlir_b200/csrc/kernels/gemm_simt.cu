@@ -70,16 +70,22 @@ __device__ __forceinline__ float requant_scale(const RequantScale &rq, int64_t i
 
 // One warp per row, a 16-byte chunk per lane and trip; with dst, the row is also
 // copied into an aligned row of `pitch` bytes whose tail is zero.  The column
-// scales of a QLinearMatMul ride along (rq.len != 0): a launch of their own was
-// 2.1 us for a few thousand divides.
+// scales of a QLinearMatMul ride along (rq.len != 0) in blocks behind those of
+// the rows: a launch of their own was 2.1 us for a few thousand divides, and made
+// by the blocks of the rows, one of them for up to 8 rows, they were a serial chain
+// (1 x 256 x 32768: 45 us a call so, 19 now).
 template <bool kSigned>
 __global__ void __launch_bounds__(256)
     rowsum_kernel(const uint8_t *__restrict__ A, int64_t M, int64_t K,
         int32_t *__restrict__ rowsum, uint8_t *__restrict__ dst, int64_t pitch,
         RequantScale rq) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rq.len;
-       i += (int64_t)gridDim.x * blockDim.x)
-    rq.S[i] = requant_scale(rq, i);
+  const int64_t row_blocks = ceil_div(M, (int64_t)(blockDim.x >> 5));
+  if (blockIdx.x >= row_blocks) {
+    const int64_t i = ((int64_t)blockIdx.x - row_blocks) * blockDim.x + threadIdx.x;
+    if (i < rq.len)
+      rq.S[i] = requant_scale(rq, i);
+    return;
+  }
   const int64_t m = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (m >= M)
     return;
@@ -694,7 +700,7 @@ int launch_gemm_simt(const GemmCall &a, cudaStream_t st) {
 
 int launch_repitch(const void *A, int a_signed, int64_t M, int64_t K, int64_t pitch,
     uint8_t *dst, int32_t *rowsum, const RequantScale &rq, cudaStream_t st) {
-  const unsigned grid = (unsigned)ceil_div(M, 8);
+  const unsigned grid = (unsigned)(ceil_div(M, 8) + ceil_div(rq.len, 256));
   if (a_signed)
     rowsum_kernel<true><<<grid, 256, 0, st>>>((const uint8_t *)A, M, K, rowsum, dst, pitch, rq);
   else

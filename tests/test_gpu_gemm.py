@@ -635,6 +635,18 @@ def test_qlinear_parameters_on_the_device(gpu, orc, ydt, M, K, N, per_column):
     assert np.array_equal(gpu.qlinear_matmul(*args, device=True).numpy(), want)
 
 
+@pytest.mark.parametrize("M,K,N", [(1, 64, 255), (1, 33, 256), (8, 64, 257), (9, 40, 5000),
+                                   (70, 64, 40)])
+def test_qlinear_scales_beside_row_sums(gpu, orc, M, K, N):
+    # One launch makes the row sums (8 rows a block) and the column scales (256 a
+    # block): more blocks of either, and the edges of both.
+    rng = np.random.default_rng(M + N)
+    A, B, bs, _ = qlinear_case(rng, (M,), K, N)
+    bz = rand8(rng, N, np.int8)
+    args = (A, np.float32(0.02), np.uint8(128), B, bs, bz, np.float32(0.5), np.uint8(11))
+    assert np.array_equal(gpu.qlinear_matmul(*args, device=True).numpy(), orc.qlinear_matmul(*args))
+
+
 @pytest.mark.parametrize("scale", [0.9, 70.0, 3e7])
 def test_qlinear_large_results(gpu, orc, scale):
     # Results around and beyond 2^22 (and 2^31, where the conversion saturates):
