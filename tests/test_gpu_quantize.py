@@ -195,3 +195,30 @@ def test_pass_run_edges(gpu, orc, n, shift):
         out = y.cpu().numpy()
         assert out[shift:shift + n].tobytes() == orc.dequantize_linear(vals, 0.37, 5).tobytes()
         assert (out[:shift] == -1).all() and (out[shift + n:] == -1).all()
+
+
+@pytest.mark.parametrize("dt", [np.uint8, np.int8, np.int32])
+@pytest.mark.parametrize("xs,ys", [(0, 0), (4, 4), (4, 1), (1, 4), (3, 2)])
+@pytest.mark.parametrize("n", [1, 3, 5, 1023, 40001])
+def test_dequantize_alignments(gpu, orc, dt, xs, ys, n):
+    # Groups of four values where both tensors start on one, single values
+    # where either does not; the last one to three values of a ragged size.
+    import torch
+    rng = np.random.default_rng(n)
+    info = np.iinfo(dt)
+    vals = rng.integers(max(info.min, -10**6), min(info.max, 10**6), size=n).astype(dt)
+    src = torch.zeros(n + 8, dtype=getattr(torch, np.dtype(dt).name), device="cuda")
+    src[xs:xs + n] = torch.from_numpy(vals).cuda()
+    y = torch.full((n + 8,), -1.0, device="cuda")
+    torch.cuda.synchronize()
+    t = [gpu.Tensor.from_cuda_array(y[ys:ys + n]), gpu.Tensor.from_cuda_array(src[xs:xs + n]),
+         gpu.Tensor.from_numpy(np.array(0.0123, np.float32))]
+    for zp in (np.array(5, dt), None):
+        z = gpu.Tensor.from_numpy(zp) if zp is not None else None
+        gpu.lib().omcudaDequantizeLinear(*[a.handle for a in t], z.handle if z else None)
+        gpu.check()
+        torch.cuda.synchronize()
+        out = y.cpu().numpy()
+        want = orc.dequantize_linear(vals, 0.0123, 5 if zp is not None else 0)
+        assert out[ys:ys + n].tobytes() == want.tobytes()
+        assert (out[:ys] == -1).all() and (out[ys + n:] == -1).all()
