@@ -697,7 +697,7 @@ void omcudaMatMulInteger(OMTensor *Y, const OMTensor *A, const OMTensor *B,
   BatchedGemm bg;
   memset(&bg, 0, sizeof(bg));
   if (azn <= 1 && batched_dims(d, &bg) &&
-      gemm_batched_wanted(dA, dB, d.batch, d.M, d.N, d.K, &bg) &&
+      gemm_batched_wanted(dA, dB, d.batch, d.M, d.N, d.K, st, &bg) &&
       !is_registered_constant(omTensorGetDataPtr(B))) {
     bg.a_zp = dAz;
     bg.a_zp_len = (int)azn;

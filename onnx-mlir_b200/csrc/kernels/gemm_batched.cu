@@ -298,7 +298,7 @@ constexpr int64_t kPreparedMaxK = int64_t(65535) * 64;
 // this kernel was never slower (three of 1 x 65536 x 63 2190 / 2217), and two in
 // whole words of B never either.
 bool gemm_batched_wanted(const void *A, const void *B, int64_t batch, int64_t M, int64_t N,
-    int64_t K, BatchedGemm *g) {
+    int64_t K, cudaStream_t st, BatchedGemm *g) {
   if (K <= 0 || M >= (int64_t(1) << 30) || N >= (int64_t(1) << 30) || K >= (int64_t(1) << 30))
     return false;
   const int64_t blocks = batch * ceil_div(M, kTile) * ceil_div(N, kTile);
@@ -319,12 +319,23 @@ bool gemm_batched_wanted(const void *A, const void *B, int64_t batch, int64_t M,
   g->vec_b = (b_low & 3u) == 0;
   if (batch > 2 || K > kPreparedMaxK)
     return true;
+  bool faster;
   if (batch == 2)
-    return g->vec_b || K <= 2048;
-  if (!g->vec_b)
-    return K <= 384;
-  // (up to 16 rows a thread reads one of them, in single bytes as fast)
-  return g->vec_a || M <= 16 ? K <= 16384 || N > kTile : K <= 2048;
+    faster = g->vec_b || K <= 2048;
+  else if (!g->vec_b)
+    faster = K <= 384;
+  else // (up to 16 rows a thread reads one of them, in single bytes as fast)
+    faster = g->vec_a || M <= 16 ? K <= 16384 || N > kTile : K <= 2048;
+  if (faster)
+    return true;
+  // The prepared path takes blocks of the pool, which a captured call must not
+  // (its replays would write to them after they were given back).
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return cs != cudaStreamCaptureStatusNone;
 }
 
 template <bool kASigned, bool kBSigned, bool kVecA, bool kVecB>

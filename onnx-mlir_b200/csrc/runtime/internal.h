@@ -110,10 +110,10 @@ struct BatchedGemm {
   // set by the launcher
   int tiles_m, tiles_n, y_vec;
 };
-// Whether this kernel is the one for these products; g has its batch dimensions
-// and gets its sizes and alignment.
+// Whether this kernel is the one for these products on this stream; g has its
+// batch dimensions and gets its sizes and alignment.
 bool gemm_batched_wanted(const void *A, const void *B, int64_t batch, int64_t M, int64_t N,
-    int64_t K, BatchedGemm *g);
+    int64_t K, cudaStream_t st, BatchedGemm *g);
 int launch_gemm_batched(const void *A, int a_signed, const void *B, int b_signed,
     int32_t *Y, int64_t batch, BatchedGemm g, cudaStream_t st);
 

@@ -568,6 +568,49 @@ def test_which_products_run_in_one_launch(gpu, orc, batch, M, K, N, one):
     assert np.array_equal(got.numpy(), orc.matmul_integer(A, B, az, bz))
 
 
+def test_captured_product_needs_no_pool(gpu, orc):
+    # A product with a long K, which would go to the prepared path, stays one launch
+    # on the operands as they lie while its stream is being captured: a replay
+    # reads what the tensors hold then and writes nothing but Y.
+    import torch
+    M, K, N = 3, 4099, 63
+    rng = np.random.default_rng(37)
+    a, b = (torch.empty(s, dtype=torch.uint8, device="cuda") for s in ((M, K), (K, N)))
+    y = torch.zeros((M, N), dtype=torch.int32, device="cuda")
+    az, bz = (torch.tensor(v, dtype=torch.uint8, device="cuda") for v in (7, 200))
+    t = [gpu.Tensor.from_cuda_array(x) for x in (y, a, b, az, bz)]
+    call = [x.handle for x in t]
+    L = gpu.lib()
+    before = gpu.launch_count()
+    L.omcudaMatMulInteger(*call)
+    assert gpu.launch_count() - before > 1
+    gpu.check()
+    # (a short K loads the one-launch kernel outside the capture)
+    gpu.matmul_integer(rand8(rng, (M, 301), np.uint8), rand8(rng, (301, N), np.uint8),
+                       np.array(7, np.uint8), np.array(200, np.uint8))
+    gpu.synchronize()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    try:
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            L.omcudaSetStream(stream.cuda_stream)
+            before = gpu.launch_count()
+            L.omcudaMatMulInteger(*call)
+            assert gpu.launch_count() - before == 1
+    finally:
+        L.omcudaSetStream(None)
+    gpu.check()
+    for _ in range(2):
+        A, B = rand8(rng, (M, K), np.uint8), rand8(rng, (K, N), np.uint8)
+        a.copy_(torch.from_numpy(A))
+        b.copy_(torch.from_numpy(B))
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        want = orc.matmul_integer(A, B, np.array(7, np.uint8), np.array(200, np.uint8))
+        assert np.array_equal(y.cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("M,K,N", [(1, 2, (1 << 27) + 4),  # 28 rows of B are beyond 2^31
                                    (1, 17 << 21, 1)])       # 63 rows of A are
 def test_batched_b_operand_offsets(gpu, M, K, N):
