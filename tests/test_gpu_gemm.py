@@ -545,6 +545,71 @@ def test_batched_b_operand(gpu, orc, lead, M, K, N, adt, bdt):
     assert np.array_equal(got.numpy(), orc.matmul_integer(A, B, az, bz))
 
 
+def device_view(gpu, x, shift):
+    """x on the device, `shift` bytes past an aligned address; and its buffer."""
+    import torch
+    buf = torch.zeros(x.size + shift, dtype=torch.uint8, device="cuda")
+    buf[shift:] = torch.from_numpy(np.ascontiguousarray(x).view(np.uint8).reshape(-1)).cuda()
+    torch.cuda.synchronize()
+    view = buf[shift:].view(torch.int8 if x.dtype == np.int8 else torch.uint8).view(x.shape)
+    return gpu.Tensor.from_cuda_array(view), buf
+
+
+@pytest.mark.parametrize("adt,bdt", [(np.uint8, np.int8), (np.int8, np.uint8)])
+@pytest.mark.parametrize("M,K,N", [(1, 101, 70), (9, 101, 70), (16, 96, 33), (17, 101, 64),
+                                   (40, 1001, 70), (40, 96, 300)])
+def test_registered_weight(gpu, orc, M, K, N, adt, bdt):
+    # A weight that is a registered constant takes the prepared path whatever its
+    # size: A in aligned rows as it lies, in others read as it lies by the kernels
+    # for few rows and copied into aligned rows otherwise, with row sums in that
+    # pass or without; the second call uses the prepared form of the first.
+    rng = np.random.default_rng(M * K + N)
+    A, B = rand8(rng, (M, K), adt), rand8(rng, (K, N), bdt)
+    az, bz, bzn = rand8(rng, (), adt), rand8(rng, (), bdt), rand8(rng, N, bdt)
+    Bd = gpu.Tensor.from_numpy(B).to_device()
+    gpu.lib().omcudaRegisterConstant(Bd.handle)
+    try:
+        for shift in (0, 1, 3):
+            Ad, keep = device_view(gpu, A, shift)
+            for a_zp, b_zp in ((None, None), (az, None), (None, bz), (az, bzn)):
+                before = gpu.launch_count()
+                got = gpu.matmul_integer(Ad, Bd, a_zp, b_zp, device=True).numpy()
+                assert gpu.launch_count() > before
+                assert np.array_equal(got, orc.matmul_integer(A, B, a_zp, b_zp)), (shift, a_zp, b_zp)
+    finally:
+        gpu.synchronize()
+        gpu.lib().omcudaForgetConstants()
+
+
+@pytest.mark.parametrize("lead_a,lead_b,M,K,N,constant", [
+    # more batch dimensions than the one-launch kernel's argument block holds;
+    # eight B slices for 128 products
+    ((2, 1, 2, 1, 2, 1, 2), (1, 2, 1, 2, 1, 2, 1), 5, 33, 7, False),
+    ((2, 1, 2, 1, 2, 1, 2), (1, 2, 1, 2, 1, 2, 1), 19, 33, 16, False),
+    ((3,), (3,), 20, 48, 24, True),          # a batched weight
+    ((2, 3), (3,), 4, 31, 9, True),          # ... shared by the outer dimension
+    ((2,), (2,), 1024, 1025, 1032, False),   # products too large for mma.sync
+])
+def test_products_one_after_another(gpu, orc, lead_a, lead_b, M, K, N, constant):
+    # The prepared path of a batched B: a loop over the products, A slices at
+    # whatever address they start, B slices prepared once each.
+    rng = np.random.default_rng(M * K + N)
+    A, B = rand8(rng, lead_a + (M, K), np.uint8), rand8(rng, lead_b + (K, N), np.int8)
+    Bd = gpu.Tensor.from_numpy(B).to_device()
+    if constant:
+        gpu.lib().omcudaRegisterConstant(Bd.handle)
+    try:
+        for a_zp, b_zp in ((None, None), (np.array(9, np.uint8), None),
+                           (np.array(9, np.uint8), rand8(rng, N, np.int8))):
+            before = gpu.launch_count()
+            got = gpu.matmul_integer(gpu.Tensor.from_numpy(A).to_device(), Bd, a_zp, b_zp, device=True)
+            assert gpu.launch_count() - before > 1
+            assert np.array_equal(got.numpy(), orc.matmul_integer(A, B, a_zp, b_zp))
+    finally:
+        gpu.synchronize()
+        gpu.lib().omcudaForgetConstants()
+
+
 @pytest.mark.parametrize("batch,M,K,N,one", [
     (1, 1, 16384, 64, True), (1, 1, 16400, 64, False), (1, 1, 16400, 68, True),  # whole words
     (1, 17, 2047, 64, True), (1, 17, 2049, 64, False),      # A in single bytes

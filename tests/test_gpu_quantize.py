@@ -161,8 +161,8 @@ def test_one_cluster_sizes(gpu, orc, n):
 @pytest.mark.parametrize("shift", [0, 1])
 def test_pass_run_edges(gpu, orc, n, shift):
     # QuantizeLinear and DequantizeLinear take runs of 4096 values per block: part
-    # of a run, whole runs, several runs per block, and addresses that allow no
-    # vector access.
+    # of a run, one whole run, one for each of many blocks (more than one per block:
+    # test_pass_grid_wraps), and addresses that allow no vector access.
     import torch
     rng = np.random.default_rng(n)
     x = rng.normal(0, 20, size=n).astype(np.float32)
@@ -222,3 +222,50 @@ def test_dequantize_alignments(gpu, orc, dt, xs, ys, n):
         want = orc.dequantize_linear(vals, 0.0123, 5 if zp is not None else 0)
         assert out[ys:ys + n].tobytes() == want.tobytes()
         assert (out[:ys] == -1).all() and (out[ys + n:] == -1).all()
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+def test_pass_grid_wraps(gpu, orc, shift):
+    # More values than one run of 4096 for each of the 64 blocks per SM a pass has at
+    # most: some blocks take a second run, the last one a part of one.
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = sms * 64 * 4096 + 5 * 4096 + 1027
+    rng = np.random.default_rng(36)
+    x = rng.normal(0, 20, size=n).astype(np.float32)
+    xt = torch.zeros(n + 1, device="cuda")
+    xt[shift:shift + n] = torch.from_numpy(x).cuda()
+    L = gpu.lib()
+    xd = gpu.Tensor.from_cuda_array(xt[shift:shift + n])
+    s = gpu.Tensor.from_numpy(np.array(0.37, np.float32))
+
+    def out(dtype):
+        buf = torch.zeros(n + 1, dtype=dtype, device="cuda")
+        return buf, gpu.Tensor.from_cuda_array(buf[shift:shift + n])
+
+    for dt, zp in ((torch.uint8, np.array(131, np.uint8)), (torch.int8, np.array(-3, np.int8))):
+        q, qd = out(dt)
+        z = gpu.Tensor.from_numpy(zp)
+        torch.cuda.synchronize()
+        L.omcudaQuantizeLinear(qd.handle, xd.handle, s.handle, z.handle)
+        gpu.check()
+        torch.cuda.synchronize()
+        want = orc.quantize(x, 0.37, float(zp), dt == torch.int8)
+        assert np.array_equal(q.cpu().numpy()[shift:shift + n], want)
+        y, yd = out(torch.float32)
+        torch.cuda.synchronize()
+        L.omcudaDequantizeLinear(yd.handle, qd.handle, s.handle, z.handle)
+        gpu.check()
+        torch.cuda.synchronize()
+        assert np.array_equal(y.cpu().numpy()[shift:shift + n],
+                              orc.dequantize_linear(want, 0.37, int(zp)))
+    q, qd = out(torch.uint8)
+    ys, yz = torch.zeros((), device="cuda"), torch.zeros((), dtype=torch.uint8, device="cuda")
+    t = [gpu.Tensor.from_cuda_array(a) for a in (ys, yz)]
+    torch.cuda.synchronize()
+    L.omcudaDynamicQuantizeLinear(qd.handle, t[0].handle, t[1].handle, xd.handle)
+    gpu.check()
+    torch.cuda.synchronize()
+    want_y, want_s, want_z = orc.dynamic_quantize_linear(x)
+    assert np.array_equal(q.cpu().numpy()[shift:shift + n], want_y)
+    assert ys.item() == want_s and yz.item() == want_z
