@@ -38,12 +38,12 @@ __host__ __device__
 static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 #ifdef __CUDACC__
-// Whether a kernel that makes this many values is launched with launch_pdl's overlap.  Kernels of
-// a few tens of microseconds gain what their launch takes (linear 128 x 768 x 768 16.9
-// -> 12.3 us, an encoder run of 32 x 128 tokens 2.03 -> 1.97 ms); in long ones
-// the early blocks only hold registers and shared memory of the SMs that
-// finish their predecessor: without this rule an encoder run of 256 x 512 tokens
-// took 119.7 ms instead of 113.2.
+// Whether a kernel that makes this many values is launched with launch_pdl's
+// overlap.  Kernels of a few tens of microseconds gain what their launch takes
+// (linear 128 x 768 x 768 16.9 -> 12.3 us, an encoder run of 32 x 128 tokens 2.03
+// -> 1.97 ms); in long ones the early blocks only hold registers and shared
+// memory of the SMs that finish their predecessor: without this rule an encoder
+// run of 256 x 512 tokens took 119.7 ms instead of 113.2.
 inline bool pdl_pays(int64_t values) { return values <= ((int64_t)16 << 20); }
 
 // Launches a kernel that may be set up while the kernel before it on the stream
@@ -92,10 +92,10 @@ __device__ __forceinline__ void pdl_sync() {
 // __restrict__) may legally be moved across a memory clobber; through the
 // pointer this returns they depend on what follows the wait.  Every pointer
 // that such a kernel reads through passes through here, since any of a caller's
-// tensors may be its predecessor's output.  Not needed for copies issued by volatile asm
-// (TMA, cp.async), nor where a branch that is decided after the wait guards the
-// load: a bounds check on thread and block indices is not one, the wait for an
-// mbarrier that those copies complete is.
+// tensors may be its predecessor's output.  Not needed for copies issued by
+// volatile asm (TMA, cp.async), nor where a branch that is decided after the
+// wait guards the load: a bounds check on thread and block indices is not one,
+// the wait for an mbarrier that those copies complete is.
 template <typename T>
 __device__ __forceinline__ T *after_pdl(T *p) {
   // an offset of zero that the compiler cannot know: the pointer keeps what

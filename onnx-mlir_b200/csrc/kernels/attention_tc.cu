@@ -607,7 +607,8 @@ int launch_attention_tc(const void *hi, const void *lo, int64_t ld_planes,
   const int64_t resident = (int64_t)sm_count() * 2;
   const unsigned grid = (unsigned)(n_items < resident ? n_items : resident);
   OMCUDA_CHECK(launch_pdl(attention_tc_kernel, grid, kTcAttThreads, kTcAttSmem, st, 0,
-      pdl_pays(B * S * heads * kTDh), map_hi, map_lo, map_out, (int32_t)q_col, (int32_t)k_col, (int32_t)v_col, S, heads, n_items, scale_log2e,
+      pdl_pays(B * S * heads * kTDh), map_hi, map_lo, map_out, (int32_t)q_col,
+      (int32_t)k_col, (int32_t)v_col, S, heads, n_items, scale_log2e,
       (uint32_t *)out_range, status, tc_wait_limit_ns()));
   OMCUDA_CHECK_LAUNCH("attention_tc_kernel");
   return OMCUDA_OK;

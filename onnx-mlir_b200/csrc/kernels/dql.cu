@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kDqlThreads)
   // that a launch on a small tensor would otherwise spend before it asks for data.
   // Runs and not a stride of the whole grid, and only four loads in flight per
   // thread so that more blocks fit: 64 Mi values 67.0 -> 64.1 us, an encoder run of
-  // 1 x 61 tokens 741 -> 659 us, of 32 x 128 1903 -> 1839.
+  // 1 x 61 resident tokens 741 -> 659 us, of 32 x 128 1903 -> 1839.
   const bool aligned = (((uintptr_t)x & 15u) == 0) && (((uintptr_t)y & 3u) == 0);
   const int64_t n4 = aligned ? n >> 2 : 0;
   const float4 *x4 = reinterpret_cast<const float4 *>(x);
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(kSmallThreads) dql_small_kernel(SmallDql p) {
 // y = (x - zp) * scale, bound by HBM.  Four values a lane, so that a warp stores
 // whole 512-byte lines (one value a lane: 128 bytes from 32 loads of one byte),
 // and runs of kDequantUnroll * 256 such groups per block:
-// 8191 x 3073 values of 8 bits 31.4 -> 23.9 us (5.4 TB/s), of 32 bits 37.5 -> 35.3.
+// 8191 x 3073 values of 8 bits 31.4 -> 22.7 us (5.5 TB/s), of 32 bits 37.5 -> 35.3.
 constexpr int kDequantUnroll = 4;
 
 // Values i .. i + 3 of x as floats, i a multiple of 4.

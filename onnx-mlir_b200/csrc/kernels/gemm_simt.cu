@@ -592,16 +592,20 @@ static void launch_gemv(const GemmCall &a, cudaStream_t st) {
   int sel = (a.a_signed ? 2 : 0) | (a.B.b_signed ? 1 : 0);
   switch (sel) {
   case 0:
-    (void)launch_pdl(gemm_i8_gemv_kernel<MT, CB, false, false>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
+    (void)launch_pdl(
+        gemm_i8_gemv_kernel<MT, CB, false, false>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   case 1:
-    (void)launch_pdl(gemm_i8_gemv_kernel<MT, CB, false, true>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
+    (void)launch_pdl(
+        gemm_i8_gemv_kernel<MT, CB, false, true>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   case 2:
-    (void)launch_pdl(gemm_i8_gemv_kernel<MT, CB, true, false>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
+    (void)launch_pdl(
+        gemm_i8_gemv_kernel<MT, CB, true, false>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   default:
-    (void)launch_pdl(gemm_i8_gemv_kernel<MT, CB, true, true>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
+    (void)launch_pdl(
+        gemm_i8_gemv_kernel<MT, CB, true, true>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   }
 }
@@ -619,16 +623,20 @@ static void launch_gemv_mma(const GemmCall &a, cudaStream_t st) {
   int sel = (a.a_signed ? 2 : 0) | (a.B.b_signed ? 1 : 0);
   switch (sel) {
   case 0:
-    (void)launch_pdl(gemm_i8_gemv_mma_kernel<CG, false, false>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
+    (void)launch_pdl(
+        gemm_i8_gemv_mma_kernel<CG, false, false>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   case 1:
-    (void)launch_pdl(gemm_i8_gemv_mma_kernel<CG, false, true>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
+    (void)launch_pdl(
+        gemm_i8_gemv_mma_kernel<CG, false, true>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   case 2:
-    (void)launch_pdl(gemm_i8_gemv_mma_kernel<CG, true, false>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
+    (void)launch_pdl(
+        gemm_i8_gemv_mma_kernel<CG, true, false>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   default:
-    (void)launch_pdl(gemm_i8_gemv_mma_kernel<CG, true, true>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
+    (void)launch_pdl(
+        gemm_i8_gemv_mma_kernel<CG, true, true>, grid, threads, 0, st, 0, true, A, Bt, a.B.kp, p);
     break;
   }
 }
@@ -804,14 +812,14 @@ int omcuda::gemm_i8(const GemmCall &a, cudaStream_t st) {
   bool tc_ok = gemm_tc_supported(a);
   if (a.kernel_choice == 1 && !tc_ok)
     return fail(OMCUDA_ENOTSUP,
-        "GemmI8: tensor-core kernel needs K %% 16 == 0 and 16-byte aligned A");
+        "GemmI8: the tensor-core kernel needs 16-byte aligned rows of A");
   const bool tc_only = a.epilogue == OMCUDA_EPI_DEQUANT_SPLIT ||
                        a.epilogue == OMCUDA_EPI_DEQUANT_RANGE ||
                        a.epilogue == OMCUDA_EPI_DEQUANT_QUANT;
   if (tc_only && (!tc_ok || a.kernel_choice == 2))
     return fail(OMCUDA_ENOTSUP,
         "GemmI8: the split-bf16, range-only and quantizing tails exist on the "
-        "tensor-core kernel only (K %% 16 == 0, 16-byte aligned A)");
+        "tensor-core kernel only (16-byte aligned rows of A)");
   // With a handful of rows the GEMM is one read of the weight, which the
   // GEMV-shaped kernels stream faster than 128-row tensor-core tiles on a few
   // SMs (measured: M = 1 19 us against 23-27 us on the 58 MB weights).

@@ -455,9 +455,7 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
   } else {
     // The row pitch of Y is not a multiple of 16 bytes (a ragged N), so no TMA
     // store: a 32 x 32 block passes through the slab and every row leaves as
-    // one coalesced warp-wide store, instead of 32 rows in 32 sectors each
-    // (777 x 1001 x 1537, f32: the whole call 687 -> 27.7 us with padded rows
-    // on these kernels instead of the dp4a one).
+    // one coalesced warp-wide store, instead of 32 rows in 32 sectors each.
 #pragma unroll 1
     for (int c = 0; c < kHalfCols; c += 32) {
       uint32_t v[32];
@@ -1438,8 +1436,8 @@ int launch_pair_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan
   if (rc != OMCUDA_OK)
     return rc;
   OMCUDA_CHECK(launch_pdl(gemm_i8_tc2_kernel<EPI, EW>, (unsigned)(2 * clusters), kThreads,
-      kPairSmemBytes, st, 2, pdl_pays(a.M * a.N), map_a, map_b, map_b_half, map_y, map_y2, p, idesc, idesc_half,
-      full_units, num_units, status, tc_wait_limit_ns()));
+      kPairSmemBytes, st, 2, pdl_pays(a.M * a.N), map_a, map_b, map_b_half, map_y, map_y2,
+      p, idesc, idesc_half, full_units, num_units, status, tc_wait_limit_ns()));
   count_launch();
   return OMCUDA_OK;
 }
