@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kDqlThreads)
     else
       zp_f = (float)*reinterpret_cast<const uint8_t *>(zp8);
   }
-  const QuantConsts qc = make_quant_consts(scale, zp_f, mode);
+  const QuantConsts qc = make_quant_consts<kSigned>(scale, zp_f, mode);
   while (base < n4) {
 #pragma unroll
     for (int u = 0; u < kQuantUnroll; ++u)
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kDqlThreads)
   x = after_pdl(x);
   params = after_pdl(params);
   __shared__ int32_t part[kDqlThreads / 32];
-  const QuantConsts qc = make_quant_consts(__ldg(params), __ldg(params + 1), mode);
+  const QuantConsts qc = make_quant_consts<false>(__ldg(params), __ldg(params + 1), mode);
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
     const float *xr = x + r * cols;
     uint32_t *yr = reinterpret_cast<uint32_t *>(y + r * pitch);
@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(kSmallThreads) dql_small_kernel(SmallDql p) {
     if (p.y_zp)
       *p.y_zp = (uint8_t)(unsigned int)zp_f; // fptoui; zp_f is in [0,255]
   }
-  const QuantConsts qc = make_quant_consts(scale, zp_f, p.mode);
+  const QuantConsts qc = make_quant_consts<false>(scale, zp_f, p.mode);
 #pragma unroll
   for (int u = 0; u < kWords; ++u) {
     const int w = tid + u * nthreads;

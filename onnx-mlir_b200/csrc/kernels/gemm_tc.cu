@@ -314,7 +314,7 @@ __device__ __forceinline__ void split_words_bf16(uint32_t (&v)[32]) {
 template <int EPI>
 __device__ __forceinline__ QuantConsts epi_quant_consts(const EpiParams &p, bool publish) {
   if (EPI != OMCUDA_EPI_DEQUANT_QUANT)
-    return QuantConsts{1.0f, 1.0f, 0.0f, true};
+    return QuantConsts{};
   float scale, zp_f;
   const uint32_t *range = after_pdl(p.q_range);
   dql_params_from_range(ordered_to_f32(__ldg(range)), ordered_to_f32(__ldg(range + 1)),
@@ -327,7 +327,7 @@ __device__ __forceinline__ QuantConsts epi_quant_consts(const EpiParams &p, bool
     if (p.q_zp)
       *p.q_zp = (uint8_t)(unsigned int)zp_f; // fptoui; zp_f is in [0,255]
   }
-  return make_quant_consts(scale, zp_f, p.quant_mode);
+  return make_quant_consts<false>(scale, zp_f, p.quant_mode);
 }
 
 // Drains one accumulator tile half (this warp's 32 TMEM lanes x kHalfCols

@@ -47,10 +47,21 @@ __device__ __forceinline__ uint32_t quantize_one_exact(
 // Per-launch constants of the fast path.
 struct QuantConsts {
   float scale, rcp, zp_f;
+  float x_lo, x_hi; // inputs beyond these saturate
   bool fast;
   bool use_rcp; // fast-math mode: the reference multiplies by RN(1 / scale)
 };
 
+// The smallest and the largest result; integers up to 2^22 on either side of
+// kQuantMagic lie in the low mantissa bits of a float that has it added.
+template <bool kSigned>
+struct QuantBounds {
+  static constexpr float lo = kSigned ? -128.0f : 0.0f;
+  static constexpr float hi = kSigned ? 127.0f : 255.0f;
+};
+constexpr float kQuantMagic = 12582912.0f; // 1.5 * 2^23
+
+template <bool kSigned>
 __device__ __forceinline__ QuantConsts make_quant_consts(
     float scale, float zp_f, int mode = 0) {
   QuantConsts c;
@@ -58,56 +69,43 @@ __device__ __forceinline__ QuantConsts make_quant_consts(
   c.zp_f = (mode & OMCUDA_MODE_NO_ZERO_POINT) ? 0.0f : zp_f;
   c.use_rcp = (mode & OMCUDA_MODE_FAST_MATH) != 0;
   c.rcp = __fdiv_rn(1.0f, scale);
-  // The shortcut needs a normal, finite reciprocal; anything else (scale 0
-  // from an all-zero tensor, denormal or huge scales) takes the exact path.
-  const float as = fabsf(scale);
-  c.fast = (as > 1e-30f) && (as < 1e30f);
+  // A quarter beyond the last integer: a clamped input still rounds to it.
+  c.x_lo = __fmul_rn(QuantBounds<kSigned>::lo - c.zp_f - 0.25f, scale);
+  c.x_hi = __fmul_rn(QuantBounds<kSigned>::hi - c.zp_f + 0.25f, scale);
+  // The shortcut needs a normal, finite reciprocal and residuals that do not
+  // underflow; anything else (scale 0 from an all-zero tensor, negative,
+  // denormal or huge scales) takes the exact path.
+  c.fast = (scale > 1e-30f) && (scale < 1e30f);
   return c;
 }
 
-// Same result as quantize_one_exact with no divide or convert instruction on
-// the common path (those run on the quarter-rate special-function pipe and
-// would bound the kernel instead of HBM):
-//  * t = fma(x, RN(1/scale), 1.5 * 2^23) rounds the product half-even to an
-//    integer held in the mantissa (exact while |product| < 2^22); r = t - 1.5 *
-//    2^23 is that integer and d = fma(x, RN(1/scale), -r) the exact distance
-//    of the product from it.
-//  * x * RN(1/scale) is within 2.5 ulp of the IEEE quotient q = x / scale.
-//    Where |q| <= 512 that is below 2e-4, so unless |d| > 0.499 (the product
-//    lies within 1e-3 of a tie) q rounds to the same integer r; the rare
-//    near-tie element is redone with the exact divide.  Where |q| > 512 the
-//    result saturates whatever the rounding (zero point and bounds lie in
-//    [-128, 255]), and |d| <= 0.499 still holds or the exact path runs.
-//  * the zero point is added and the clip applied while the value still
-//    carries the 1.5 * 2^23 offset (integers below 2^24, or large values that
-//    the clip cuts off either way), and the result is the low byte of the
-//    mantissa (two's complement for the signed type).
-// In fast-math mode the reference's quotient is RN(x * RN(1/scale)), the
-// rounded value of the very product the fma holds exactly: away from a tie it
-// rounds to the same integer, near one the redo uses that product.
-// +-inf saturate through the clip; a NaN product fails the |d| test, passes
-// through fmaxf as the lower clip bound, which is where maxnum/minnum send a
-// NaN in the reference as well.
-template <bool kSigned>
-__device__ __forceinline__ uint32_t quantize_one(float x, const QuantConsts &c) {
-  if (!c.fast)
-    return quantize_one_exact<kSigned>(x, c.scale, c.zp_f, c.use_rcp);
-  const float kMagic = 12582912.0f; // 1.5 * 2^23
-  float t = __fmaf_rn(x, c.rcp, kMagic);
-  const float r = __fsub_rn(t, kMagic);
-  const float d = __fmaf_rn(x, c.rcp, -r);
-  if (fabsf(d) > 0.499f) // near a tie, or too large for the mantissa trick
-    t = __fadd_rn(round_even(c.use_rcp ? __fmul_rn(x, c.rcp) : __fdiv_rn(x, c.scale)),
-        kMagic);
-  const float u = __fadd_rn(t, c.zp_f);
-  const float s = kSigned ? clipf(u, kMagic - 128.0f, kMagic + 127.0f)
-                          : clipf(u, kMagic, kMagic + 255.0f);
-  return __float_as_uint(s) & 0xffu;
+// The quotients x / scale of two values, rounded as the IEEE divide rounds them,
+// by multiplications only (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", 1990): with y = RN(1/scale), one
+// correction q + (x - q scale) y of q = RN(x y) leaves it within an ulp of the
+// quotient, and from such a q the same correction gives RN(x / scale).  The
+// second residual is exact, as that asks: with |q| >= 1/4 (anything smaller
+// rounds to zero whatever its last bits are) and scale > 1e-30 its last bit is
+// at least 2^-149.
+// In fast-math mode the reference's quotient is RN(x y) itself.
+__device__ __forceinline__ uint64_t quotient_x2(uint64_t x, const QuantConsts &c) {
+  const uint64_t y = pack_f32x2(c.rcp, c.rcp), ns = pack_f32x2(-c.scale, -c.scale);
+  uint64_t q = mul_f32x2(x, y);
+  if (!c.use_rcp) {
+    q = fma_f32x2(fma_f32x2(q, ns, x), y, q);
+    q = fma_f32x2(fma_f32x2(q, ns, x), y, q);
+  }
+  return q;
 }
 
-// Four elements by the exact formula, out of line: the fast path below calls
-// it for the rare float4 that holds a near-tie element, and must not carry the
-// divide's instructions as predicated code.
+// Inputs that saturate, cut back to where they still do (a NaN goes to the lower
+// bound, where maxnum/minnum send it in the reference as well).
+__device__ __forceinline__ float quant_clamp(float x, const QuantConsts &c) {
+  return fminf(fmaxf(x, c.x_lo), c.x_hi);
+}
+
+// Four elements by the exact formula, out of line: scales the fast path below
+// does not take.
 template <bool kSigned>
 __device__ __noinline__ uint32_t quantize_four_exact(
     float4 v, float scale, float zp_f, bool use_rcp) {
@@ -117,31 +115,32 @@ __device__ __noinline__ uint32_t quantize_four_exact(
          (quantize_one_exact<kSigned>(v.w, scale, zp_f, use_rcp) << 24);
 }
 
-// quantize_one on the four elements of a float4 with one near-tie test for
-// all of them.
+// Same result as quantize_one_exact on the four elements of a float4, with no
+// divide or convert instruction and no branch per element: the quotient as
+// above, rounded half-even by adding kQuantMagic, the zero point added to that,
+// and the result is the low byte (two's complement for the signed type) of the
+// mantissa.  About six instructions an element.  (An approximate quotient with
+// the exact divide for elements near a tie costs less on paper, but with a test
+// at 0.499 a fifth of the warps had such an element among their 128 and took the
+// divide: 16 Mi values 16.4 us, 7.3 without any arithmetic.)
 template <bool kSigned>
 __device__ __forceinline__ uint32_t quantize_four(float4 v, const QuantConsts &c) {
   if (!c.fast)
     return quantize_four_exact<kSigned>(v, c.scale, c.zp_f, c.use_rcp);
-  const float kMagic = 12582912.0f; // 1.5 * 2^23
-  const float t0 = __fmaf_rn(v.x, c.rcp, kMagic), t1 = __fmaf_rn(v.y, c.rcp, kMagic);
-  const float t2 = __fmaf_rn(v.z, c.rcp, kMagic), t3 = __fmaf_rn(v.w, c.rcp, kMagic);
-  const float d0 = __fmaf_rn(v.x, c.rcp, -__fsub_rn(t0, kMagic));
-  const float d1 = __fmaf_rn(v.y, c.rcp, -__fsub_rn(t1, kMagic));
-  const float d2 = __fmaf_rn(v.z, c.rcp, -__fsub_rn(t2, kMagic));
-  const float d3 = __fmaf_rn(v.w, c.rcp, -__fsub_rn(t3, kMagic));
-  // NaN distances (infinite or NaN inputs) fall through fmaxf and take the
-  // fast path, which saturates them as the exact formula does.
-  const float dmax = fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(d2), fabsf(d3)));
-  if (dmax > 0.499f) // a near tie, or a value too large for the mantissa trick
-    return quantize_four_exact<kSigned>(v, c.scale, c.zp_f, c.use_rcp);
-  const float lo = kSigned ? kMagic - 128.0f : kMagic;
-  const float hi = kSigned ? kMagic + 127.0f : kMagic + 255.0f;
-  const uint32_t b0 = __float_as_uint(clipf(__fadd_rn(t0, c.zp_f), lo, hi)) & 0xffu;
-  const uint32_t b1 = __float_as_uint(clipf(__fadd_rn(t1, c.zp_f), lo, hi)) & 0xffu;
-  const uint32_t b2 = __float_as_uint(clipf(__fadd_rn(t2, c.zp_f), lo, hi)) & 0xffu;
-  const uint32_t b3 = __float_as_uint(clipf(__fadd_rn(t3, c.zp_f), lo, hi));
-  return b0 | (b1 << 8) | (b2 << 16) | (b3 << 24);
+  const uint64_t magic = pack_f32x2(kQuantMagic, kQuantMagic);
+  const uint64_t zp = pack_f32x2(c.zp_f, c.zp_f);
+  const uint64_t q01 = quotient_x2(pack_f32x2(quant_clamp(v.x, c), quant_clamp(v.y, c)), c);
+  const uint64_t q23 = quotient_x2(pack_f32x2(quant_clamp(v.z, c), quant_clamp(v.w, c)), c);
+  const uint64_t t01 = add_f32x2(add_f32x2(q01, magic), zp);
+  const uint64_t t23 = add_f32x2(add_f32x2(q23, magic), zp);
+  const uint32_t b01 = __byte_perm((uint32_t)t01, (uint32_t)(t01 >> 32), 0x0040);
+  const uint32_t b23 = __byte_perm((uint32_t)t23, (uint32_t)(t23 >> 32), 0x0040);
+  return __byte_perm(b01, b23, 0x5410);
+}
+
+template <bool kSigned>
+__device__ __forceinline__ uint32_t quantize_one(float x, const QuantConsts &c) {
+  return quantize_four<kSigned>(make_float4(x, x, x, x), c) & 0xffu;
 }
 
 } // namespace omcuda

@@ -105,6 +105,25 @@ def test_quantize_linear(gpu, orc, signed):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("scale", [2e-31, 1.1e-30, 3.3e-7, 0.1, 1 / 3, 0.99999994, 1.9999999, 255 / 7,
+                                   8e29, 2e30, -0.3])
+@pytest.mark.parametrize("zp,signed", [(0, False), (255, False), (77, False), (-128, True), (5, True)])
+def test_quotients_next_to_ties(gpu, orc, scale, zp, signed):
+    """Values whose quotient by the scale lies on a tie or a few ulps beside it, and
+    values far beyond what saturates, for scales that take the divide-free
+    arithmetic and for such that do not."""
+    s = np.float32(scale)
+    tie = ((np.arange(-300, 300) + 0.5).astype(np.float32) * s).astype(np.float32)
+    near = [(tie.view(np.int32) + d).view(np.float32) for d in range(-3, 4)]
+    far = np.array([0.0, -0.0, 1e-40, -1e-40, 1e38, -1e38, 3e38, -3e38, np.inf, -np.inf, np.nan],
+                   np.float32)
+    x = np.concatenate(near + [far, (np.arange(-300, 300) * s).astype(np.float32)])
+    dt = np.int8 if signed else np.uint8
+    got = gpu.quantize_linear(x, s, np.array(zp, dt), out_dtype=dt)
+    want = orc.quantize(x, s, float(zp), signed)
+    assert np.array_equal(got, want), (x[got != want][:8], got[got != want][:8], want[got != want][:8])
+
+
 @pytest.mark.parametrize("dt", [np.uint8, np.int8, np.int32])
 def test_dequantize_linear(gpu, orc, dt):
     rng = np.random.default_rng(8)
