@@ -249,9 +249,8 @@ void omcudaAttention(OMTensor *y, const OMTensor *q, const OMTensor *k,
 /* Bytes of scratch omcudaDevDynamicQuantizeLinear needs for n elements. */
 int64_t omcudaDevDqlScratchBytes(int64_t n);
 /* DynamicQuantizeLinear on device buffers.  scratch: device memory of at
- * least omcudaDevDqlScratchBytes(n) whose first 64 bytes are zero before the
- * first use (the kernel leaves them zeroed); calls that overlap on the GPU
- * need a scratch block each. */
+ * least omcudaDevDqlScratchBytes(n), whatever it holds; calls that overlap on
+ * the GPU need a scratch block each. */
 int omcudaDevDynamicQuantizeLinear(const float *x, int64_t n, uint8_t *y,
     float *y_scale, uint8_t *y_zp, void *scratch, void *stream);
 /* DynamicQuantizeLinear for callers that cannot allocate device memory (a
@@ -267,10 +266,9 @@ int omcudaDevDynamicQuantizeLinear(const float *x, int64_t n, uint8_t *y,
  *  - The first call on each device looks up the array's device address
  *    (with that device current); make that first call before any stream
  *    capture begins.
- *  - All calls on a device share the one array, which keeps the previous
- *    call's contents; the entry point re-zeroes the part that must start at
- *    zero.  Two calls whose kernels overlap on the GPU (different streams,
- *    no ordering between them) race on it: order them. */
+ *  - All calls on a device share the one array.  Two calls whose kernels
+ *    overlap on the GPU (different streams, no ordering between them) race on
+ *    it: order them. */
 #define OMCUDA_DQL_NOALLOC_MAX_ELEMS ((int64_t)1 << 31)
 int omcudaDevDynamicQuantizeLinearNoAlloc(const float *x, int64_t n, uint8_t *y,
     float *y_scale, uint8_t *y_zp, void *stream);

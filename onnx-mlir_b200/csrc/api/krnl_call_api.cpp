@@ -180,18 +180,10 @@ private:
 // ---- DynamicQuantizeLinear scratch ------------------------------------------------------
 //
 // One block per call (not per stream): two host threads may interleave their
-// launches on the shared library stream, and the reduction leaves the scale
-// and zero point in its scratch for the quantize pass that follows.
+// launches on the shared library stream, and the reduction leaves its partials
+// in its scratch for the quantize pass that follows.
 
-void *dql_scratch_for(Stage &sg, cudaStream_t st) {
-  void *p = sg.scratch((size_t)omcudaDevDqlScratchBytes(0));
-  if (!p)
-    return nullptr;
-  // Only the ticket line has to start at zero.
-  if (check_cuda(cudaMemsetAsync(p, 0, 64, st), "cudaMemsetAsync(dql scratch)") != OMCUDA_OK)
-    return nullptr;
-  return p;
-}
+void *dql_scratch_for(Stage &sg) { return sg.scratch((size_t)omcudaDevDqlScratchBytes(0)); }
 
 // ---- constants: prepared B operands cached by buffer ----------------------------------
 
@@ -560,7 +552,7 @@ void omcudaDynamicQuantizeLinear(
     sg.finish(false);
     return;
   }
-  void *scr = dql_scratch_for(sg, st);
+  void *scr = dql_scratch_for(sg);
   if (!sg.ok() || !scr)
     return;
   sg.set(omcudaDevDynamicQuantizeLinear(dx, n, dy, ds, dz, scr, st));
@@ -900,7 +892,7 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
   uint8_t *xq = (uint8_t *)sg.scratch((size_t)(d.M * g.lda));
   float *xs = (float *)sg.scratch(16);
   const bool small = dql_small_wanted(d.M, g.lda);
-  void *scr = small ? nullptr : dql_scratch_for(sg, st);
+  void *scr = small ? nullptr : dql_scratch_for(sg);
   if (!sg.ok() || (!small && !scr))
     return;
   uint8_t *xz = (uint8_t *)(xs + 1);
@@ -914,16 +906,11 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
   if (small) {
     sg.set(launch_dql_small(
         dX, d.M, d.K, g.lda, xq, (int32_t *)g.a_rowsum, xs, xz, st));
-  } else if (g.lda == d.K) {
+  } else if (g.lda == d.K && !wzn) {
     sg.set(omcudaDevDynamicQuantizeLinear(dX, d.M * d.K, xq, xs, xz, scr, st));
-    if (wzn && sg.ok())
-      sg.set(omcudaDevRowSum(xq, 0, d.M, d.K, (int32_t *)g.a_rowsum, st));
   } else {
-    const float *params = nullptr;
-    sg.set(launch_dql_range(dX, d.M * d.K, scr, xs, xz, &params, st));
-    if (sg.ok())
-      sg.set(launch_quantize_rows(
-          dX, d.M, d.K, g.lda, xq, (int32_t *)g.a_rowsum, params, st));
+    sg.set(launch_dql_rows(
+        dX, d.M, d.K, g.lda, xq, (int32_t *)g.a_rowsum, xs, xz, scr, st));
   }
   g.A = xq;
   g.a_signed = 0;

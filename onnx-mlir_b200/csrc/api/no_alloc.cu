@@ -8,8 +8,7 @@
 // sandboxing layer.  The ordinary entry point
 // omcudaDevDynamicQuantizeLinear makes such a caller bring its own scratch
 // buffer; this variant needs none: its scratch (the per-block partial min/max
-// table, the ticket counter and the two derived scalars of the single-pass
-// grid reduction) lives in a fixed array that is part of the library image.
+// table of the reduction) lives in a fixed array that is part of the library image.
 // Every GPU that loads the library therefore holds kScratchBytes (32 KiB) of
 // device memory for it until the process exits.
 //
@@ -85,12 +84,6 @@ extern "C" int omcudaDevDynamicQuantizeLinearNoAlloc(const float *x, int64_t n,
         (long long)omcudaDevDqlScratchBytes(n), (long long)kScratchBytes);
   void *scratch = nullptr;
   int rc = scratch_for_current_device(&scratch);
-  if (rc != OMCUDA_OK)
-    return rc;
-  // The array still holds whatever the previous call left.  The reduction only
-  // requires its ticket counter (first 64-byte line) to start at zero.
-  rc = omcuda::check_cuda(
-      cudaMemsetAsync(scratch, 0, 64, (cudaStream_t)stream), "cudaMemsetAsync");
   if (rc != OMCUDA_OK)
     return rc;
   return omcudaDevDynamicQuantizeLinear(x, n, y, y_scale, y_zp, scratch, stream);

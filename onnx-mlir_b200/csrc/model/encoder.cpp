@@ -303,10 +303,6 @@ int ensure_workspace(omcudaEncoder *e, int64_t T, cudaStream_t st) {
     e->dql_scratch.ensure((size_t)omcudaDevDqlScratchBytes(0), st);
     if (!e->ranges.p || !e->params.p || !e->dql_scratch.p)
       return OMCUDA_ENOMEM;
-    int rc = check_cuda(cudaMemsetAsync(e->dql_scratch.p, 0, e->dql_scratch.bytes, st),
-        "encoder: scratch");
-    if (rc != OMCUDA_OK)
-      return rc;
   }
   return OMCUDA_OK;
 }

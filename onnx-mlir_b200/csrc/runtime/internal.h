@@ -40,21 +40,15 @@ int quant_mode();
 uint64_t tc_wait_limit_ns();
 
 // dql.cu
-int launch_quantize_with_params(const float *x, int64_t n, uint8_t *y,
-    const float *params, cudaStream_t st);
+//
+// DynamicQuantizeLinear of a [rows, cols] matrix into rows of `pitch` bytes (a
+// multiple of 16, y 16-byte aligned), the tail of a row zero: the form the GEMM
+// kernels take.  rowsum (i32 [rows], sums of a row's bytes) may be null; scratch
+// as for omcudaDevDynamicQuantizeLinear.
+int launch_dql_rows(const float *x, int64_t rows, int64_t cols, int64_t pitch, uint8_t *y,
+    int32_t *rowsum, float *y_scale, uint8_t *y_zp, void *scratch, cudaStream_t st);
 
-// DynamicQuantizeLinear's reduction alone: scale and zero point of x.  *params
-// (in scratch, see omcudaDevDynamicQuantizeLinear) is what the quantize passes take.
-int launch_dql_range(const float *x, int64_t n, void *scratch, float *y_scale,
-    uint8_t *y_zp, const float **params, cudaStream_t st);
-// The quantize pass of a [rows, cols] matrix into rows of
-// `pitch` bytes (a multiple of 16, y 16-byte aligned), the tail of a row zero:
-// the form the GEMM kernels take when cols is no multiple of 16.  rowsum (i32
-// [rows], sums of a row's bytes) may be null.
-int launch_quantize_rows(const float *x, int64_t rows, int64_t cols, int64_t pitch,
-    uint8_t *y, int32_t *rowsum, const float *params, cudaStream_t st);
-
-// Both in one launch, without scratch, for a tensor that one cluster holds in
+// The same in one launch, without scratch, for a tensor that one cluster holds in
 // its registers.  [rows, cols] into rows of `pitch` bytes as above, or one row
 // of pitch == cols of any alignment.
 bool dql_small_wanted(int64_t rows, int64_t pitch);

@@ -288,3 +288,26 @@ def test_pass_grid_wraps(gpu, orc, shift):
     want_y, want_s, want_z = orc.dynamic_quantize_linear(x)
     assert np.array_equal(q.cpu().numpy()[shift:shift + n], want_y)
     assert ys.item() == want_s and yz.item() == want_z
+
+
+@pytest.mark.parametrize("m,k", [(8, 1001), (9, 1001), (591, 1001), (592, 1001), (593, 1024), (591, 1024),
+                                 (40, 8200), (5000, 67), (21, 4099),
+                                 (1, 16381), (4, 4096), (16, 1009)])
+@pytest.mark.parametrize("wt", [np.int8, np.uint8])
+def test_quantized_rows(gpu, orc, m, k, wt):
+    """The quantize pass by rows inside a linear, with (unsigned weights with a zero
+    point) and without the rows' sums: one block's worth, a block and a warp per
+    row and the line between the two, rows that take wide loads and rows that do not."""
+    rng = np.random.default_rng(m * 7 + k)
+    x = rng.normal(0.3, 2, size=(m, k)).astype(np.float32)
+    n = 33
+    w = rng.integers(-127, 128, (k, n)).astype(np.int8) if wt == np.int8 else \
+        rng.integers(0, 256, (k, n)).astype(np.uint8)
+    zp = None if wt == np.int8 else np.array(131, np.uint8)
+    bias = rng.normal(size=n).astype(np.float32)
+    xq, xs, xz = orc.dynamic_quantize_linear(x)
+    wi = w.astype(np.int64) - (0 if zp is None else 131)
+    acc = (xq.astype(np.int64) - int(xz)) @ wi
+    want = (acc.astype(np.float32) * np.float32(np.float32(xs) * np.float32(0.0157))) + bias
+    got = gpu.dyn_quant_linear(x, w, np.float32(0.0157), zp, bias, 0)
+    assert got.tobytes() == want.astype(np.float32).tobytes()
