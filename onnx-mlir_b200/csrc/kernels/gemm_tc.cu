@@ -195,10 +195,10 @@ __device__ __forceinline__ void epilogue_chunk(const EpiParams &p,
     if (p.bias) {
       float b[32];
       load_cols32(p.bias, nc, valid, vec, b);
+      // (single sums: a packed one could be fused with the packed product above)
 #pragma unroll
-      for (int j = 0; j < 32; j += 2)
-        unpack_f32x2(add_f32x2(pack_f32x2(f[j], f[j + 1]), pack_f32x2(b[j], b[j + 1])),
-            f[j], f[j + 1]);
+      for (int j = 0; j < 32; ++j)
+        f[j] = __fadd_rn(f[j], b[j]);
     }
     if (p.gelu) {
 #pragma unroll

@@ -87,15 +87,18 @@ __device__ __forceinline__ QuantConsts make_quant_consts(
 // second residual is exact, as that asks: with |q| >= 1/4 (anything smaller
 // rounds to zero whatever its last bits are) and scale > 1e-30 its last bit is
 // at least 2^-149.
-// In fast-math mode the reference's quotient is RN(x y) itself.
+// In fast-math mode the reference's quotient is RN(x y) itself: two plain products,
+// for the sums that follow would take a packed one in (see mul_f32x2).
 __device__ __forceinline__ uint64_t quotient_x2(uint64_t x, const QuantConsts &c) {
+  if (c.use_rcp) {
+    float x0, x1;
+    unpack_f32x2(x, x0, x1);
+    return pack_f32x2(__fmul_rn(x0, c.rcp), __fmul_rn(x1, c.rcp));
+  }
   const uint64_t y = pack_f32x2(c.rcp, c.rcp), ns = pack_f32x2(-c.scale, -c.scale);
   uint64_t q = mul_f32x2(x, y);
-  if (!c.use_rcp) {
-    q = fma_f32x2(fma_f32x2(q, ns, x), y, q);
-    q = fma_f32x2(fma_f32x2(q, ns, x), y, q);
-  }
-  return q;
+  q = fma_f32x2(fma_f32x2(q, ns, x), y, q);
+  return fma_f32x2(fma_f32x2(q, ns, x), y, q);
 }
 
 // Inputs that saturate, cut back to where they still do (a NaN goes to the lower
