@@ -19,7 +19,7 @@
 //              (M=128, N=BN, K=32 per instruction, four per stage) into one of
 //              two TMEM accumulator buffers and commits to mbarriers to free
 //              the smem stage / publish the accumulator.
-//   warps 2-9  epilogue: tcgen05.ld the accumulator (a warp may read the 32
+//   the others epilogue: tcgen05.ld the accumulator (a warp may read the 32
 //              TMEM lanes its id modulo 4 selects; the two warps of a lane
 //              quadrant split the tile's columns), apply the epilogue, stage
 //              the results in shared memory and store whole 128-byte lines.
@@ -47,20 +47,21 @@ namespace omcuda {
 
 namespace {
 
+// The DEQUANT tail with a residual, as a kernel of its own: its loads take
+// registers that the others would spill.
+constexpr int kEpiDequantResidual = 100;
+__host__ __device__ constexpr bool tail_is_dequant(int epi) {
+  return epi == kEpiDequantResidual || epi_is_dequant(epi);
+}
 constexpr int kBM = 128;       // rows of A per tile
 constexpr int kBK = 128;       // bytes (= int8 elements) of K per stage
 constexpr int kUmmaK = 32;     // K of one tcgen05.mma kind::i8
 // The kernels are built with 8 or 16 epilogue warps (EW).  Sixteen hide the
 // epilogue's latency better, which decides shapes with a short K loop; eight
 // leave shared memory for a deeper operand pipeline, which decides long K.
-// Columns of a tile that one epilogue warp drains: the EW/4 warps that may
-// read a TMEM lane quadrant split the tile's columns, 32 columns at least.
-__host__ __device__ constexpr int epi_cols_per_warp(int bn, int ew) {
-  return bn / (ew / 4) >= 32 ? bn / (ew / 4) : 32;
-}
-__host__ __device__ constexpr int epi_active_warps(int bn, int ew) {
-  return 4 * (bn / epi_cols_per_warp(bn, ew));
-}
+// Columns of a tile that one epilogue warp drains: the EW / 4 warps that may
+// read a TMEM lane quadrant split the tile's columns.
+__host__ __device__ constexpr int epi_cols_per_warp(int bn, int ew) { return bn / (ew / 4); }
 __host__ __device__ constexpr int tc_threads(int ew) { return 32 * (2 + ew); }
 constexpr int kSmemBudget = 232448 - 1024 - 512; // per CTA, minus slack and barriers
 __host__ __device__ constexpr int tc_stages(int stage_bytes, int ew) {
@@ -92,63 +93,126 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a,
                : "memory");
 }
 
+__device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+
 __device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
   return v;
 }
 
+// A load for its effect on L1 alone.
+__device__ __forceinline__ void touch(const void *p) {
+  [[maybe_unused]] uint32_t v;
+  asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(p));
+}
+
+// ---- one tile, one warp ----------------------------------------------------------------
+
+// Where a warp's part of a tile lies: its first row and column, and how many rows
+// further down the slice of a split-K pass is stored.
+struct WarpPlace {
+  int64_t m, n;
+  int32_t store_row;
+};
+
+// Brings what a warp will need for a tile, kCols columns of the per-column vectors,
+// into L1 while the tile before it is worked on: every thread reads all of them, 32
+// per chunk.  Returns the values of the lane's own row, row at.m + lane.
+//
+// What bounds the kernels while K is short is the epilogue: 16384 x 4096 outputs
+// took 74 to 135 us whatever K was, against 8 us of MMAs at K = 128.  Most of that
+// was waiting, per warp and tile: for a release at cluster scope (mbar_arrive_cluster),
+// for the row's values, for 64-bit divisions by run-time tile counts.  Dequantized
+// 74 -> 54 us at K = 128, 92 -> 80 at 1024; to bf16 planes 104 -> 83; with Gelu and
+// range 108 -> 89; requantized with zero points 90 -> 72.  Tried and not taken:
+// a table of the warp's columns in shared memory (cheaper reads, 58 against 72 us for
+// bf16 planes at K = 128, but it takes a stage of the operand ring: 91 against 83 at
+// 1024); slabs of half the size for a sixth stage (gains where there is no
+// arithmetic, loses with Gelu, 100 against 89); accumulators in the shape of MMA
+// fragments, a quarter of the column reads (more moves than it saves: 90, Gelu 115).
+template <int kCols>
+__device__ __forceinline__ EpiRow fetch_ahead(const EpiParams &p, const WarpPlace &at, int lane) {
+#pragma unroll
+  for (int i = 0; i < kCols / 32; ++i) {
+    const int64_t n = at.n + 32 * i + lane;
+    if (n < p.N) {
+      if (p.a_zp_len != 0)
+        touch(p.colsum + n);
+      if (p.sb && p.sb_len != 1)
+        touch(p.sb + n);
+      if (p.bias)
+        touch(p.bias + n);
+    }
+  }
+  EpiRow row = {0, 0};
+  if (at.m + lane < p.M)
+    row = epi_row(p, at.m + lane);
+  return row;
+}
+
 // ---- epilogue arithmetic on one 32-column chunk ---------------------------------------
 
-// Loads 32 consecutive per-column values with 16-byte loads when allowed.
-template <typename T>
-__device__ __forceinline__ void load_cols32(
-    const T *base, int64_t n, int valid, bool vec_ok, T (&out)[32]) {
-  if (vec_ok && valid == 32) {
-    const uint4 *p4 = reinterpret_cast<const uint4 *>(base + n);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      uint4 q = __ldg(p4 + j);
-      out[4 * j + 0] = *reinterpret_cast<T *>(&q.x);
-      out[4 * j + 1] = *reinterpret_cast<T *>(&q.y);
-      out[4 * j + 2] = *reinterpret_cast<T *>(&q.z);
-      out[4 * j + 3] = *reinterpret_cast<T *>(&q.w);
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      out[j] = (j < valid) ? __ldg(base + n + j) : T(0);
-  }
+// Columns 4 j .. 4 j + 3 of a chunk that starts at base.  kWhole: the chunk's 32
+// columns exist and start on 16 bytes; else the last of the `valid` first stands for
+// those behind it (whose results nothing uses): loads without a condition, which the
+// compiler asks for together.
+template <bool kWhole>
+__device__ __forceinline__ float4 col_four(const float *base, int j, int valid) {
+  if (kWhole)
+    return __ldg(reinterpret_cast<const float4 *>(base) + j);
+  const int last = valid - 1;
+  return make_float4(__ldg(base + min(4 * j, last)), __ldg(base + min(4 * j + 1, last)),
+      __ldg(base + min(4 * j + 2, last)), __ldg(base + min(4 * j + 3, last)));
+}
+template <bool kWhole>
+__device__ __forceinline__ int4 col_four(const int32_t *base, int j, int valid) {
+  if (kWhole)
+    return __ldg(reinterpret_cast<const int4 *>(base) + j);
+  const int last = valid - 1;
+  return make_int4(__ldg(base + min(4 * j, last)), __ldg(base + min(4 * j + 1, last)),
+      __ldg(base + min(4 * j + 2, last)), __ldg(base + min(4 * j + 3, last)));
 }
 
 // Turns 32 raw accumulators of one row into 32 output words (EPI_I32: the
-// corrected i32; EPI_DEQUANT, EPI_DEQUANT_SPLIT and EPI_DEQUANT_RANGE: f32
-// bits; EPI_REQUANT: one byte per word; EPI_DEQUANT_QUANT: words 0..7 hold
-// the 32 output bytes, four to a word).
-template <int EPI>
+// corrected i32; the f32 tails, EPI_DEQUANT_SPLIT and EPI_DEQUANT_RANGE: f32
+// bits; EPI_REQUANT and EPI_DEQUANT_QUANT: words 0..7 hold the 32 output bytes,
+// four to a word).  nc: the chunk's first column, of which `valid` exist.  The
+// range (lo, hi) of the f32 tails is left to the caller where a residual follows.
+template <int EPI, bool kWhole>
 __device__ __forceinline__ void epilogue_chunk(const EpiParams &p,
-    const EpiScalars &sc, const QuantConsts &qc, const EpiRow &row,
-    const float *res_row, int64_t nc, int valid, uint32_t (&v)[32], float &lo,
-    float &hi) {
-  const bool vec = p.vec_ok != 0;
+    const EpiScalars &sc, const QuantConsts &qc, const EpiRow &row, int64_t nc, int valid,
+    uint32_t (&v)[32], float &lo, float &hi) {
   if (p.b_zp_len != 0) {
     // - bz[n] * rowsum[m] + K * az * bz[n]  =  bz[n] * (K * az - rowsum[m])
     const uint32_t tr = (uint32_t)p.K * (uint32_t)row.az - (uint32_t)row.rs;
     if (p.b_zp_len == 1) {
       const uint32_t bz = (uint32_t)load_zp8(p.b_zp, 0, p.b_signed);
+      if (bz != 0) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        v[j] += bz * tr;
-    } else if (vec && valid == 32 && (((uintptr_t)p.b_zp + (uintptr_t)nc) & 15u) == 0) {
+        for (int j = 0; j < 32; ++j)
+          v[j] += bz * tr;
+      }
+    } else if (kWhole && (((uintptr_t)p.b_zp + (uintptr_t)nc) & 15u) == 0) {
+      // Weights are mostly symmetric: 32 zero points that are all zero cost a look.
       const uint4 *src = reinterpret_cast<const uint4 *>(
           reinterpret_cast<const uint8_t *>(p.b_zp) + nc);
       const uint4 q0 = __ldg(src), q1 = __ldg(src + 1);
       const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+      if ((w[0] | w[1] | w[2] | w[3] | w[4] | w[5] | w[6] | w[7]) != 0) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const uint32_t byte = (w[j >> 2] >> (8 * (j & 3))) & 0xffu;
-        const uint32_t bz = p.b_signed ? (uint32_t)(int32_t)(int8_t)byte : byte;
-        v[j] += bz * tr;
+        for (int j = 0; j < 32; ++j) {
+          const uint32_t byte = (w[j >> 2] >> (8 * (j & 3))) & 0xffu;
+          const uint32_t bz = p.b_signed ? (uint32_t)(int32_t)(int8_t)byte : byte;
+          v[j] += bz * tr;
+        }
       }
     } else {
 #pragma unroll
@@ -158,62 +222,67 @@ __device__ __forceinline__ void epilogue_chunk(const EpiParams &p,
     }
   }
   if (p.a_zp_len != 0) {
-    int32_t cs[32];
-    load_cols32(p.colsum, nc, valid, vec, cs);
+    const uint32_t naz = 0u - (uint32_t)row.az;
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-      v[j] -= (uint32_t)row.az * (uint32_t)cs[j];
+    for (int j = 0; j < 32; j += 4) {
+      const int4 q = col_four<kWhole>(p.colsum + nc, j >> 2, valid);
+      v[j] += naz * (uint32_t)q.x;
+      v[j + 1] += naz * (uint32_t)q.y;
+      v[j + 2] += naz * (uint32_t)q.z;
+      v[j + 3] += naz * (uint32_t)q.w;
+    }
   }
   if (EPI == OMCUDA_EPI_I32)
     return;
-  if (epi_is_dequant(EPI)) {
+  if (tail_is_dequant(EPI)) {
+    // (packed products: two exactly rounded ones per instruction)
     float f[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j)
       f[j] = __int2float_rn((int32_t)v[j]);
+    const uint64_t sa2 = pack_f32x2(sc.sa, sc.sa);
+    if (p.form != 0) {
+#pragma unroll
+      for (int j = 0; j < 32; j += 2)
+        unpack_f32x2(mul_f32x2(pack_f32x2(f[j], f[j + 1]), sa2), f[j], f[j + 1]);
+    }
     if (p.sb_len == 1) {
-      if (p.form == 0) {
-        // (packed fp32: two exactly rounded products per instruction)
-        const uint64_t s2 = pack_f32x2(sc.s0, sc.s0);
+      const float s = p.form == 0 ? sc.s0 : __ldg(p.sb);
+      const uint64_t s2 = pack_f32x2(s, s);
 #pragma unroll
-        for (int j = 0; j < 32; j += 2)
-          unpack_f32x2(mul_f32x2(pack_f32x2(f[j], f[j + 1]), s2), f[j], f[j + 1]);
-      } else {
-        const float sb = __ldg(p.sb);
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          f[j] = __fmul_rn(__fmul_rn(f[j], sc.sa), sb);
-      }
+      for (int j = 0; j < 32; j += 2)
+        unpack_f32x2(mul_f32x2(pack_f32x2(f[j], f[j + 1]), s2), f[j], f[j + 1]);
     } else {
-      float sb[32];
-      load_cols32(p.sb, nc, valid, vec, sb);
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        f[j] = (p.form == 0) ? __fmul_rn(f[j], __fmul_rn(sc.sa, sb[j]))
-                             : __fmul_rn(__fmul_rn(f[j], sc.sa), sb[j]);
+      for (int j = 0; j < 32; j += 4) {
+        const float4 q = col_four<kWhole>(p.sb + nc, j >> 2, valid);
+        uint64_t s01 = pack_f32x2(q.x, q.y), s23 = pack_f32x2(q.z, q.w);
+        if (p.form == 0) { // onnx.Mul of the two scales
+          s01 = mul_f32x2(s01, sa2);
+          s23 = mul_f32x2(s23, sa2);
+        }
+        unpack_f32x2(mul_f32x2(pack_f32x2(f[j], f[j + 1]), s01), f[j], f[j + 1]);
+        unpack_f32x2(mul_f32x2(pack_f32x2(f[j + 2], f[j + 3]), s23), f[j + 2], f[j + 3]);
+      }
     }
     if (p.bias) {
-      float b[32];
-      load_cols32(p.bias, nc, valid, vec, b);
       // (single sums: a packed one could be fused with the packed product above)
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        f[j] = __fadd_rn(f[j], b[j]);
+      for (int j = 0; j < 32; j += 4) {
+        const float4 q = col_four<kWhole>(p.bias + nc, j >> 2, valid);
+        f[j] = __fadd_rn(f[j], q.x);
+        f[j + 1] = __fadd_rn(f[j + 1], q.y);
+        f[j + 2] = __fadd_rn(f[j + 2], q.z);
+        f[j + 3] = __fadd_rn(f[j + 3], q.w);
+      }
     }
     if (p.gelu) {
 #pragma unroll
       for (int j = 0; j < 32; j += 2)
         gelu_erf_x2(f[j], f[j + 1]);
     }
-    if (EPI == OMCUDA_EPI_DEQUANT && res_row) {
-      float r[32];
-      load_cols32(res_row, nc, valid, p.res_vec_ok != 0, r);
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        f[j] = __fadd_rn(f[j], r[j]);
-    }
-    if (p.out_range) {
-      if (valid == 32) {
+    if (p.out_range && EPI != kEpiDequantResidual) {
+      if (kWhole || valid == 32) {
         // three-input min / max: one instruction per two values
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
@@ -243,38 +312,47 @@ __device__ __forceinline__ void epilogue_chunk(const EpiParams &p,
     return;
   }
   // EPI_REQUANT
-  float S[32];
-  if (p.sb_len == 1) {
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      S[j] = sc.s0;
-  } else {
-    load_cols32(p.sb, nc, valid, vec, S);
-  }
   // round_even, fptosi and the truncation to 8 bits in one addition: x + 1.5 * 2^23
   // holds rint(x), two's complement, in its low mantissa bits while |x| < 2^22.
-  // Rounding and conversion run at a quarter of the ALU's rate, as the int to
-  // float conversion before them does: three of those per output are 6144 clocks
-  // for a 128 x 256 tile, more than its MMAs at K = 1024.  16384 x 1024 x
-  // 4096: 104.7 -> 99.2 us.
+  // Rounding and conversion run at a quarter of the ALU's rate.  The zero point is
+  // added to four packed bytes at once, without carries between them.
+  float x[32];
   float top = 0.0f; // largest |x|; a NaN stays
 #pragma unroll
-  for (int j = 0; j < 32; j += 2) {
+  for (int j = 0; j < 32; j += 4) {
+    const float4 q = p.sb_len == 1 ? make_float4(sc.s0, sc.s0, sc.s0, sc.s0)
+                                   : col_four<kWhole>(p.sb + nc, j >> 2, valid);
     unpack_f32x2(mul_f32x2(pack_f32x2(__int2float_rn((int32_t)v[j]),
                                __int2float_rn((int32_t)v[j + 1])),
-                     pack_f32x2(S[j], S[j + 1])),
-        S[j], S[j + 1]);
-    asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(S[j])));
-    asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(S[j + 1])));
+                     pack_f32x2(q.x, q.y)),
+        x[j], x[j + 1]);
+    unpack_f32x2(mul_f32x2(pack_f32x2(__int2float_rn((int32_t)v[j + 2]),
+                               __int2float_rn((int32_t)v[j + 3])),
+                     pack_f32x2(q.z, q.w)),
+        x[j + 2], x[j + 3]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(x[j + e])));
   }
   if (top < 4194304.0f) {
+    const uint32_t yz4 = (sc.yz & 0xffu) * 0x01010101u;
+    // (single sums, see mul_f32x2)
+    const auto low = [&](int j) { return __float_as_uint(__fadd_rn(x[j], 12582912.0f)); };
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-      v[j] = (__float_as_uint(__fadd_rn(S[j], 12582912.0f)) + sc.yz) & 0xffu;
+    for (int j = 0; j < 32; j += 4) {
+      const uint32_t w = __byte_perm(__byte_perm(low(j), low(j + 1), 0x0040),
+          __byte_perm(low(j + 2), low(j + 3), 0x0040), 0x5410);
+      v[j >> 2] = ((w & 0x7f7f7f7fu) + (yz4 & 0x7f7f7f7fu)) ^ ((w ^ yz4) & 0x80808080u);
+    }
   } else {
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-      v[j] = ((uint32_t)__float2int_rz(round_even(S[j])) + sc.yz) & 0xffu;
+    for (int j = 0; j < 32; j += 4) {
+      uint32_t w = 0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        w |= (((uint32_t)__float2int_rz(round_even(x[j + e])) + sc.yz) & 0xffu) << (8 * e);
+      v[j >> 2] = w;
+    }
   }
 }
 
@@ -330,22 +408,38 @@ __device__ __forceinline__ QuantConsts epi_quant_consts(const EpiParams &p, bool
   return make_quant_consts<false>(scale, zp_f, p.quant_mode);
 }
 
-// Drains one accumulator tile half (this warp's 32 TMEM lanes x kHalfCols
-// columns starting at taddr) through the epilogue into Y.
-//   m_warp   first output row of this warp's 32 rows
-//   n0       first output column of this warp's column range
+// Asks for row m of a warp's block of the residual (kCols columns from n0 on) in
+// L2 while the MMAs of the tile are still running.
+template <int kCols>
+__device__ __forceinline__ void prefetch_residual(const EpiParams &p, int64_t m, int64_t n0) {
+  if (m >= p.M)
+    return;
+  const float *rr = p.residual + m * p.N + n0;
+  for (int c = 0; c < kCols && n0 + c < p.N; c += 32)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(rr + c));
+}
+
+// Drains this warp's share of one accumulator tile (its 32 TMEM lanes x kHalfCols
+// columns starting at taddr) through the epilogue into Y, 32 or (with eight warps,
+// which have the registers) 64 columns at a time.
+//   at       this warp's 32 rows and first column
+//   row      this thread's row's values
 //   slab0    this warp's 4 KiB staging slab in shared memory
 //   release  called once, right after the last tensor-memory load of the
 //            tile: the accumulator buffer is handed back to the MMA issuer
-//            before the arithmetic and the stores of the last chunk, which
+//            before the arithmetic and the stores of the last columns, which
 //            keeps those off the path that decides when the next tile's MMAs
 //            may start
+//
+// A residual is added to the values where they lie in the slab, by lanes that
+// stand on neighbouring columns: whole 128-byte lines of it per load.  (One row per
+// thread, as the accumulator comes, touched 32 lines per load.)
 template <int BN, int EPI, int EW, typename Release>
 __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
-    const EpiScalars &sc, const QuantConsts &qc, uint32_t taddr, int64_t m_warp,
-    int64_t n0, uint32_t slab0, int lane, bool use_slab, float &lo, float &hi,
-    const CUtensorMap *map_y, const CUtensorMap *map_y2, Release &&release,
-    int32_t store_row_off = 0) {
+    const EpiScalars &sc, const QuantConsts &qc, uint32_t taddr, const WarpPlace &at,
+    const EpiRow &row, uint32_t slab0, int lane, bool use_slab, float &lo, float &hi,
+    const CUtensorMap *map_y, const CUtensorMap *map_y2, Release &&release) {
+  const int64_t m_warp = at.m, n0 = at.n;
   const bool hint_store = (p.l2_hints & 1) != 0;
   const uint64_t pol_out = hint_store ? l2_policy_evict_first() : 0;
   // EPI_DEQUANT_SPLIT stages like the 4-byte tails (32 columns per 128-byte
@@ -353,59 +447,102 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
   constexpr bool kSplit = EPI == OMCUDA_EPI_DEQUANT_SPLIT;
   // EPI_DEQUANT_RANGE walks the tile like the f32 tail and stores nothing.
   constexpr bool kNoStore = EPI == OMCUDA_EPI_DEQUANT_RANGE;
-  constexpr bool kPacked = EPI == OMCUDA_EPI_DEQUANT_QUANT; // bytes arrive four to a word
-  constexpr int kOutBytes =
-      (EPI == OMCUDA_EPI_REQUANT || EPI == OMCUDA_EPI_DEQUANT_QUANT) ? 1 : 4;
+  constexpr bool kBytesOut = EPI == OMCUDA_EPI_REQUANT || EPI == OMCUDA_EPI_DEQUANT_QUANT;
+  constexpr bool kRes = EPI == kEpiDequantResidual;
+  constexpr int kOutBytes = kBytesOut ? 1 : 4;
   constexpr int kHalfCols = epi_cols_per_warp(BN, EW);
   constexpr int kSlabCols =
       (128 / kOutBytes) < kHalfCols ? (128 / kOutBytes) : kHalfCols;
-  constexpr int kSlabsPerHalf = kHalfCols / kSlabCols;
-  static_assert(kHalfCols % 32 == 0 && kHalfCols % kSlabCols == 0, "tile shape");
+  constexpr int kStep = EW > 8 || kHalfCols < 64 ? 32 : 64; // columns read at a time
+  static_assert(kHalfCols % kStep == 0 && kHalfCols % kSlabCols == 0, "tile shape");
+  // Results pass through a shared-memory slab (32 rows per warp, rows of
+  // kRowB bytes in the swizzle pattern of that width) and leave with one TMA
+  // store per slab, which writes whole lines and clips rows and columns
+  // beyond the matrix.  EPI_DEQUANT_SPLIT uses the two halves of the slab
+  // for the hi and the lo plane.
+  constexpr int kRowB = kSplit ? 64 : kSlabCols * kOutBytes;
+  static_assert(kRowB == 32 || kRowB == 64 || kRowB == 128,
+      "slab rows span one swizzle width");
+  // 16-byte piece index XOR address bits 7.. (3, 2 or 1 bits for the 128-,
+  // 64- and 32-byte swizzle), as the store's tensor map expects.
+  constexpr uint32_t kSwzMask = (uint32_t)kRowB / 16u - 1u;
+  const uint32_t row_off = (uint32_t)lane * kRowB;
+  const uint32_t swz = ((row_off >> 7) & kSwzMask) << 4;
+  const uint32_t my_row = slab0 + row_off;
   const int64_t m = m_warp + lane;
-  const bool row_ok = m < p.M;
-  EpiRow row;
-  row.az = 0;
-  row.rs = 0;
-  if (row_ok)
-    row = epi_row(p, m);
-  const float *res_row = (row_ok && p.residual) ? p.residual + m * p.N : nullptr;
-  if (use_slab) {
-    // Results pass through a shared-memory slab (32 rows per warp, rows of
-    // kRowB bytes in the 128-byte-swizzle pattern) and leave with one TMA
-    // store per slab, which writes whole lines and clips rows and columns
-    // beyond the matrix.  EPI_DEQUANT_SPLIT uses the two halves of the slab
-    // for the hi and the lo plane.
-    constexpr int kRowB = kSplit ? 64 : kSlabCols * kOutBytes;
-    static_assert(kRowB == 32 || kRowB == 64 || kRowB == 128,
-        "slab rows span one swizzle width");
-    // 16-byte piece index XOR address bits 7.. (3, 2 or 1 bits for the 128-,
-    // 64- and 32-byte swizzle), as the store's tensor map expects.
-    constexpr uint32_t kSwzMask = (uint32_t)kRowB / 16u - 1u;
-    const uint32_t row_off = (uint32_t)lane * kRowB;
-    // The XOR term of this thread's row (pieces of a row stay inside it).
-    const uint32_t swz = ((row_off >> 7) & kSwzMask) << 4;
-    const uint32_t my_row = slab0 + row_off;
-    const bool warp_in = m_warp < p.M;
+  const int rows = (int)(p.M - m_warp < 32 ? p.M - m_warp : 32); // (may be negative)
 #pragma unroll 1
-    for (int g = 0; g < kSlabsPerHalf; ++g) {
-      const int64_t ng = n0 + (int64_t)g * kSlabCols;
-#pragma unroll 1
-      for (int cc = 0; cc < kSlabCols; cc += 32) {
-        uint32_t v[32];
-        __syncwarp(); // tcgen05.ld is warp-collective: enter it converged
-        tmem_ld32(taddr + (uint32_t)(g * kSlabCols + cc), v);
-        tmem_ld_wait();
-        if (g == kSlabsPerHalf - 1 && cc + 32 >= kSlabCols)
-          release();
-        const int64_t nc = ng + cc;
-        const int valid = (int)((p.N - nc) < 32 ? (p.N - nc) : 32);
-        if (row_ok && valid > 0)
-          epilogue_chunk<EPI>(p, sc, qc, row, res_row, nc, valid, v, lo, hi);
-        if (kNoStore)
-          continue;
-        if (kSplit)
-          split_words_bf16(v);
-        if (cc == 0) {
+  for (int g = 0; g < kHalfCols; g += kStep) {
+    // A residual: lane l stands on columns 4 (l % 8) .. + 3 of rows l / 8 + 4 i of a
+    // 32 x 32 block.  Half of it (i < 4) is asked for before the accumulator is read,
+    // the rest once that has left the registers.
+    float4 res[4];
+    const auto load_res = [&](int c, int i0) {
+      const int64_t n = n0 + c + 4 * (lane & 7);
+      const float *src = p.residual + (m_warp + (lane >> 3) + 4 * i0) * p.N + n;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        res[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if ((lane >> 3) + 4 * (i0 + i) < rows && n < p.N) {
+          if (p.res_vec_ok)
+            res[i] = __ldg(reinterpret_cast<const float4 *>(src));
+          else // (a slab's columns come in fours: N is a multiple of 4)
+            res[i] = make_float4(__ldg(src), __ldg(src + 1), __ldg(src + 2), __ldg(src + 3));
+        }
+        src += 4 * p.N;
+      }
+    };
+    const auto add_res = [&](int c, int i0) {
+      const bool col_in = n0 + c + 4 * (lane & 7) < p.N;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t r = 4 * (i0 + i) + (lane >> 3);
+        const uint32_t word = slab0 + r * 128u + ((((uint32_t)lane & 7u) ^ (r & 7u)) << 4);
+        float4 f = ld_shared_f4(word);
+        f.x = __fadd_rn(f.x, res[i].x);
+        f.y = __fadd_rn(f.y, res[i].y);
+        f.z = __fadd_rn(f.z, res[i].z);
+        f.w = __fadd_rn(f.w, res[i].w);
+        if (p.out_range && col_in && (int)r < rows) {
+          lo = min3f(min3f(lo, f.x, f.y), f.z, f.w);
+          hi = max3f(max3f(hi, f.x, f.y), f.z, f.w);
+        }
+        st_shared_v4(word, __float_as_uint(f.x), __float_as_uint(f.y), __float_as_uint(f.z),
+            __float_as_uint(f.w));
+      }
+    };
+    if (kRes && use_slab)
+      load_res(g, 0);
+    uint32_t v[kStep / 32][32];
+    __syncwarp(); // tcgen05.ld is warp-collective: enter it converged
+#pragma unroll
+    for (int h = 0; h < kStep / 32; ++h)
+      tmem_ld32(taddr + (uint32_t)(g + 32 * h), v[h]);
+    tmem_ld_wait();
+    if (g + kStep >= kHalfCols)
+      release();
+#pragma unroll
+    for (int h = 0; h < kStep / 32; ++h) {
+      const int c = g + 32 * h;
+      const int64_t nc = n0 + c;
+      const int valid = (int)((p.N - nc) < 32 ? (p.N - nc) : 32);
+      if (valid <= 0)
+        break; // (uniform; what a slab holds by then has been stored)
+      float l = lo, u = hi;
+      if (p.vec_ok != 0 && valid == 32)
+        epilogue_chunk<EPI, true>(p, sc, qc, row, nc, valid, v[h], l, u);
+      else
+        epilogue_chunk<EPI, false>(p, sc, qc, row, nc, valid, v[h], l, u);
+      if (lane < rows) {
+        lo = l;
+        hi = u;
+      }
+      if (kNoStore)
+        continue;
+      if (kSplit)
+        split_words_bf16(v[h]);
+      if (use_slab) {
+        if (c % kSlabCols == 0) {
           // The previous store must have read the slab before it is rewritten.
           if (lane == 0)
             tma_store_wait_read();
@@ -415,100 +552,87 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const uint32_t so = my_row + (((uint32_t)j * 16u) ^ swz);
-            st_shared_v4(so, v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-            st_shared_v4(so + 2048u, v[16 + 4 * j], v[17 + 4 * j], v[18 + 4 * j],
-                v[19 + 4 * j]);
+            st_shared_v4(so, v[h][4 * j], v[h][4 * j + 1], v[h][4 * j + 2], v[h][4 * j + 3]);
+            st_shared_v4(so + 2048u, v[h][16 + 4 * j], v[h][17 + 4 * j], v[h][18 + 4 * j],
+                v[h][19 + 4 * j]);
           }
-        } else if (kOutBytes == 4) {
+        } else if (!kBytesOut) {
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            st_shared_v4(my_row + (((uint32_t)j * 16u) ^ swz), v[4 * j], v[4 * j + 1],
-                v[4 * j + 2], v[4 * j + 3]);
+            st_shared_v4(my_row + (((uint32_t)j * 16u) ^ swz), v[h][4 * j], v[h][4 * j + 1],
+                v[h][4 * j + 2], v[h][4 * j + 3]);
+          if (kRes) {
+            __syncwarp();
+            add_res(c, 0);
+            load_res(c, 4);
+            add_res(c, 4);
+            if (h + 1 < kStep / 32)
+              load_res(c + 32, 0);
+          }
         } else {
-          uint32_t w[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            w[j] = kPacked ? v[j]
-                           : (v[4 * j] | (v[4 * j + 1] << 8) | (v[4 * j + 2] << 16) |
-                                 (v[4 * j + 3] << 24));
-          st_shared_v4(my_row + ((uint32_t)cc ^ swz), w[0], w[1], w[2], w[3]);
-          st_shared_v4(my_row + (((uint32_t)cc + 16u) ^ swz), w[4], w[5], w[6], w[7]);
+          const uint32_t cc = (uint32_t)(c % kSlabCols);
+          st_shared_v4(my_row + (cc ^ swz), v[h][0], v[h][1], v[h][2], v[h][3]);
+          st_shared_v4(my_row + ((cc + 16u) ^ swz), v[h][4], v[h][5], v[h][6], v[h][7]);
         }
-      }
-      if (kNoStore)
-        continue;
-      fence_proxy_async_smem(); // the slab was written through the generic proxy
-      __syncwarp();
-      if (lane == 0 && warp_in && ng < p.N) {
-        if (hint_store) {
-          tma_store_2d_hint(map_y, slab0, (int32_t)ng, (int32_t)m_warp + store_row_off, pol_out);
-          if (kSplit)
-            tma_store_2d_hint(map_y2, slab0 + 2048u, (int32_t)ng, (int32_t)m_warp, pol_out);
-        } else {
-          tma_store_2d(map_y, slab0, (int32_t)ng, (int32_t)m_warp + store_row_off);
-          if (kSplit)
-            tma_store_2d(map_y2, slab0 + 2048u, (int32_t)ng, (int32_t)m_warp);
+        if ((c + 32) % kSlabCols != 0 && nc + 32 < p.N)
+          continue; // the slab takes more columns
+        fence_proxy_async_smem(); // the slab was written through the generic proxy
+        __syncwarp();
+        if (lane == 0 && rows > 0) {
+          const int32_t x = (int32_t)(n0 + c - c % kSlabCols);
+          if (hint_store) {
+            tma_store_2d_hint(map_y, slab0, x, (int32_t)m_warp + at.store_row, pol_out);
+            if (kSplit)
+              tma_store_2d_hint(map_y2, slab0 + 2048u, x, (int32_t)m_warp, pol_out);
+          } else {
+            tma_store_2d(map_y, slab0, x, (int32_t)m_warp + at.store_row);
+            if (kSplit)
+              tma_store_2d(map_y2, slab0 + 2048u, x, (int32_t)m_warp);
+          }
+          tma_store_commit();
         }
-        tma_store_commit();
+        continue;
       }
-    }
-  } else {
-    // The row pitch of Y is not a multiple of 16 bytes (a ragged N), so no TMA
-    // store: a 32 x 32 block passes through the slab and every row leaves as
-    // one coalesced warp-wide store, instead of 32 rows in 32 sectors each.
-#pragma unroll 1
-    for (int c = 0; c < kHalfCols; c += 32) {
-      uint32_t v[32];
-      __syncwarp();
-      tmem_ld32(taddr + (uint32_t)c, v);
-      tmem_ld_wait();
-      if (c + 32 >= kHalfCols)
-        release();
-      const int64_t nc = n0 + c;
-      const int valid = (int)((p.N - nc) < 32 ? (p.N - nc) : 32);
-      if (valid <= 0)
-        continue;
-      if (row_ok)
-        epilogue_chunk<EPI>(p, sc, qc, row, res_row, nc, valid, v, lo, hi);
-      if (kNoStore)
-        continue;
+      // The row pitch of Y is not a multiple of 16 bytes (a ragged N), so no TMA
+      // store: a 32 x 32 block passes through the slab and every row leaves as
+      // one coalesced warp-wide store, instead of 32 rows in 32 sectors each.
       if (kSplit) {
-        if (!row_ok)
+        if (lane >= rows)
           continue;
-        split_words_bf16(v);
         uint16_t *dhi = reinterpret_cast<uint16_t *>(p.Y) + m * p.N + nc;
         uint16_t *dlo = dhi + p.M * p.N;
 #pragma unroll
         for (int j = 0; j < 32; ++j)
           if (j < valid) {
-            dhi[j] = (uint16_t)(v[j >> 1] >> (16 * (j & 1)));
-            dlo[j] = (uint16_t)(v[16 + (j >> 1)] >> (16 * (j & 1)));
+            dhi[j] = (uint16_t)(v[h][j >> 1] >> (16 * (j & 1)));
+            dlo[j] = (uint16_t)(v[h][16 + (j >> 1)] >> (16 * (j & 1)));
           }
         continue;
       }
       // slab word (r, j) sits at piece (j / 4) ^ (r % 8) of row r
-      const int rows = (int)(p.M - m_warp < 32 ? p.M - m_warp : 32);
+      __syncwarp(); // the block before has been read
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (!kPacked)
-          st_shared_v4(slab0 + (uint32_t)lane * 128u + (uint32_t)((j ^ (lane & 7)) * 16),
-              v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-        else if (j < 2)
-          st_shared_v4(slab0 + (uint32_t)lane * 128u + (uint32_t)((j ^ (lane & 7)) * 16),
-              v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      for (int j = 0; j < (kBytesOut ? 2 : 8); ++j)
+        st_shared_v4(slab0 + (uint32_t)lane * 128u + (uint32_t)((j ^ (lane & 7)) * 16),
+            v[h][4 * j], v[h][4 * j + 1], v[h][4 * j + 2], v[h][4 * j + 3]);
       __syncwarp();
-      const int piece = kPacked ? lane >> 4 : lane >> 2;
-      const uint32_t in_piece = kPacked ? (uint32_t)(lane & 15) & ~3u : (uint32_t)(lane & 3) * 4u;
+      const int piece = kBytesOut ? lane >> 4 : lane >> 2;
+      const uint32_t in_piece = kBytesOut ? (uint32_t)(lane & 15) & ~3u : (uint32_t)(lane & 3) * 4u;
       for (int r = 0; r < rows; ++r) {
         const uint32_t w = ld_shared_u32(
             slab0 + (uint32_t)r * 128u + (uint32_t)((piece ^ (r & 7)) * 16) + in_piece);
         if (lane < valid) {
-          const int64_t at = (m_warp + r) * p.N + nc + lane;
-          if (kOutBytes == 4)
-            reinterpret_cast<uint32_t *>(p.Y)[at] = w;
-          else
-            reinterpret_cast<uint8_t *>(p.Y)[at] =
-                (uint8_t)(kPacked ? w >> (8 * (lane & 3)) : w);
+          const int64_t y_at = (m_warp + r) * p.N + nc + lane;
+          if (kRes) {
+            const float f = __fadd_rn(__uint_as_float(w), __ldg(p.residual + y_at));
+            lo = fminf(lo, f);
+            hi = fmaxf(hi, f);
+            reinterpret_cast<float *>(p.Y)[y_at] = f;
+          } else if (!kBytesOut) {
+            reinterpret_cast<uint32_t *>(p.Y)[y_at] = w;
+          } else {
+            reinterpret_cast<uint8_t *>(p.Y)[y_at] = (uint8_t)(w >> (8 * (lane & 3)));
+          }
         }
       }
     }
@@ -528,7 +652,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
         int *status, uint64_t wait_ns) {
   using Cfg = TcConfig<BN, EW>;
   constexpr int kStages = Cfg::kStages;
-  constexpr int kHalfCols = epi_cols_per_warp(BN, EW); // columns per epilogue warp of a lane quadrant
+  constexpr int kHalfCols = epi_cols_per_warp(BN, EW);
 
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[kStages];
@@ -570,7 +694,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&bar_acc_full[b]), 1);
-      mbar_init(smem_u32(&bar_acc_empty[b]), epi_active_warps(BN, EW)); // one arrive per active epilogue warp
+      mbar_init(smem_u32(&bar_acc_empty[b]), EW);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -667,49 +791,37 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
       }
     }
   } else {
-    // ---------------- epilogue (warps 2..9) ----------------
+    // ---------------- epilogue (the other warps) ----------------
     const int quad = warp & 3;       // TMEM lanes [32*quad, 32*quad+32)
-    const int ew = warp - 2;         // 0..7
+    const int ew = warp - 2;
     const int c_lo = (ew >> 2) * kHalfCols; // this warp's share of the columns
-    const bool active = c_lo < BN;          // narrow tiles leave some warps idle
     const EpiScalars sc = epi_scalars(p);
     const QuantConsts qc = epi_quant_consts<EPI>(p, warp == 2 && lane == 0 && blockIdx.x == 0);
     const bool use_slab = p.line_store != 0;
     const uint32_t slab0 = staging_base + (uint32_t)ew * Cfg::kSlabBytes;
-    bool ok = active;
+    const EpiParams ahead = epi_after_pdl(p); // (its loads are not behind an mbarrier)
+    bool ok = true;
     int64_t it = 0;
     float lo = INFINITY, hi = -INFINITY; // range of this warp's f32 outputs
+    const auto place = [&](int64_t u) { // (units are far fewer than 2^32)
+      const uint32_t t = (uint32_t)u / (uint32_t)split, tm = t / (uint32_t)tiles_n;
+      return WarpPlace{(int64_t)tm * kBM + quad * 32,
+          (int64_t)(t - tm * (uint32_t)tiles_n) * BN + c_lo,
+          (int32_t)(((uint32_t)u - t * (uint32_t)split) * p.ws_rows)};
+    };
+    WarpPlace at_next = place(blockIdx.x);
+    EpiRow row_next = fetch_ahead<kHalfCols>(ahead, at_next, lane);
     for (int64_t u = blockIdx.x; u < num_units && ok; u += gridDim.x, ++it) {
-      const int64_t t = split > 1 ? u / split : u;
-      const int32_t row_off = split > 1 ? (int32_t)((u % split) * p.ws_rows) : 0;
       const int buf = (int)(it & 1);
       const uint32_t acc_phase = (uint32_t)((it >> 1) & 1);
-      const int64_t m_warp = (t / tiles_n) * kBM + quad * 32;
-      const int64_t n0 = (t % tiles_n) * BN + c_lo;
-      // While the MMAs of this tile are still running, pull the per-column
-      // vectors this warp will need into L1.
-      {
-        const int line = lane & 7, which = lane >> 3;
-        const int64_t nl = n0 + 32 * line;
-        const void *src = nullptr;
-        if (32 * line < kHalfCols && nl < p.N) {
-          if (which == 0 && p.a_zp_len != 0)
-            src = p.colsum + nl;
-          else if (which == 1 && p.bias)
-            src = p.bias + nl;
-          else if (which == 2 && p.sb && p.sb_len != 1)
-            src = p.sb + nl;
-        }
-        if (src)
-          asm volatile("prefetch.global.L1 [%0];" ::"l"(src));
-        // ... and this warp's block of the residual (32 rows x kHalfCols f32)
-        // towards L2: the epilogue reads it one row per thread.
-        if (p.residual && m_warp + lane < p.M) {
-          const float *rr = p.residual + (m_warp + lane) * p.N + n0;
-          for (int c = 0; c < kHalfCols && n0 + c < p.N; c += 32)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(rr + c));
-        }
+      const WarpPlace at = at_next;
+      const EpiRow row = row_next;
+      if (u + gridDim.x < num_units) {
+        at_next = place(u + gridDim.x);
+        row_next = fetch_ahead<kHalfCols>(ahead, at_next, lane);
       }
+      if (EPI == kEpiDequantResidual)
+        prefetch_residual<kHalfCols>(p, at.m + lane, at.n);
       if (!mbar_wait(smem_u32(&bar_acc_full[buf]), acc_phase, abortp, wait_ns)) {
         ok = false;
         break;
@@ -719,17 +831,17 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
           tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN + c_lo);
       // The accumulator buffer may be overwritten once every warp has read
       // its share of it.
-      epilogue_tile<BN, EPI, EW>(p, sc, qc, taddr, m_warp, n0, slab0, lane, use_slab,
-          lo, hi, &map_y, &map_y2, [&] {
+      epilogue_tile<BN, EPI, EW>(p, sc, qc, taddr, at, row, slab0, lane, use_slab, lo, hi,
+          &map_y, &map_y2, [&] {
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0)
               mbar_arrive(smem_u32(&bar_acc_empty[buf]));
-          }, row_off);
+          });
     }
     // One commit of the running range per warp, and every store of this warp
     // complete before the CTA may exit.
-    if (active && p.out_range && epi_is_dequant(EPI) && EPI != OMCUDA_EPI_DEQUANT_QUANT)
+    if (p.out_range && tail_is_dequant(EPI) && EPI != OMCUDA_EPI_DEQUANT_QUANT)
       epi_range_commit(p.out_range, lo, hi);
     if (lane == 0)
       tma_store_wait_all();
@@ -845,7 +957,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&bar_acc_full[b]), 1);
-      mbar_init(smem_u32(&bar_acc_empty[b]), 2 * epi_active_warps(BN, EW));
+      mbar_init(smem_u32(&bar_acc_empty[b]), 2 * EW);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -948,50 +1060,40 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
       }
     }
   } else {
-    // ---------------- epilogue (warps 2..9 of both CTAs) ----------------
+    // ---------------- epilogue (the other warps of both CTAs) ----------------
     const int quad = warp & 3;
     const int ew = warp - 2;
     const int c_lo = (ew >> 2) * kHalfCols;
-    const bool active = c_lo < BN;
     const EpiScalars sc = epi_scalars(p);
     const QuantConsts qc = epi_quant_consts<EPI>(p, warp == 2 && lane == 0 && blockIdx.x == 0);
     const bool use_slab = p.line_store != 0;
     const uint32_t slab0 = staging_base + (uint32_t)ew * kSlabBytes;
-    bool ok = active;
+    const EpiParams ahead = epi_after_pdl(p); // (its loads are not behind an mbarrier)
+    bool ok = true;
     int64_t it = 0;
     float lo = INFINITY, hi = -INFINITY; // range of this warp's f32 outputs
-    for (int64_t u = cluster_id; u < num_units && ok; u += num_clusters, ++it) {
+    const auto place = [&](int64_t u) { // (units are far fewer than 2^32)
       const PairUnit un = pair_unit(u, full_units);
-      const int64_t t = split > 1 ? un.tile / split : un.tile;
-      const int32_t row_off = split > 1 ? (int32_t)((un.tile % split) * p.ws_rows) : 0;
+      const uint32_t t = (uint32_t)un.tile / (uint32_t)split, tm = t / (uint32_t)tiles_n;
+      return WarpPlace{(int64_t)tm * (2 * kBM) + rank * kBM + quad * 32,
+          (int64_t)(t - tm * (uint32_t)tiles_n) * BN + un.half * (BN / 2) + c_lo,
+          (int32_t)(((uint32_t)un.tile - t * (uint32_t)split) * p.ws_rows)};
+    };
+    WarpPlace at_next = place(cluster_id);
+    EpiRow row_next = fetch_ahead<kHalfCols>(ahead, at_next, lane);
+    for (int64_t u = cluster_id; u < num_units && ok; u += num_clusters, ++it) {
       const int buf = (int)(it & 1);
       const uint32_t acc_phase = (uint32_t)((it >> 1) & 1);
-      const int64_t m_warp = (t / tiles_n) * (2 * kBM) + rank * kBM + quad * 32;
-      const int64_t n0 = (t % tiles_n) * BN + un.half * (BN / 2) + c_lo;
       // a half tile keeps only the warps of accumulator columns 0..127 busy
-      const bool mine = !un.narrow || c_lo < BN / 2;
-      if (mine) {
-        const int line = lane & 7, which = lane >> 3;
-        const int64_t nl = n0 + 32 * line;
-        const void *src = nullptr;
-        if (32 * line < kHalfCols && nl < p.N) {
-          if (which == 0 && p.a_zp_len != 0)
-            src = p.colsum + nl;
-          else if (which == 1 && p.bias)
-            src = p.bias + nl;
-          else if (which == 2 && p.sb && p.sb_len != 1)
-            src = p.sb + nl;
-        }
-        if (src)
-          asm volatile("prefetch.global.L1 [%0];" ::"l"(src));
-        // ... and this warp's block of the residual (32 rows x kHalfCols f32)
-        // towards L2: the epilogue reads it one row per thread.
-        if (p.residual && m_warp + lane < p.M) {
-          const float *rr = p.residual + (m_warp + lane) * p.N + n0;
-          for (int c = 0; c < kHalfCols && n0 + c < p.N; c += 32)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(rr + c));
-        }
+      const bool mine = u < full_units || c_lo < BN / 2;
+      const WarpPlace at = at_next;
+      const EpiRow row = row_next;
+      if (u + num_clusters < num_units) {
+        at_next = place(u + num_clusters);
+        row_next = fetch_ahead<kHalfCols>(ahead, at_next, lane);
       }
+      if (EPI == kEpiDequantResidual && mine)
+        prefetch_residual<kHalfCols>(p, at.m + lane, at.n);
       if (!mbar_wait(smem_u32(&bar_acc_full[buf]), acc_phase, abortp, wait_ns)) {
         ok = false;
         break;
@@ -1006,12 +1108,12 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
           mbar_arrive_cluster(mapa_shared(smem_u32(&bar_acc_empty[buf]), 0));
       };
       if (mine)
-        epilogue_tile<BN, EPI, EW>(p, sc, qc, taddr, m_warp, n0, slab0, lane, use_slab,
-            lo, hi, &map_y, &map_y2, release, row_off);
+        epilogue_tile<BN, EPI, EW>(p, sc, qc, taddr, at, row, slab0, lane, use_slab, lo, hi,
+            &map_y, &map_y2, release);
       else
         release();
     }
-    if (active && p.out_range && epi_is_dequant(EPI) && EPI != OMCUDA_EPI_DEQUANT_QUANT)
+    if (p.out_range && tail_is_dequant(EPI) && EPI != OMCUDA_EPI_DEQUANT_QUANT)
       epi_range_commit(p.out_range, lo, hi);
     if (lane == 0)
       tma_store_wait_all();
@@ -1317,7 +1419,9 @@ int launch_bn_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan =
 }
 
 // A long K loop hides the epilogue behind the MMAs and wants pipeline depth;
-// a short one is bounded by the epilogue and wants more warps on it.
+// a short one is bounded by the epilogue and wants more warps on it, except for
+// raw sums, which leave no arithmetic to share (16384 x 1024 x 4096: 70 us with eight
+// warps, 85 with sixteen, whose slabs take a stage of the operand ring).
 // (OMCUDA_GEMM_EW=8|16 overrides the choice, for experiments.)
 inline bool want_wide_epilogue(const GemmCall &a) {
   static const int forced = [] {
@@ -1331,7 +1435,9 @@ inline bool want_wide_epilogue(const GemmCall &a) {
 
 template <int BN, int EPI>
 int launch_bn_epi(const GemmCall &a, cudaStream_t st) {
-  return want_wide_epilogue(a) ? launch_bn_epi_ew<BN, EPI, 16>(a, st)
+  // (tiles of 64 columns have no work for more than eight warps)
+  constexpr int kWide = BN == 64 || EPI == OMCUDA_EPI_I32 ? 8 : 16;
+  return want_wide_epilogue(a) ? launch_bn_epi_ew<BN, EPI, kWide>(a, st)
                                : launch_bn_epi_ew<BN, EPI, 8>(a, st);
 }
 
@@ -1341,7 +1447,8 @@ int launch_bn(const GemmCall &a, cudaStream_t st) {
   case OMCUDA_EPI_I32:
     return launch_bn_epi<BN, OMCUDA_EPI_I32>(a, st);
   case OMCUDA_EPI_DEQUANT:
-    return launch_bn_epi<BN, OMCUDA_EPI_DEQUANT>(a, st);
+    return a.residual ? launch_bn_epi<BN, kEpiDequantResidual>(a, st)
+                      : launch_bn_epi<BN, OMCUDA_EPI_DEQUANT>(a, st);
   case OMCUDA_EPI_REQUANT:
     return launch_bn_epi<BN, OMCUDA_EPI_REQUANT>(a, st);
   case OMCUDA_EPI_DEQUANT_SPLIT:
@@ -1444,7 +1551,8 @@ int launch_pair_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan
 
 template <int EPI>
 int launch_pair_epi(const GemmCall &a, cudaStream_t st) {
-  return want_wide_epilogue(a) ? launch_pair_epi_ew<EPI, 16>(a, st)
+  constexpr int kWide = EPI == OMCUDA_EPI_I32 ? 8 : 16;
+  return want_wide_epilogue(a) ? launch_pair_epi_ew<EPI, kWide>(a, st)
                                : launch_pair_epi_ew<EPI, 8>(a, st);
 }
 
@@ -1453,7 +1561,8 @@ int launch_pair(const GemmCall &a, cudaStream_t st) {
   case OMCUDA_EPI_I32:
     return launch_pair_epi<OMCUDA_EPI_I32>(a, st);
   case OMCUDA_EPI_DEQUANT:
-    return launch_pair_epi<OMCUDA_EPI_DEQUANT>(a, st);
+    return a.residual ? launch_pair_epi<kEpiDequantResidual>(a, st)
+                      : launch_pair_epi<OMCUDA_EPI_DEQUANT>(a, st);
   case OMCUDA_EPI_REQUANT:
     return launch_pair_epi<OMCUDA_EPI_REQUANT>(a, st);
   case OMCUDA_EPI_DEQUANT_SPLIT:
@@ -1526,11 +1635,9 @@ int launch_split_k(const GemmCall &a, cudaStream_t st, int split) {
   const GemmCall part = split_pass_args(a, plan);
   int rc;
   if (a.M > kBM)
-    rc = want_wide_epilogue(a) ? launch_pair_epi_ew<OMCUDA_EPI_I32, 16>(part, st, plan)
-                               : launch_pair_epi_ew<OMCUDA_EPI_I32, 8>(part, st, plan);
+    rc = launch_pair_epi_ew<OMCUDA_EPI_I32, 8>(part, st, plan);
   else
-    rc = want_wide_epilogue(a) ? launch_bn_epi_ew<256, OMCUDA_EPI_I32, 16>(part, st, plan)
-                               : launch_bn_epi_ew<256, OMCUDA_EPI_I32, 8>(part, st, plan);
+    rc = launch_bn_epi_ew<256, OMCUDA_EPI_I32, 8>(part, st, plan);
   if (rc == OMCUDA_OK) {
     const EpiParams p = make_epi_params(a);
     const int64_t total = a.M * (a.N >> 2);
