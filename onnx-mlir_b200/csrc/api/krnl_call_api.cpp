@@ -293,7 +293,8 @@ void set_a_operand(Stage &sg, GemmCall *g, const void *A, cudaStream_t st,
   }
   if (!sg.ok())
     return;
-  sg.set(launch_repitch(A, g->a_signed, g->M, g->K, g->lda, rows, rs, rq, st));
+  sg.set(launch_repitch(
+      A, g->a_signed, g->M, g->K, g->lda, rows, rs, rq, st, g->b_zp, g->b_zp_len));
   g->a_rowsum = rs;
 }
 

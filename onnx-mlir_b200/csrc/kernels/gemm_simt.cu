@@ -22,45 +22,62 @@ namespace omcuda {
 
 // ---- B preparation -----------------------------------------------------------
 
+// Bound by the read and the write of B.  A thread takes a 4 x 4 block of a 64(k) x
+// 64(n) tile: four words of neighbouring columns (or bytes, where rows of B do not
+// start on words), turned in registers into words of neighbouring k, which pass
+// through shared memory to leave row by row.  With the column sums below 14336 x 4096
+// (59 MB) take 40 us; byte by byte, and sums of a column per thread, 485.
 __global__ void __launch_bounds__(256)
     transpose_b_kernel(const uint8_t *__restrict__ B, int64_t K, int64_t N,
         int64_t kp, uint8_t *__restrict__ Bt) {
-  // 64(k) x 64(n) byte tile through shared memory; reads are coalesced along
-  // n, writes along k.
-  __shared__ uint8_t tile[64][65];
+  __shared__ uint32_t tile[64][17]; // [column][word of k]
   const int64_t k0 = (int64_t)blockIdx.y * 64, n0 = (int64_t)blockIdx.x * 64;
-  const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6; // 64 x 4
-  for (int r = ty; r < 64; r += 4) {
-    int64_t k = k0 + r, n = n0 + tx;
-    tile[r][tx] = (k < K && n < N) ? B[k * N + n] : (uint8_t)0;
+  const bool words = (((uintptr_t)B | (uintptr_t)N) & 3u) == 0;
+  {
+    const int nb = threadIdx.x & 15, kb = threadIdx.x >> 4;
+    const int64_t n = n0 + 4 * nb;
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int64_t k = k0 + 4 * kb + i;
+      w[i] = 0;
+      if (k < K && n < N) {
+        const uint8_t *src = B + k * N + n;
+        if (words) {
+          w[i] = __ldcs(reinterpret_cast<const uint32_t *>(src));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (n + j < N)
+              w[i] |= (uint32_t)__ldg(src + j) << (8 * j);
+        }
+      }
+    }
+    // 4 x 4 bytes transposed
+    const uint32_t a0 = __byte_perm(w[0], w[1], 0x5140), a1 = __byte_perm(w[0], w[1], 0x7362);
+    const uint32_t b0 = __byte_perm(w[2], w[3], 0x5140), b1 = __byte_perm(w[2], w[3], 0x7362);
+    tile[4 * nb][kb] = __byte_perm(a0, b0, 0x5410);
+    tile[4 * nb + 1][kb] = __byte_perm(a0, b0, 0x7632);
+    tile[4 * nb + 2][kb] = __byte_perm(a1, b1, 0x5410);
+    tile[4 * nb + 3][kb] = __byte_perm(a1, b1, 0x7632);
   }
   __syncthreads();
-  for (int r = ty; r < 64; r += 4) {
-    int64_t n = n0 + r, k = k0 + tx;
-    if (n < N && k < kp)
-      Bt[n * kp + k] = tile[tx][r];
-  }
-}
-
-template <bool kSigned>
-__global__ void __launch_bounds__(256)
-    colsum_kernel(const uint8_t *__restrict__ B, int64_t K, int64_t N,
-        int32_t *__restrict__ colsum) {
-  // blockDim = (64, 4): 64 columns per block, K split four ways.
-  __shared__ int32_t part[4][64];
-  const int64_t n = (int64_t)blockIdx.x * 64 + threadIdx.x;
-  int32_t s = 0;
-  if (n < N) {
-    for (int64_t k = threadIdx.y; k < K; k += 4) {
-      uint8_t b = B[k * N + n];
-      s += kSigned ? (int32_t)(int8_t)b : (int32_t)b;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = (threadIdx.x >> 4) + 16 * i, c = threadIdx.x & 15;
+    const int64_t n = n0 + r, k = k0 + 4 * c;
+    if (n >= N || k >= kp)
+      continue;
+    const uint32_t w = tile[r][c];
+    uint8_t *dst = Bt + n * kp + k;
+    if (((uintptr_t)Bt & 3u) == 0) {
+      *reinterpret_cast<uint32_t *>(dst) = w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        dst[j] = (uint8_t)(w >> (8 * j));
     }
   }
-  part[threadIdx.y][threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.y == 0 && n < N)
-    colsum[n] = part[0][threadIdx.x] + part[1][threadIdx.x] +
-                part[2][threadIdx.x] + part[3][threadIdx.x];
 }
 
 // QLinearMatMul's column scales (src/Conversion/ONNXToKrnl/Math/QLinearMatMul.cpp:123-138).
@@ -74,17 +91,42 @@ __device__ __forceinline__ float requant_scale(const RequantScale &rq, int64_t i
 // the rows: a launch of their own was 2.1 us for a few thousand divides, and made
 // by the blocks of the rows, one of them for up to 8 rows, they were a serial chain
 // (1 x 256 x 32768: 45 us a call so, 19 now).
+//
+// The sums serve the zero points of the weight, which are mostly all zero: with zp
+// (zp_len bytes), a block first looks at those and leaves without its sums, which
+// nothing reads then, if it finds nothing else.  QLinearMatMul 512 x 1024 x 1024 12.3
+// -> 8.3 us a call, together with the launch that overlaps; 16384 x 1024 x 4096 77 -> 72.
 template <bool kSigned>
 __global__ void __launch_bounds__(256)
     rowsum_kernel(const uint8_t *__restrict__ A, int64_t M, int64_t K,
         int32_t *__restrict__ rowsum, uint8_t *__restrict__ dst, int64_t pitch,
-        RequantScale rq) {
+        const uint8_t *__restrict__ zp, int64_t zp_len, RequantScale rq) {
+  pdl_sync();
+  A = after_pdl(A);
+  zp = after_pdl(zp);
   const int64_t row_blocks = ceil_div(M, (int64_t)(blockDim.x >> 5));
   if (blockIdx.x >= row_blocks) {
     const int64_t i = ((int64_t)blockIdx.x - row_blocks) * blockDim.x + threadIdx.x;
     if (i < rq.len)
       rq.S[i] = requant_scale(rq, i);
     return;
+  }
+  if (zp) {
+    uint32_t any = 0;
+    for (int64_t i = 16 * (int64_t)threadIdx.x; i < zp_len; i += 16 * 256) {
+      if ((((uintptr_t)zp) & 15u) == 0 && i + 16 <= zp_len) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(zp + i));
+        any |= q.x | q.y | q.z | q.w;
+      } else {
+        for (int64_t j = i; j < i + 16 && j < zp_len; ++j)
+          any |= __ldg(zp + j);
+      }
+    }
+    if (!__syncthreads_or((int)any)) {
+      if (!dst)
+        return;
+      rowsum = nullptr;
+    }
   }
   const int64_t m = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (m >= M)
@@ -707,12 +749,13 @@ int launch_gemm_simt(const GemmCall &a, cudaStream_t st) {
 }
 
 int launch_repitch(const void *A, int a_signed, int64_t M, int64_t K, int64_t pitch,
-    uint8_t *dst, int32_t *rowsum, const RequantScale &rq, cudaStream_t st) {
+    uint8_t *dst, int32_t *rowsum, const RequantScale &rq, cudaStream_t st, const void *zp,
+    int64_t zp_len) {
   const unsigned grid = (unsigned)(ceil_div(M, 8) + ceil_div(rq.len, 256));
-  if (a_signed)
-    rowsum_kernel<true><<<grid, 256, 0, st>>>((const uint8_t *)A, M, K, rowsum, dst, pitch, rq);
-  else
-    rowsum_kernel<false><<<grid, 256, 0, st>>>((const uint8_t *)A, M, K, rowsum, dst, pitch, rq);
+  // (a block's rows are 8 K bytes: more zero points than that cost more than they save)
+  const uint8_t *look = zp_len <= 8 * K ? (const uint8_t *)zp : nullptr;
+  OMCUDA_CHECK(launch_pdl(a_signed ? rowsum_kernel<true> : rowsum_kernel<false>, grid, 256, 0,
+      st, 0, pdl_pays(M * K), (const uint8_t *)A, M, K, rowsum, dst, pitch, look, zp_len, rq));
   OMCUDA_CHECK_LAUNCH("rowsum_kernel");
   return OMCUDA_OK;
 }
@@ -743,16 +786,9 @@ extern "C" int omcudaDevPrepareB(const void *B, int b_signed, int64_t K,
   transpose_b_kernel<<<tgrid, 256, 0, st>>>(
       (const uint8_t *)B, K, N, kp, (uint8_t *)out->bt);
   OMCUDA_CHECK_LAUNCH("transpose_b_kernel");
-  dim3 cblock(64, 4);
-  unsigned cgrid = (unsigned)ceil_div(N, 64);
-  if (b_signed)
-    colsum_kernel<true><<<cgrid, cblock, 0, st>>>(
-        (const uint8_t *)B, K, N, out->colsum);
-  else
-    colsum_kernel<false><<<cgrid, cblock, 0, st>>>(
-        (const uint8_t *)B, K, N, out->colsum);
-  OMCUDA_CHECK_LAUNCH("colsum_kernel");
-  return OMCUDA_OK;
+  // Column sums of B are row sums of its copy (whose padding is zero): coalesced
+  // 16-byte loads of what has just been written, on the whole machine.
+  return launch_repitch(out->bt, b_signed, N, kp, 0, nullptr, out->colsum, RequantScale(), st);
 }
 
 extern "C" int omcudaDevRowSum(const void *A, int a_signed, int64_t M,

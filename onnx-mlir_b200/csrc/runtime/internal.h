@@ -82,9 +82,12 @@ struct RequantScale {
 };
 // Copies an 8-bit [M,K] matrix of any alignment into rows of `pitch` bytes (a
 // multiple of 16, dst 16-byte aligned), zero from K on; dst or rowsum may be
-// null.  Makes the scales of rq in the same launch.
+// null.  Makes the scales of rq in the same launch.  zp (zp_len bytes, may be
+// null): what the sums are for; when all of it is zero they may be left out, and
+// rowsum then holds anything.
 int launch_repitch(const void *A, int a_signed, int64_t M, int64_t K, int64_t pitch,
-    uint8_t *dst, int32_t *rowsum, const RequantScale &rq, cudaStream_t st);
+    uint8_t *dst, int32_t *rowsum, const RequantScale &rq, cudaStream_t st,
+    const void *zp = nullptr, int64_t zp_len = 0);
 
 // gemm_batched.cu: every product of a MatMulInteger whose B is an activation in
 // one launch, operands read as they lie.  Product i (row-major over size[])

@@ -769,3 +769,47 @@ def test_qlinear_large_results(gpu, orc, scale):
     got, want = gpu.qlinear_matmul(*args), orc.qlinear_matmul(*args)
     assert np.array_equal(got[inside], want[inside]) and inside.any()
     assert (x > 2**22).any() or scale < 1
+
+
+@pytest.mark.parametrize("m,k,n", [(40, 64, 128), (300, 192, 144), (9, 1024, 96), (150, 77, 133)])
+@pytest.mark.parametrize("zeros", ["all", "chunks", "none"])
+@pytest.mark.parametrize("yt", [np.uint8, np.int8])
+def test_weight_zero_points_partly_zero(gpu, orc, m, k, n, zeros, yt):
+    """Zero points of the weight that are all zero, zero in whole runs of 32 columns
+    (which the tails skip), or nowhere; output zero points at the end of their type."""
+    rng = np.random.default_rng(m + k + n)
+    a = rng.integers(0, 256, (m, k)).astype(np.uint8)
+    b = rng.integers(-128, 128, (k, n)).astype(np.int8)
+    bz = np.zeros(n, np.int8) if zeros == "all" else rng.integers(1, 100, n).astype(np.int8)
+    if zeros == "chunks":
+        bz[32:96] = 0
+    bs = (rng.random(n) * 0.009 + 0.001).astype(np.float32)
+    yz = yt(np.iinfo(yt).max)
+    args = (a, np.float32(0.02), np.uint8(131), b, bs, bz, np.float32(0.37), yz)
+    want = orc.qlinear_matmul(*args)
+    assert np.array_equal(gpu.qlinear_matmul(*args), want)
+    assert np.array_equal(gpu.qlinear_matmul(*args, device=True).numpy(), want)
+
+
+@pytest.mark.parametrize("k,n", [(1, 1), (3, 5), (16, 4), (63, 65), (64, 64), (65, 130), (200, 67),
+                                 (130, 256)])
+@pytest.mark.parametrize("signed", [False, True])
+def test_prepared_weight(gpu, k, n, signed):
+    """The K-major copy of a weight, its zero padding and its column sums."""
+    import torch
+    from omcuda import dev
+    rng = np.random.default_rng(k * 300 + n)
+    w = rng.integers(0, 256, (k, n)).astype(np.uint8)
+    nbytes, kp = dev.prepared_b_bytes(k, n)
+    for shift in (0, 1):
+        src = torch.zeros(k * n + 1, dtype=torch.uint8, device="cuda")
+        src[shift:shift + k * n] = torch.from_numpy(w.ravel()).cuda()
+        bt = torch.full((nbytes,), 255, dtype=torch.uint8, device="cuda")
+        cs = torch.empty(n, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        dev.prepare_b(src.data_ptr() + shift, int(signed), k, n, bt.data_ptr(), cs.data_ptr(), None)
+        torch.cuda.synchronize()
+        got = bt.cpu().numpy().reshape(n, kp)
+        assert np.array_equal(got[:, :k], w.T) and not got[:, k:].any()
+        v = w.view(np.int8) if signed else w
+        assert np.array_equal(cs.cpu().numpy(), v.astype(np.int64).sum(0))
