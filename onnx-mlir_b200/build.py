@@ -28,6 +28,7 @@ SOURCES = [
     "kernels/dql.cu",
     "kernels/gemm_simt.cu",
     "kernels/gemm_batched.cu",
+    "kernels/linear_rows.cu",
     "kernels/gemm_tc.cu",
     "kernels/encoder_ops.cu",
     "kernels/attention_mma.cu",

@@ -890,6 +890,24 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
   g.N = d.N;
   g.K = d.K;
   g.lda = (d.K + 15) & ~int64_t(15);
+  if (d.K > 0 && linear_rows_wanted(d.M, d.N, g.lda)) {
+    if (wzn) {
+      g.b_zp = dWz;
+      g.b_zp_len = wzn;
+    }
+    if (sg.ok())
+      sg.set(prepared_b(sg, omTensorGetDataPtr(Wq), dW, wt == ONNX_TYPE_INT8, d.K, d.N, st, &g.B));
+    g.epilogue = OMCUDA_EPI_DEQUANT;
+    g.Y = dY;
+    g.sb = dWs;
+    g.sb_len = wsn;
+    g.scale_form = (int)scaleForm;
+    g.bias = dBias;
+    if (sg.ok())
+      sg.set(launch_linear_rows(dX, g, st));
+    sg.finish(false);
+    return;
+  }
   uint8_t *xq = (uint8_t *)sg.scratch((size_t)(d.M * g.lda));
   float *xs = (float *)sg.scratch(16);
   const bool small = dql_small_wanted(d.M, g.lda);

@@ -426,31 +426,6 @@ __global__ void __launch_bounds__(32 * kGemvWarps)
 constexpr int kGemvMmaWarps = 8;
 constexpr int kGemvMmaUnroll = 4; // 64-byte blocks of K in flight per warp
 
-template <bool kASigned, bool kBSigned>
-__device__ __forceinline__ void mma_m16n8k32(int32_t (&c)[4], uint32_t a0,
-    uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  if (kASigned && kBSigned)
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 "
-                 "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-  else if (kASigned && !kBSigned)
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 "
-                 "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-  else if (!kASigned && kBSigned)
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 "
-                 "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-  else
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 "
-                 "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 template <int CG, bool kASigned, bool kBSigned>
 __global__ void __launch_bounds__(32 * kGemvMmaWarps)
     gemm_i8_gemv_mma_kernel(const uint8_t *__restrict__ A,

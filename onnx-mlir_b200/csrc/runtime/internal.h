@@ -89,6 +89,11 @@ int launch_repitch(const void *A, int a_signed, int64_t M, int64_t K, int64_t pi
     uint8_t *dst, int32_t *rowsum, const RequantScale &rq, cudaStream_t st,
     const void *zp = nullptr, int64_t zp_len = 0);
 
+// linear_rows.cu: DynamicQuantizeLinear, product and DEQUANT tail of up to 16 f32 rows
+// in one launch (a: as for gemm_i8, but for its A and what describes it).
+bool linear_rows_wanted(int64_t M, int64_t N, int64_t kp);
+int launch_linear_rows(const float *x, const GemmCall &a, cudaStream_t st);
+
 // gemm_batched.cu: every product of a MatMulInteger whose B is an activation in
 // one launch, operands read as they lie.  Product i (row-major over size[])
 // reads A and B at the element offsets its strides give (0 along a broadcast

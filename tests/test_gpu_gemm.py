@@ -813,3 +813,34 @@ def test_prepared_weight(gpu, k, n, signed):
         assert np.array_equal(got[:, :k], w.T) and not got[:, k:].any()
         v = w.view(np.int8) if signed else w
         assert np.array_equal(cs.cpu().numpy(), v.astype(np.int64).sum(0))
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (1, 15, 63), (2, 64, 64), (16, 512, 65), (16, 513, 200), (3, 1040, 128),
+                                   (7, 4099, 130), (16, 8200, 96), (2, 16001, 2100), (3, 5461, 33), (2, 500, 18000),
+                                   (16, 1024, 2496), (4, 768, 3072)])
+@pytest.mark.parametrize("wt,per_column", [(np.int8, False), (np.uint8, True), (np.uint8, False)])
+@pytest.mark.parametrize("form", [0, 1])
+def test_linear_of_few_rows(gpu, orc, m, k, n, wt, per_column, form):
+    """Up to 16 rows in one launch, K split over a cluster: slices that are empty, that
+    end inside a 64-byte block, more of x than a thread keeps, several column groups
+    per cluster, and sizes that are left to the separate kernels."""
+    rng = np.random.default_rng(m * 31 + k + n)
+    x = rng.normal(0.2, 2, size=(m, k)).astype(np.float32)
+    w = rng.integers(-127, 128, (k, n)).astype(np.int8) if wt == np.int8 else \
+        rng.integers(0, 256, (k, n)).astype(np.uint8)
+    zp = None if wt == np.int8 else (rng.integers(0, 256, n).astype(np.uint8) if per_column
+                                     else np.array(131, np.uint8))
+    ws = (rng.random(n) * 0.009 + 0.001).astype(np.float32) if per_column else np.float32(0.0157)
+    bias = rng.normal(size=n).astype(np.float32) if m % 2 else None
+    xq, xs, xz = orc.dynamic_quantize_linear(x)
+    xi = (xq.astype(np.float64) - float(xz))
+    wi = w.astype(np.float64) - (0.0 if zp is None else zp.astype(np.float64))
+    f = (xi @ wi).astype(np.int64).astype(np.float32)  # exact: |sum| < 2^53
+    want = f * (np.float32(xs) * ws) if form == 0 else (f * np.float32(xs)) * ws
+    want = want.astype(np.float32)
+    if bias is not None:
+        want = want + bias
+    for device in (False, True):
+        got = gpu.dyn_quant_linear(x, w, ws, zp, bias, form, device=device)
+        got = got.numpy() if device else got
+        assert got.tobytes() == want.astype(np.float32).tobytes()
