@@ -530,10 +530,9 @@ static int grid_for(int64_t work_items, int per_block) {
 // fastest with the blocks that are resident at once (16 Mi values: 13.0 us, with
 // a short block per run 15.8); what comes from HBM with short blocks, up to 64 per
 // SM, of which the last round is a small part (64 Mi: 51.6, resident ones 54.6).
-static int pass_grid(int64_t n, int run, bool resident = false) {
+static int pass_grid(int64_t n, int run, bool resident) {
   int64_t want = ceil_div(n, run);
-  const int64_t cap =
-      (int64_t)sm_count() * (resident || n <= ((int64_t)24 << 20) ? 8 : 64);
+  const int64_t cap = (int64_t)sm_count() * (resident ? 8 : 64);
   if (want < 1)
     want = 1;
   return (int)(want < cap ? want : cap);
@@ -551,7 +550,7 @@ static void launch_dequantize(const T *x, int64_t n, const float *scale, const T
     float *y, cudaStream_t st) {
   const bool whole = ((uintptr_t)x & (4 * sizeof(T) - 1)) == 0 && ((uintptr_t)y & 15u) == 0;
   if (whole)
-    dequantize_kernel<<<pass_grid(n, 256 * 4 * kDequantUnroll), 256, 0, st>>>(x, n, scale, zp, y);
+    dequantize_kernel<<<pass_grid(n, 256 * 4 * kDequantUnroll, false), 256, 0, st>>>(x, n, scale, zp, y);
   else
     dequantize_single_kernel<<<grid_for(n, 256 * 4), 256, 0, st>>>(x, n, scale, zp, y);
 }
@@ -568,7 +567,10 @@ int launch_quantize_pass(const float *x, int64_t n, uint8_t *y, const RangeParts
   // matters; 64 Mi values 115 us with short blocks, 106 with resident ones, 103
   // with the overlap).
   const bool folds = parts.count > 0;
-  const int grid = pass_grid(n, kDqlThreads * 4 * unroll, folds);
+  // (what a producer on the device has just left lies in L2 up to some 100 MB; a
+  // caller's own tensor may come from anywhere)
+  const bool in_l2 = range && n <= ((int64_t)24 << 20);
+  const int grid = pass_grid(n, kDqlThreads * 4 * unroll, folds || in_l2);
   OMCUDA_CHECK(launch_pdl(quantize_kernel<kSigned>, grid, kDqlThreads, 0, st, 0,
       folds || pdl_pays(n),
       x, n, y, parts, scale, zp, range, outs, quant_mode(), unroll));
