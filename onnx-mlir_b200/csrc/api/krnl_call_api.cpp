@@ -183,6 +183,19 @@ private:
 // launches on the shared library stream, and the reduction leaves its partials
 // in its scratch for the quantize pass that follows.
 
+//
+// A captured call must not take one: its replays would write to the block after it
+// was given back.
+
+bool is_capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return cs != cudaStreamCaptureStatusNone;
+}
+
 void *dql_scratch_for(Stage &sg) { return sg.scratch((size_t)omcudaDevDqlScratchBytes(0)); }
 
 // ---- constants: prepared B operands cached by buffer ----------------------------------
@@ -547,7 +560,8 @@ void omcudaDynamicQuantizeLinear(
   float *ds = (float *)sg.out(yScale);
   uint8_t *dz = (uint8_t *)sg.out(yZp);
   const int64_t n = omTensorGetNumElems(x);
-  if (dql_small_wanted(1, n)) {
+  if (dql_small_wanted(1, n) || (dql_one_cluster_holds(n) && (is_capturing(st) ||
+                                    dql_in_place(dx, n, dy, ds, dz)))) {
     if (sg.ok())
       sg.set(launch_dql_small(dx, 1, n, n, dy, nullptr, ds, dz, st));
     sg.finish(false);

@@ -327,18 +327,21 @@ __global__ void __launch_bounds__(kDqlThreads)
 }
 
 // DynamicQuantizeLinear of a tensor of which every thread of one cluster holds
-// one word of four values: what bounds small tensors is launches and round trips
+// kWords words of four values: what bounds small tensors is launches and round trips
 // through memory.  Here every thread loads its values once, the CTAs exchange their
 // {min,max} through distributed shared memory, every thread derives the two
 // scalars and quantizes what it still holds: one launch for two, no scratch.  The
 // same minima, maxima and per-element arithmetic as the passes above, so the same
-// bytes.  The line where it ends is explained at dql_small_wanted.
+// bytes.  One word is the fast form, the line where it ends is explained at
+// dql_small_wanted; four are for calls that must not take the two passes
+// (dql_one_cluster_holds).
 //
 // The tensor is [rows, cols], written in rows of `pitch` bytes (zero from cols
 // on); a flat tensor is one row of pitch == cols.  rowsum (may be null) gets
 // the sums of the quantized rows.
 constexpr int kSmallThreads = 1024;
 constexpr int kSmallMaxCluster = 16;
+constexpr int kSmallMaxWords = 4; // per thread
 
 struct SmallDql {
   const float *x;
@@ -354,6 +357,7 @@ struct SmallDql {
   int mode;
 };
 
+template <int kWords>
 __global__ void __launch_bounds__(kSmallThreads) dql_small_kernel(SmallDql p) {
   __shared__ float s_lo[kSmallThreads / 32], s_hi[kSmallThreads / 32];
   __shared__ float c_lo[kSmallMaxCluster], c_hi[kSmallMaxCluster];
@@ -364,33 +368,45 @@ __global__ void __launch_bounds__(kSmallThreads) dql_small_kernel(SmallDql p) {
   cluster.barrier_arrive(); // "has started": waited for before the first remote store
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tid = (int)(rank * kSmallThreads + threadIdx.x);
+  const int nthreads = (int)(ctas * kSmallThreads);
   if (p.rowsum)
-    for (int i = tid; i < p.rows; i += (int)(ctas * kSmallThreads))
+    for (int i = tid; i < p.rows; i += nthreads)
       p.rowsum[i] = 0;
   // Zeros that stand for no element change neither scalar: the range is
   // widened to hold 0 before anything is derived from it.
-  float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  const bool in = tid < p.words;
-  const int r = in ? tid / p.row_words : p.rows - 1;
-  const int c = 4 * (tid - r * p.row_words);
-  const int have = in ? p.cols - c : 0;
-  {
-    const float *src = x + (int64_t)r * p.cols + c;
-    if (have >= 4 && p.vec_in) {
-      v = __ldg(reinterpret_cast<const float4 *>(src));
+  float4 v[kWords];
+  int row[kWords], col[kWords], have[kWords];
+#pragma unroll
+  for (int u = 0; u < kWords; ++u) {
+    const int w = tid + u * nthreads;
+    const bool in = w < p.words;
+    row[u] = in ? w / p.row_words : p.rows - 1;
+    col[u] = 4 * (w - row[u] * p.row_words);
+    have[u] = in ? p.cols - col[u] : 0;
+    v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float *src = x + (int64_t)row[u] * p.cols + col[u];
+    if (have[u] >= 4 && p.vec_in) {
+      v[u] = __ldg(reinterpret_cast<const float4 *>(src));
     } else {
-      if (have > 0)
-        v.x = __ldg(src);
-      if (have > 1)
-        v.y = __ldg(src + 1);
-      if (have > 2)
-        v.z = __ldg(src + 2);
-      if (have > 3)
-        v.w = __ldg(src + 3);
+      if (have[u] > 0)
+        v[u].x = __ldg(src);
+      if (have[u] > 1)
+        v[u].y = __ldg(src + 1);
+      if (have[u] > 2)
+        v[u].z = __ldg(src + 2);
+      if (have[u] > 3)
+        v[u].w = __ldg(src + 3);
     }
   }
-  float lo = warp_min(min3f(fminf(v.x, v.y), v.z, v.w));
-  float hi = warp_max(max3f(fmaxf(v.x, v.y), v.z, v.w));
+  float lo = min3f(fminf(v[0].x, v[0].y), v[0].z, v[0].w);
+  float hi = max3f(fmaxf(v[0].x, v[0].y), v[0].z, v[0].w);
+#pragma unroll
+  for (int u = 1; u < kWords; ++u) {
+    lo = min3f(min3f(lo, v[u].x, v[u].y), v[u].z, v[u].w);
+    hi = max3f(max3f(hi, v[u].x, v[u].y), v[u].z, v[u].w);
+  }
+  lo = warp_min(lo);
+  hi = warp_max(hi);
   if (lane == 0) {
     s_lo[warp] = lo;
     s_hi[warp] = hi;
@@ -406,7 +422,7 @@ __global__ void __launch_bounds__(kSmallThreads) dql_small_kernel(SmallDql p) {
       *cluster.map_shared_rank(&c_hi[rank], lane) = hi;
     }
   }
-  cluster.sync(); // orders the remote stores, and the zeroes in rowsum
+  cluster.sync(); // orders the remote stores, the zeroes in rowsum, and all loads before all stores
   lo = c_lo[0];
   hi = c_hi[0];
   for (unsigned i = 1; i < ctas; ++i) {
@@ -420,27 +436,34 @@ __global__ void __launch_bounds__(kSmallThreads) dql_small_kernel(SmallDql p) {
   if (tid - lane >= p.words)
     return; // the whole warp is past the end
   const QuantConsts qc = make_quant_consts<false>(scale, zp_f, p.mode);
-  uint32_t q = have > 0 ? quantize_four<false>(v, qc) : 0u;
-  if (have < 4)
-    q = have > 0 ? q & ((1u << (8 * have)) - 1u) : 0u;
-  if (in) {
-    uint8_t *dst = p.y + (int64_t)r * p.pitch + c;
-    if (p.vec_out && c + 4 <= p.pitch) {
-      *reinterpret_cast<uint32_t *>(dst) = q;
-    } else {
-      for (int e = 0; e < 4 && c + e < p.pitch; ++e)
-        dst[e] = (uint8_t)(q >> (8 * e));
+#pragma unroll
+  for (int u = 0; u < kWords; ++u) {
+    if (tid + u * nthreads - lane >= p.words)
+      break;
+    const bool in = tid + u * nthreads < p.words;
+    const int r = row[u], c = col[u];
+    uint32_t q = have[u] > 0 ? quantize_four<false>(v[u], qc) : 0u;
+    if (have[u] < 4)
+      q = have[u] > 0 ? q & ((1u << (8 * have[u])) - 1u) : 0u;
+    if (in) {
+      uint8_t *dst = p.y + (int64_t)r * p.pitch + c;
+      if (p.vec_out && c + 4 <= p.pitch) {
+        *reinterpret_cast<uint32_t *>(dst) = q;
+      } else {
+        for (int e = 0; e < 4 && c + e < p.pitch; ++e)
+          dst[e] = (uint8_t)(q >> (8 * e));
+      }
     }
-  }
-  if (p.rowsum) {
-    int32_t sum = add_bytes<false>(q, 0);
-    // rows grow with the lane: first and last alike means one row
-    if (__shfl_sync(0xffffffffu, r, 0) == __shfl_sync(0xffffffffu, r, 31)) {
-      sum = __reduce_add_sync(0xffffffffu, sum);
-      if (lane == 0)
+    if (p.rowsum) {
+      int32_t sum = add_bytes<false>(q, 0);
+      // rows grow with the lane: first and last alike means one row
+      if (__shfl_sync(0xffffffffu, r, 0) == __shfl_sync(0xffffffffu, r, 31)) {
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (lane == 0)
+          atomicAdd(p.rowsum + r, sum);
+      } else if (in) {
         atomicAdd(p.rowsum + r, sum);
-    } else if (in) {
-      atomicAdd(p.rowsum + r, sum);
+      }
     }
   }
 }
@@ -633,11 +656,15 @@ int small_cluster_limit() {
     at[0].val.clusterDim.z = 1;
     q.attrs = at;
     q.numAttrs = 1;
-    int clusters = 0;
-    if (cudaFuncSetAttribute(dql_small_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed,
-            1) == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&clusters, dql_small_kernel, &q) == cudaSuccess &&
-        clusters > 0)
+    int a = 0, b = 0;
+    if (cudaFuncSetAttribute(dql_small_kernel<1>,
+            cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaFuncSetAttribute(dql_small_kernel<kSmallMaxWords>,
+            cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&a, dql_small_kernel<1>, &q) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&b, dql_small_kernel<kSmallMaxWords>, &q) ==
+            cudaSuccess &&
+        a > 0 && b > 0)
       n = kSmallMaxCluster;
     (void)cudaGetLastError();
     limit.set(n);
@@ -653,6 +680,17 @@ bool dql_small_wanted(int64_t rows, int64_t pitch) {
   // few SMs of one cluster lose to the whole machine: two, 131072 values, 5.0 us.
   const int64_t words = (int64_t)kSmallThreads * small_cluster_limit();
   return rows <= words && pitch <= 4 * words && rows * ceil_div(pitch, 4) <= words;
+}
+
+bool dql_one_cluster_holds(int64_t n) {
+  return n <= (int64_t)4 * kSmallMaxWords * kSmallThreads * small_cluster_limit();
+}
+
+bool dql_in_place(const float *x, int64_t n, const uint8_t *y, const float *y_scale,
+    const uint8_t *y_zp) {
+  const int64_t bytes = n * (int64_t)sizeof(float);
+  return ranges_overlap(x, bytes, y, n) || ranges_overlap(x, bytes, y_scale, sizeof(float)) ||
+         ranges_overlap(x, bytes, y_zp, 1);
 }
 
 int launch_dql_small(const float *x, int64_t rows, int64_t cols, int64_t pitch,
@@ -672,9 +710,12 @@ int launch_dql_small(const float *x, int64_t rows, int64_t cols, int64_t pitch,
   p.vec_out = ((uintptr_t)y & 3u) == 0 && (rows == 1 || pitch % 4 == 0);
   p.mode = quant_mode();
   unsigned ctas = 1;
-  while (ctas * kSmallThreads < (unsigned)p.words)
+  while (ctas * kSmallThreads < (unsigned)p.words && ctas < (unsigned)small_cluster_limit())
     ctas *= 2;
-  OMCUDA_CHECK(launch_pdl(dql_small_kernel, ctas, kSmallThreads, 0, st, ctas, true, p));
+  OMCUDA_CHECK(launch_pdl((unsigned)p.words <= ctas * kSmallThreads
+                              ? dql_small_kernel<1>
+                              : dql_small_kernel<kSmallMaxWords>,
+      ctas, kSmallThreads, 0, st, ctas, true, p));
   count_launch();
   return OMCUDA_OK;
 }
@@ -692,7 +733,8 @@ extern "C" int omcudaDevDynamicQuantizeLinear(const float *x, int64_t n,
   if (n < 0 || (n > 0 && (!x || !y)) || !scratch)
     return fail(OMCUDA_EINVAL, "DynamicQuantizeLinear: bad argument");
   cudaStream_t st = (cudaStream_t)stream;
-  if (dql_small_wanted(1, n))
+  if (dql_small_wanted(1, n) ||
+      (dql_one_cluster_holds(n) && dql_in_place(x, n, y, y_scale, y_zp)))
     return launch_dql_small(x, 1, n, n, y, nullptr, y_scale, y_zp, st);
   RangeParts parts;
   int rc = launch_range_parts(x, n, scratch, &parts, st);

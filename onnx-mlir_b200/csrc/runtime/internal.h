@@ -39,6 +39,13 @@ int quant_mode();
 // Wait limit the tensor-core kernels are launched with (gemm_tc.cu).
 uint64_t tc_wait_limit_ns();
 
+// Whether two ranges of memory share a byte.
+inline bool ranges_overlap(const void *a, int64_t a_bytes, const void *b, int64_t b_bytes) {
+  const uintptr_t p = (uintptr_t)a, q = (uintptr_t)b;
+  return a_bytes > 0 && b_bytes > 0 && p < q + (uintptr_t)b_bytes &&
+         q < p + (uintptr_t)a_bytes;
+}
+
 // dql.cu
 //
 // DynamicQuantizeLinear of a [rows, cols] matrix into rows of `pitch` bytes (a
@@ -54,6 +61,14 @@ int launch_dql_rows(const float *x, int64_t rows, int64_t cols, int64_t pitch, u
 bool dql_small_wanted(int64_t rows, int64_t pitch);
 int launch_dql_small(const float *x, int64_t rows, int64_t cols, int64_t pitch,
     uint8_t *y, int32_t *rowsum, float *y_scale, uint8_t *y_zp, cudaStream_t st);
+// Whether launch_dql_small takes a flat tensor of n values at all.  Up to four times
+// the size that is faster so, it serves calls for which the two passes are wrong:
+// one on a stream that is being captured, whose replays would write the partials to
+// a pool block that was given back, and one that writes onto x, which the second
+// pass reads again.
+bool dql_one_cluster_holds(int64_t n);
+bool dql_in_place(const float *x, int64_t n, const uint8_t *y, const float *y_scale,
+    const uint8_t *y_zp);
 
 // gemm_tc.cu / gemm_simt.cu
 //

@@ -311,3 +311,61 @@ def test_quantized_rows(gpu, orc, m, k, wt):
     want = (acc.astype(np.float32) * np.float32(np.float32(xs) * np.float32(0.0157))) + bias
     got = gpu.dyn_quant_linear(x, w, np.float32(0.0157), zp, bias, 0)
     assert got.tobytes() == want.astype(np.float32).tobytes()
+
+
+@pytest.mark.parametrize("n", [65537, 100001, 262144])
+def test_captured_dynamic_quantize_needs_no_pool(gpu, orc, n):
+    """Above the size that is fastest in one launch a captured call stays one all the
+    same: two passes would leave their partials in a pool block, which the replays
+    would write to after it was given back."""
+    import torch
+    rng = np.random.default_rng(n)
+    x = torch.empty(n, device="cuda")
+    y = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    s, z = torch.zeros((), device="cuda"), torch.zeros((), dtype=torch.uint8, device="cuda")
+    call = [gpu.Tensor.from_cuda_array(t) for t in (y, s, z, x)]
+    L = gpu.lib()
+    gpu.dynamic_quantize_linear(np.ones(n, np.float32))  # (kernels loaded, a free pool block)
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    try:
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            L.omcudaSetStream(stream.cuda_stream)
+            before = gpu.launch_count()
+            L.omcudaDynamicQuantizeLinear(*[t.handle for t in call])
+            launches = gpu.launch_count() - before
+    finally:
+        L.omcudaSetStream(None)
+    gpu.check()
+    assert launches == 1
+    for _ in range(2):
+        v = rng.normal(0.1, 3, size=n).astype(np.float32)
+        x.copy_(torch.from_numpy(v))
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        want_y, want_s, want_z = orc.dynamic_quantize_linear(v)
+        assert np.array_equal(y.cpu().numpy(), want_y)
+        assert s.item() == want_s and z.item() == want_z
+
+
+@pytest.mark.parametrize("n", [1000, 65537, 131072, 262144])
+@pytest.mark.parametrize("where", ["y", "y_end", "scalars"])
+def test_dynamic_quantize_onto_its_input(gpu, orc, n, where):
+    """Outputs in the memory of x, for sizes that one cluster holds."""
+    import torch
+    v = np.random.default_rng(n).normal(-0.2, 3, size=n).astype(np.float32)
+    xt = torch.from_numpy(v).cuda()
+    raw = xt.view(torch.uint8)
+    y = {"y": raw[:n], "y_end": raw[3 * n:], "scalars": torch.zeros(n, dtype=torch.uint8, device="cuda")}[where]
+    s, z = torch.zeros(1, device="cuda"), torch.zeros(1, dtype=torch.uint8, device="cuda")
+    if where == "scalars":
+        s, z = xt[n - 1:], raw[:1]
+    t = [gpu.Tensor.from_cuda_array(a) for a in (y, s, z, xt)]
+    torch.cuda.synchronize()
+    gpu.lib().omcudaDynamicQuantizeLinear(*[a.handle for a in t])
+    gpu.synchronize()
+    torch.cuda.synchronize()
+    want_y, want_s, want_z = orc.dynamic_quantize_linear(v)
+    assert np.array_equal(y.cpu().numpy(), want_y)
+    assert s.item() == want_s and z.item() == want_z
