@@ -904,7 +904,9 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
   g.N = d.N;
   g.K = d.K;
   g.lda = (d.K + 15) & ~int64_t(15);
-  if (d.K > 0 && linear_rows_wanted(d.M, d.N, g.lda)) {
+  // (one launch writes parts of Y while others still read X, so not onto X)
+  if (d.K > 0 && linear_rows_wanted(d.M, d.N, g.lda) &&
+      !ranges_overlap(dX, d.M * d.K * 4, dY, d.M * d.N * 4)) {
     if (wzn) {
       g.b_zp = dWz;
       g.b_zp_len = wzn;

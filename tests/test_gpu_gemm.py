@@ -844,3 +844,39 @@ def test_linear_of_few_rows(gpu, orc, m, k, n, wt, per_column, form):
         got = gpu.dyn_quant_linear(x, w, ws, zp, bias, form, device=device)
         got = got.numpy() if device else got
         assert got.tobytes() == want.astype(np.float32).tobytes()
+
+
+@pytest.mark.parametrize("m,k,n,at", [(2, 1024, 1024, 0), (8, 1024, 1024, 0), (16, 512, 512, 0), (4, 2048, 1000, 0),
+                                      (4, 1000, 1500, 500), (4, 1000, 1500, 3999), (3, 64, 64, 191)])
+def test_linear_onto_its_input(gpu, orc, m, k, n, at):
+    """Y in the memory of X, from element `at` of X on: X is read completely before Y
+    is written."""
+    import torch
+    rng = np.random.default_rng(m + k + n)
+    x = rng.normal(0.2, 2, size=(m, k)).astype(np.float32)
+    w = rng.integers(-127, 128, (k, n)).astype(np.int8)
+    xq, xs, xz = orc.dynamic_quantize_linear(x)
+    acc = (xq.astype(np.int64) - int(xz)) @ w.astype(np.int64)
+    want = acc.astype(np.float32) * (np.float32(xs) * np.float32(0.0157))
+    wd = gpu.Tensor.from_numpy(w).to_device()
+    ws = gpu.Tensor.from_numpy(np.array(0.0157, np.float32)).to_device()
+    L = gpu.lib()
+    L.omcudaRegisterConstant(wd.handle)
+    try:
+        for inside in (False, True, True):
+            buf = torch.zeros(at + 2 * m * max(k, n), device="cuda")
+            buf[:m * k] = torch.from_numpy(x.ravel()).cuda()
+            first = at if inside else m * k
+            xd = gpu.Tensor.from_cuda_array(buf[:m * k].view(m, k))
+            yd = gpu.Tensor.from_cuda_array(buf[first:first + m * n].view(m, n))
+            torch.cuda.synchronize()
+            before = gpu.launch_count()
+            L.omcudaDynQuantLinear(yd.handle, xd.handle, wd.handle, ws.handle, None, None, 0)
+            gpu.synchronize()
+            launches = gpu.launch_count() - before
+            got = buf[first:first + m * n].cpu().numpy().reshape(m, n)
+            assert got.tobytes() == want.astype(np.float32).tobytes()
+        assert launches == 2  # (quantize and product; the weight is prepared by now)
+    finally:
+        gpu.synchronize()
+        L.omcudaForgetConstants()
