@@ -92,10 +92,13 @@ __global__ void __launch_bounds__(kRangeThreads)
       hi = max3f(max3f(hi, v[u].x, v[u].y), v[u].z, v[u].w);
     }
   }
-  for (; j < n; j += nthreads) {
-    lo = fminf(lo, tail);
-    hi = fmaxf(hi, tail);
-    tail = j + nthreads < n ? __ldg(x + j + nthreads) : 0.0f;
+  lo = fminf(lo, tail);
+  hi = fmaxf(hi, tail);
+#pragma unroll 8
+  for (j += nthreads; j < n; j += nthreads) {
+    const float f = __ldg(x + j);
+    lo = fminf(lo, f);
+    hi = fmaxf(hi, f);
   }
   block_range<kRangeThreads>(lo, hi);
   if (threadIdx.x == 0)
@@ -167,29 +170,60 @@ struct QuantOutputs {
   }
 };
 
-// Scale and zero point are derived as DynamicQuantizeLinear does from `parts`
-// (count > 0: the reduction's partials) or from `range` (a producer's running
-// {min,max}, ordered-uint encoding, see f32_to_ordered), or are the given scale
-// and 8-bit zero point (zp8 may be null).
+// What a quantize pass takes its scale and zero point from: as DynamicQuantizeLinear
+// derives them from `parts` (count > 0: the reduction's partials) or from `range` (a
+// producer's running {min,max}, ordered-uint encoding, see f32_to_ordered), or
+// the given scale and 8-bit zero point (zp8 may be null).
+struct QuantSource {
+  RangeParts parts;
+  const uint32_t *range;
+  const float *scale;
+  const void *zp8;
+};
+template <bool kSigned>
+__device__ __forceinline__ QuantConsts quant_scalars(
+    const QuantSource &src, const QuantOutputs &outs, int mode) {
+  float scale, zp_f;
+  if (src.parts.count > 0 || src.range) {
+    // (every thread derives the same two scalars)
+    float lo, hi;
+    if (src.parts.count > 0) {
+      fold_parts(src.parts, lo, hi);
+    } else {
+      const uint32_t *range = after_pdl(src.range);
+      lo = ordered_to_f32(__ldg(range));
+      hi = ordered_to_f32(__ldg(range + 1));
+    }
+    dql_params_from_range(lo, hi, &scale, &zp_f, mode);
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+      outs.publish(scale, zp_f);
+  } else {
+    scale = __ldg(after_pdl(src.scale));
+    const void *zp8 = after_pdl(src.zp8);
+    if (!zp8)
+      zp_f = 0.0f;
+    else if (kSigned)
+      zp_f = (float)*reinterpret_cast<const int8_t *>(zp8);
+    else
+      zp_f = (float)*reinterpret_cast<const uint8_t *>(zp8);
+  }
+  return make_quant_consts<kSigned>(scale, zp_f, mode);
+}
+
+// x 16-byte and y 4-byte aligned.
 template <bool kSigned>
 __global__ void __launch_bounds__(kDqlThreads)
-    quantize_kernel(const float *__restrict__ x, int64_t n,
-        uint8_t *__restrict__ y, RangeParts parts,
-        const float *__restrict__ scale_ptr, const void *__restrict__ zp8,
-        const uint32_t *__restrict__ range, QuantOutputs outs, int mode, int unroll) {
+    quantize_kernel(const float *__restrict__ x, int64_t n, uint8_t *__restrict__ y,
+        QuantSource src, QuantOutputs outs, int mode, int unroll) {
   pdl_sync();
   x = after_pdl(x);
-  scale_ptr = after_pdl(scale_ptr);
-  zp8 = after_pdl(zp8);
-  range = after_pdl(range);
   // A block takes runs of unroll * 256 neighbouring float4 (16 KiB at most), the
   // loads of the first before it derives the scalars: three dependent divides
   // that a launch on a small tensor would otherwise spend before it asks for data.
   // Runs and not a stride of the whole grid, and only four loads in flight per
   // thread so that more blocks fit: 64 Mi values 67.0 -> 64.1 us, an encoder run of
   // 1 x 61 resident tokens 741 -> 659 us, of 32 x 128 1903 -> 1839.
-  const bool aligned = (((uintptr_t)x & 15u) == 0) && (((uintptr_t)y & 3u) == 0);
-  const int64_t n4 = aligned ? n >> 2 : 0;
+  const int64_t n4 = n >> 2;
   const float4 *x4 = reinterpret_cast<const float4 *>(x);
   uint32_t *y4 = reinterpret_cast<uint32_t *>(y);
   const int run = unroll * kDqlThreads;
@@ -199,34 +233,11 @@ __global__ void __launch_bounds__(kDqlThreads)
   for (int u = 0; u < kQuantUnroll; ++u)
     if (u < unroll && base + u * kDqlThreads < n4)
       v[u] = __ldcs(x4 + base + u * kDqlThreads);
-  // what is left of a word, or everything when the addresses are not aligned
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
-  int64_t j = (n4 << 2) + tid;
-  float tail = j < n ? __ldg(x + j) : 0.0f;
-  float scale, zp_f;
-  if (parts.count > 0 || range) {
-    // (every thread derives the same two scalars)
-    float lo, hi;
-    if (parts.count > 0) {
-      fold_parts(parts, lo, hi);
-    } else {
-      lo = ordered_to_f32(__ldg(range));
-      hi = ordered_to_f32(__ldg(range + 1));
-    }
-    dql_params_from_range(lo, hi, &scale, &zp_f, mode);
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-      outs.publish(scale, zp_f);
-  } else {
-    scale = __ldg(scale_ptr);
-    if (!zp8)
-      zp_f = 0.0f;
-    else if (kSigned)
-      zp_f = (float)*reinterpret_cast<const int8_t *>(zp8);
-    else
-      zp_f = (float)*reinterpret_cast<const uint8_t *>(zp8);
-  }
-  const QuantConsts qc = make_quant_consts<kSigned>(scale, zp_f, mode);
+  // what is left of a word
+  const int64_t rest = (n4 << 2) + threadIdx.x;
+  const bool takes_rest = blockIdx.x == 0 && rest < n;
+  const float last = takes_rest ? __ldg(x + rest) : 0.0f;
+  const QuantConsts qc = quant_scalars<kSigned>(src, outs, mode);
   while (base < n4) {
 #pragma unroll
     for (int u = 0; u < kQuantUnroll; ++u)
@@ -238,10 +249,32 @@ __global__ void __launch_bounds__(kDqlThreads)
       if (u < unroll && base + u * kDqlThreads < n4)
         v[u] = __ldcs(x4 + base + u * kDqlThreads);
   }
-  for (; j < n; j += nthreads) {
-    y[j] = (uint8_t)quantize_one<kSigned>(tail, qc);
-    tail = j + nthreads < n ? __ldg(x + j + nthreads) : 0.0f;
-  }
+  if (takes_rest)
+    y[rest] = (uint8_t)quantize_one<kSigned>(last, qc);
+}
+
+// The same one value at a time, for tensors that are not aligned so.  A kernel of
+// its own, as for dequantize: the loads of several trips together take registers
+// that the one above would miss (in it, 64 Mi aligned values went from 54 to 57 us),
+// and one value asked for ahead of the one in work is too little to hide memory
+// behind.  64 Mi values quantized 224 -> 131 us, dynamically 364 -> 179, 1 Mi 6.1 ->
+// 4.4 and 13.1 -> 9.8, on resident blocks (short ones 139, 187, 5.2 and 14.5).
+template <bool kSigned>
+__global__ void __launch_bounds__(kDqlThreads)
+    quantize_single_kernel(const float *__restrict__ x, int64_t n, uint8_t *__restrict__ y,
+        QuantSource src, QuantOutputs outs, int mode) {
+  pdl_sync();
+  x = after_pdl(x);
+  const int64_t step = (int64_t)gridDim.x * kDqlThreads;
+  int64_t j = (int64_t)blockIdx.x * kDqlThreads + threadIdx.x;
+  const float first = j < n ? __ldg(x + j) : 0.0f;
+  const QuantConsts qc = quant_scalars<kSigned>(src, outs, mode);
+  if (j >= n)
+    return;
+  y[j] = (uint8_t)quantize_one<kSigned>(first, qc);
+#pragma unroll 4
+  for (j += step; j < n; j += step)
+    y[j] = (uint8_t)quantize_one<kSigned>(__ldg(x + j), qc);
 }
 
 // The quantize pass by rows, written in the aligned rows the GEMM kernels take
@@ -581,22 +614,25 @@ static void launch_dequantize(const T *x, int64_t n, const float *scale, const T
 namespace {
 
 template <bool kSigned>
-int launch_quantize_pass(const float *x, int64_t n, uint8_t *y, const RangeParts &parts,
-    const float *scale, const void *zp, const uint32_t *range, const QuantOutputs &outs,
-    cudaStream_t st) {
+int launch_quantize_pass(const float *x, int64_t n, uint8_t *y, const QuantSource &src,
+    const QuantOutputs &outs, cudaStream_t st) {
   const int unroll = quant_unroll(n);
   // Behind the reduction: resident blocks, for each block folds all partials, and
   // set up while it runs, whatever the size (it holds no shared memory that
   // matters; 64 Mi values 115 us with short blocks, 106 with resident ones, 103
   // with the overlap).
-  const bool folds = parts.count > 0;
+  const bool folds = src.parts.count > 0;
   // (what a producer on the device has just left lies in L2 up to some 100 MB; a
   // caller's own tensor may come from anywhere)
-  const bool in_l2 = range && n <= ((int64_t)24 << 20);
-  const int grid = pass_grid(n, kDqlThreads * 4 * unroll, folds || in_l2);
-  OMCUDA_CHECK(launch_pdl(quantize_kernel<kSigned>, grid, kDqlThreads, 0, st, 0,
-      folds || pdl_pays(n),
-      x, n, y, parts, scale, zp, range, outs, quant_mode(), unroll));
+  const bool in_l2 = src.range && n <= ((int64_t)24 << 20);
+  const bool overlap = folds || pdl_pays(n);
+  if (((uintptr_t)x & 15u) == 0 && ((uintptr_t)y & 3u) == 0)
+    OMCUDA_CHECK(launch_pdl(quantize_kernel<kSigned>,
+        pass_grid(n, kDqlThreads * 4 * unroll, folds || in_l2), kDqlThreads, 0, st, 0, overlap,
+        x, n, y, src, outs, quant_mode(), unroll));
+  else
+    OMCUDA_CHECK(launch_pdl(quantize_single_kernel<kSigned>, grid_for(n, kDqlThreads * 4),
+        kDqlThreads, 0, st, 0, overlap, x, n, y, src, outs, quant_mode()));
   OMCUDA_CHECK_LAUNCH("quantize_kernel");
   return OMCUDA_OK;
 }
@@ -740,7 +776,7 @@ extern "C" int omcudaDevDynamicQuantizeLinear(const float *x, int64_t n,
   int rc = launch_range_parts(x, n, scratch, &parts, st);
   if (rc != OMCUDA_OK)
     return rc;
-  return launch_quantize_pass<false>(x, n, y, parts, nullptr, nullptr, nullptr,
+  return launch_quantize_pass<false>(x, n, y, QuantSource{parts, nullptr, nullptr, nullptr},
       QuantOutputs{nullptr, y_scale, y_zp}, st);
 }
 
@@ -762,8 +798,9 @@ extern "C" int omcudaDevQuantizeFromRange(const float *x, int64_t n, void *range
   cudaStream_t st = (cudaStream_t)stream;
   // One launch: every block derives the scalars from the range itself (a
   // block of its own when there is nothing to quantize).
-  return launch_quantize_pass<false>(x, n, y, RangeParts{nullptr, 0}, nullptr, nullptr,
-      (const uint32_t *)range, QuantOutputs{params, y_scale, y_zp}, st);
+  return launch_quantize_pass<false>(x, n, y,
+      QuantSource{RangeParts{nullptr, 0}, (const uint32_t *)range, nullptr, nullptr},
+      QuantOutputs{params, y_scale, y_zp}, st);
 }
 
 extern "C" int omcudaDevQuantizeLinear(const float *x, int64_t n, void *y,
@@ -773,11 +810,9 @@ extern "C" int omcudaDevQuantizeLinear(const float *x, int64_t n, void *y,
   if (n == 0)
     return OMCUDA_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const RangeParts none{nullptr, 0};
-  return y_signed ? launch_quantize_pass<true>(
-                        x, n, (uint8_t *)y, none, scale, zp, nullptr, QuantOutputs{}, st)
-                  : launch_quantize_pass<false>(
-                        x, n, (uint8_t *)y, none, scale, zp, nullptr, QuantOutputs{}, st);
+  const QuantSource src{RangeParts{nullptr, 0}, nullptr, scale, zp};
+  return y_signed ? launch_quantize_pass<true>(x, n, (uint8_t *)y, src, QuantOutputs{}, st)
+                  : launch_quantize_pass<false>(x, n, (uint8_t *)y, src, QuantOutputs{}, st);
 }
 
 extern "C" int omcudaDevDequantizeLinear(const void *x, int dtype, int64_t n,

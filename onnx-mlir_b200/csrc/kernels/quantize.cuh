@@ -143,6 +143,8 @@ __device__ __forceinline__ uint32_t quantize_four(float4 v, const QuantConsts &c
 
 template <bool kSigned>
 __device__ __forceinline__ uint32_t quantize_one(float x, const QuantConsts &c) {
+  if (!c.fast)
+    return quantize_one_exact<kSigned>(x, c.scale, c.zp_f, c.use_rcp);
   return quantize_four<kSigned>(make_float4(x, x, x, x), c) & 0xffu;
 }
 

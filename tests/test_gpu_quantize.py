@@ -369,3 +369,44 @@ def test_dynamic_quantize_onto_its_input(gpu, orc, n, where):
     want_y, want_s, want_z = orc.dynamic_quantize_linear(v)
     assert np.array_equal(y.cpu().numpy(), want_y)
     assert s.item() == want_s and z.item() == want_z
+
+
+@pytest.mark.parametrize("n", [1, 3, 255, 1025, 70001, 1300001])
+@pytest.mark.parametrize("xs,ys", [(1, 0), (2, 1), (3, 3), (0, 1), (0, 2), (0, 4)])
+def test_quantize_alignments(gpu, orc, n, xs, ys):
+    """Tensors that start anywhere, with scales that take the divide-free arithmetic
+    and one that does not; nothing beside the result is written."""
+    import torch
+    rng = np.random.default_rng(n + xs + 4 * ys)
+    v = rng.normal(0, 20, size=n).astype(np.float32)
+    xt = torch.zeros(n + 4, device="cuda")
+    xt[xs:xs + n] = torch.from_numpy(v).cuda()
+    xd = gpu.Tensor.from_cuda_array(xt[xs:xs + n])
+    L = gpu.lib()
+
+    def result(dtype):
+        buf = torch.full((n + 16,), 99, dtype=dtype, device="cuda")
+        return buf, gpu.Tensor.from_cuda_array(buf[ys:ys + n])
+
+    def check(buf, want):
+        got = buf.cpu().numpy()
+        assert np.array_equal(got[ys:ys + n], want)
+        assert (got[:ys] == 99).all() and (got[ys + n:] == 99).all()
+
+    for scale, zp in ((0.37, np.array(131, np.uint8)), (0.21, np.array(-3, np.int8)),
+                      (1e-33, np.array(7, np.uint8))):
+        buf, yd = result(getattr(torch, zp.dtype.name))
+        s, z = gpu.Tensor.from_numpy(np.array(scale, np.float32)), gpu.Tensor.from_numpy(zp)
+        torch.cuda.synchronize()
+        L.omcudaQuantizeLinear(yd.handle, xd.handle, s.handle, z.handle)
+        gpu.synchronize()
+        check(buf, orc.quantize(v, scale, float(zp), zp.dtype == np.int8))
+    buf, yd = result(torch.uint8)
+    s, z = torch.zeros((), device="cuda"), torch.zeros((), dtype=torch.uint8, device="cuda")
+    t = [gpu.Tensor.from_cuda_array(a) for a in (s, z)]
+    torch.cuda.synchronize()
+    L.omcudaDynamicQuantizeLinear(yd.handle, t[0].handle, t[1].handle, xd.handle)
+    gpu.synchronize()
+    want_y, want_s, want_z = orc.dynamic_quantize_linear(v)
+    check(buf, want_y)
+    assert s.item() == want_s and z.item() == want_z
