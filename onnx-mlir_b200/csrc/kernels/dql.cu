@@ -61,11 +61,18 @@ __device__ __forceinline__ void block_range(float &lo, float &hi) {
 
 // Bound by the read of x: 64 Mi values in 39 us (6.9 TB/s), 16 Mi that lie in L2 in
 // 6 (11 TB/s).  Plain loads and not streaming ones: the quantize pass finds in
-// L2 what still fits there.
+// L2 what still fits there.  kZero: sets the `zeros` words of `sums` to zero as well,
+// for a pass behind it that adds to them.
+template <bool kZero>
 __global__ void __launch_bounds__(kRangeThreads)
-    dql_minmax_kernel(const float *__restrict__ x, int64_t n, float2 *__restrict__ part) {
+    dql_minmax_kernel(const float *__restrict__ x, int64_t n, float2 *__restrict__ part,
+        int32_t *__restrict__ sums, int zeros) {
   pdl_sync();
   x = after_pdl(x);
+  if (kZero)
+    for (int i = blockIdx.x * kRangeThreads + threadIdx.x; i < zeros;
+         i += gridDim.x * kRangeThreads)
+      sums[i] = 0;
   float lo = INFINITY, hi = -INFINITY;
   const bool aligned = ((uintptr_t)x & 15u) == 0;
   const int64_t n4 = aligned ? n >> 2 : 0;
@@ -280,19 +287,20 @@ __global__ void __launch_bounds__(kDqlThreads)
 // The quantize pass by rows, written in the aligned rows the GEMM kernels take
 // (zero from cols up to pitch), with the sums of the quantized rows where the
 // weight has a zero point.  kWarps warps make a row at a time: one while that
-// keeps the machine busy, for there is nothing to wait for then, else a block.  A
-// thread makes one output word from four neighbouring values, four words in
-// flight.  The linear 777 x 1001 x 1537 22.6 -> 19.4 us
+// keeps the machine busy, for there is nothing to wait for then, else a block, and
+// where the rows are few, `split` blocks, whose sums are added up in memory that the
+// reduction has cleared.  A thread makes one output word from four neighbouring
+// values, four words in flight.  The linear 777 x 1001 x 1537 22.6 -> 19.4 us
 // together with the reduction above, 777 x 1024 x 1536 23.6 -> 15.7.
-template <int kWarps>
+constexpr int kRowsUnroll = 4;
+template <int kWarps, bool kSplit>
 __global__ void __launch_bounds__(kDqlThreads)
     quantize_rows_kernel(const float *__restrict__ x, int64_t rows, int cols, int pitch,
         uint8_t *__restrict__ y, int32_t *__restrict__ rowsum, RangeParts parts,
-        QuantOutputs outs, int vec_in, int mode) {
+        QuantOutputs outs, int vec_in, int split, int mode) {
   pdl_sync();
   x = after_pdl(x);
   constexpr int kThreads = 32 * kWarps, kRows = kDqlThreads / kThreads;
-  constexpr int kUnroll = 4;
   __shared__ int32_t part[kDqlThreads / 32];
   float lo, hi, scale, zp_f;
   fold_parts(parts, lo, hi);
@@ -302,16 +310,20 @@ __global__ void __launch_bounds__(kDqlThreads)
   const QuantConsts qc = make_quant_consts<false>(scale, zp_f, mode);
   const int t = threadIdx.x % kThreads, warp = threadIdx.x >> 5;
   const int words = pitch >> 2;
-  for (int64_t r = (int64_t)blockIdx.x * kRows + threadIdx.x / kThreads; r < rows;
-       r += (int64_t)gridDim.x * kRows) {
+  // (a split row: every grid has a block for each part of it)
+  const int step = kSplit ? split * kThreads : kThreads; // words apart
+  const int first = kSplit ? (int)(blockIdx.x % (unsigned)split) * kThreads + t : t;
+  for (int64_t r = kSplit ? (int64_t)(blockIdx.x / (unsigned)split)
+                          : (int64_t)blockIdx.x * kRows + threadIdx.x / kThreads;
+       r < rows; r += kSplit ? rows : (int64_t)gridDim.x * kRows) {
     const float *xr = x + r * cols;
     uint32_t *yr = reinterpret_cast<uint32_t *>(y + r * pitch);
     int32_t sum = 0;
-    for (int j0 = t; j0 < words; j0 += kUnroll * kThreads) {
-      float4 v[kUnroll];
+    for (int j0 = first; j0 < words; j0 += kRowsUnroll * step) {
+      float4 v[kRowsUnroll];
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
-        const int c = 4 * (j0 + u * kThreads), have = cols - c;
+      for (int u = 0; u < kRowsUnroll; ++u) {
+        const int c = 4 * (j0 + u * step), have = cols - c;
         v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (have >= 4 && vec_in) {
           v[u] = __ldcs(reinterpret_cast<const float4 *>(xr + c));
@@ -327,8 +339,8 @@ __global__ void __launch_bounds__(kDqlThreads)
         }
       }
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
-        const int j = j0 + u * kThreads, have = cols - 4 * j;
+      for (int u = 0; u < kRowsUnroll; ++u) {
+        const int j = j0 + u * step, have = cols - 4 * j;
         if (j >= words)
           break;
         uint32_t w = have > 0 ? quantize_four<false>(v[u], qc) : 0u;
@@ -353,7 +365,10 @@ __global__ void __launch_bounds__(kDqlThreads)
         int32_t s = 0;
         for (int w = 0; w < kDqlThreads / 32; ++w)
           s += part[w];
-        rowsum[r] = s;
+        if (kSplit)
+          atomicAdd(rowsum + r, s);
+        else
+          rowsum[r] = s;
       }
     }
   }
@@ -638,16 +653,16 @@ int launch_quantize_pass(const float *x, int64_t n, uint8_t *y, const QuantSourc
 }
 
 // DynamicQuantizeLinear's reduction alone.
-int launch_range_parts(
-    const float *x, int64_t n, void *scratch, RangeParts *parts, cudaStream_t st) {
+int launch_range_parts(const float *x, int64_t n, void *scratch, RangeParts *parts,
+    cudaStream_t st, int32_t *sums = nullptr, int zeros = 0) {
   float2 *part = scratch_parts(scratch);
   int64_t grid = ceil_div(n, (int64_t)kRangeThreads * 4);
   const int64_t cap = (int64_t)sm_count() * kRangeBlocksPerSm;
   grid = grid < 1 ? 1 : grid < cap ? grid : cap;
   if (grid > kRangeMaxParts)
     grid = kRangeMaxParts;
-  OMCUDA_CHECK(launch_pdl(dql_minmax_kernel, (unsigned)grid, kRangeThreads, 0, st, 0,
-      pdl_pays(n), x, n, part));
+  OMCUDA_CHECK(launch_pdl(sums ? dql_minmax_kernel<true> : dql_minmax_kernel<false>,
+      (unsigned)grid, kRangeThreads, 0, st, 0, pdl_pays(n), x, n, part, sums, zeros));
   OMCUDA_CHECK_LAUNCH("dql_minmax_kernel");
   parts->part = part;
   parts->count = (int)grid;
@@ -658,18 +673,30 @@ int launch_range_parts(
 
 int launch_dql_rows(const float *x, int64_t rows, int64_t cols, int64_t pitch, uint8_t *y,
     int32_t *rowsum, float *y_scale, uint8_t *y_zp, void *scratch, cudaStream_t st) {
+  const bool warps = rows >= (int64_t)sm_count() * 4;
+  // Few rows, long ones: about one block per SM, but none with less than the four
+  // words a thread keeps in flight.  u8 weights, N = 256: 1 x 100000 40 -> 21 us, 8 x
+  // 14336 19.8 -> 18.6, 16 x 14336 21.2 -> 19.8; two per SM cost 128 x 8192 0.5.
+  int64_t split = 1;
+  if (rows > 0 && rows < sm_count()) {
+    const int64_t most = ceil_div(pitch, kRowsUnroll * 4 * kDqlThreads);
+    split = sm_count() / rows;
+    split = split < most ? split : most > 0 ? most : 1;
+  }
   RangeParts parts;
-  int rc = launch_range_parts(x, rows * cols, scratch, &parts, st);
+  int rc = launch_range_parts(x, rows * cols, scratch, &parts, st,
+      split > 1 ? rowsum : nullptr, (int)rows);
   if (rc != OMCUDA_OK)
     return rc;
-  const bool warps = rows >= (int64_t)sm_count() * 4;
-  const int64_t blocks = warps ? ceil_div(rows, kDqlThreads / 32) : rows;
+  const int64_t blocks = warps ? ceil_div(rows, kDqlThreads / 32) : rows * split;
   const int64_t cap = (int64_t)sm_count() * 8;
   const int vec_in = ((uintptr_t)x & 15u) == 0 && cols % 4 == 0;
-  OMCUDA_CHECK(launch_pdl(warps ? quantize_rows_kernel<1> : quantize_rows_kernel<8>,
+  OMCUDA_CHECK(launch_pdl(warps       ? quantize_rows_kernel<1, false>
+                          : split > 1 ? quantize_rows_kernel<8, true>
+                                      : quantize_rows_kernel<8, false>,
       (unsigned)(blocks < cap ? blocks : cap), kDqlThreads, 0, st, 0, pdl_pays(rows * cols), x,
       rows, (int)cols, (int)pitch, y, rowsum, parts, QuantOutputs{nullptr, y_scale, y_zp},
-      vec_in, quant_mode()));
+      vec_in, (int)split, quant_mode()));
   OMCUDA_CHECK_LAUNCH("quantize_rows_kernel");
   return OMCUDA_OK;
 }

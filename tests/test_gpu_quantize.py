@@ -292,12 +292,13 @@ def test_pass_grid_wraps(gpu, orc, shift):
 
 @pytest.mark.parametrize("m,k", [(8, 1001), (9, 1001), (591, 1001), (592, 1001), (593, 1024), (591, 1024),
                                  (40, 8200), (5000, 67), (21, 4099),
-                                 (1, 16381), (4, 4096), (16, 1009)])
+                                 (1, 16381), (4, 4096), (16, 1009),
+                                 (1, 70001), (3, 40000), (16, 4112), (17, 8192), (74, 4113), (75, 4113)])
 @pytest.mark.parametrize("wt", [np.int8, np.uint8])
 def test_quantized_rows(gpu, orc, m, k, wt):
     """The quantize pass by rows inside a linear, with (unsigned weights with a zero
-    point) and without the rows' sums: one block's worth, a block and a warp per
-    row and the line between the two, rows that take wide loads and rows that do not."""
+    point) and without the rows' sums: one block's worth, several blocks, a block and a
+    warp per row and the lines between them, rows that take wide loads and rows that do not."""
     rng = np.random.default_rng(m * 7 + k)
     x = rng.normal(0.3, 2, size=(m, k)).astype(np.float32)
     n = 33
