@@ -25,6 +25,7 @@ namespace omcuda {
 
 static constexpr int kDqlThreads = 256;
 static constexpr int kQuantUnroll = 4;
+static constexpr int kSingleUnroll = 4; // values in flight where a thread takes single ones
 // The reduction's blocks, and so the partials every block of the pass behind it
 // folds: four of 512 threads fill an SM.
 static constexpr int kRangeThreads = 512;
@@ -264,8 +265,8 @@ __global__ void __launch_bounds__(kDqlThreads)
 // its own, as for dequantize: the loads of several trips together take registers
 // that the one above would miss (in it, 64 Mi aligned values went from 54 to 57 us),
 // and one value asked for ahead of the one in work is too little to hide memory
-// behind.  64 Mi values quantized 224 -> 131 us, dynamically 364 -> 179, 1 Mi 6.1 ->
-// 4.4 and 13.1 -> 9.8, on resident blocks (short ones 139, 187, 5.2 and 14.5).
+// behind.  64 Mi values quantized 224 -> 109 us, dynamically 365 -> 159, 1 Mi 6.1 ->
+// 3.5 and 13.1 -> 8.8, on resident blocks and with four loads together.
 template <bool kSigned>
 __global__ void __launch_bounds__(kDqlThreads)
     quantize_single_kernel(const float *__restrict__ x, int64_t n, uint8_t *__restrict__ y,
@@ -279,9 +280,17 @@ __global__ void __launch_bounds__(kDqlThreads)
   if (j >= n)
     return;
   y[j] = (uint8_t)quantize_one<kSigned>(first, qc);
-#pragma unroll 4
-  for (j += step; j < n; j += step)
-    y[j] = (uint8_t)quantize_one<kSigned>(__ldg(x + j), qc);
+  for (j += step; j < n; j += kSingleUnroll * step) {
+    float f[kSingleUnroll];
+#pragma unroll
+    for (int u = 0; u < kSingleUnroll; ++u)
+      if (j + u * step < n)
+        f[u] = __ldg(x + j + u * step);
+#pragma unroll
+    for (int u = 0; u < kSingleUnroll; ++u)
+      if (j + u * step < n)
+        y[j + u * step] = (uint8_t)quantize_one<kSigned>(f[u], qc);
+  }
 }
 
 // The quantize pass by rows, written in the aligned rows the GEMM kernels take
