@@ -62,12 +62,13 @@ __device__ __forceinline__ void block_range(float &lo, float &hi) {
 
 // Bound by the read of x: 64 Mi values in 39 us (6.9 TB/s), 16 Mi that lie in L2 in
 // 6 (11 TB/s).  Plain loads and not streaming ones: the quantize pass finds in
-// L2 what still fits there.  kZero: sets the `zeros` words of `sums` to zero as well,
+// L2 what still fits there.  kFull: the run is kRangeUnroll float4 a thread, known to
+// the compiler (64 Mi values 104 us the whole call without that, 101 with).  kZero: sets the `zeros` words of `sums` to zero as well,
 // for a pass behind it that adds to them.
-template <bool kZero>
+template <bool kFull, bool kZero>
 __global__ void __launch_bounds__(kRangeThreads)
     dql_minmax_kernel(const float *__restrict__ x, int64_t n, float2 *__restrict__ part,
-        int32_t *__restrict__ sums, int zeros) {
+        int unroll, int32_t *__restrict__ sums, int zeros) {
   pdl_sync();
   x = after_pdl(x);
   if (kZero)
@@ -84,16 +85,17 @@ __global__ void __launch_bounds__(kRangeThreads)
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
   int64_t j = (n4 << 2) + tid;
   float tail = j < n ? __ldg(x + j) : 0.0f;
-  constexpr int kRun = kRangeUnroll * kRangeThreads;
-  for (int64_t base = (int64_t)blockIdx.x * kRun + threadIdx.x; base < n4;
-       base += (int64_t)gridDim.x * kRun) {
+  const int run = (kFull ? kRangeUnroll : unroll) * kRangeThreads;
+  for (int64_t base = (int64_t)blockIdx.x * run + threadIdx.x; base < n4;
+       base += (int64_t)gridDim.x * run) {
     // (what lies past the end counts as zero, which changes neither scalar: the
     // range is widened to hold 0 before anything is derived from it)
     float4 v[kRangeUnroll];
 #pragma unroll
     for (int u = 0; u < kRangeUnroll; ++u)
-      v[u] = base + u * kRangeThreads < n4 ? __ldg(x4 + base + u * kRangeThreads)
-                                           : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      v[u] = (kFull || u < unroll) && base + u * kRangeThreads < n4
+                 ? __ldg(x4 + base + u * kRangeThreads)
+                 : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
     for (int u = 0; u < kRangeUnroll; ++u) {
       lo = min3f(min3f(lo, v[u].x, v[u].y), v[u].z, v[u].w);
@@ -665,13 +667,26 @@ int launch_quantize_pass(const float *x, int64_t n, uint8_t *y, const QuantSourc
 int launch_range_parts(const float *x, int64_t n, void *scratch, RangeParts *parts,
     cudaStream_t st, int32_t *sums = nullptr, int zeros = 0) {
   float2 *part = scratch_parts(scratch);
-  int64_t grid = ceil_div(n, (int64_t)kRangeThreads * 4);
+  // Runs of one to eight float4 a thread, so that about a third of the SMs has a
+  // block until those are full: no block without work, whose empty partial every
+  // block behind would fold.  1 Mi values (the whole call) 7.7 -> 5.3 us, 524288 5.7 ->
+  // 5.1, 98304 4.5 -> 4.3 against runs of eight and a block per 2048 values, most of
+  // them empty.  With a block per SM the call alone gains as much (5.2), but what is
+  // set up behind loses: linear 777 x 1001 x 1537 20.3 so, 19.4 with one per SM, 18.7.
+  const int64_t per = ceil_div(n, (int64_t)(sm_count() / 3) * kRangeThreads * 4);
+  const int unroll = (int)(per < 1 ? 1 : per < kRangeUnroll ? per : kRangeUnroll);
+  const bool aligned = ((uintptr_t)x & 15u) == 0; // (else four single values a thread)
+  int64_t grid = ceil_div(n, (int64_t)kRangeThreads * 4 * (aligned ? unroll : 1));
   const int64_t cap = (int64_t)sm_count() * kRangeBlocksPerSm;
   grid = grid < 1 ? 1 : grid < cap ? grid : cap;
   if (grid > kRangeMaxParts)
     grid = kRangeMaxParts;
-  OMCUDA_CHECK(launch_pdl(sums ? dql_minmax_kernel<true> : dql_minmax_kernel<false>,
-      (unsigned)grid, kRangeThreads, 0, st, 0, pdl_pays(n), x, n, part, sums, zeros));
+  const bool full = unroll == kRangeUnroll;
+  OMCUDA_CHECK(launch_pdl(full ? (sums ? dql_minmax_kernel<true, true>
+                                       : dql_minmax_kernel<true, false>)
+                               : (sums ? dql_minmax_kernel<false, true>
+                                       : dql_minmax_kernel<false, false>),
+      (unsigned)grid, kRangeThreads, 0, st, 0, pdl_pays(n), x, n, part, unroll, sums, zeros));
   OMCUDA_CHECK_LAUNCH("dql_minmax_kernel");
   parts->part = part;
   parts->count = (int)grid;
