@@ -1420,9 +1420,13 @@ int launch_bn_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan =
 
 // A long K loop hides the epilogue behind the MMAs and wants pipeline depth;
 // a short one is bounded by the epilogue and wants more warps on it, except for
-// raw sums, which leave no arithmetic to share (16384 x 1024 x 4096: 70 us with eight
-// warps, 85 with sixteen, whose slabs take a stage of the operand ring).
+// raw sums that leave by line stores, which have no arithmetic to share (16384 x
+// 1024 x 4096: 70 us with eight warps, 85 with sixteen, whose slabs take a stage of
+// the operand ring).  Rows of a ragged N leave one by one, and that is work to
+// share (raw sums 4096 x 1001 x 1537 with zero points: 39.5 us with eight, 32.8 with
+// sixteen).
 // (OMCUDA_GEMM_EW=8|16 overrides the choice, for experiments.)
+template <int EPI>
 inline bool want_wide_epilogue(const GemmCall &a) {
   static const int forced = [] {
     const char *s = getenv("OMCUDA_GEMM_EW");
@@ -1430,15 +1434,15 @@ inline bool want_wide_epilogue(const GemmCall &a) {
   }();
   if (forced == 8 || forced == 16)
     return forced == 16;
-  return a.K < 2048;
+  return a.K < 2048 && !(EPI == OMCUDA_EPI_I32 && y_takes_line_stores<EPI>(a));
 }
 
 template <int BN, int EPI>
 int launch_bn_epi(const GemmCall &a, cudaStream_t st) {
   // (tiles of 64 columns have no work for more than eight warps)
-  constexpr int kWide = BN == 64 || EPI == OMCUDA_EPI_I32 ? 8 : 16;
-  return want_wide_epilogue(a) ? launch_bn_epi_ew<BN, EPI, kWide>(a, st)
-                               : launch_bn_epi_ew<BN, EPI, 8>(a, st);
+  constexpr int kWide = BN == 64 ? 8 : 16;
+  return want_wide_epilogue<EPI>(a) ? launch_bn_epi_ew<BN, EPI, kWide>(a, st)
+                                    : launch_bn_epi_ew<BN, EPI, 8>(a, st);
 }
 
 template <int BN>
@@ -1551,9 +1555,8 @@ int launch_pair_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan
 
 template <int EPI>
 int launch_pair_epi(const GemmCall &a, cudaStream_t st) {
-  constexpr int kWide = EPI == OMCUDA_EPI_I32 ? 8 : 16;
-  return want_wide_epilogue(a) ? launch_pair_epi_ew<EPI, kWide>(a, st)
-                               : launch_pair_epi_ew<EPI, 8>(a, st);
+  return want_wide_epilogue<EPI>(a) ? launch_pair_epi_ew<EPI, 16>(a, st)
+                                    : launch_pair_epi_ew<EPI, 8>(a, st);
 }
 
 int launch_pair(const GemmCall &a, cudaStream_t st) {
