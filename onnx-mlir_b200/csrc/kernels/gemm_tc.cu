@@ -610,7 +610,8 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
         continue;
       }
       // slab word (r, j) sits at piece (j / 4) ^ (r % 8) of row r
-      __syncwarp(); // the block before has been read
+      if (kStep > 32)
+        __syncwarp(); // the block before has been read
 #pragma unroll
       for (int j = 0; j < (kBytesOut ? 2 : 8); ++j)
         st_shared_v4(slab0 + (uint32_t)lane * 128u + (uint32_t)((j ^ (lane & 7)) * 16),
