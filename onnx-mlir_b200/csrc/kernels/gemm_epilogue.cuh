@@ -42,7 +42,8 @@ struct EpiParams {
   int b_zp_len; // 0, 1, or N
   int b_signed;
   const int32_t *colsum; // [N]
-  const int32_t *rowsum; // [M], needed when b_zp_len != 0
+  const int32_t *rowsum; // [M], needed when b_zp_len != 0; where all of b_zp is zero
+                         // they may hold anything: used only in products with it
   int kind;              // omcudaEpilogue
   void *Y;
   const float *sa;

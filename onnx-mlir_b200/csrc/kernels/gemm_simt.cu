@@ -82,7 +82,8 @@ __global__ void __launch_bounds__(256)
 
 // QLinearMatMul's column scales (src/Conversion/ONNXToKrnl/Math/QLinearMatMul.cpp:123-138).
 __device__ __forceinline__ float requant_scale(const RequantScale &rq, int64_t i) {
-  return __fdiv_rn(__fmul_rn(*rq.a_scale, rq.b_scale[i]), *rq.y_scale);
+  const float *a = after_pdl(rq.a_scale), *b = after_pdl(rq.b_scale), *y = after_pdl(rq.y_scale);
+  return __fdiv_rn(__fmul_rn(*a, b[i]), *y);
 }
 
 // One warp per row, a 16-byte chunk per lane and trip; with dst, the row is also
@@ -93,9 +94,11 @@ __device__ __forceinline__ float requant_scale(const RequantScale &rq, int64_t i
 // (1 x 256 x 32768: 45 us a call so, 19 now).
 //
 // The sums serve the zero points of the weight, which are mostly all zero: with zp
-// (zp_len bytes), a block first looks at those and leaves without its sums, which
-// nothing reads then, if it finds nothing else.  QLinearMatMul 512 x 1024 x 1024 12.3
-// -> 8.3 us a call, together with the launch that overlaps; 16384 x 1024 x 4096 77 -> 72.
+// (zp_len bytes), a block first looks at those and leaves its sums as they are if it
+// finds nothing else.  The tails still load them, whatever they hold, and multiply
+// them by those zeros modulo 2^32.  QLinearMatMul 512 x 1024 x 1024 12.3 -> 8.3 us a
+// call, together with the launch that overlaps; 16384 x 1024 x 4096 with changing
+// inputs 100.2 -> 82.5, together with the GEMM's tail.
 template <bool kSigned>
 __global__ void __launch_bounds__(256)
     rowsum_kernel(const uint8_t *__restrict__ A, int64_t M, int64_t K,

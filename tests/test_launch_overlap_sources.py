@@ -12,7 +12,8 @@ CSRC = os.path.join(ROOT, "onnx-mlir_b200", "csrc")
 
 def sources():
     text = ""
-    for path in sorted(glob.glob(os.path.join(CSRC, "**", "*.cu*"), recursive=True)):
+    for path in sorted(p for kind in ("*.cu*", "*.h")
+                       for p in glob.glob(os.path.join(CSRC, "**", kind), recursive=True)):
         text += re.sub(r"//[^\n]*", "", open(path).read()) + "\n"
     return text
 
@@ -49,6 +50,16 @@ def const_pointer_members(text, struct):
     body, _ = block(text, m.end() - 1, "{", "}")
     return [name for decl in re.findall(r"\bconst\s+\w+\s*(\*[^;(]*);", body)
             for name in re.findall(r"\*\s*(\w+)", decl)]
+
+
+def functions_taking(text, struct):
+    """(argument name, body) of the kernels and device functions that take `struct`."""
+    for m in re.finditer(r"\b\w+\s*\((?=[^(){};]*\b%s\b)" % struct, text):
+        params, at = block(text, m.end() - 1, "(", ")")
+        brace = re.compile(r"\s*\{").match(text, at)
+        arg = re.search(r"\b%s\s*&?\s*(\w+)" % struct, params)
+        if brace and arg:
+            yield arg.group(1), block(text, brace.end() - 1, "{", "}")[0]
 
 
 def test_every_overlapped_kernel_waits():
@@ -89,6 +100,18 @@ def test_loads_depend_on_the_wait():
                     done = "after_pdl(%s.%s)" % (arg, member) in behind
                 if not done:
                     missing.append((name, "%s.%s" % (arg, member)))
+    # Blocks of arguments that device functions read for the kernel.
+    for struct in ("RequantScale", "RangeParts", "QuantSource"):
+        bodies = list(functions_taking(text, struct))
+        for member in const_pointer_members(text, struct):
+            wrapped = False
+            for arg, body in bodies:
+                read = r"%s\.%s\b" % (arg, member)
+                wrapped |= bool(re.search(r"after_pdl\(%s\)" % read, body))
+                if re.search(r"(?<![\w)])\*\s*%s|%s\s*\[|__ld\w+\(%s" % (read, read, read), body):
+                    missing.append((struct, member))
+            if not wrapped:
+                missing.append((struct, member))
     assert not missing, missing
     for name, members in (("epi_scalars", ("sa", "sb", "y_zp_dev")),
                           ("epi_quant_consts", ("q_range",))):
