@@ -32,7 +32,7 @@ constexpr int kRowsCluster = 8;   // CTAs that split K
 constexpr int kRowsThreads = 256; // eight warps, eight columns each
 constexpr int kRowsGroup = 64;    // columns a CTA takes at a time
 constexpr int kRowsUnroll = 8;    // 64-byte blocks of K in flight per warp
-constexpr int kRowsHeld = 8;      // words of x a thread keeps between its two looks
+constexpr int kRowsHeld = 5;      // words of x a thread keeps: all of its slice
 constexpr int kRowsMaxRounds = 8; // column groups per cluster
 constexpr int64_t kRowsMaxSmem = 100 * 1024; // two CTAs per SM
 
@@ -133,9 +133,6 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
 #pragma unroll
   for (int u = 0; u < kRowsHeld; ++u)
     fold(held[u]);
-#pragma unroll 4
-  for (int w = threadIdx.x + kRowsHeld * kRowsThreads; w < total; w += kRowsThreads)
-    fold(load(w));
   lo = warp_min(lo);
   hi = warp_max(hi);
   if (lane == 0) {
@@ -184,9 +181,6 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
     if (w < total)
       store(w, held[u]);
   }
-#pragma unroll 4
-  for (int w = threadIdx.x + kRowsHeld * kRowsThreads; w < total; w += kRowsThreads)
-    store(w, load(w));
   __syncthreads();
 
   // ---- products: rows 0..15 (those from M on are whatever the memory holds, and
@@ -296,10 +290,17 @@ bool linear_rows_wanted(int64_t M, int64_t N, int64_t kp) {
   // reads: 8 x 1024 x 1024 6.3 us here and 7.1 as two kernels, 16 x 256 x 256 5.8 and
   // 7.0, 2 x 8192 x 8192 17.2 and 19.6, 6 x 5000 x 12000 19.8 and 22.8, but 8 x 4096 x
   // 4096 10.1 and 9.5, 16 x 14336 x 4096 31 and 20.  One row is quantized so fast that
-  // the dp4a kernel behind it is as good (1 x 2048 x 2048: 6.2 and 5.9).
+  // the dp4a kernel behind it is as good (1 x 2048 x 2048: 6.2 and 5.9).  The line is
+  // drawn well inside: of 710 sizes up to 32768 values, weights in L2, it chooses none
+  // that the two kernels run more than 2 % faster, and leaves many to them that would
+  // be faster here (4 x 7000 x 300 7.9 and 12.2, 12 x 300 x 14336 10.9 and 14.4).
   if (M < 2 || M > kRowsMax || N > (int64_t)1 << 24)
     return false;
   if (M * kp > 16384 && (M * kp > 32768 || N < 1024 * M))
+    return false;
+  // A thread holds its part of the slice: up to 1200 words a CTA within the line above
+  // (15 x 2176), slices being rounded up to 64 values a row.
+  if (M * (rows_slice(kp) / 4) > kRowsHeld * kRowsThreads)
     return false;
   // More than one column group per cluster: not for weights of a few MB (4 x 768 x 3072:
   // 7.1 us here, 6.9 as two kernels).

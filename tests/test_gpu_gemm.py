@@ -822,8 +822,8 @@ def test_prepared_weight(gpu, k, n, signed):
 @pytest.mark.parametrize("form", [0, 1])
 def test_linear_of_few_rows(gpu, orc, m, k, n, wt, per_column, form):
     """Up to 16 rows in one launch, K split over a cluster: slices that are empty, that
-    end inside a 64-byte block, more of x than a thread keeps, several column groups
-    per cluster, and sizes that are left to the separate kernels."""
+    end inside a 64-byte block, several column groups per cluster, and sizes that are
+    left to the separate kernels (which is which: the test below)."""
     rng = np.random.default_rng(m * 31 + k + n)
     x = rng.normal(0.2, 2, size=(m, k)).astype(np.float32)
     w = rng.integers(-127, 128, (k, n)).astype(np.int8) if wt == np.int8 else \
@@ -877,6 +877,68 @@ def test_linear_onto_its_input(gpu, orc, m, k, n, at):
             got = buf[first:first + m * n].cpu().numpy().reshape(m, n)
             assert got.tobytes() == want.astype(np.float32).tobytes()
         assert launches == 2  # (quantize and product; the weight is prepared by now)
+    finally:
+        gpu.synchronize()
+        L.omcudaForgetConstants()
+
+
+@pytest.mark.parametrize("m,k,n,one", [
+    (2, 64, 64, True), (16, 1009, 65, True), (3, 1040, 128, True), (16, 1024, 1984, True),
+    (15, 2176, 15400, True),   # all five words of x that a thread can hold
+    (2, 16001, 2100, True), (2, 8192, 9000, True),  # several column groups per cluster
+    (1, 64, 64, False), (17, 64, 64, False), (24, 1001, 130, False), (4, 768, 3072, False),
+    (16, 1040, 96, False), (4, 8208, 5000, False), (16, 2048, 400, False)])
+@pytest.mark.parametrize("data", ["normal", "zero", "negative", "nan", "inf", "tiny"])
+def test_linear_of_few_rows_values(gpu, orc, m, k, n, one, data):
+    """One launch for a prepared weight or not, by the sizes, and either way the values
+    of the separate operators: activations that quantize with a scale of zero or
+    beyond the divide-free range, infinities and NaNs, rows that do not start on 16
+    bytes, and the modes without zero point and with the reciprocal."""
+    import torch
+    rng = np.random.default_rng(m * 31 + k + n)
+    x = rng.normal(0.2, 2, size=(m, k)).astype(np.float32)
+    if data == "zero":
+        x[:] = 0
+    elif data == "negative":
+        x = -np.abs(x) - 1
+    elif data == "nan":
+        x.ravel()[::61] = np.nan
+    elif data == "inf":
+        x.ravel()[m * k // 2] = np.inf
+    elif data == "tiny":
+        x *= np.float32(1e-35)
+    w = rng.integers(0, 256, (k, n)).astype(np.uint8)
+    zp = rng.integers(0, 256, n).astype(np.uint8)
+    ws = (rng.random(n) * 0.009 + 0.001).astype(np.float32)
+    wi = (w.astype(np.float64) - zp)
+    t = [gpu.Tensor.from_numpy(a).to_device() for a in (w, ws, zp)]
+    L = gpu.lib()
+    L.omcudaRegisterConstant(t[0].handle)
+    try:
+        for mode, shift in ((0, 0), (0, 1), (1, 0), (2, 0), (3, 0)):
+            buf = torch.zeros(m * k + 1, device="cuda")
+            buf[shift:shift + m * k] = torch.from_numpy(x.ravel()).cuda()
+            y = torch.zeros((m, n), device="cuda")
+            xd = gpu.Tensor.from_cuda_array(buf[shift:shift + m * k].view(m, k))
+            yd = gpu.Tensor.from_cuda_array(y)
+            torch.cuda.synchronize()
+            orc.L.orc_set_quant_mode(mode)
+            L.omcudaSetQuantizationMode(mode)
+            try:
+                xq, xs, xz = orc.dynamic_quantize_linear(x)
+                for _ in range(2):
+                    before = gpu.launch_count()
+                    L.omcudaDynQuantLinear(yd.handle, xd.handle, *[a.handle for a in t], None, 0)
+                    launches = gpu.launch_count() - before
+            finally:
+                L.omcudaSetQuantizationMode(0)
+                orc.L.orc_set_quant_mode(0)
+            gpu.synchronize()
+            assert (launches == 1) == one
+            acc = ((xq.astype(np.float64) - float(xz)) @ wi).astype(np.int64)  # exact: below 2^53
+            with np.errstate(invalid="ignore"):
+                want = acc.astype(np.float32) * (np.float32(xs) * ws)
+            assert np.array_equal(y.cpu().numpy(), want.astype(np.float32), equal_nan=True), (mode, shift)
     finally:
         gpu.synchronize()
         L.omcudaForgetConstants()
