@@ -301,8 +301,8 @@ __global__ void __launch_bounds__(kDqlThreads)
 // keeps the machine busy, for there is nothing to wait for then, else a block, and
 // where the rows are few, `split` blocks, whose sums are added up in memory that the
 // reduction has cleared.  A thread makes one output word from four neighbouring
-// values, four words in flight.  The linear 777 x 1001 x 1537 22.6 -> 19.4 us
-// together with the reduction above, 777 x 1024 x 1536 23.6 -> 15.7.
+// values, four words in flight.  The linear 777 x 1001 x 1537 22.5 -> 17.5 us
+// together with the reduction above, 777 x 1024 x 1536 19.8 -> 14.3.
 constexpr int kRowsUnroll = 4;
 template <int kWarps, bool kSplit>
 __global__ void __launch_bounds__(kDqlThreads)
@@ -763,7 +763,7 @@ int small_cluster_limit() {
 
 bool dql_small_wanted(int64_t rows, int64_t pitch) {
   // One word a thread, 65536 values in 16 CTAs: 8192 values 3.5 us, 32768 3.6, where
-  // two launches take 4.6 at any size up to 200 000.  With more words a thread the
+  // two launches take 4.4 at any size up to 200 000.  With more words a thread the
   // few SMs of one cluster lose to the whole machine: two, 131072 values, 5.0 us.
   const int64_t words = (int64_t)kSmallThreads * small_cluster_limit();
   return rows <= words && pitch <= 4 * words && rows * ceil_div(pitch, 4) <= words;
