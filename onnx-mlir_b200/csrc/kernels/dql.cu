@@ -702,7 +702,7 @@ int launch_dql_rows(const float *x, int64_t rows, int64_t cols, int64_t pitch, u
   // words a thread keeps in flight.  u8 weights, N = 256: 1 x 100000 40 -> 21 us, 8 x
   // 14336 19.8 -> 18.6, 16 x 14336 21.2 -> 19.8; two per SM cost 128 x 8192 0.5.
   int64_t split = 1;
-  if (rows > 0 && rows < sm_count()) {
+  if (rows > 0 && rows < sm_count() && pitch < (int64_t)1 << 30) { // (32-bit columns)
     const int64_t most = ceil_div(pitch, kRowsUnroll * 4 * kDqlThreads);
     split = sm_count() / rows;
     split = split < most ? split : most > 0 ? most : 1;
