@@ -489,6 +489,9 @@ int omcudaEncoderSetLayer(
  * output of the same shape and on the same side.  Returns NULL and sets errno
  * on failure. */
 OMTensorList *omcudaEncoderRun(omcudaEncoder *enc, OMTensorList *inputs);
+/* The same for host tensors with the output supplied by the caller: the HBM
+ * staging of x and y goes back to the pool when the call returns, y complete. */
+int omcudaEncoderRunHost(omcudaEncoder *enc, OMTensor *y, const OMTensor *x);
 /* The same with the output tensor supplied by the caller, as a krnl.call
  * callee receives it (outputs first, preallocated; src/Dialect/Krnl/Krnl.td:52-96):
  * x and y are f32 [batch, seq, hidden], each in host or device memory.  Host

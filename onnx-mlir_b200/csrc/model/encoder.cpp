@@ -698,6 +698,39 @@ int run_launches(omcudaEncoder *e, const float *x, int64_t batch, int64_t seq, f
 
 } // namespace
 
+namespace {
+
+// A run of host memory whose HBM staging goes back to the pool with the call (256 x 512
+// tokens of 1024 values: 1.07 GB that an encoder would otherwise sit on).  Complete when it
+// returns.
+int run_host(omcudaEncoder *e, const float *x, int64_t B, int64_t S, float *y, cudaStream_t st) {
+  const size_t bytes = (size_t)(B * S * e->cfg.hidden) * 4;
+  DevBuf dx, dy;
+  dx.ensure(bytes);
+  dy.ensure(bytes);
+  int rc = OMCUDA_OK;
+  if (!dx.p || !dy.p)
+    rc = sticky_error() ? omcudaGetLastError()
+                        : fail(OMCUDA_ENOMEM, "EncoderRun: allocation failed");
+  if (rc == OMCUDA_OK)
+    rc = check_cuda(
+        cudaMemcpyAsync(dx.p, x, bytes, cudaMemcpyHostToDevice, st), "encoder: H2D");
+  if (rc == OMCUDA_OK)
+    rc = omcudaEncoderRunDev(e, (const float *)dx.p, B, S, (float *)dy.p, st);
+  if (rc == OMCUDA_OK)
+    rc = check_cuda(
+        cudaMemcpyAsync(y, dy.p, bytes, cudaMemcpyDeviceToHost, st), "encoder: D2H");
+  if (rc == OMCUDA_OK) {
+    omcudaSynchronize();
+    rc = omcudaGetLastError();
+  }
+  dx.release();
+  dy.release();
+  return rc;
+}
+
+} // namespace
+
 extern "C" OMTensorList *omcudaEncoderRun(omcudaEncoder *e, OMTensorList *inputs) {
   if (sticky_error() || ensure_init() != OMCUDA_OK)
     return nullptr;
@@ -715,7 +748,6 @@ extern "C" OMTensorList *omcudaEncoderRun(omcudaEncoder *e, OMTensorList *inputs
     return nullptr;
   }
   const int64_t B = omTensorGetShape(x)[0], S = omTensorGetShape(x)[1];
-  const int64_t n = B * S * e->cfg.hidden;
   cudaStream_t st = current_stream();
   const bool on_dev = omcudaTensorIsOnDevice(x) != 0;
   OMTensor *out = nullptr;
@@ -729,30 +761,14 @@ extern "C" OMTensorList *omcudaEncoderRun(omcudaEncoder *e, OMTensorList *inputs
       return nullptr;
     }
   } else {
-    DevBuf dx, dy;
-    dx.ensure((size_t)n * 4);
-    dy.ensure((size_t)n * 4);
     out = omTensorCreateEmpty(omTensorGetShape(x), 3, ONNX_TYPE_FLOAT);
-    bool ok = dx.p && dy.p && out;
-    ok = ok && check_cuda(cudaMemcpyAsync(dx.p, omTensorGetDataPtr(x),
-                              (size_t)n * 4, cudaMemcpyHostToDevice, st),
-                   "encoder: H2D") == OMCUDA_OK;
-    ok = ok && omcudaEncoderRunDev(e, (const float *)dx.p, B, S, (float *)dy.p,
-                   st) == OMCUDA_OK;
-    ok = ok && check_cuda(cudaMemcpyAsync(omTensorGetDataPtr(out), dy.p,
-                              (size_t)n * 4, cudaMemcpyDeviceToHost, st),
-                   "encoder: D2H") == OMCUDA_OK;
-    if (ok) {
-      omcudaSynchronize();
-      ok = !sticky_error();
+    if (!out) {
+      fail(OMCUDA_ENOMEM, "EncoderRun: host allocation failed");
+      return nullptr;
     }
-    dx.release();
-    dy.release();
-    if (!ok) {
-      if (out)
-        omTensorDestroy(out);
-      if (!sticky_error())
-        fail(OMCUDA_ENOMEM, "EncoderRun: allocation failed");
+    if (run_host(e, (const float *)omTensorGetDataPtr(x), B, S,
+            (float *)omTensorGetDataPtr(out), st) != OMCUDA_OK) {
+      omTensorDestroy(out);
       return nullptr;
     }
   }
@@ -763,6 +779,27 @@ extern "C" OMTensorList *omcudaEncoderRun(omcudaEncoder *e, OMTensorList *inputs
     return nullptr;
   }
   return res;
+}
+
+extern "C" int omcudaEncoderRunHost(
+    omcudaEncoder *e, OMTensor *y, const OMTensor *x) {
+  if (sticky_error())
+    return omcudaGetLastError();
+  int rc = ensure_init();
+  if (rc != OMCUDA_OK)
+    return rc;
+  if (!e || !x || !y || omTensorGetDataType(x) != ONNX_TYPE_FLOAT ||
+      omTensorGetDataType(y) != ONNX_TYPE_FLOAT || omTensorGetRank(x) != 3 ||
+      omTensorGetRank(y) != 3 || omTensorGetShape(x)[2] != e->cfg.hidden)
+    return fail(OMCUDA_EINVAL, "EncoderRunHost: x and y must be f32 [batch, seq, hidden]");
+  for (int i = 0; i < 3; ++i)
+    if (omTensorGetShape(x)[i] != omTensorGetShape(y)[i])
+      return fail(OMCUDA_EINVAL, "EncoderRunHost: y must have the shape of x");
+  if (omcudaTensorIsOnDevice(x) || omcudaTensorIsOnDevice(y))
+    return fail(OMCUDA_EINVAL,
+        "EncoderRunHost: host tensors only (device tensors: omcudaEncoderRunInto)");
+  return run_host(e, (const float *)omTensorGetDataPtr(x), omTensorGetShape(x)[0],
+      omTensorGetShape(x)[1], (float *)omTensorGetDataPtr(y), current_stream());
 }
 
 extern "C" int omcudaEncoderRunInto(

@@ -496,17 +496,22 @@ class Encoder:
                 raise OmcudaError(rc, "omcudaEncoderSetLayer failed")
 
     def run(self, x):
-        """run_main_graph: numpy [B,S,H] in, numpy out (staged through HBM), or
-        a device Tensor in, device Tensor out."""
+        """run_main_graph: numpy [B,S,H] in, numpy out (staged through HBM that goes
+        back to the library's pool with the call), or a device Tensor in, device
+        Tensor out."""
+        L = lib()
         if not isinstance(x, Tensor):
             # The library copies into the array that is returned: the output it would
             # make itself had to be copied once more, into memory as cold (batch 4 x 512
             # tokens, 6 MB: 2520 -> 1900 us).
             t = Tensor.from_numpy(np.asarray(x, np.float32))
             out = Tensor.empty(t.shape, np.float32)
-            self.run_into(t, out)
+            L.omcudaEncoderRunHost.argtypes = [ctypes.c_void_p] * 3
+            rc = L.omcudaEncoderRunHost(self.handle, out.handle, t.handle)
+            if rc != 0:
+                check()
+                raise OmcudaError(rc, "omcudaEncoderRunHost failed")
             return out.numpy()
-        L = lib()
         arr = (ctypes.c_void_p * 1)(x.handle)
         ins = L.omTensorListCreate(arr, 1)
         outs = L.omcudaEncoderRun(self.handle, ins)
@@ -520,7 +525,8 @@ class Encoder:
 
     def run_into(self, x, y):
         """run_main_graph with the caller's output: x, y are Tensors (host or
-        device) of shape [B,S,H]; y is filled in place."""
+        device) of shape [B,S,H]; y is filled in place.  The encoder keeps the HBM
+        staging of host Tensors."""
         L = lib()
         L.omcudaEncoderRunInto.argtypes = [ctypes.c_void_p] * 3
         rc = L.omcudaEncoderRunInto(self.handle, y.handle, x.handle)

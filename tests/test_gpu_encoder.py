@@ -236,3 +236,28 @@ def test_ragged_sequence_alone_equals_many(gpu, S, B):
     many = enc.run(np.repeat(x, B, axis=0))
     assert many.tobytes() == np.repeat(one, B, axis=0).tobytes()
     enc.close()
+
+
+def test_run_of_host_arrays_gives_its_staging_back(gpu):
+    # run() stages a numpy batch through HBM for the length of the call: two tensors of
+    # the batch's size find their memory in the pool afterwards, with the encoder alive.
+    import torch
+    H, heads, F, B, S = 128, 2, 256, 512, 130
+    enc = gpu.Encoder(H, heads, F, make_encoder(29, H, F, 1))
+    x = np.random.default_rng(30).normal(size=(B, S, H)).astype(np.float32)
+    y = enc.run(x)
+    free = torch.cuda.mem_get_info()[0]
+    kept = [gpu.Tensor.device_empty(x.shape, np.float32) for _ in range(2)]
+    assert free - torch.cuda.mem_get_info()[0] < x.nbytes
+    # the array is the caller's: the next run does not write to it
+    before = y.copy()
+    enc.run(2 * x)
+    assert np.array_equal(y, before)
+    z = np.zeros_like(x)
+    enc.run_into(gpu.Tensor.from_numpy(x), gpu.Tensor.from_numpy(z))
+    assert z.tobytes() == y.tobytes()
+    with pytest.raises(gpu.OmcudaError) as ei:
+        enc.run(x[0])
+    assert ei.value.code == gpu.EINVAL
+    del kept
+    enc.close()
