@@ -203,7 +203,9 @@ void *dql_scratch_for(Stage &sg) { return sg.scratch((size_t)omcudaDevDqlScratch
 struct PreparedEntry {
   omcudaPreparedB pb;
   cudaStream_t stream; // where the prepare kernels ran
-  cudaEvent_t ready;   // recorded behind them
+  cudaEvent_t ready;   // recorded behind them; null: they have finished
+  bool captured;       // they were captured: the event must not be asked
+  bool done;           // the host has seen them finish
 };
 std::mutex g_const_mutex;
 std::set<const void *> g_const_ptrs;
@@ -214,11 +216,27 @@ bool is_registered_constant(const void *p) {
   return g_const_ptrs.count(p) != 0;
 }
 
+// Whether what the event was recorded behind has finished.  (A stream capture anywhere in the
+// process may forbid the question to a thread that has not relaxed its own mode.)
+bool event_passed(cudaEvent_t ev) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  const bool passed = cudaEventQuery(ev) == cudaSuccess;
+  (void)cudaGetLastError(); // cudaErrorNotReady is not an error
+  (void)cudaThreadExchangeStreamCaptureMode(&mode);
+  return passed;
+}
+
 // Returns a prepared form of B ([K,N], 8-bit).  `key_ptr` is the tensor's own
 // pointer (the cache key); `b_dev` the staged device copy.  A cache hit from a
 // stream other than the one that prepared the entry first waits for that
-// prepare to finish.  *settled (may be null): set when the entry was there and needed no
-// wait, for GemmCall::b_settled; else left alone.
+// prepare to finish.  *settled (may be null): set when the host has seen the entry's
+// prepare finish, for GemmCall::b_settled; else left alone.  That it was asked for on this
+// stream is not enough: with several threads on a stream the prepare can have been queued
+// between this call's own kernels, right in front of the GEMM that reads ahead.
 int prepared_b(Stage &sg, const void *key_ptr, const void *b_dev, int b_signed,
     int64_t K, int64_t N, cudaStream_t st, omcudaPreparedB *out, bool *settled = nullptr) {
   bool cacheable = is_registered_constant(key_ptr);
@@ -227,12 +245,14 @@ int prepared_b(Stage &sg, const void *key_ptr, const void *b_dev, int b_signed,
     std::lock_guard<std::mutex> lock(g_const_mutex);
     auto it = g_prepared.find(key);
     if (it != g_prepared.end()) {
-      const bool wait = it->second.stream != st && it->second.ready;
-      if (wait)
-        OMCUDA_CHECK(cudaStreamWaitEvent(st, it->second.ready, 0));
-      if (settled)
-        *settled = !wait;
-      *out = it->second.pb;
+      PreparedEntry &e = it->second;
+      if (e.stream != st && e.ready)
+        OMCUDA_CHECK(cudaStreamWaitEvent(st, e.ready, 0));
+      if (settled) {
+        e.done = e.done || (!e.captured && !is_capturing(st) && (!e.ready || event_passed(e.ready)));
+        *settled = e.done;
+      }
+      *out = e.pb;
       return OMCUDA_OK;
     }
   }
@@ -282,7 +302,7 @@ int prepared_b(Stage &sg, const void *key_ptr, const void *b_dev, int b_signed,
       if (ev)
         cudaEventDestroy(ev);
     } else {
-      g_prepared[key] = PreparedEntry{pb, st, ev};
+      g_prepared[key] = PreparedEntry{pb, st, ev, is_capturing(st), false};
     }
   }
   *out = pb;
@@ -955,7 +975,7 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
   g.a_signed = 0;
   if (sg.ok())
     sg.set(prepared_b(sg, omTensorGetDataPtr(Wq), dW, wt == ONNX_TYPE_INT8, d.K,
-        d.N, st, &g.B, &g.b_settled));
+        d.N, st, &g.B, gemm_few_wanted(d.M, d.N, d.K) ? &g.b_settled : nullptr));
   g.a_zp = xz;
   g.a_zp_len = 1;
   g.epilogue = OMCUDA_EPI_DEQUANT;

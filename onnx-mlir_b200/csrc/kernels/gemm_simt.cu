@@ -847,7 +847,8 @@ extern "C" int omcudaDevPrepareB(const void *B, int b_signed, int64_t K,
       (const uint8_t *)B, K, N, kp, (uint8_t *)out->bt);
   OMCUDA_CHECK_LAUNCH("transpose_b_kernel");
   // Column sums of B are row sums of its copy (whose padding is zero): coalesced
-  // 16-byte loads of what has just been written, on the whole machine.
+  // 16-byte loads of what has just been written, on the whole machine.  (Last, and it
+  // does not write the copy: whoever is launched behind it with overlap may start once it has.)
   return launch_repitch(out->bt, b_signed, N, kp, 0, nullptr, out->colsum, RequantScale(), st);
 }
 

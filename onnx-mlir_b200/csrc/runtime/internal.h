@@ -85,8 +85,8 @@ struct GemmCall : omcudaGemmArgs {
   // output's type); null: y_zp.  Read by the kernel, so that the host never
   // waits for it.
   const uint8_t *y_zp_dev;
-  // B was prepared long ago: no kernel that may still be running when this GEMM is set
-  // up (the one right before it on the stream) writes it.
+  // The host has seen the preparation of B finish: no kernel that may still be running when
+  // this GEMM is set up writes it.
   bool b_settled;
   GemmCall() : omcudaGemmArgs(), lda(0), y_zp_dev(nullptr), b_settled(false) {}
   explicit GemmCall(const omcudaGemmArgs &a)

@@ -104,3 +104,48 @@ def test_concurrent_host_threads(gpu, orc):
         th.join()
     L.omcudaForgetConstants()
     assert not errors, errors[:5]
+
+
+def test_threads_of_one_stream_share_a_first_use(gpu, orc):
+    # Two host threads on the shared library stream whose first calls use the same fresh
+    # weight: the preparation one of them queues may stand between the other's quantize
+    # kernel and its product, which reads settled weights ahead of its wait.  Sizes of the
+    # few-rows kernel, several weights, several calls behind each.
+    L = gpu.lib()
+    rng = np.random.default_rng(5)
+    K, N, rounds = 1024, 768, 24
+    x = rng.normal(size=(48, K)).astype(np.float32)
+    dx = gpu.Tensor.from_numpy(x).to_device()
+    Ws = [rng.integers(-127, 128, (K, N), dtype=np.int8) for _ in range(rounds)]
+    tW = [gpu.Tensor.from_numpy(W).to_device() for W in Ws]
+    for t in tW:
+        L.omcudaRegisterConstant(t.handle)
+    gpu.synchronize()
+    barrier = threading.Barrier(2)
+    got, errors = [[None] * rounds, [None] * rounds], []
+
+    def worker(t):
+        try:
+            for i in range(rounds):
+                barrier.wait()
+                got[t][i] = [gpu.dyn_quant_linear(dx, tW[i], np.float32(0.01), None, None, 0,
+                                                  device=True) for _ in range(3)]
+            gpu.synchronize()
+        except Exception as exc:  # noqa: BLE001 - reported by the main thread
+            errors.append((t, repr(exc)))
+            barrier.abort()
+
+    threads = [threading.Thread(target=worker, args=(t,)) for t in range(2)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not errors, errors
+    xq, xs, xz = orc.dynamic_quantize_linear(x)
+    for i, W in enumerate(Ws):
+        acc = (xq.astype(np.int64) - int(xz)) @ W.astype(np.int64)
+        want = (acc.astype(np.float32) * (xs * np.float32(0.01))).astype(np.float32)
+        for t in range(2):
+            for y in got[t][i]:
+                assert y.numpy().tobytes() == want.tobytes(), (t, i)
+    L.omcudaForgetConstants()
