@@ -364,6 +364,10 @@ typedef struct {
 } omcudaGemmArgs;
 
 int omcudaDevGemmI8(const omcudaGemmArgs *args, void *stream);
+/* Whether kernel_choice 0 runs M x K x N products with 16-byte aligned rows of A and an i32,
+ * dequant, requant or split tail on the kernel for few rows (1, else 0; negative: error), and
+ * how: rows of A per tile, CTAs that share a tile's K loop. */
+int omcudaDevGemmFewPlan(int64_t M, int64_t N, int64_t K, int *rows, int *split);
 
 /* Bounded device-side waits.  Every wait of the tensor-core kernels (int8
  * GEMM, bf16 attention) on an mbarrier gives up after a limit -- two seconds

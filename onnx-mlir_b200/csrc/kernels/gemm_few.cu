@@ -587,6 +587,12 @@ bool gemm_few_wanted(int64_t M, int64_t N, int64_t K) {
   return M > 1 && (N >= 4800 || K >= 2304);
 }
 
+void gemm_few_plan(int64_t M, int64_t N, int64_t K, int *rows, int *split) {
+  const FewPlan plan = few_plan(M, N, K);
+  *rows = plan.t;
+  *split = plan.split;
+}
+
 bool gemm_few_supported(const GemmCall &a) {
   return (a.epilogue == OMCUDA_EPI_I32 || a.epilogue == OMCUDA_EPI_DEQUANT ||
              a.epilogue == OMCUDA_EPI_REQUANT || a.epilogue == OMCUDA_EPI_DEQUANT_SPLIT) &&

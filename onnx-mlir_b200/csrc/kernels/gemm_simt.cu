@@ -876,6 +876,23 @@ extern "C" int omcudaDevGemmI8(const omcudaGemmArgs *args, void *stream) {
   return gemm_i8(GemmCall(*args), (cudaStream_t)stream);
 }
 
+// Whether a product that the few-rows kernel can run goes there; otherwise it runs on the
+// 128- and 256-row tiles (use_tc), which a switch may have asked for, or the kernels for
+// at most 16 rows.
+static bool few_takes(int64_t M, int64_t N, int64_t K, bool use_tc) {
+  return gemm_few_wanted(M, N, K) && !(use_tc && gemm_tc_forced());
+}
+
+extern "C" int omcudaDevGemmFewPlan(int64_t M, int64_t N, int64_t K, int *rows, int *split) {
+  if (M <= 0 || N <= 0 || K <= 0 || !rows || !split)
+    return fail(OMCUDA_EINVAL, "GemmFewPlan: bad argument"), -1;
+  *rows = *split = 0;
+  if (!few_takes(M, N, K, M > gemv_max_m()))
+    return 0;
+  gemm_few_plan(M, N, K, rows, split);
+  return 1;
+}
+
 int omcuda::gemm_i8(const GemmCall &a, cudaStream_t st) {
   if (a.M < 0 || a.N <= 0 || a.K <= 0 || !a.A || !a.B.bt ||
       (!a.Y && a.epilogue != OMCUDA_EPI_DEQUANT_RANGE))
@@ -917,12 +934,12 @@ int omcuda::gemm_i8(const GemmCall &a, cudaStream_t st) {
     return fail(OMCUDA_ENOTSUP,
         "GemmI8: the split-bf16, range-only and quantizing tails exist on the "
         "tensor-core kernel only (16-byte aligned rows of A)");
-  if (a.kernel_choice == 0 && gemm_few_supported(a) && gemm_few_wanted(a.M, a.N, a.K))
-    return launch_gemm_few(a, st);
   // With a handful of rows the GEMM is one read of the weight, which the
   // GEMV-shaped kernels stream faster than 128-row tensor-core tiles on a few
   // SMs (a row by 4096 x 14336: 14 us, on the few-rows kernel 15.3, on 128-row tiles 23-27).
-  bool use_tc = (a.kernel_choice == 1) || tc_only ||
-                (a.kernel_choice == 0 && tc_ok && a.M > gemv_max_m());
+  const bool use_tc = (a.kernel_choice == 1) || tc_only ||
+                      (a.kernel_choice == 0 && tc_ok && a.M > gemv_max_m());
+  if (a.kernel_choice == 0 && gemm_few_supported(a) && few_takes(a.M, a.N, a.K, use_tc))
+    return launch_gemm_few(a, st);
   return use_tc ? launch_gemm_tc(a, st) : launch_gemm_simt(a, st);
 }

@@ -1419,6 +1419,16 @@ int launch_bn_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan =
   return OMCUDA_OK;
 }
 
+// OMCUDA_GEMM_EW=8|16 overrides the choice below, for experiments; else 0.
+inline int forced_epilogue_warps() {
+  static const int v = [] {
+    const char *s = getenv("OMCUDA_GEMM_EW");
+    const int n = s ? atoi(s) : 0;
+    return n == 8 || n == 16 ? n : 0;
+  }();
+  return v;
+}
+
 // A long K loop hides the epilogue behind the MMAs and wants pipeline depth;
 // a short one is bounded by the epilogue and wants more warps on it, except for
 // raw sums that leave by line stores, which have no arithmetic to share (16384 x
@@ -1429,15 +1439,10 @@ int launch_bn_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan =
 // in work at a time) the last tile's epilogue has no MMAs to hide behind, however long
 // K is: 4096 x 3072 x 768 42.9 -> 41.3, 700 x 4096 x 4096 34.1 -> 32.3, 2048 x 8192 x 2304 70 -> 66,
 // but 4096 x 4096 x 4096, three and a half, 89.3 and 91.9.
-// (OMCUDA_GEMM_EW=8|16 overrides the choice, for experiments.)
 template <int EPI>
 inline bool want_wide_epilogue(const GemmCall &a, int64_t units, int64_t slots) {
-  static const int forced = [] {
-    const char *s = getenv("OMCUDA_GEMM_EW");
-    return s ? atoi(s) : 0;
-  }();
-  if (forced == 8 || forced == 16)
-    return forced == 16;
+  if (forced_epilogue_warps() != 0)
+    return forced_epilogue_warps() == 16;
   return (a.K < 2048 || units <= 2 * slots) &&
          !(EPI == OMCUDA_EPI_I32 && y_takes_line_stores<EPI>(a));
 }
@@ -1596,6 +1601,17 @@ inline int split_k_forced() {
   return v;
 }
 
+// OMCUDA_GEMM_BN=64|128|256 overrides the choice of the tile width, 512 selects the
+// 2-CTA kernel (experiments); else 0.
+inline int forced_tile_width() {
+  static const int v = [] {
+    const char *s = getenv("OMCUDA_GEMM_BN");
+    const int n = s ? atoi(s) : 0;
+    return n == 64 || n == 128 || n == 256 || n == 512 ? n : 0;
+  }();
+  return v;
+}
+
 // How many K slices a GEMM of up to 512 rows should run as (1: none).  The
 // partial pass uses 128 x 256 tiles on single CTAs up to 128 rows and 256 x
 // 256 tiles on CTA pairs above.  The second launch and the round trip of the
@@ -1673,14 +1689,13 @@ bool gemm_tc_supported(const GemmCall &a) {
          a.N < (int64_t(1) << 31);
 }
 
+bool gemm_tc_forced() {
+  return forced_tile_width() != 0 || forced_epilogue_warps() != 0 || split_k_forced() > 1;
+}
+
 int launch_gemm_tc(const GemmCall &a, cudaStream_t st) {
-  // Tile width: the widest tile that still gives every SM work
-  // (OMCUDA_GEMM_BN=64|128|256 overrides the choice, 512 selects the 2-CTA
-  // kernel, for experiments).
-  static const int forced_bn = [] {
-    const char *s = getenv("OMCUDA_GEMM_BN");
-    return s ? atoi(s) : 0;
-  }();
+  // Tile width: the widest tile that still gives every SM work.
+  const int forced_bn = forced_tile_width();
   if (forced_bn == 0 || split_k_forced() > 1) {
     const int split = split_k_for(a, st);
     if (split > 1)

@@ -94,9 +94,13 @@ struct GemmCall : omcudaGemmArgs {
 };
 int gemm_i8(const GemmCall &a, cudaStream_t st);
 bool gemm_tc_supported(const GemmCall &a);
+// A switch asks for a tile width, epilogue warps or slices of gemm_tc.cu.
+bool gemm_tc_forced();
 int launch_gemm_tc(const GemmCall &a, cudaStream_t st);
 // gemm_few.cu: few rows of A, on the tensor cores.
 bool gemm_few_wanted(int64_t M, int64_t N, int64_t K);
+// Rows per tile and CTAs per cluster that it would run with.
+void gemm_few_plan(int64_t M, int64_t N, int64_t K, int *rows, int *split);
 bool gemm_few_supported(const GemmCall &a);
 int launch_gemm_few(const GemmCall &a, cudaStream_t st);
 int launch_gemm_simt(const GemmCall &a, cudaStream_t st);

@@ -115,6 +115,18 @@ def gemm_i8(args, stream):
     _ok(_bind().omcudaDevGemmI8(ctypes.byref(args), stream))
 
 
+def gemm_few_plan(M, N, K):
+    """(rows per tile, CTAs per cluster) of the few-rows kernel where it is the choice
+    for such products, else None."""
+    rows, split = _i32(0), _i32(0)
+    L = _bind()
+    L.omcudaDevGemmFewPlan.argtypes = [_i64] * 3 + [ctypes.POINTER(_i32)] * 2
+    rc = L.omcudaDevGemmFewPlan(M, N, K, ctypes.byref(rows), ctypes.byref(split))
+    if rc < 0:
+        check()
+    return (rows.value, split.value) if rc == 1 else None
+
+
 def range_init(ranges, count, stream):
     L = _bind()
     L.omcudaDevRangeInit.argtypes = [_vp, _i64, _vp]
