@@ -96,11 +96,13 @@ def test_gemv_shaped_rows_1_to_32(gpu, orc, adt, bdt, choice):
 @pytest.mark.parametrize("M,K,N", [(17, 8192, 256), (100, 8208, 260), (128, 16384, 512),
                                    (129, 8192, 512), (300, 8208, 768), (512, 9216, 1024)])
 def test_split_k_shapes(gpu, orc, M, K, N):
-    # Up to 512 rows, with few output tiles and K of 8192 or more, the
-    # tensor-core kernels deal each tile's K loop to several work units (raw partial sums through a
+    # Up to 512 rows, with few output tiles and K of 8192 or more, the kernels of 128 and
+    # 256 rows deal each tile's K loop to several work units (raw partial sums through a
     # workspace, then one reduce pass with the real tail): on single CTAs up to
-    # 128 rows, on CTA pairs above.  All three tails against the oracle, every
-    # zero-point form, K not a multiple of the 128-byte K step.
+    # 128 rows, on CTA pairs above.  The raw sums of choice 1 run that way; choice 0 and
+    # the operators take the few-rows kernel at these sizes.  All three tails against the
+    # oracle, every zero-point form, K not a multiple of the 128-byte K step.  (The real
+    # tails of split sums: test_split_k_tails.)
     rng = np.random.default_rng(M + K + N)
     dg = DevGemm(gpu)
     for adt, bdt in [(np.uint8, np.int8), (np.int8, np.uint8)]:
@@ -458,15 +460,8 @@ def test_dequant_tail_with_residual(gpu, M, K, N, choice):
     assert y1.tobytes() == (y0 + res).astype(np.float32).tobytes()
 
 
-@pytest.mark.parametrize("M,K,N", [
-    (17, 16, 8), (17, 128, 128), (32, 144, 129), (33, 1040, 257), (64, 2064, 100), (65, 4096, 130),
-    (128, 14336, 72), (129, 640, 1000), (200, 3072, 260), (256, 4112, 3700), (640, 48, 240),
-    (16, 3600, 4801), (2, 16384, 4), (48, 64, 12300), (63, 1024, 520)])
-@pytest.mark.parametrize("adt,bdt", [(np.uint8, np.int8), (np.int8, np.uint8)])
-def test_few_rows_on_the_tensor_cores(gpu, M, K, N, adt, bdt):
-    """gemm_few.cu at the edges of its row tiles (16 to 128) and of its 128 columns,
-    with slices of K of one block and of uneven lengths and rows that no CTA of a
-    cluster owns: the sums against the exact product, every tail against the
+def check_few_rows(gpu, M, K, N, adt, bdt):
+    """The few-rows kernel's sums against the exact product, every tail against the
     128-row tensor-core kernel's, whose arithmetic is the same, bit for bit."""
     rng = np.random.default_rng(M + K + N)
     A, B = rand8(rng, (M, K), adt), rand8(rng, (K, N), bdt)
@@ -512,6 +507,79 @@ def test_few_rows_on_the_tensor_cores(gpu, M, K, N, adt, bdt):
             out.append((Y.numpy().tobytes(), ranges.numpy().tobytes() if "range" in extra else b""))
         gpu.synchronize()
         assert out[0] == out[1], (epi, form, extra)
+
+
+@pytest.mark.parametrize("M,K,N", [
+    (17, 16, 8), (17, 128, 128), (32, 144, 129), (33, 1040, 257), (64, 2064, 100), (65, 4096, 130),
+    (128, 14336, 72), (129, 640, 1000), (200, 3072, 260), (256, 4112, 3700), (640, 48, 240),
+    (16, 3600, 4801), (2, 16384, 4), (48, 64, 12300), (63, 1024, 520)])
+@pytest.mark.parametrize("adt,bdt", [(np.uint8, np.int8), (np.int8, np.uint8)])
+def test_few_rows_on_the_tensor_cores(gpu, M, K, N, adt, bdt):
+    """gemm_few.cu at the edges of its row tiles and of its 128 columns, with slices of K of
+    one block and of uneven lengths (tiles of 16 rows, and of 64 in two of them)."""
+    check_few_rows(gpu, M, K, N, adt, bdt)
+
+
+@pytest.mark.parametrize("rows,split,M,K,N", [
+    (16, 1, 223, 64, 4), (16, 2, 119, 320, 2), (16, 3, 33, 544, 2), (16, 4, 43, 992, 12),
+    (16, 6, 31, 2864, 4), (16, 8, 77, 4656, 4),
+    (32, 1, 21, 160, 4136), (32, 2, 17, 336, 490), (32, 3, 17, 608, 839), (32, 4, 594, 4176, 4),
+    (32, 6, 457, 4528, 1), (32, 8, 322, 7344, 1),
+    (64, 1, 591, 1296, 921), (64, 2, 618, 2544, 389), (64, 3, 575, 2784, 388),
+    (64, 4, 599, 4640, 129), (64, 6, 515, 8512, 130), (64, 8, 131, 9264, 385),
+    (128, 1, 581, 4208, 1855), (128, 2, 513, 6960, 1028), (128, 3, 500, 6608, 1029),
+    (128, 4, 625, 14032, 388), (128, 6, 386, 13488, 386), (128, 8, 71, 9600, 1208)])
+@pytest.mark.parametrize("adt,bdt", [(np.uint8, np.int8), (np.int8, np.uint8)])
+def test_few_rows_every_cut(gpu, rows, split, M, K, N, adt, bdt):
+    """Every row tile with every number of CTAs to its K loop, among them last tiles of one
+    to three rows, which most CTAs of the cluster own none of."""
+    from omcuda import dev
+    assert dev.gemm_few_plan(M, N, K) == (rows, split), "the plan moved: take other sizes"
+    check_few_rows(gpu, M, K, N, adt, bdt)
+
+
+@pytest.mark.parametrize("M,K,N,choice", [
+    (17, 8192, 256, 1), (100, 8208, 260, 1), (128, 16384, 512, 1), (129, 8192, 512, 1),
+    (300, 8208, 768, 1), (512, 9216, 1024, 1), (100, 14336, 2400, 0), (300, 14336, 2400, 0)])
+@pytest.mark.parametrize("adt,bdt", [(np.uint8, np.int8), (np.int8, np.uint8)])
+def test_split_k_tails(gpu, M, K, N, choice, adt, bdt):
+    """The dequantize and requantize tails behind split sums, on single CTAs (up to 128 rows)
+    and on pairs, with bias, per-column scales and zero points, against the same float
+    operations on the exact sums, bit for bit; two launches each, the sums and the tail."""
+    rng = np.random.default_rng(M + K + N)
+    A, B = rand8(rng, (M, K), adt), rand8(rng, (K, N), bdt)
+    zp_a, zp_b = rand8(rng, 1, adt), rand8(rng, N, bdt)
+    f32 = np.float32
+    # sums of at most 255^2 K: exact in float64, below 2^31
+    acc = ((A.astype(np.float64) - zp_a) @ (B.astype(np.float64) - zp_b)).astype(f32)
+    sb, bias = rng.uniform(1e-4, 1e-3, N).astype(f32), rng.normal(0, 0.5, N).astype(f32)
+    dg = DevGemm(gpu)
+    D = dg.dev
+    pb, keep = dg.prepare(B)
+    dA, az, bz = dg.dtensor(A), dg.dtensor(zp_a), dg.dtensor(zp_b)
+    rs = gpu.Tensor.device_empty((M,), np.int32)
+    D.row_sum(dA.data_ptr, int(adt == np.int8), M, K, rs.data_ptr, dg.stream)
+    dsa, dsb, dbias = dg.dtensor(np.array([0.013], f32)), dg.dtensor(sb), dg.dtensor(bias)
+    for epi in (D.EPI_DEQUANT, D.EPI_REQUANT):
+        g = D.GemmArgs()
+        g.M, g.N, g.K, g.A, g.a_signed, g.B = M, N, K, dA.data_ptr, int(adt == np.int8), pb
+        g.a_zp, g.a_zp_len = az.data_ptr, 1
+        g.b_zp, g.b_zp_len, g.a_rowsum = bz.data_ptr, N, rs.data_ptr
+        g.epilogue, g.kernel_choice = epi, choice
+        g.sa, g.sb, g.sb_len, g.y_zp = dsa.data_ptr, dsb.data_ptr, N, 7
+        if epi == D.EPI_DEQUANT:
+            g.bias = dbias.data_ptr
+        Y = gpu.Tensor.device_empty((M, N), np.uint8 if epi == D.EPI_REQUANT else f32)
+        g.Y = Y.data_ptr
+        before = gpu.launch_count()
+        D.gemm_i8(g, dg.stream)
+        assert gpu.launch_count() - before == 2
+        if epi == D.EPI_DEQUANT:
+            want = acc * (f32(0.013) * sb) + bias
+        else:
+            want = (np.rint(acc * sb).astype(np.int64) + 7).astype(np.uint8)
+        assert Y.numpy().tobytes() == want.tobytes()
+    gpu.synchronize()
 
 
 @pytest.mark.parametrize("K,N", [
@@ -572,10 +640,10 @@ def test_random_shapes_against_exact_products(gpu, seed):
 @pytest.mark.parametrize("seed", range(24))
 def test_random_few_rows_long_k_auto_dispatch(gpu, seed):
     # The dispatcher's small-M territory at random: 1..600 rows, K up to 16384,
-    # ragged N -- GEMV-shaped kernels (1..16 rows), split-K on single CTAs and
-    # on CTA pairs (K >= 8192, few tiles), narrow tiles, the 2-CTA kernel at
-    # three quarters occupancy.  Every output element against the exact integer
-    # product (float64 holds it exactly), per-row A zero points included.
+    # ragged N -- GEMV-shaped kernels (1..16 rows), the few-rows kernel and, for products
+    # it leaves, split-K (K >= 8192, few tiles), narrow tiles and the 2-CTA kernel.  Every
+    # output element against the exact integer product (float64 holds it exactly), per-row
+    # A zero points included.
     from gpu_util import DevGemm
     rng = np.random.default_rng(2000 + seed)
     M = int(rng.choice([1, 2, 3, 7, 8, 15, 16, 17, 31, 64, 100, 128, 129, 200, 256, 300,
@@ -587,7 +655,7 @@ def test_random_few_rows_long_k_auto_dispatch(gpu, seed):
         N = (N + 3) & ~3
     K = 16 * int(rng.integers(1, 1025))
     if seed % 4 == 1:
-        K = 16 * int(rng.integers(512, 1025))  # split-K territory
+        K = 16 * int(rng.integers(512, 1025))  # long K
     a_signed, b_signed = bool(rng.integers(0, 2)), bool(rng.integers(0, 2))
     A = rng.integers(-128 if a_signed else 0, 128 if a_signed else 256, (M, K)).astype(
         np.int8 if a_signed else np.uint8)
