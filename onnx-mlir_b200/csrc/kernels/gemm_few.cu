@@ -518,37 +518,43 @@ int launch_few_epi(const GemmCall &a, const FewPlan &plan, cudaStream_t st) {
 // such CTAs takes in us, fitted to 10000 launches (M 1 to 512, K and N 256 to 14336, all t
 // and split, weights in L2 or not): the choice takes 1.1 % more than the best one in the
 // mean, 18 % at most.
+// The search runs on the host in every call: 32-bit divisions, and none where one round of
+// CTAs does (128 x 768 x 768, 24 cuts: 0.54 -> 0.18 us of a 2.7 GHz core).
 FewPlan few_plan(int64_t M, int64_t N, int64_t K) {
-  const int64_t num_kb = ceil_div(K, kFewBK);
+  const uint32_t num_kb = (uint32_t)ceil_div(K, kFewBK);
+  const int64_t col_tiles = ceil_div(N, kFewCols);
+  const int sm = sm_count();
+  const auto ceil_few = [](int64_t a, int64_t b) { return a <= b ? 1 : ceil_div(a, b); };
   FewPlan best = {0, 0, 0};
   double least = 0.0;
   for (int t = 16; t <= 128 && (t == 16 || t < 2 * M); t *= 2) {
+    const int64_t tiles = col_tiles * ((uint32_t)(M + t - 1) / (uint32_t)t);
     for (int split : {1, 2, 3, 4, 6, 8}) {
-      if (split > num_kb)
+      if ((uint32_t)split > num_kb)
         break;
-      const int64_t ctas = ceil_div(N, kFewCols) * ceil_div(M, t) * split;
-      const int64_t kbs = ceil_div(num_kb, split);
+      const int64_t ctas = tiles * split;
+      const int kbs = (int)((num_kb + split - 1) / (uint32_t)split);
       // SMs that clusters find together: with one CTA to an SM 16 clusters of eight, 32 of
       // four or 46 of three do not always fit, and the launch takes two rounds (64 x
       // 1536 x 6144 in 48 clusters of three 17.5 us, of two 12.2).
-      const int64_t sms = sm_count() * (split > 2 ? 3 : 4) / 4 - (split == 2 ? 8 : 0);
-      const int64_t share = ceil_div(ctas, sms);
+      const int64_t sms = sm * (split > 2 ? 3 : 4) / 4 - (split == 2 ? 8 : 0);
       // Stages: as many as the slice has, while all CTAs that an SM gets (three at most:
       // registers) fit.
-      const int64_t wanted = share < 3 ? share : 3;
-      const int64_t steps = ceil_div(kbs, kFewBlocks);
-      int stages = (int)(steps < kFewMaxStages ? steps : kFewMaxStages);
+      const int64_t wanted = ctas <= sms ? 1 : ctas <= 2 * sms ? 2 : 3;
+      const int steps = (kbs + kFewBlocks - 1) / kFewBlocks;
+      int stages = steps < kFewMaxStages ? steps : kFewMaxStages;
+      const int64_t besides = few_besides(t, split) + 1024;
       int64_t smem;
       for (;; --stages) {
-        smem = few_ring(t, stages) + few_besides(t, split) + 1024;
+        smem = few_ring(t, stages) + besides;
         if (stages <= 1 || (smem <= kFewMaxSmem && smem * wanted <= kFewSmemPerSm))
           break;
       }
       if (smem > kFewMaxSmem)
         continue;
-      const int64_t fit = kFewSmemPerSm / smem < 3 ? kFewSmemPerSm / smem : 3;
-      const int64_t rounds = ceil_div(ctas, sms * fit);
-      const double per_sm = (double)ceil_div(ceil_div(ctas, rounds), sm_count());
+      const int64_t fit = 3 * smem <= kFewSmemPerSm ? 3 : 2 * smem <= kFewSmemPerSm ? 2 : 1;
+      const int64_t rounds = ceil_few(ctas, sms * fit);
+      const double per_sm = (double)ceil_few(rounds == 1 ? ctas : ceil_div(ctas, rounds), sm);
       const double load = per_sm * kbs * (16.0 + t / 8.0) * 0.0014; // KiB
       const double mma = per_sm * kbs * 0.07;
       const double chain = steps * 0.109 * (1.0 + 3.86 / stages);

@@ -1,6 +1,7 @@
 """Which products the kernel for few rows takes, and that the switches which name a tile
 width, epilogue warps or a number of slices of the other tensor-core kernels reach those."""
 import os
+import random
 import subprocess
 import sys
 
@@ -64,3 +65,46 @@ print(omcuda.launch_count() - before,
 """ % os.path.join(ROOT, "tests")
     assert child(code, OMCUDA_GEMM_SPLIT_K="2") == ["2", "True"]
     assert child(code) == ["1", "True"]
+
+
+def cheapest_cut(M, N, K, sms=148):
+    """The cut with the least estimate (whole ceilings, no shortcuts)."""
+    ceil = lambda a, b: -(-a // b)
+    kb, best = ceil(K, 128), None
+    for t in (16, 32, 64, 128):
+        if t > 16 and t >= 2 * M:
+            break
+        for split in (1, 2, 3, 4, 6, 8):
+            if split > kb:
+                break
+            ctas, kbs = ceil(N, 128) * ceil(M, t) * split, ceil(kb, split)
+            found = sms * (3 if split > 2 else 4) // 4 - (8 if split == 2 else 0)
+            steps = ceil(kbs, 2)
+            besides = 2048 + (split * ceil(t, split) * 512 if split > 1 else 0)
+            for stages in range(min(steps, 6), 0, -1):
+                smem = max(stages * 256 * (128 + t), t * 512) + besides
+                if smem <= 226 << 10 and smem * min(ceil(ctas, found), 3) <= 228 << 10:
+                    break
+            if smem > 226 << 10:
+                continue
+            rounds = ceil(ctas, found * min((228 << 10) // smem, 3))
+            per_sm = float(ceil(ceil(ctas, rounds), sms))
+            us = rounds * (max(per_sm * kbs * (16.0 + t / 8.0) * 0.0014, per_sm * kbs * 0.07,
+                               steps * 0.109 * (1.0 + 3.86 / stages)) +
+                           per_sm * min(t, M) * 0.0229) + ctas * 0.0037
+            if best is None or us < best[0]:
+                best = (us, t, split)
+    return best[1:]
+
+
+def test_the_plan_is_the_cheapest_cut(omcuda):
+    from omcuda import dev
+    rng, seen = random.Random(3), set()
+    for _ in range(6000):
+        M = rng.choice((rng.randint(2, 64), rng.randint(2, 640)))
+        K, N = rng.randint(1, rng.choice((600, 16384))), rng.randint(1, rng.choice((600, 16384, 1 << 20)))
+        plan = dev.gemm_few_plan(M, N, K)
+        if plan is not None:
+            seen.add(plan)
+            assert plan == cheapest_cut(M, N, K), (M, N, K)
+    assert len(seen) > 20
