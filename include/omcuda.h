@@ -341,10 +341,10 @@ typedef struct {
   void *out_minmax;
   /* 0 = choose (one row, and few rows of small weights: GEMV-shaped kernels;
    * 2 to 640 rows where the products are few: the tcgen05 kernel for few rows,
-   * which needs no workspace; tcgen05 tiles of 128 and 256 rows above, with a
-   * split-K pass through a pool workspace for up to 512 rows, K >= 8192 and
-   * few tiles -- not inside a stream capture; the SIMT kernels when K is not
-   * a multiple of 16 or A is not 16-byte aligned); 1 = force the tcgen05
+   * which needs no workspace; tcgen05 tiles of 128 and 256 rows for what it
+   * leaves, with a split-K pass through a pool workspace for up to 512 rows,
+   * K >= 8192 and few tiles -- not inside a stream capture; the SIMT kernels
+   * when K is not a multiple of 16 or A is not 16-byte aligned); 1 = force the tcgen05
    * kernels of 128 and 256 rows; 2 = force the SIMT (dp4a / mma.sync) kernels.
    * Every choice gives the same bytes. */
   int kernel_choice;

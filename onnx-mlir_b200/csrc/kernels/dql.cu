@@ -700,9 +700,10 @@ int launch_range_parts(const float *x, int64_t n, void *scratch, RangeParts *par
     grid = kRangeMaxParts;
   const bool full = unroll == kRangeUnroll;
   // Small blocks, one float4 a thread, while they are few enough to be folded: the fewer
-  // warps an SM has, the sooner each is through.  70000 values (the whole call) 4.27 -> 3.92
-  // us, 100000 4.27 -> 4.09, linear 128 x 768 x 768 8.8 -> 8.5, 35 x 2500 x 640 9.3 -> 8.8;
-  // 150000 4.32 and 4.49.
+  // warps an SM has, the sooner each is through.  What the device takes for the whole call
+  // (a caller's host may take longer: some 10 us for a linear through the Python binding):
+  // 70000 values 4.21 -> 3.96 us, 100000 4.23 -> 4.06, linear 128 x 768 x 768 8.71 -> 8.59, 35 x
+  // 2500 x 640 9.42 -> 9.08, but 100 x 1024 x 1024 9.16 and 9.25; 150000 4.32 and 4.49.
   const int64_t small_blocks = ceil_div(n, (int64_t)kRangeFewThreads * 4);
   if (aligned && 2 * small_blocks <= 3 * sm_count()) {
     grid = small_blocks < 1 ? 1 : small_blocks;

@@ -5,9 +5,10 @@
 // not amortise, and at small sizes by latency: of launches, and of what has to happen in
 // turn inside one.  So the operands change places: a tile is 128 output columns (rows of
 // Bt, the MMA's M) by T rows of A (its N, 16 to 128), which wastes little on rows that do
-// not exist, and the K loop of a tile is dealt to the CTAs of a cluster, as many as it
-// takes to have the whole machine read.  A CTA lives for one slice of one tile,
-// several are resident per SM:
+// not exist, and the K loop of a tile is dealt to the CTAs of a cluster, so that more SMs
+// read: as many as few_plan() finds cheapest, which for clusters of three and more counts on
+// three quarters of the SMs (16 x 14336 x 4096: 32 tiles, 96 CTAs in clusters of three).  A CTA
+// lives for one slice of one tile, several are resident per SM:
 //   warp 8      asks for the slices of Bt as soon as it starts, before the kernel it
 //               follows has finished (see `settled`), and for A behind pdl_sync()
 //   warp 9      issues the MMAs, four K slices of 32 bytes per block of 128, two blocks

@@ -287,13 +287,16 @@ int rows_rounds(int64_t N) {
 
 bool linear_rows_wanted(int64_t M, int64_t N, int64_t kp) {
   // Every cluster reads all of x, so x has to be small next to the weight a cluster
-  // reads: 8 x 1024 x 1024 6.3 us here and 7.1 as two kernels, 16 x 256 x 256 5.8 and
-  // 7.0, 2 x 8192 x 8192 17.2 and 19.6, 6 x 5000 x 12000 19.8 and 22.8, but 8 x 4096 x
-  // 4096 10.1 and 9.5, 16 x 14336 x 4096 31 and 20.  One row is quantized so fast that
-  // the dp4a kernel behind it is as good (1 x 2048 x 2048: 6.2 and 5.9).  The line is
-  // drawn well inside: of 710 sizes up to 32768 values, weights in L2, it chooses none
-  // that the two kernels run more than 2 % faster, and leaves many to them that would
-  // be faster here (4 x 7000 x 300 7.9 and 12.2, 12 x 300 x 14336 10.9 and 14.4).
+  // reads: 16 x 256 x 256 5.8 us here and 7.0 as quantize and product, 16 x 768 x 768 5.8
+  // and 7.5, 6 x 2062 x 1072 7.1 and 8.2.  One row is quantized so fast that the dp4a
+  // kernel behind it is as good (1 x 2048 x 2048: 6.2 and 5.9).  The line was drawn
+  // against the GEMV-shaped products, well inside: none of 710 sizes up to 32768 values
+  // was more than 2 % faster as two kernels.  Against the few-rows kernel, which now makes
+  // the product of large weights, that holds for one column group per cluster (0.55 to
+  // 0.94 of the two kernels' time on 39 sizes), not for more (1.02 to 1.8 on 19): 2 x
+  // 8192 x 8192 16.6 and 12.0 with the weight in L2, 19.4 and 16.9 beyond, 2 x 4096 x 14336
+  // 15.5 and 11.1, 18.0 and 15.4, 15 x 2176 x 15360 17.2 and 9.5, 19.7 and 12.1, 5 x 1650 x 5419
+  // 8.7 and 8.4, 9.4 and 8.8.
   if (M < 2 || M > kRowsMax || N > (int64_t)1 << 24)
     return false;
   if (M * kp > 16384 && (M * kp > 32768 || N < 1024 * M))
@@ -303,7 +306,7 @@ bool linear_rows_wanted(int64_t M, int64_t N, int64_t kp) {
   if (M * (rows_slice(kp) / 4) > kRowsHeld * kRowsThreads)
     return false;
   // More than one column group per cluster: not for weights of a few MB (4 x 768 x 3072:
-  // 7.1 us here, 6.9 as two kernels).
+  // 7.1 us here, 6.9 as two kernels).  (Nor, by the times above, for larger ones.)
   const int rounds = rows_rounds(N);
   if (rounds > 1 && N * kp < (int64_t)8 << 20)
     return false;

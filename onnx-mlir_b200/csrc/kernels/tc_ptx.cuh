@@ -24,7 +24,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
 // One lane of the (whole, converged) warp, always the same.  Of a branch on it in a
 // warp-uniform one the compiler knows that one thread runs it, and keeps addresses and
 // descriptors of what is issued there in uniform registers, where tcgen05 and TMA
-// instructions take them; on `lane == 0` it moves each there.
+// instructions take them; on `lane == 0` it moves each there.  All tensor-core kernels,
+// lane 0 against this: linear 4096 x 4096 x 4096 96.0 -> 91.6 us, QLinearMatMul 16384 x 1024 x
+// 4096 81.6 -> 77.3, encoder base 32 x 128 1517 -> 1405, large 256 x 512 101.3 -> 97.2 ms.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t"
