@@ -503,15 +503,15 @@ __global__ void __launch_bounds__(32 * kTiles * (kShared ? 2 : 1))
     m0 = mn0;
     m1 = mn1;
     float ps0 = 0.0f, ps1 = 0.0f;
-    float q0[NT_S], q1[NT_S]; // sums of a tile's two values of a row
+    float pair0[NT_S], pair1[NT_S]; // sums of a tile's two values of a row
 #pragma unroll
     for (int nt = 0; nt < NT_S; ++nt) {
       s[nt][0] = expf(s[nt][0] - mn0);
       s[nt][1] = expf(s[nt][1] - mn0);
       s[nt][2] = expf(s[nt][2] - mn1);
       s[nt][3] = expf(s[nt][3] - mn1);
-      q0[nt] = s[nt][0] + s[nt][1];
-      q1[nt] = s[nt][2] + s[nt][3];
+      pair0[nt] = s[nt][0] + s[nt][1];
+      pair1[nt] = s[nt][2] + s[nt][3];
     }
     // P of 16 keys at a time: the accumulator layout of two adjacent score tiles is the A
     // operand layout of one such step.
@@ -529,8 +529,8 @@ __global__ void __launch_bounds__(32 * kTiles * (kShared ? 2 : 1))
         return make_uint4(__float_as_uint(a), __float_as_uint(b), __float_as_uint(c),
             __float_as_uint(d));
       };
-      xch_mine[0] = bits(q0[0], q0[1], q0[2], q0[3]);
-      xch_mine[32] = bits(q1[0], q1[1], q1[2], q1[3]);
+      xch_mine[0] = bits(pair0[0], pair0[1], pair0[2], pair0[3]);
+      xch_mine[32] = bits(pair1[0], pair1[1], pair1[2], pair1[3]);
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         xch_mine[32 * (2 + 2 * k)] = make_uint4(ph[k][0], ph[k][1], ph[k][2], ph[k][3]);
@@ -545,8 +545,8 @@ __global__ void __launch_bounds__(32 * kTiles * (kShared ? 2 : 1))
 #pragma unroll
       for (int i = 0; i < 8; ++i) { // keys in order, whoever made their sums
         const bool mine = (i >> 2) == half;
-        ps0 += mine ? q0[i & 3] : z0[i & 3];
-        ps1 += mine ? q1[i & 3] : z1[i & 3];
+        ps0 += mine ? pair0[i & 3] : z0[i & 3];
+        ps1 += mine ? pair1[i & 3] : z1[i & 3];
       }
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
@@ -564,8 +564,8 @@ __global__ void __launch_bounds__(32 * kTiles * (kShared ? 2 : 1))
     } else {
 #pragma unroll
       for (int nt = 0; nt < NT_S; ++nt) {
-        ps0 += q0[nt];
-        ps1 += q1[nt];
+        ps0 += pair0[nt];
+        ps1 += pair1[nt];
       }
     }
     ps0 += __shfl_xor_sync(0xffffffffu, ps0, 1);
