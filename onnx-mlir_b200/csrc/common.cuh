@@ -88,6 +88,9 @@ __device__ __forceinline__ void pdl_sync() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The wait alone: the kernel after this one is set up when this one's blocks have left.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // The pointer, for use after pdl_sync().  Read-only loads (__ldg, const
 // __restrict__) may legally be moved across a memory clobber; through the
 // pointer this returns they depend on what follows the wait.  Every pointer

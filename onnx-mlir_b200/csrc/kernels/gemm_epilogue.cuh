@@ -66,6 +66,7 @@ struct EpiParams {
   // L2 eviction hints of the tensor-core kernels' TMA copies: bit 0 output
   // stores evict_first, bit 1 A loads evict_first, bit 2 B loads evict_last.
   int l2_hints;
+  int early_next; // GemmCall::early_next
   int quant_mode; // OMCUDA_MODE_* flags for the quantizing tail
   // Split-K pass of the tensor-core kernels: a work unit is one of split_k
   // slices of a tile's K loop and stores its raw sums (EPI_I32 without zero

@@ -583,6 +583,7 @@ EpiParams make_epi_params(const GemmCall &a) {
              (a.N % 4 == 0);
   p.line_store = 0;
   p.l2_hints = 0;
+  p.early_next = a.early_next;
   p.quant_mode = quant_mode();
   p.split_k = 1;
   p.ws_rows = 0;

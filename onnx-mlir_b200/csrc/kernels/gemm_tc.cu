@@ -706,7 +706,10 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   tcgen05_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
   volatile int *abortp = &abort_flag;
-  pdl_sync(); // (loads below: see epi_after_pdl)
+  if (p.early_next) // (loads below: see epi_after_pdl)
+    pdl_sync();
+  else
+    pdl_wait();
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -970,7 +973,10 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   tcgen05_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
   volatile int *abortp = &abort_flag;
-  pdl_sync(); // (loads below: see epi_after_pdl)
+  if (p.early_next) // (loads below: see epi_after_pdl)
+    pdl_sync();
+  else
+    pdl_wait();
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------

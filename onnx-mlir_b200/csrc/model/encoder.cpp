@@ -234,6 +234,7 @@ int gemm(omcudaEncoder *e, const uint8_t *A, const uint8_t *a_zp,
   }
   GemmCall call(g);
   call.b_settled = true; // (omcudaEncoderSetLayer waits for what it prepares)
+  call.early_next = true;
   int rc = gemm_i8(call, st);
   if (e1)
     cudaEventRecord(e1, st);

@@ -88,9 +88,25 @@ struct GemmCall : omcudaGemmArgs {
   // The host has seen the preparation of B finish: no kernel that may still be running when
   // this GEMM is set up writes it.
   bool b_settled;
-  GemmCall() : omcudaGemmArgs(), lda(0), y_zp_dev(nullptr), b_settled(false) {}
+  // The kernel behind may be set up while this product runs (gemm_tc.cu).  Not for the
+  // operators, whose successor may be anything: the blocks of a pass that come early find
+  // the SMs of this kernel's last tiles taken and stay together on those that were free.  us
+  // of a chain of calls, set up early / at the end (and before dequantize and the passes of
+  // more than 16 Mi values overlapped at all):
+  //   16384 x 1024 x 4096  linear, DynamicQuantizeLinear                 222 / 203 (211)
+  //                        DynamicQuantizeLinear, product, dequantize    199 / 181 (183)
+  //   2048 x 1024 x 4096   the same three                                32.2 / 30.4 (31.1)
+  //   4096 x 4096 x 4096   linear after linear                           168 / 159 (180)
+  //   777 x 1001 x 1537                                                  35.7 / 33.1 (37.2)
+  //   700 x 768 x 768                                                    23.5 / 22.9 (25.0)
+  // For the encoder's, behind which LayerNorm, attention and the quantize pass that folds
+  // nothing wait: base 32 x 128 tokens 1400 / 1479, large 32 x 128 3384 / 3527, base 8 x 128 787 /
+  // 802 us.
+  bool early_next;
+  GemmCall()
+      : omcudaGemmArgs(), lda(0), y_zp_dev(nullptr), b_settled(false), early_next(false) {}
   explicit GemmCall(const omcudaGemmArgs &a)
-      : omcudaGemmArgs(a), lda(a.K), y_zp_dev(nullptr), b_settled(false) {}
+      : omcudaGemmArgs(a), lda(a.K), y_zp_dev(nullptr), b_settled(false), early_next(false) {}
 };
 int gemm_i8(const GemmCall &a, cudaStream_t st);
 bool gemm_tc_supported(const GemmCall &a);

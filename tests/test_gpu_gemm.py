@@ -582,6 +582,34 @@ def test_split_k_tails(gpu, M, K, N, choice, adt, bdt):
     gpu.synchronize()
 
 
+@pytest.mark.parametrize("M,K,N", [(700, 768, 768), (2048, 256, 2048), (5000, 128, 4100), (777, 80, 1537)])
+def test_passes_behind_a_product(gpu, orc, M, K, N):
+    """Products on the tensor cores and the passes that read them, queued without waiting
+    (single CTAs and pairs; results on both sides of 16 Mi values): each pass finds its
+    product complete, in every one of four rounds over the same buffers."""
+    rng = np.random.default_rng(M + N)
+    L = gpu.lib()
+    B = rand8(rng, (K, N), np.int8)
+    As = [rand8(rng, (M, K), np.uint8) for _ in range(4)]
+    d = lambda a: gpu.Tensor.from_numpy(np.asarray(a)).to_device()
+    dB, dA, sc = d(B), [d(A) for A in As], d(np.float32(0.25))
+    L.omcudaRegisterConstant(dB.handle)
+    acc, f = gpu.Tensor.device_empty((M, N), np.int32), gpu.Tensor.device_empty((M, N), np.float32)
+    q = [gpu.Tensor.device_empty((M, N), np.uint8) for _ in As]
+    ys = [(gpu.Tensor.device_empty((), np.float32), gpu.Tensor.device_empty((), np.uint8)) for _ in As]
+    for a, y, (s, z) in zip(dA, q, ys):
+        L.omcudaMatMulInteger(acc.handle, a.handle, dB.handle, None, None)
+        L.omcudaDequantizeLinear(f.handle, acc.handle, sc.handle, None)
+        L.omcudaDynamicQuantizeLinear(y.handle, s.handle, z.handle, f.handle)
+    gpu.synchronize()
+    for A, y, (s, z) in zip(As, q, ys):
+        # (sums below 2^24: exact in fp32)
+        wy, ws, wz = orc.dynamic_quantize_linear(
+            (A.astype(np.float32) @ B.astype(np.float32)) * np.float32(0.25))
+        assert s.numpy() == ws and z.numpy() == wz and np.array_equal(y.numpy(), wy)
+    L.omcudaForgetConstants()
+
+
 @pytest.mark.parametrize("K,N", [
     (16, 1), (3000, 5), (2912, 1776), (2913, 1776), (2928, 1777), (1024, 4736), (1025, 4736), (1040, 4737),
     (8192, 4740), (100, 9472), (100, 9473), (2064, 20003)])
