@@ -23,30 +23,40 @@
 //
 // A work item = 128 query rows of one (batch, head).  Two persistent CTAs
 // share an SM, so that one's softmax (CUDA cores) overlaps the other's matrix
-// products (tensor pipe); each walks its share of the items and requests the
-// Q and first K tiles of its next item while the current one is in its last
-// key block.  Per block of 128 keys:
-//   thread 0   waits for the K tiles (TMA, 128-byte swizzle), issues
-//              S = Q K^T as 12 MMAs (3 split terms x 4 k-steps) into tensor
-//              memory, commits to an mbarrier, refills the K buffers;
+// products (tensor pipe); each walks its share of the items.  Per block of 128
+// keys:
+//   the product warp (att_products) issues S = Q K^T as 12 MMAs (3 split terms
+//              x 4 k-steps) into tensor memory;
 //   8 warps    two threads per query row (its TMEM lane), 64 keys each: row
 //              maximum (exchanged through shared memory), p = 2^(s*c - m),
 //              running sum, p split into bf16 hi/lo and stored back over the
 //              scores in tensor memory;
-//   thread 0   issues O_j = P V as 16 MMAs with P read from tensor memory and
-//              V (keys x 64, MN-major) from shared memory: P_hi against
+//   the product warp issues O_j = P V as 16 MMAs with P read from tensor memory
+//              and V (keys x 64, MN-major) from shared memory: P_hi against
 //              [V_hi | V_lo] as one N = 128 product per 16-key slice (into
 //              128 columns of tensor memory), P_lo V_hi on top of the first
-//              64 columns; refills V;
+//              64 columns; and right behind them the next block's S;
+//   the load warp (att_loads) refills each buffer (TMA, 128-byte swizzle) once
+//              the products that read it are done, and sends results off.
 // O accumulates in tensor memory over the key blocks of an item (the P V MMAs
 // add to it); the exponent offset of a row follows its running maximum lazily,
 // moving only when a block's maximum exceeds it by more than 2^8, and only
 // then are O and the row sum rescaled (a tensor-memory load / multiply /
 // store pass): on typical data one pass or none per item instead of one
 // register fold per block.  At the end of the item the 8 warps read O (the sum
-// of its two 64-column halves), normalise and store.
-// The normalised 128 x 64 result of an item is staged in the (then free) V
-// buffers and leaves with two TMA stores of whole 128-byte lines.
+// of its two 64-column halves), normalise and stage it in shared memory, from
+// which it leaves with two TMA stores of whole 128-byte lines.
+//
+// What bounds it: the chain of a CTA (scores -> softmax -> P V -> scores), two of
+// which share an SM.  One warp used to issue products and copies beside its rows,
+// with a CTA barrier between any two phases: of some 5100 clocks per block 1180 were
+// spent issuing copies and waking up, and 2600 more per item on its results.  With warps
+// of their own for products and copies, mbarriers between the phases, S queued behind
+// P V and the results out of V's way, a block takes some 4400 and an item 500 more (two
+// CTAs share the SM meanwhile: 1536 clocks of MMAs per block each).  Batch x sequence x
+// heads, us: 256 x 512 x 16 835 -> 750, 64 x 384 x 16 138 -> 112, 1 x 512 x 16 16.5 ->
+// 13.1, 32 x 128 x 12 11.3 -> 11.0, 1024 x 128 x 16 338 -> 326 (HBM).  The largest runs
+// at the power limit, clocks at 1.35 GHz.  Every sum is in the order it was in.
 // Every wait on an mbarrier is bounded (tc_ptx.cuh); a timeout raises the
 // CTA's abort flag, the CTA frees its tensor memory, writes the status word
 // and returns.
@@ -69,7 +79,8 @@ constexpr int kTDh = 64;            // head size
 constexpr int kTile = 128 * 128;    // bytes of one 128-row x 64-bf16 tile
 constexpr int kTcAttSmem = 6 * kTile + 1024;
 constexpr uint32_t kTmemColsAtt = 256; // S/P: 0..127, O_j: 128..255
-constexpr int kTcAttThreads = 256;     // two threads per query row
+constexpr int kTcAttWarps = 8;         // two threads per query row
+constexpr int kTcAttThreads = 32 * kTcAttWarps + 64; // and the two warps that feed them
 
 // S = Q K^T of a block: twelve MMAs over the four 16-element K slices (32 bytes,
 // descriptor + 2) of three pairs of operands, small terms first: Ql Kh, Qh Kl, Qh Kh.
@@ -158,6 +169,17 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
       : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+        "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr)
+      : "memory");
+}
+
 __device__ __forceinline__ void tmem_st_wait() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
@@ -206,6 +228,19 @@ struct AttItem {
   int32_t row_q, row_kv, cq, ck, cv, col_out;
 };
 
+// Shared-memory addresses of the operand tiles, and of the mbarriers: tiles loaded (q, k, v),
+// scores ready (s), P in tensor memory (p), P V done (o), results staged (r), and one for a CTA
+// that gives up.
+struct AttTiles {
+  uint32_t qh, ql, kh, kl, vh, vl;
+};
+struct AttBars {
+  uint32_t q, k, v, s, p, o, r, end;
+};
+struct AttLoads { // requested so far
+  uint32_t q, k, v;
+};
+
 __device__ __forceinline__ AttItem att_item(int64_t item, int nq, int64_t S,
     int64_t heads, int32_t q_col, int32_t k_col, int32_t v_col) {
   const int64_t bh = item / nq, qt = item % nq;
@@ -220,6 +255,152 @@ __device__ __forceinline__ AttItem att_item(int64_t item, int nq, int64_t S,
   return it;
 }
 
+// For the product warp, whose wait is part of the chain: polls without being suspended for
+// the first 4096 (mbarrier.try_wait wakes up some 100 clocks late: 1 x 512 x 16 14.9 -> 13.1 us,
+// 256 x 512 x 16 746 -> 750), then waits like the others.
+__device__ __forceinline__ bool mbar_spin(
+    uint32_t bar, uint32_t parity, volatile int *abort_flag, uint64_t limit_ns) {
+  for (int i = 0; i < 4096; ++i)
+    if (mbar_test_wait(bar, parity))
+      return true;
+  return mbar_wait(bar, parity, abort_flag, limit_ns);
+}
+
+// The tensor pipe's part, by one elected thread of a warp that does nothing else.  Returns
+// false when a wait ran out (or the CTA is aborting).
+//
+// Products of one thread run in the order of issue, so the next block's S = Q K^T is queued
+// right behind P V, which still reads P from the columns that it overwrites: no wait between
+// the two, and the first block of the next item runs while the softmax warps are still busy
+// with the results of the one before.
+__device__ __forceinline__ bool att_products(const AttTiles &s, const AttBars &bar,
+    uint32_t tmem, int nkb, int64_t n_items, volatile int *abortp, uint64_t wait_ns) {
+  constexpr uint32_t kIdescQK = att_idesc(kTK, 0);
+  constexpr uint32_t kIdescPV = att_idesc(kTDh, 1);
+  // P_hi against V_hi and V_lo in one MMA of N = 128: the B descriptor's
+  // leading-dimension offset (stride between 64-element groups along N) is
+  // the distance from the V_hi tile to the V_lo tile, so output columns
+  // 0..63 hold P_hi V_hi and 64..127 hold P_hi V_lo.
+  constexpr uint32_t kIdescPV2 = att_idesc(2 * kTDh, 1);
+  constexpr uint64_t kLboField = (uint64_t)0x3fff << 16;
+  static_assert(kTDh == 64, "four K slices per operand row");
+  static_assert(kTK == 128, "eight 16-key slices per block");
+  const uint32_t t_s = tmem, t_o = tmem + 128u;
+  const uint64_t dqh = make_smem_desc(s.qh), dql = make_smem_desc(s.ql),
+                 dkh = make_smem_desc(s.kh), dkl = make_smem_desc(s.kl),
+                 dvh = make_smem_desc(s.vh);
+  const uint64_t dv2 = (dvh & ~kLboField) | ((uint64_t)((s.vl - s.vh) >> 4) << 16);
+  auto wait = [&](uint32_t b, uint32_t parity) {
+    return mbar_spin(b, parity & 1u, abortp, wait_ns);
+  };
+  uint32_t n = 0;     // key blocks, parity of bar.k / v / s / p / o
+  uint32_t nitem = 0; // items, parity of bar.q
+  if (!wait(bar.q, 0) || !wait(bar.k, 0))
+    return false;
+  tcgen05_fence_after();
+  umma_scores(t_s, dql, dqh, dkh, dkl, kIdescQK);
+  umma_commit(bar.s);
+  for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x, ++nitem) {
+    const bool has_next = item + gridDim.x < n_items;
+    for (int j = 0; j < nkb; ++j, ++n) {
+      const bool last = j + 1 == nkb;
+      if (!wait(bar.v, n) || !wait(bar.p, n))
+        return false;
+      tcgen05_fence_after();
+      umma_values(t_o, t_s, dv2, dvh, kIdescPV2, kIdescPV, j != 0 ? 1u : 0u);
+      umma_commit(bar.o);
+      if (!last || has_next) {
+        if ((last && !wait(bar.q, nitem + 1)) || !wait(bar.k, n + 1))
+          return false;
+        umma_scores(t_s, dql, dqh, dkh, dkl, kIdescQK);
+        umma_commit(bar.s);
+      }
+    }
+  }
+  return true;
+}
+
+// The copies' part, by one elected thread of another warp: every buffer is refilled as soon as
+// the products that read it are done.  loads: what it requested, for one that gives up.
+__device__ __forceinline__ bool att_loads(const CUtensorMap &map_hi, const CUtensorMap &map_lo,
+    const CUtensorMap &map_out, const AttTiles &s, const AttBars &bar, int32_t q_col,
+    int32_t k_col, int32_t v_col, int nkb, int nq, int64_t S, int64_t heads, int64_t n_items,
+    AttLoads &loads, volatile int *abortp, uint64_t wait_ns) {
+  auto load = [&](uint32_t b, uint32_t hi, uint32_t lo, int32_t col, int32_t row) {
+    mbar_expect_tx(b, 2 * kTile);
+    tma_load_2d(hi, &map_hi, col, row, b);
+    tma_load_2d(lo, &map_lo, col, row, b);
+  };
+  auto load_q = [&](const AttItem &it) {
+    load(bar.q, s.qh, s.ql, it.cq, it.row_q), ++loads.q;
+  };
+  auto load_k = [&](const AttItem &it, int j) {
+    load(bar.k, s.kh, s.kl, it.ck, it.row_kv + j * kTK), ++loads.k;
+  };
+  auto load_v = [&](const AttItem &it, int j) {
+    load(bar.v, s.vh, s.vl, it.cv, it.row_kv + j * kTK), ++loads.v;
+  };
+  auto wait = [&](uint32_t b, uint32_t parity) {
+    return mbar_wait(b, parity & 1u, abortp, wait_ns);
+  };
+  AttItem it = att_item(blockIdx.x, nq, S, heads, q_col, k_col, v_col);
+  load_q(it);
+  load_k(it, 0);
+  load_v(it, 0);
+  // The results of an item take a turn in the K buffers, once the next item's first scores are
+  // done with them: the next K has the longest time to arrive.  Items of one key block have no
+  // such next K; theirs take it in the V buffers.
+  const bool in_v = nkb == 1;
+  auto store = [&](const AttItem &at) {
+    tma_store_2d(&map_out, in_v ? s.vh : s.kh, at.col_out, at.row_q);
+    tma_store_2d(&map_out, in_v ? s.vl : s.kl, at.col_out + 32, at.row_q);
+    tma_store_commit();
+  };
+  uint32_t n = 0, nitem = 0;
+  AttItem before = it;
+  for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x, ++nitem) {
+    const bool has_next = item + gridDim.x < n_items;
+    AttItem nx = it;
+    if (has_next)
+      nx = att_item(item + gridDim.x, nq, S, heads, q_col, k_col, v_col);
+    for (int j = 0; j < nkb; ++j, ++n) {
+      const bool last = j + 1 == nkb, more = !last || has_next;
+      const AttItem &at = last ? nx : it; // of the next block
+      const int jn = last ? 0 : j + 1;
+      if (!wait(bar.s, n)) // the K buffers are free, behind an item's last block the Q buffers too
+        return false;
+      if (last && has_next)
+        load_q(nx);
+      if (j == 0 && nitem != 0 && !in_v) {
+        if (!wait(bar.r, nitem - 1))
+          return false;
+        store(before);
+        tma_store_wait_read();
+      }
+      if (more)
+        load_k(at, jn);
+      if (in_v) {
+        if (!wait(bar.r, nitem))
+          return false;
+        store(it);
+        tma_store_wait_read();
+      } else if (more && !wait(bar.o, n)) {
+        return false;
+      }
+      if (more)
+        load_v(at, jn);
+    }
+    before = it;
+    it = nx;
+  }
+  if (!in_v) {
+    if (!wait(bar.r, nitem - 1))
+      return false;
+    store(before);
+  }
+  return true;
+}
+
 __global__ void __launch_bounds__(kTcAttThreads, 2)
     attention_tc_kernel(const __grid_constant__ CUtensorMap map_hi,
         const __grid_constant__ CUtensorMap map_lo,
@@ -227,10 +408,13 @@ __global__ void __launch_bounds__(kTcAttThreads, 2)
         int32_t v_col, int64_t S, int64_t heads, int64_t n_items, float scale_log2e,
         uint32_t *__restrict__ out_range, int *status, uint64_t wait_ns) {
   extern __shared__ uint8_t att_tc_smem[];
-  __shared__ uint64_t bar_q, bar_k, bar_v, bar_s, bar_o;
+  __shared__ uint64_t bars[8];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
-  __shared__ float xch[2][kTQ]; // row maximum / row sum of each half of the keys
+  // What the two threads of a row tell each other.  The maxima of a block lie where those of
+  // the block before last did: a thread gets there past a barrier that its partner reaches
+  // after having read them.  So do the sums, for there is a block between any two.
+  __shared__ float xch_max[2][2][kTQ], xch_sum[2][kTQ];
 
   const int tid = threadIdx.x, warp = warp_number(), lane = tid & 31;
   // Warps w and w + 4 share the 32 query rows (TMEM lanes) of quadrant w & 3:
@@ -242,9 +426,11 @@ __global__ void __launch_bounds__(kTcAttThreads, 2)
   const int nq = (int)(S / kTQ);
 
   const uint32_t smem0 = (smem_u32(att_tc_smem) + 1023u) & ~1023u;
-  const uint32_t s_qh = smem0, s_ql = smem0 + kTile, s_kh = smem0 + 2 * kTile,
-                 s_kl = smem0 + 3 * kTile, s_vh = smem0 + 4 * kTile,
-                 s_vl = smem0 + 5 * kTile;
+  const AttTiles tiles = {smem0, smem0 + kTile, smem0 + 2 * kTile, smem0 + 3 * kTile,
+      smem0 + 4 * kTile, smem0 + 5 * kTile};
+  const uint32_t bar0 = smem_u32(bars);
+  const AttBars bar = {bar0, bar0 + 8, bar0 + 16, bar0 + 24, bar0 + 32, bar0 + 40, bar0 + 48,
+      bar0 + 56};
 
   if (tid == 32) {
     prefetch_tensormap(&map_hi);
@@ -253,11 +439,14 @@ __global__ void __launch_bounds__(kTcAttThreads, 2)
   }
   if (tid == 0) {
     abort_flag = 0;
-    mbar_init(smem_u32(&bar_q), 1);
-    mbar_init(smem_u32(&bar_k), 1);
-    mbar_init(smem_u32(&bar_v), 1);
-    mbar_init(smem_u32(&bar_s), 1);
-    mbar_init(smem_u32(&bar_o), 1);
+    mbar_init(bar.q, 1);
+    mbar_init(bar.k, 1);
+    mbar_init(bar.v, 1);
+    mbar_init(bar.s, 1);
+    mbar_init(bar.p, kTcAttWarps);
+    mbar_init(bar.o, 1);
+    mbar_init(bar.r, kTcAttWarps);
+    mbar_init(bar.end, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0)
@@ -267,277 +456,208 @@ __global__ void __launch_bounds__(kTcAttThreads, 2)
   tcgen05_fence_after();
   const uint32_t tmem = tmem_slot;
   pdl_sync();
-  const uint32_t t_s = tmem;          // scores, then P, columns 0..127
-  const uint32_t t_o = tmem + 128u;   // P V of the current key block
-  const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
-  const int kc0 = half * (kTK / 2); // first key column of this thread's share
   volatile int *abortp = &abort_flag;
 
-  // The CTA walks the items blockIdx.x, blockIdx.x + gridDim.x, ...; the
-  // operands of an item's first key block are requested while the item
-  // before it is still in its last block, as soon as their buffers are free.
-  if (warp == 0 && elect_one() && (int64_t)blockIdx.x < n_items) {
-    const AttItem it = att_item(blockIdx.x, nq, S, heads, q_col, k_col, v_col);
-    mbar_expect_tx(smem_u32(&bar_q), 2 * kTile);
-    tma_load_2d(s_qh, &map_hi, it.cq, it.row_q, smem_u32(&bar_q));
-    tma_load_2d(s_ql, &map_lo, it.cq, it.row_q, smem_u32(&bar_q));
-    mbar_expect_tx(smem_u32(&bar_k), 2 * kTile);
-    tma_load_2d(s_kh, &map_hi, it.ck, it.row_kv, smem_u32(&bar_k));
-    tma_load_2d(s_kl, &map_lo, it.ck, it.row_kv, smem_u32(&bar_k));
-    mbar_expect_tx(smem_u32(&bar_v), 2 * kTile);
-    tma_load_2d(s_vh, &map_hi, it.cv, it.row_kv, smem_u32(&bar_v));
-    tma_load_2d(s_vl, &map_lo, it.cv, it.row_kv, smem_u32(&bar_v));
-  }
-
-  constexpr uint32_t kIdescQK = att_idesc(kTK, 0);
-  constexpr uint32_t kIdescPV = att_idesc(kTDh, 1);
-  // P_hi against V_hi and V_lo in one MMA of N = 128: the B descriptor's
-  // leading-dimension offset (stride between 64-element groups along N) is
-  // the distance from the V_hi tile to the V_lo tile, so output columns
-  // 0..63 hold P_hi V_hi and 64..127 hold P_hi V_lo.
-  constexpr uint32_t kIdescPV2 = att_idesc(2 * kTDh, 1);
-  constexpr uint64_t kLboField = (uint64_t)0x3fff << 16;
-
-  bool ok = true;
-  uint32_t nblk = 0;  // key blocks done by this CTA: parity of bar_k / s / v / o
-  uint32_t nitem = 0; // items done by this CTA: parity of bar_q
-  float lo_run = INFINITY, hi_run = -INFINITY; // range of this thread's outputs
-
-  for (int64_t item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++nitem) {
-    const AttItem it = att_item(item, nq, S, heads, q_col, k_col, v_col);
-    const bool has_next = item + gridDim.x < n_items;
-    AttItem nx = it;
-    if (has_next)
-      nx = att_item(item + gridDim.x, nq, S, heads, q_col, k_col, v_col);
-
-    // O accumulates in tensor memory over the key blocks of the item.  The
-    // exponent offset m_ref of a row follows its running maximum lazily: it
-    // moves (and O and the row sum are rescaled) only when a block's maximum
-    // exceeds it by more than 2^8, so p never exceeds 256 and most blocks
-    // need no pass over O at all.  Any offset gives the same softmax once
-    // the sum over the same p normalises the result.
-    float m_ref = -INFINITY; // exponent offset, in units of s * scale * log2(e)
-    float l_run = 0.0f;      // running sum of p
-
-    for (int j = 0; j < nkb; ++j, ++nblk) {
-      const uint32_t ph = nblk & 1u;
-      // ---- S = Q K_j^T ----
-      __syncwarp();
-      if (warp == 0 && elect_one()) {
-        if (j == 0)
-          ok = mbar_wait(smem_u32(&bar_q), nitem & 1u, abortp, wait_ns);
-        ok = ok && mbar_wait(smem_u32(&bar_k), ph, abortp, wait_ns);
-        if (ok) {
-          tcgen05_fence_after();
-          static_assert(kTDh == 64, "four K slices per operand row");
-          umma_scores(t_s, make_smem_desc(s_ql), make_smem_desc(s_qh), make_smem_desc(s_kh),
-              make_smem_desc(s_kl), kIdescQK);
-          umma_commit(smem_u32(&bar_s));
-          if (j == 0 && nitem != 0) {
-            // The V buffers held the previous item's output for its TMA
-            // store: refill them once the store has read them.
-            tma_store_wait_read();
-            mbar_expect_tx(smem_u32(&bar_v), 2 * kTile);
-            tma_load_2d(s_vh, &map_hi, it.cv, it.row_kv, smem_u32(&bar_v));
-            tma_load_2d(s_vl, &map_lo, it.cv, it.row_kv, smem_u32(&bar_v));
-          }
-          ok = mbar_wait(smem_u32(&bar_s), ph, abortp, wait_ns);
-          if (ok && j + 1 < nkb) { // the K buffers are free again
-            mbar_expect_tx(smem_u32(&bar_k), 2 * kTile);
-            tma_load_2d(s_kh, &map_hi, it.ck, it.row_kv + (j + 1) * kTK, smem_u32(&bar_k));
-            tma_load_2d(s_kl, &map_lo, it.ck, it.row_kv + (j + 1) * kTK, smem_u32(&bar_k));
-          } else if (ok && has_next) { // so are the Q buffers: next item
-            mbar_expect_tx(smem_u32(&bar_q), 2 * kTile);
-            tma_load_2d(s_qh, &map_hi, nx.cq, nx.row_q, smem_u32(&bar_q));
-            tma_load_2d(s_ql, &map_lo, nx.cq, nx.row_q, smem_u32(&bar_q));
-            mbar_expect_tx(smem_u32(&bar_k), 2 * kTile);
-            tma_load_2d(s_kh, &map_hi, nx.ck, nx.row_kv, smem_u32(&bar_k));
-            tma_load_2d(s_kl, &map_lo, nx.ck, nx.row_kv, smem_u32(&bar_k));
-          }
-        }
-      }
-      ok = __syncthreads_and(ok) != 0;
-      if (!ok)
-        break;
-      tcgen05_fence_after();
-
-      // ---- online softmax: this thread's half of its row ----
-      __syncwarp(); // tcgen05.ld / st are warp-collective: enter them converged
-      // The thread's 64 scores are read from tensor memory once and stay in
-      // registers for both passes (maximum, then exponentials).
-      static_assert(kTK / 2 == 64, "two 32-column loads per thread");
-      uint32_t sv[2][32];
-      tmem_ld32(t_s + lane_base + (uint32_t)kc0, sv[0]);
-      tmem_ld32(t_s + lane_base + (uint32_t)kc0 + 32u, sv[1]);
-      tmem_ld_wait();
-      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}; // (no chain of 32)
-#pragma unroll
-      for (int h2 = 0; h2 < 2; ++h2)
-#pragma unroll
-        for (int i = 0; i < 32; i += 2)
-          m4[(i >> 1) & 3] = max3f(m4[(i >> 1) & 3], __uint_as_float(sv[h2][i]),
-              __uint_as_float(sv[h2][i + 1]));
-      float mx = max3f(m4[0], m4[1], fmaxf(m4[2], m4[3]));
-      // Row maximum over both halves (the two threads of a row sit in warps w
-      // and w + 4: a 64-thread named barrier per quadrant).
-      xch[half][row] = mx;
-      pair_barrier(quad);
-      mx = fmaxf(mx, xch[half ^ 1][row]);
-      const float m_blk = __fmul_rn(mx, scale_log2e);
-      // (true for every row on the first block: m_ref is -inf)
-      const bool move = m_blk > __fadd_rn(m_ref, 8.0f);
-      // Both threads of a row and both warps of a quadrant see the same rows
-      // and maxima, so they take this branch together.
-      if (j > 0 && __any_sync(0xffffffffu, move)) {
-        const float f = move ? ex2_approx(__fsub_rn(m_ref, m_blk)) : 1.0f;
-        l_run = __fmul_rn(l_run, f);
-        const uint64_t f2 = pack_f32x2(f, f);
-#pragma unroll 1
-        for (uint32_t part = 0; part < 2; ++part) { // P_hi V_hi + P_lo V_hi | P_hi V_lo
-          const uint32_t ta = t_o + part * 64u + lane_base + (uint32_t)(half * 32);
-          uint32_t v[32];
-          tmem_ld32(ta, v);
-          tmem_ld_wait();
-          uint32_t w0[16], w1[16];
-#pragma unroll
-          for (int i = 0; i < 16; i += 2) {
-            float a, b;
-            unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), f2), a, b);
-            w0[i] = __float_as_uint(a);
-            w0[i + 1] = __float_as_uint(b);
-            unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(v[16 + i]), __uint_as_float(v[17 + i])), f2), a, b);
-            w1[i] = __float_as_uint(a);
-            w1[i + 1] = __float_as_uint(b);
-          }
-          tmem_st16(ta, w0);
-          tmem_st16(ta + 16u, w1);
-        }
-        tmem_st_wait();
-      }
-      if (move)
-        m_ref = m_blk;
-      // (packed fp32 below: two individually rounded operations per instruction)
-      const uint64_t scale2 = pack_f32x2(scale_log2e, scale_log2e);
-      const uint64_t neg_m2 = pack_f32x2(-m_ref, -m_ref);
-      const uint64_t minus1 = pack_f32x2(-1.0f, -1.0f);
-      uint64_t psum2 = pack_f32x2(0.0f, 0.0f);
-#pragma unroll
-      for (int h2 = 0; h2 < 2; ++h2) {
-        const int c = kc0 + 32 * h2;
-        const uint32_t(&v)[32] = sv[h2];
-        uint32_t whi[16], wlo[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float a0, a1;
-          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[2 * i]),
-                                     __uint_as_float(v[2 * i + 1])),
-                           scale2, neg_m2),
-              a0, a1);
-          const float p0 = ex2_approx(a0), p1 = ex2_approx(a1);
-          const uint64_t p2 = pack_f32x2(p0, p1);
-          psum2 = add_f32x2(psum2, p2);
-          const uint32_t hi = cvt_bf16x2(p0, p1);
-          // p - hi: one rounding, as the subtraction has
-          float r0, r1;
-          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(hi << 16),
-                                     __uint_as_float(hi & 0xffff0000u)),
-                           minus1, p2),
-              r0, r1);
-          whi[i] = hi;
-          wlo[i] = cvt_bf16x2(r0, r1);
-        }
-        // P of keys c..c+31: hi in columns c..c+15, lo in c+16..c+31 (the
-        // scores of those columns are already consumed).
-        tmem_st16(t_s + lane_base + (uint32_t)c, whi);
-        tmem_st16(t_s + lane_base + (uint32_t)c + 16u, wlo);
-      }
-      float ps0, ps1;
-      unpack_f32x2(psum2, ps0, ps1);
-      l_run = __fadd_rn(l_run, __fadd_rn(ps0, ps1));
-      tmem_st_wait();
-      tcgen05_fence_before();
-      __syncthreads(); // every row of P is in tensor memory
-
-      // ---- O_j = P V_j ----
-      if (warp == 0 && elect_one()) {
-        tcgen05_fence_after();
-        ok = mbar_wait(smem_u32(&bar_v), ph, abortp, wait_ns);
-        if (ok) {
-          tcgen05_fence_after();
-          static_assert(kTK == 128, "two groups of four 16-key slices per block");
-          const uint64_t dvh = make_smem_desc(s_vh);
-          const uint64_t dv2 = (dvh & ~kLboField) | ((uint64_t)((s_vl - s_vh) >> 4) << 16);
-          umma_values(t_o, t_s, dv2, dvh, kIdescPV2, kIdescPV, j != 0 ? 1u : 0u);
-          umma_commit(smem_u32(&bar_o));
-          ok = mbar_wait(smem_u32(&bar_o), ph, abortp, wait_ns);
-          if (ok && j + 1 < nkb) { // the V buffers are free again
-            mbar_expect_tx(smem_u32(&bar_v), 2 * kTile);
-            tma_load_2d(s_vh, &map_hi, it.cv, it.row_kv + (j + 1) * kTK, smem_u32(&bar_v));
-            tma_load_2d(s_vl, &map_lo, it.cv, it.row_kv + (j + 1) * kTK, smem_u32(&bar_v));
-          }
-        }
-      }
-      // No CTA barrier here: the other threads go on to wait for the next
-      // block's scores, which thread 0 requests only once this P V is done.
+  // The CTA walks the items blockIdx.x, blockIdx.x + gridDim.x, ... (the grid has no more
+  // CTAs than there are items).
+  if (warp == kTcAttWarps) {
+    if (elect_one() && !att_products(tiles, bar, tmem, nkb, n_items, abortp, wait_ns)) {
+      // Gave up: tell the others, then let what is under way end before tensor memory goes.
+      abort_flag = 1;
+      volatile int own = 0;
+      umma_commit(bar.end);
+      (void)mbar_wait(bar.end, 0, &own, wait_ns);
     }
-    ok = __syncthreads_and(ok) != 0; // the item's last P V is complete
-    if (!ok)
-      break;
-    tcgen05_fence_after();
     __syncwarp();
-    float o[kTDh / 2];
-    {
-      uint32_t v[32];
-      tmem_ld32(t_o + lane_base + (uint32_t)(half * 32), v);
-      tmem_ld_wait();
+  } else if (warp == kTcAttWarps + 1) {
+    AttLoads loads = {0, 0, 0};
+    const bool mine = elect_one();
+    if (mine && !att_loads(map_hi, map_lo, map_out, tiles, bar, q_col, k_col, v_col, nkb, nq, S,
+                           heads, n_items, loads, abortp, wait_ns)) {
+      abort_flag = 1; // (as above, for the copies)
+      const uint32_t b[3] = {bar.q, bar.k, bar.v}, asked[3] = {loads.q, loads.k, loads.v};
 #pragma unroll
-      for (int i = 0; i < 32; ++i)
-        o[i] = __uint_as_float(v[i]);
-      // ... plus the P_hi V_lo part from the upper 64 columns
-      tmem_ld32(t_o + 64u + lane_base + (uint32_t)(half * 32), v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int i = 0; i < 32; i += 2)
-        unpack_f32x2(add_f32x2(pack_f32x2(o[i], o[i + 1]),
-                         pack_f32x2(__uint_as_float(v[i]), __uint_as_float(v[i + 1]))),
-            o[i], o[i + 1]);
+      for (int i = 0; i < 3; ++i) {
+        volatile int own = 0;
+        (void)mbar_wait(b[i], (asked[i] - 1u) & 1u, &own, wait_ns);
+      }
     }
-    tcgen05_fence_before();
+    if (mine)
+      tma_store_wait_all();
+    __syncwarp();
+  } else {
+    const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
+    const uint32_t t_row = tmem + lane_base + (uint32_t)(half * (kTK / 2)); // its scores, then P
+    const uint32_t t_out = tmem + 128u + lane_base + (uint32_t)(32 * half); // its part of O
+    // A warp whose wait ran out goes on to the end all the same, with whatever tensor memory
+    // holds: its partner meets it at every barrier of the pair, and the waits that follow end
+    // as soon as they see the flag.
+    bool ok = true;
+    uint32_t n = 0;                              // key blocks
+    float lo_run = INFINITY, hi_run = -INFINITY; // range of this thread's outputs
 
-    // Row sum over both halves, then normalise.  The 128 x 64 result leaves
-    // through the V buffers (free after the last P V): half 0's 32 columns in
-    // the first 16 KiB tile, half 1's in the second, rows of 128 bytes in the
-    // 128-byte swizzle pattern, one TMA store per tile, which writes whole
-    // lines.  The next item's V load waits for the store to have read them.
-    xch[half][row] = l_run;
-    pair_barrier(quad);
-    const float inv = __fdiv_rn(1.0f, __fadd_rn(xch[0][row], xch[1][row]));
-    const uint32_t my_row = (half ? s_vl : s_vh) + (uint32_t)row * 128u;
-    const uint32_t swz = ((uint32_t)row & 7u) << 4;
+    for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x) {
+      // O accumulates in tensor memory over the key blocks of the item.  The
+      // exponent offset m_ref of a row follows its running maximum lazily: it
+      // moves (and O and the row sum are rescaled) only when a block's maximum
+      // exceeds it by more than 2^8, so p never exceeds 256 and most blocks
+      // need no pass over O at all.  Any offset gives the same softmax once
+      // the sum over the same p normalises the result.
+      float m_ref = -INFINITY; // exponent offset, in units of s * scale * log2(e)
+      float l_run = 0.0f;      // running sum of p
+
+      for (int j = 0; j < nkb; ++j, ++n) {
+        // (the scores come behind P V of the block before on the tensor pipe, so that is done too)
+        ok = mbar_wait(bar.s, n & 1u, abortp, wait_ns) && ok;
+        tcgen05_fence_after();
+
+        // ---- online softmax: this thread's half of its row ----
+        __syncwarp(); // tcgen05.ld / st are warp-collective: enter them converged
+        // The thread's 64 scores are read from tensor memory once and stay in
+        // registers for both passes (maximum, then exponentials).
+        static_assert(kTK / 2 == 64, "two 32-column loads per thread");
+        uint32_t sv[2][32];
+        tmem_ld32(t_row, sv[0]);
+        tmem_ld32(t_row + 32u, sv[1]);
+        tmem_ld_wait();
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}; // (no chain of 32)
 #pragma unroll
-    for (int i = 0; i < kTDh / 2; i += 4) {
-      const float4 v = make_float4(__fmul_rn(o[i], inv), __fmul_rn(o[i + 1], inv),
-          __fmul_rn(o[i + 2], inv), __fmul_rn(o[i + 3], inv));
-      asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(
-                       my_row + (((uint32_t)i * 4u) ^ swz)),
-                   "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
-                   : "memory");
-      lo_run = fminf(lo_run, fminf(fminf(v.x, v.y), fminf(v.z, v.w)));
-      hi_run = fmaxf(hi_run, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int i = 0; i < 32; i += 2)
+            m4[(i >> 1) & 3] = max3f(m4[(i >> 1) & 3], __uint_as_float(sv[h][i]),
+                __uint_as_float(sv[h][i + 1]));
+        float mx = max3f(m4[0], m4[1], fmaxf(m4[2], m4[3]));
+        // Row maximum over both halves (a named barrier per quadrant).
+        xch_max[n & 1u][half][row] = mx;
+        pair_barrier(quad);
+        mx = fmaxf(mx, xch_max[n & 1u][half ^ 1][row]);
+        const float m_blk = __fmul_rn(mx, scale_log2e);
+        // (true for every row on the first block: m_ref is -inf)
+        const bool move = m_blk > __fadd_rn(m_ref, 8.0f);
+        // Both threads of a row and both warps of a quadrant see the same rows
+        // and maxima, so they take this branch together.
+        if (j > 0 && __any_sync(0xffffffffu, move)) {
+          const float f = move ? ex2_approx(__fsub_rn(m_ref, m_blk)) : 1.0f;
+          l_run = __fmul_rn(l_run, f);
+          const uint64_t f2 = pack_f32x2(f, f);
+#pragma unroll 1
+          for (uint32_t part = 0; part < 4; ++part) { // P_hi V_hi + P_lo V_hi | P_hi V_lo
+            const uint32_t ta = t_out + (part >> 1) * 64u + (part & 1u) * 16u;
+            uint32_t v[16];
+            tmem_ld16(ta, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              float a, b;
+              unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), f2), a, b);
+              v[i] = __float_as_uint(a);
+              v[i + 1] = __float_as_uint(b);
+            }
+            tmem_st16(ta, v);
+          }
+          tmem_st_wait();
+        }
+        if (move)
+          m_ref = m_blk;
+        // (packed fp32 below: two individually rounded operations per instruction)
+        const uint64_t scale2 = pack_f32x2(scale_log2e, scale_log2e);
+        const uint64_t neg_m2 = pack_f32x2(-m_ref, -m_ref);
+        const uint64_t minus1 = pack_f32x2(-1.0f, -1.0f);
+        uint64_t psum2 = pack_f32x2(0.0f, 0.0f);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t(&v)[32] = sv[h];
+          uint32_t whi[16], wlo[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            float a0, a1;
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[2 * i]),
+                                       __uint_as_float(v[2 * i + 1])),
+                             scale2, neg_m2),
+                a0, a1);
+            const float p0 = ex2_approx(a0), p1 = ex2_approx(a1);
+            const uint64_t p2 = pack_f32x2(p0, p1);
+            psum2 = add_f32x2(psum2, p2);
+            const uint32_t hi = cvt_bf16x2(p0, p1);
+            // p - hi: one rounding, as the subtraction has
+            float r0, r1;
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(hi << 16),
+                                       __uint_as_float(hi & 0xffff0000u)),
+                             minus1, p2),
+                r0, r1);
+            whi[i] = hi;
+            wlo[i] = cvt_bf16x2(r0, r1);
+          }
+          // P of 32 keys: hi in columns 0..15 of theirs, lo in 16..31 (the scores of those
+          // columns are already consumed).
+          tmem_st16(t_row + (uint32_t)(32 * h), whi);
+          tmem_st16(t_row + (uint32_t)(32 * h) + 16u, wlo);
+        }
+        float ps0, ps1;
+        unpack_f32x2(psum2, ps0, ps1);
+        l_run = __fadd_rn(l_run, __fadd_rn(ps0, ps1));
+        tmem_st_wait();
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0)
+          mbar_arrive(bar.p); // this warp's part of P is in tensor memory
+      }
+      ok = mbar_wait(bar.o, (n - 1u) & 1u, abortp, wait_ns) && ok; // the item's last P V
+      tcgen05_fence_after();
+      __syncwarp();
+      uint32_t o[32];
+      {
+        uint32_t v[32];
+        tmem_ld32(t_out, o); // P_hi V_hi + P_lo V_hi
+        tmem_ld32(t_out + 64u, v); // P_hi V_lo
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          float a, b;
+          unpack_f32x2(add_f32x2(pack_f32x2(__uint_as_float(o[i]), __uint_as_float(o[i + 1])),
+                           pack_f32x2(__uint_as_float(v[i]), __uint_as_float(v[i + 1]))),
+              a, b);
+          o[i] = __float_as_uint(a);
+          o[i + 1] = __float_as_uint(b);
+        }
+      }
+      tcgen05_fence_before(); // (what the next item's first arrival at bar.p publishes)
+
+      // Row sum over both halves, then normalise.
+      xch_sum[half][row] = l_run;
+      pair_barrier(quad);
+      const float inv = __fdiv_rn(1.0f, __fadd_rn(xch_sum[0][row], xch_sum[1][row]));
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const float f = __fmul_rn(__uint_as_float(o[i]), inv);
+        lo_run = fminf(lo_run, f);
+        hi_run = fmaxf(hi_run, f);
+        o[i] = __float_as_uint(f);
+      }
+      // The 128 x 64 result leaves through the K or the V buffers (att_loads): half 0's
+      // 32 columns in the first 16 KiB tile, half 1's in the second, rows of 128 bytes in the
+      // 128-byte swizzle pattern, one TMA store per tile, which writes whole lines.
+      const bool in_v = nkb == 1;
+      if (!in_v && item + gridDim.x < n_items)
+        ok = mbar_wait(bar.s, n & 1u, abortp, wait_ns) && ok;
+      const uint32_t my_row =
+          (in_v ? (half ? tiles.vl : tiles.vh) : (half ? tiles.kl : tiles.kh)) + (uint32_t)row * 128u;
+      const uint32_t swz = ((uint32_t)row & 7u) << 4;
+#pragma unroll
+      for (int i = 0; i < 32; i += 4)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(
+                         my_row + (((uint32_t)i * 4u) ^ swz)),
+                     "r"(o[i]), "r"(o[i + 1]), "r"(o[i + 2]), "r"(o[i + 3])
+                     : "memory");
+      fence_proxy_async_smem(); // the tiles were written through the generic proxy
+      __syncwarp();
+      if (lane == 0)
+        mbar_arrive(bar.r);
     }
-    fence_proxy_async_smem(); // the tiles were written through the generic proxy
-    __syncthreads();
-    if (warp == 0 && elect_one()) {
-      tma_store_2d(&map_out, s_vh, it.col_out, it.row_q);
-      tma_store_2d(&map_out, s_vl, it.col_out + 32, it.row_q);
-      tma_store_commit();
-    }
+    if (__all_sync(0xffffffffu, ok) && out_range)
+      range_commit_warp(out_range, lo_run, hi_run);
   }
-
-  if (ok && out_range && (int64_t)blockIdx.x < n_items)
-    range_commit_warp(out_range, lo_run, hi_run);
-  if (warp == 0 && elect_one())
-    tma_store_wait_all();
 
   // ---- teardown ----
   tcgen05_fence_before();

@@ -142,6 +142,23 @@ def test_attention_growing_and_shrinking_key_blocks(gpu, orc, scales):
           1e-3, 1e-3)
 
 
+@pytest.mark.parametrize("B,S", [(1, 128), (19, 128), (40, 128), (10, 256), (20, 256), (7, 384)])
+def test_attention_of_many_items(gpu, orc, B, S):
+    # 128 query rows of a head are an item of the tcgen05 kernel, two CTAs per SM (296 on a
+    # B200) walk them: one item each, a second and a third for some, whose copies, scores and
+    # results take turns in the same buffers.  A sequence alone takes the same sums in the
+    # same order, so its results are the same bits.
+    rng = np.random.default_rng(B + S)
+    heads, dh = 16, 64
+    q, k, v = (rng.normal(size=(B, S, heads * dh)).astype(np.float32) for _ in range(3))
+    scale = 1.0 / np.sqrt(dh)
+    got = gpu.attention(q, k, v, heads, scale)
+    for b in {0, B // 2, B - 1}:
+        alone = gpu.attention(q[b:b + 1], k[b:b + 1], v[b:b + 1], heads, scale)
+        assert np.array_equal(got[b:b + 1], alone)
+    close(alone, orc.attention(q[b:b + 1], k[b:b + 1], v[b:b + 1], heads, scale), 1e-3, 1e-5)
+
+
 def test_attention_peaked_scores(gpu, orc):
     # Head size 64 with a sequence that is a multiple of 128 runs on the
     # tcgen05 kernel; peaked scores (large logits) exercise the online
