@@ -264,6 +264,120 @@ __global__ void __launch_bounds__(kDqlThreads)
     y[rest] = (uint8_t)quantize_one<kSigned>(last, qc);
 }
 
+// Eight neighbouring values, p 32-byte aligned.  kOnce: they are not asked for again soon, L2
+// may let go of them first.
+struct Eight {
+  float4 a, b;
+};
+template <bool kOnce>
+__device__ __forceinline__ Eight load_eight(const float *p) {
+  Eight v;
+  if (kOnce)
+    asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.f32 {%0, %1, %2, %3, %4, %5, %6, "
+                 "%7}, [%8];"
+                 : "=f"(v.a.x), "=f"(v.a.y), "=f"(v.a.z), "=f"(v.a.w), "=f"(v.b.x), "=f"(v.b.y),
+                   "=f"(v.b.z), "=f"(v.b.w)
+                 : "l"(p));
+  else
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v.a.x), "=f"(v.a.y), "=f"(v.a.z), "=f"(v.a.w), "=f"(v.b.x), "=f"(v.b.y),
+                   "=f"(v.b.z), "=f"(v.b.w)
+                 : "l"(p));
+  return v;
+}
+
+// The pass by the exact formula, for scales quantize_four_fast does not take (of a tensor of
+// zeros, say).  Out of line, as the kernel below is short of registers.
+template <bool kSigned>
+__device__ __noinline__ void quantize_pass_exact(
+    const float *x, int64_t n, uint8_t *y, float scale, float zp_f, bool use_rcp) {
+  const int64_t step = (int64_t)gridDim.x * kDqlThreads, n4 = n >> 2;
+  const int64_t tid = (int64_t)blockIdx.x * kDqlThreads + threadIdx.x;
+  const float4 *x4 = reinterpret_cast<const float4 *>(x);
+#pragma unroll 1
+  for (int64_t i = tid; i < n4; i += 2 * step) {
+    const bool two = i + step < n4;
+    const float4 v = __ldg(x4 + i), w = two ? __ldg(x4 + i + step) : v;
+    const uint32_t a = quantize_four_exact<kSigned>(v, scale, zp_f, use_rcp);
+    const uint32_t b = quantize_four_exact<kSigned>(w, scale, zp_f, use_rcp);
+    reinterpret_cast<uint32_t *>(y)[i] = a;
+    if (two)
+      reinterpret_cast<uint32_t *>(y)[i + step] = b;
+  }
+  if (tid < (n & 3))
+    y[(n4 << 2) + tid] =
+        (uint8_t)quantize_one_exact<kSigned>(__ldg(x + (n4 << 2) + tid), scale, zp_f, use_rcp);
+}
+
+// The pass above for many values, x 32-byte and y 8-byte aligned.  That kernel takes what
+// lies in L2 hardly faster than what comes from HBM (16 Mi values 11.5 us, 7.4 without its
+// arithmetic): it executes 72 instructions per float4, half of them predicates and 64-bit
+// addresses.  Here runs are whole (what is left goes group by group), the addresses of a
+// run are one pointer and constants, a load is 32 bytes a lane and a store 8.  Two groups a
+// thread: four take 79 registers, three blocks per SM and no less time.  Whole calls,
+// before and now: DynamicQuantizeLinear of 1 Mi values 5.2 -> 4.9 us, 6 M 13.2 -> 11.9,
+// 16 Mi 28.6 -> 24.5, 64 Mi 99.1 -> 91.3, 128 Mi 201 -> 184; a given scale 2 M 3.7 -> 2.9,
+// 64 Mi 52.6 -> 50.0 (6.7 TB/s).
+constexpr int kWideGroups = 2;
+// Resident at once.  (Five leave 51 registers, and what then goes to memory costs
+// DynamicQuantizeLinear of 64 Mi 102 us instead of 92.)
+constexpr int kWideBlocksPerSm = 4;
+template <bool kSigned, bool kOnce>
+__global__ void __launch_bounds__(kDqlThreads, kWideBlocksPerSm)
+    quantize_wide_kernel(const float *__restrict__ x, int64_t n, uint8_t *__restrict__ y,
+        QuantSource src, QuantOutputs outs, int mode) {
+  pdl_sync();
+  x = after_pdl(x);
+  constexpr int kGroups = kWideGroups, kRun = kGroups * kDqlThreads;
+  const int64_t n8 = n >> 3;
+  const unsigned runs = (unsigned)(n8 / kRun);
+  unsigned r = blockIdx.x;
+  const float *xr = x + ((int64_t)r * kRun + threadIdx.x) * 8;
+  Eight v[kGroups];
+  if (r < runs)
+#pragma unroll
+    for (int u = 0; u < kGroups; ++u)
+      v[u] = load_eight<kOnce>(xr + u * (kDqlThreads * 8));
+  const QuantConsts qc = quant_scalars<kSigned>(src, outs, mode);
+  if (!qc.fast) {
+    quantize_pass_exact<kSigned>(x, n, y, qc.scale, qc.zp_f, qc.use_rcp);
+    return;
+  }
+  uint2 *yr = reinterpret_cast<uint2 *>(y) + ((int64_t)r * kRun + threadIdx.x);
+  while (r < runs) {
+    uint2 w[kGroups];
+#pragma unroll
+    for (int u = 0; u < kGroups; ++u)
+      w[u] = make_uint2(
+          quantize_four_fast<kSigned>(v[u].a, qc), quantize_four_fast<kSigned>(v[u].b, qc));
+    uint2 *const out = yr;
+    r += gridDim.x;
+    xr += (int64_t)gridDim.x * (kRun * 8);
+    yr += (int64_t)gridDim.x * kRun;
+    if (r < runs)
+#pragma unroll
+      for (int u = 0; u < kGroups; ++u)
+        v[u] = load_eight<kOnce>(xr + u * (kDqlThreads * 8));
+#pragma unroll
+    for (int u = 0; u < kGroups; ++u)
+      out[u * kDqlThreads] = w[u];
+  }
+  // what is left, from the last block on: those have the fewest runs
+  const unsigned b = gridDim.x - 1 - blockIdx.x;
+#pragma unroll 1
+  for (int64_t g = (int64_t)runs * kRun + (int64_t)b * kDqlThreads + threadIdx.x; g < n8;
+       g += (int64_t)gridDim.x * kDqlThreads) {
+    const Eight e = load_eight<kOnce>(x + 8 * g);
+    reinterpret_cast<uint2 *>(y)[g] =
+        make_uint2(quantize_four_fast<kSigned>(e.a, qc), quantize_four_fast<kSigned>(e.b, qc));
+  }
+  const int64_t j = (n8 << 3) + threadIdx.x;
+  if (b == 0 && j < n) {
+    const float f = __ldg(x + j);
+    y[j] = (uint8_t)quantize_four_fast<kSigned>(make_float4(f, f, f, f), qc);
+  }
+}
+
 // The same one value at a time, for tensors that are not aligned so.  A kernel of
 // its own, as for dequantize: the loads of several trips together take registers
 // that the one above would miss (in it, 64 Mi aligned values went from 54 to 57 us),
@@ -621,9 +735,9 @@ static int grid_for(int64_t work_items, int per_block) {
 // fastest with the blocks that are resident at once (16 Mi values: 13.0 us, with
 // a short block per run 15.8); what comes from HBM with short blocks, up to 64 per
 // SM, of which the last round is a small part (64 Mi: 51.6, resident ones 54.6).
-static int pass_grid(int64_t n, int run, bool resident) {
+static int pass_grid(int64_t n, int run, int resident) { // blocks per SM, 0: not only those
   int64_t want = ceil_div(n, run);
-  const int64_t cap = (int64_t)sm_count() * (resident ? 8 : 64);
+  const int64_t cap = (int64_t)sm_count() * (resident ? resident : 64);
   if (want < 1)
     want = 1;
   return (int)(want < cap ? want : cap);
@@ -636,6 +750,15 @@ static int quant_unroll(int64_t n) {
   return (int)(per < 1 ? 1 : per < kQuantUnroll ? per : kQuantUnroll);
 }
 
+// Whether quantize_wide_kernel takes a pass.  Behind a producer (an encoder's) from 24000
+// values: its few blocks leave the GEMM behind it the SMs (2 x 128 tokens of 768 567 -> 544 us,
+// 33 tokens 410 -> 405, but 16 tokens 431 -> 449); else where a block per 4096 values no longer
+// leaves SMs idle (given scale: 230000 values 1.95 -> 1.84 us, 187392 1.89 and 2.00).
+static bool quant_wide(const float *x, int64_t n, const uint8_t *y, bool behind_producer) {
+  return ((uintptr_t)x & 31u) == 0 && ((uintptr_t)y & 7u) == 0 &&
+         n >= (behind_producer ? 24000 : 200000);
+}
+
 template <typename T>
 static void launch_dequantize(const T *x, int64_t n, const float *scale, const T *zp,
     float *y, cudaStream_t st) {
@@ -645,7 +768,7 @@ static void launch_dequantize(const T *x, int64_t n, const float *scale, const T
   // take nothing that one needs.  2 us of each call, 1 Mi values 4.2 -> 2.1, 8191 x 3073 of 8
   // bits 22.7 -> 20.7, 64 Mi 55.0 -> 52.3.
   if (whole)
-    (void)launch_pdl(dequantize_kernel<T>, pass_grid(n, 256 * 4 * kDequantUnroll, false), 256, 0,
+    (void)launch_pdl(dequantize_kernel<T>, pass_grid(n, 256 * 4 * kDequantUnroll, 0), 256, 0,
         st, 0, true, x, n, scale, zp, y);
   else
     (void)launch_pdl(
@@ -669,10 +792,25 @@ int launch_quantize_pass(const float *x, int64_t n, uint8_t *y, const QuantSourc
   // (a given scale: 64 Mi values 55.2 -> 52.8 us; a pass of an encoder's, between GEMMs, by
   // the rule)
   const bool overlap = folds || src.scale || pdl_pays(n);
-  if (((uintptr_t)x & 15u) == 0 && ((uintptr_t)y & 3u) == 0)
+  // What a reduction or a producer has just had: what L2 still holds of it survives
+  // until the pass gets there if what the pass has read may go first (the whole call, 16 Mi
+  // values 25.9 and so 24.0 us, 32 Mi 50.8 and 45.4; encoder large 64 x 512 24.8 and 24.6 ms,
+  // 4 x 512 2418 and 2426 us).  Beyond what L2 could hold of it plain loads are faster (128 Mi 187
+  // and 194), as for a given scale (64 Mi 49.0 and 51.4).
+  const bool once = !src.scale && n <= ((int64_t)96 << 20);
+  // Few values behind a reduction: two blocks per SM.  It still holds SMs when this is set up,
+  // and of more blocks some start a round late (3.6 M values 9.3 us with four, 7.7 with two, 5 M
+  // 9.7 and 12.5; between the kernels of an encoder four are better at any size).
+  const int resident = folds && n <= 4800000 ? 2 : folds || in_l2 ? kWideBlocksPerSm : 0;
+  if (quant_wide(x, n, y, src.range != nullptr))
+    OMCUDA_CHECK(launch_pdl(!kSigned && once ? quantize_wide_kernel<kSigned, !kSigned>
+                                             : quantize_wide_kernel<kSigned, false>,
+        pass_grid(n, kWideGroups * 8 * kDqlThreads, resident), kDqlThreads, 0, st, 0,
+        overlap, x, n, y, src, outs, quant_mode()));
+  else if (((uintptr_t)x & 15u) == 0 && ((uintptr_t)y & 3u) == 0)
     OMCUDA_CHECK(launch_pdl(quantize_kernel<kSigned>,
-        pass_grid(n, kDqlThreads * 4 * unroll, folds || in_l2), kDqlThreads, 0, st, 0, overlap,
-        x, n, y, src, outs, quant_mode(), unroll));
+        pass_grid(n, kDqlThreads * 4 * unroll, folds || in_l2 ? 8 : 0), kDqlThreads, 0, st, 0,
+        overlap, x, n, y, src, outs, quant_mode(), unroll));
   else
     OMCUDA_CHECK(launch_pdl(quantize_single_kernel<kSigned>, grid_for(n, kDqlThreads * 4),
         kDqlThreads, 0, st, 0, overlap, x, n, y, src, outs, quant_mode()));

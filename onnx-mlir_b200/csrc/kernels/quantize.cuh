@@ -47,6 +47,7 @@ __device__ __forceinline__ uint32_t quantize_one_exact(
 // Per-launch constants of the fast path.
 struct QuantConsts {
   float scale, rcp, zp_f;
+  float fix; // what a residual of the quotient is multiplied by: rcp, or 0
   float x_lo, x_hi; // inputs beyond these saturate
   bool fast;
   bool use_rcp; // fast-math mode: the reference multiplies by RN(1 / scale)
@@ -69,6 +70,7 @@ __device__ __forceinline__ QuantConsts make_quant_consts(
   c.zp_f = (mode & OMCUDA_MODE_NO_ZERO_POINT) ? 0.0f : zp_f;
   c.use_rcp = (mode & OMCUDA_MODE_FAST_MATH) != 0;
   c.rcp = __fdiv_rn(1.0f, scale);
+  c.fix = c.use_rcp ? 0.0f : c.rcp;
   // A quarter beyond the last integer: a clamped input still rounds to it.
   c.x_lo = __fmul_rn(QuantBounds<kSigned>::lo - c.zp_f - 0.25f, scale);
   c.x_hi = __fmul_rn(QuantBounds<kSigned>::hi - c.zp_f + 0.25f, scale);
@@ -87,18 +89,14 @@ __device__ __forceinline__ QuantConsts make_quant_consts(
 // second residual is exact, as that asks: with |q| >= 1/4 (anything smaller
 // rounds to zero whatever its last bits are) and scale > 1e-30 its last bit is
 // at least 2^-149.
-// In fast-math mode the reference's quotient is RN(x y) itself: two plain products,
-// for the sums that follow would take a packed one in (see mul_f32x2).
+// In fast-math mode the reference's quotient is RN(x y) itself: the corrections then
+// multiply the residuals, which are finite, by zero.
 __device__ __forceinline__ uint64_t quotient_x2(uint64_t x, const QuantConsts &c) {
-  if (c.use_rcp) {
-    float x0, x1;
-    unpack_f32x2(x, x0, x1);
-    return pack_f32x2(__fmul_rn(x0, c.rcp), __fmul_rn(x1, c.rcp));
-  }
   const uint64_t y = pack_f32x2(c.rcp, c.rcp), ns = pack_f32x2(-c.scale, -c.scale);
+  const uint64_t fix = pack_f32x2(c.fix, c.fix);
   uint64_t q = mul_f32x2(x, y);
-  q = fma_f32x2(fma_f32x2(q, ns, x), y, q);
-  return fma_f32x2(fma_f32x2(q, ns, x), y, q);
+  q = fma_f32x2(fma_f32x2(q, ns, x), fix, q);
+  return fma_f32x2(fma_f32x2(q, ns, x), fix, q);
 }
 
 // Inputs that saturate, cut back to where they still do (a NaN goes to the lower
@@ -129,9 +127,7 @@ __device__ __noinline__ uint32_t quantize_four_exact(
 // at 0.499 a fifth of the warps had such an element among their 128 and took the
 // divide: 16 Mi values 16.4 us, 7.3 without any arithmetic.)
 template <bool kSigned>
-__device__ __forceinline__ uint32_t quantize_four(float4 v, const QuantConsts &c) {
-  if (!c.fast)
-    return quantize_four_exact<kSigned>(v, c.scale, c.zp_f, c.use_rcp);
+__device__ __forceinline__ uint32_t quantize_four_fast(float4 v, const QuantConsts &c) { // c.fast
   const uint64_t magic = pack_f32x2(kQuantMagic, kQuantMagic);
   const uint64_t zp = pack_f32x2(c.zp_f, c.zp_f);
   const uint64_t q01 = quotient_x2(pack_f32x2(quant_clamp(v.x, c), quant_clamp(v.y, c)), c);
@@ -141,6 +137,12 @@ __device__ __forceinline__ uint32_t quantize_four(float4 v, const QuantConsts &c
   const uint32_t b01 = __byte_perm((uint32_t)t01, (uint32_t)(t01 >> 32), 0x0040);
   const uint32_t b23 = __byte_perm((uint32_t)t23, (uint32_t)(t23 >> 32), 0x0040);
   return __byte_perm(b01, b23, 0x5410);
+}
+template <bool kSigned>
+__device__ __forceinline__ uint32_t quantize_four(float4 v, const QuantConsts &c) {
+  if (!c.fast)
+    return quantize_four_exact<kSigned>(v, c.scale, c.zp_f, c.use_rcp);
+  return quantize_four_fast<kSigned>(v, c);
 }
 
 template <bool kSigned>

@@ -413,6 +413,51 @@ def test_quantize_alignments(gpu, orc, n, xs, ys):
     assert s.item() == want_s and z.item() == want_z
 
 
+@pytest.mark.parametrize("n", [199999, 200000, 200007, 204800, 204801, 208897, 3031041, 39010313])
+@pytest.mark.parametrize("xs,ys", [(0, 0), (8, 8), (4, 0), (0, 4)])
+def test_wide_pass(gpu, orc, n, xs, ys):
+    """The pass with 32-byte loads: from 200000 values, where x starts on 32 bytes and y on 8
+    (else the 16-byte one), runs of 4096, what is left of them, more runs than resident
+    blocks; a scale it takes, scales left to the divide, and DynamicQuantizeLinear."""
+    import torch
+    rng = np.random.default_rng(n)
+    v = np.resize(rng.normal(0, 20, size=65537).astype(np.float32), n)
+    v[-3:] = (np.inf, -1e30, np.nan)
+    xt = torch.zeros(n + 8, device="cuda")
+    xt[xs:xs + n] = torch.from_numpy(v).cuda()
+    xd = gpu.Tensor.from_cuda_array(xt[xs:xs + n])
+    L = gpu.lib()
+    buf = torch.empty(n + 16, dtype=torch.uint8, device="cuda")
+
+    def check(want):
+        got = buf.cpu().numpy()
+        assert np.array_equal(got[ys:ys + n], want.view(np.uint8))
+        assert (got[:ys] == 99).all() and (got[ys + n:] == 99).all()
+
+    for scale, zp in ((0.37, np.array(131, np.uint8)), (0.21, np.array(-3, np.int8)),
+                      (0.0, np.array(7, np.uint8)), (1e-33, np.array(-7, np.int8))):
+        buf.fill_(99)
+        yt = buf[ys:ys + n] if zp.dtype == np.uint8 else buf.view(torch.int8)[ys:ys + n]
+        s, z = gpu.Tensor.from_numpy(np.array(scale, np.float32)), gpu.Tensor.from_numpy(zp)
+        torch.cuda.synchronize()
+        yd = gpu.Tensor.from_cuda_array(yt)
+        L.omcudaQuantizeLinear(yd.handle, xd.handle, s.handle, z.handle)
+        gpu.synchronize()
+        with np.errstate(all="ignore"):
+            check(orc.quantize(v, scale, float(zp), zp.dtype == np.int8))
+    v[-3:] = 0
+    xt[xs + n - 3:xs + n] = 0
+    buf.fill_(99)
+    s, z = torch.zeros((), device="cuda"), torch.zeros((), dtype=torch.uint8, device="cuda")
+    t = [gpu.Tensor.from_cuda_array(a) for a in (s, z, buf[ys:ys + n])]
+    torch.cuda.synchronize()
+    L.omcudaDynamicQuantizeLinear(t[2].handle, t[0].handle, t[1].handle, xd.handle)
+    gpu.synchronize()
+    want_y, want_s, want_z = orc.dynamic_quantize_linear(v)
+    check(want_y)
+    assert s.item() == want_s and z.item() == want_z
+
+
 @pytest.mark.parametrize("n", [65541, 75775, 113663, 113664, 113665, 114177])
 @pytest.mark.parametrize("at", ["first", "middle", "last"])
 def test_dynamic_quantize_extremes_of_small_blocks(gpu, orc, n, at):
