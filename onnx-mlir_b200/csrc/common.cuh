@@ -343,6 +343,47 @@ __device__ __forceinline__ void range_commit_warp(
   }
 }
 
+// The same for kernels of many warps.  The warps of a block leave their {min,max} in shared
+// memory and the last to come commits for all, without a barrier.  Blocks that start together
+// end together: each warp of them used to find the range as it was initialised and to send
+// its atomics to the one address, behind which the launch then waited (LayerNorm of 4096 x 768
+// 9.3 us, 6.0 without a range, 6.9 so; 1024 x 768 5.6, 3.2, 3.3).  For the same reason they do
+// not look first (a round trip to L2); later blocks do.
+struct RangeBlock {
+  uint32_t lo, hi;
+  int left; // warps that have not come
+};
+__device__ __forceinline__ void range_block_init(RangeBlock &b, int warps) { // one thread
+  b.lo = 0xffffffffu;
+  b.hi = 0;
+  b.left = warps;
+}
+constexpr unsigned kRangeFirstBlocks = 4 * 148; // about as many as start together
+// Behind a barrier of the block that follows range_block_init.  block: this one's number.
+__device__ __forceinline__ void range_commit_block(
+    RangeBlock &b, uint32_t *range, float lo, float hi, unsigned block) {
+  lo = warp_min(lo);
+  hi = warp_max(hi);
+  if ((threadIdx.x & 31) != 0)
+    return;
+  if (lo <= hi) {
+    atomicMin(&b.lo, f32_to_ordered(lo));
+    atomicMax(&b.hi, f32_to_ordered(hi));
+  }
+  __threadfence_block();
+  if (atomicSub(&b.left, 1) != 1)
+    return;
+  __threadfence_block();
+  const uint32_t ol = *(volatile uint32_t *)&b.lo, oh = *(volatile uint32_t *)&b.hi;
+  if (ol > oh)
+    return; // nothing but NaNs
+  volatile uint32_t *vr = range;
+  if (block < kRangeFirstBlocks || ol < vr[0])
+    atomicMin(range, ol);
+  if (block < kRangeFirstBlocks || oh > vr[1])
+    atomicMax(range + 1, oh);
+}
+
 #endif // __CUDACC__
 
 } // namespace omcuda

@@ -115,6 +115,9 @@ __global__ void __launch_bounds__(128)
   constexpr int NT_S = kKeys / 8;
 
   extern __shared__ __align__(16) __nv_bfloat16 att_smem[];
+  __shared__ RangeBlock range;
+  if (threadIdx.x == 0)
+    range_block_init(range, blockDim.x >> 5); // (barriers follow)
   pdl_sync();
   in.q = after_pdl(in.q);
   in.k = after_pdl(in.k);
@@ -317,7 +320,7 @@ __global__ void __launch_bounds__(128)
     }
   }
   if (out_range)
-    range_commit_warp(out_range, lo, hi);
+    range_commit_block(range, out_range, lo, hi, blockIdx.y * gridDim.x + blockIdx.x);
 }
 
 // The bf16 hi / lo planes of a fused projection, with the columns of Q, K and V in a row.
@@ -357,6 +360,9 @@ __global__ void __launch_bounds__(32 * kTiles * (kShared ? 2 : 1))
   constexpr int kTogether = 4; // tiles whose products are interleaved
 
   extern __shared__ __align__(16) __nv_bfloat16 att_smem[];
+  __shared__ RangeBlock range;
+  if (threadIdx.x == 0)
+    range_block_init(range, blockDim.x >> 5); // (barriers follow)
   pdl_sync();
   in.hi = after_pdl(in.hi);
   in.lo = after_pdl(in.lo);
@@ -635,7 +641,7 @@ __global__ void __launch_bounds__(32 * kTiles * (kShared ? 2 : 1))
     }
   }
   if (out_range)
-    range_commit_warp(out_range, lo, hi);
+    range_commit_block(range, out_range, lo, hi, blockIdx.y * gridDim.x + blockIdx.x);
 }
 
 } // namespace

@@ -415,6 +415,7 @@ __global__ void __launch_bounds__(kTcAttThreads, 2)
   // the block before last did: a thread gets there past a barrier that its partner reaches
   // after having read them.  So do the sums, for there is a block between any two.
   __shared__ float xch_max[2][2][kTQ], xch_sum[2][kTQ];
+  __shared__ RangeBlock range;
 
   const int tid = threadIdx.x, warp = warp_number(), lane = tid & 31;
   // Warps w and w + 4 share the 32 query rows (TMEM lanes) of quadrant w & 3:
@@ -439,6 +440,7 @@ __global__ void __launch_bounds__(kTcAttThreads, 2)
   }
   if (tid == 0) {
     abort_flag = 0;
+    range_block_init(range, kTcAttWarps);
     mbar_init(bar.q, 1);
     mbar_init(bar.k, 1);
     mbar_init(bar.v, 1);
@@ -656,7 +658,7 @@ __global__ void __launch_bounds__(kTcAttThreads, 2)
         mbar_arrive(bar.r);
     }
     if (__all_sync(0xffffffffu, ok) && out_range)
-      range_commit_warp(out_range, lo_run, hi_run);
+      range_commit_block(range, out_range, lo_run, hi_run, blockIdx.x);
   }
 
   // ---- teardown ----

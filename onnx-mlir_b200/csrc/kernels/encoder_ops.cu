@@ -100,6 +100,10 @@ __global__ void __launch_bounds__(256)
         const float *__restrict__ gamma, const float *__restrict__ beta,
         float eps, float *__restrict__ y, uint32_t *__restrict__ out_range) {
   constexpr int64_t cols = (int64_t)NV * 128;
+  __shared__ RangeBlock range;
+  if (threadIdx.x == 0)
+    range_block_init(range, blockDim.x >> 5);
+  __syncthreads();
   pdl_sync();
   // (opaque: an encoder run of 1 x 61 tokens 667 us, 673 with after_pdl)
   x = after_pdl_opaque(x);
@@ -173,7 +177,7 @@ __global__ void __launch_bounds__(256)
     }
   }
   if (out_range)
-    range_commit_warp(out_range, lo, hi);
+    range_commit_block(range, out_range, lo, hi, blockIdx.x);
 }
 
 // ---- elementwise -------------------------------------------------------------------

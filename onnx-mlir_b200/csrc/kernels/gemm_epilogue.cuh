@@ -192,12 +192,6 @@ __device__ __forceinline__ uint32_t epi_requant(const EpiParams &p,
   return t & 0xffu; // arith.trunci to 8 bits: wraps, does not saturate
 }
 
-// Folds a thread's {min,max} of the fp32 outputs into the running range.
-__device__ __forceinline__ void epi_range_commit(
-    uint32_t *range, float lo, float hi) {
-  range_commit_warp(range, lo, hi);
-}
-
 // D += A B of 16 x 8 x 32 bytes on the warp-level tensor path, which is what a handful
 // of rows wants: a tcgen05 tile would be mostly padding.
 template <bool kASigned, bool kBSigned>

@@ -236,6 +236,7 @@ __global__ void __launch_bounds__(kFewThreads, 3)
   __shared__ uint64_t bar_sums; // what the cluster sends has come
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
+  __shared__ RangeBlock range;
 
   const int tid = threadIdx.x, warp = warp_number(), lane = tid & 31;
   const int rank = split > 1 ? (int)cluster_ctarank() : 0;
@@ -275,6 +276,7 @@ __global__ void __launch_bounds__(kFewThreads, 3)
 
   if (warp == kFewWarps && elect_one()) {
     abort_flag = 0;
+    range_block_init(range, kFewWarps);
     for (int s = 0; s < ahead; ++s) {
       mbar_init(smem_u32(&bar_full[s]), 1);
       mbar_init(smem_u32(&bar_empty[s]), 1);
@@ -433,7 +435,7 @@ __global__ void __launch_bounds__(kFewThreads, 3)
     }
   }
   if (epi_is_dequant(EPI) && p.out_range && warp < kFewWarps)
-    epi_range_commit(p.out_range, lo, hi);
+    range_commit_block(range, p.out_range, lo, hi, blockIdx.y * gridDim.x + blockIdx.x);
 
   // ---------------- teardown ----------------
   if (split > 1)

@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(256)
     }
   }
   if (p.out_range && p.kind == OMCUDA_EPI_DEQUANT)
-    epi_range_commit(p.out_range, lo, hi);
+    range_commit_warp(p.out_range, lo, hi);
 }
 
 
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(32 * kWarps)
     __syncthreads(); // part[] is rewritten by the next group
   }
   if (warp == 0 && p.out_range && p.kind == OMCUDA_EPI_DEQUANT)
-    epi_range_commit(p.out_range, lo, hi);
+    range_commit_warp(p.out_range, lo, hi);
 }
 
 // ---- GEMV-shaped GEMM for 2..16 rows on mma.sync ---------------------------------
@@ -455,6 +455,9 @@ __global__ void __launch_bounds__(32 * kGemvMmaWarps)
   const bool vec_ok = ((p.lda & 15) == 0) && (((uintptr_t)A & 15u) == 0);
   const int64_t blocks64 = (kp + 63) >> 6;
   __shared__ int32_t part[kGemvMmaWarps][16][kCols + 1];
+  __shared__ RangeBlock range;
+  if (threadIdx.x == 0)
+    range_block_init(range, kGemvMmaWarps); // (barriers follow: every block has a group)
   float lo = INFINITY, hi = -INFINITY;
   const int64_t groups = ceil_div(p.N, kCols);
   if (blockIdx.y == 0)
@@ -543,7 +546,7 @@ __global__ void __launch_bounds__(32 * kGemvMmaWarps)
     __syncthreads(); // part[] is rewritten by the next group
   }
   if (p.out_range && p.kind == OMCUDA_EPI_DEQUANT)
-    epi_range_commit(p.out_range, lo, hi);
+    range_commit_block(range, p.out_range, lo, hi, blockIdx.y * gridDim.x + blockIdx.x);
 }
 
 EpiParams make_epi_params(const GemmCall &a) {

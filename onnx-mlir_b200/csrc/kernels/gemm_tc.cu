@@ -662,6 +662,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   __shared__ uint64_t bar_acc_empty[2];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
+  __shared__ RangeBlock range;
 
   const int warp = warp_number();
   const int lane = threadIdx.x & 31;
@@ -689,6 +690,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   }
   if (threadIdx.x == 0) {
     abort_flag = 0;
+    range_block_init(range, EW);
     for (int s = 0; s < kStages; ++s) {
       mbar_init(smem_u32(&bar_full[s]), 1);
       mbar_init(smem_u32(&bar_empty[s]), 1);
@@ -843,10 +845,10 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
               mbar_arrive(smem_u32(&bar_acc_empty[buf]));
           });
     }
-    // One commit of the running range per warp, and every store of this warp
+    // One commit of the running range per block, and every store of this warp
     // complete before the CTA may exit.
     if (p.out_range && tail_is_dequant(EPI) && EPI != OMCUDA_EPI_DEQUANT_QUANT)
-      epi_range_commit(p.out_range, lo, hi);
+      range_commit_block(range, p.out_range, lo, hi, blockIdx.x);
     if (elect_one())
       tma_store_wait_all();
   }
@@ -929,6 +931,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   __shared__ uint64_t bar_acc_empty[2];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
+  __shared__ RangeBlock range;
 
   const int warp = warp_number();
   const int lane = threadIdx.x & 31;
@@ -955,6 +958,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   }
   if (threadIdx.x == 0) {
     abort_flag = 0;
+    range_block_init(range, EW);
     for (int s = 0; s < kStages; ++s) {
       mbar_init(smem_u32(&bar_full[s]), 1);
       mbar_init(smem_u32(&bar_empty[s]), 1);
@@ -1121,7 +1125,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
         release();
     }
     if (p.out_range && tail_is_dequant(EPI) && EPI != OMCUDA_EPI_DEQUANT_QUANT)
-      epi_range_commit(p.out_range, lo, hi);
+      range_commit_block(range, p.out_range, lo, hi, blockIdx.x);
     if (elect_one())
       tma_store_wait_all();
   }
@@ -1366,7 +1370,7 @@ __global__ void __launch_bounds__(256)
     }
   }
   if (p.out_range && p.kind == OMCUDA_EPI_DEQUANT)
-    epi_range_commit(p.out_range, lo, hi);
+    range_commit_warp(p.out_range, lo, hi);
 }
 
 // The arguments of the pass that produces the raw partial sums.

@@ -197,3 +197,61 @@ def test_layernorm_rows_do_not_depend_on_their_number(gpu, rows, hidden):
         f = np.where(u & 0x80000000, u & 0x7fffffff, ~u).astype(np.uint32).view(np.float32)
         assert f[0] == out[-1].min() and f[1] == out[-1].max()
     assert out[0].tobytes() == out[1][:rows].tobytes()
+
+
+def _range(ranges):
+    u = ranges.numpy().view(np.uint32)
+    return np.where(u & 0x80000000, u & 0x7fffffff, ~u).astype(np.uint32).view(np.float32)
+
+
+@pytest.mark.parametrize("rows", [1, 7, 1184, 1185, 4736, 4745, 10001])
+@pytest.mark.parametrize("at", [0.0, 0.5, 1.0])
+def test_running_range_of_layernorm_blocks(gpu, rows, at):
+    # The warps of a block leave their minima and maxima to the last of them, blocks that start
+    # together commit without looking, later ones (from 592: 4736 rows) look first.  The
+    # extremes sit in one row; a row of NaNs adds nothing, nothing but NaNs leaves the range.
+    from omcuda import dev
+    hidden = 768
+    rng = np.random.default_rng(rows)
+    x = rng.normal(size=(rows, hidden)).astype(np.float32)
+    r = int(at * (rows - 1))
+    x[r, 5], x[r, 700] = 1e4, -9e3
+    if rows > 2:
+        x[(r + 1) % rows] = np.nan
+    d = lambda a: gpu.Tensor.from_numpy(a).to_device()
+    gamma, beta = d(np.ones(hidden, np.float32)), d(np.zeros(hidden, np.float32))
+    stream = gpu.lib().omcudaGetStream()
+    y = gpu.Tensor.device_empty((rows, hidden), np.float32)
+    ranges = gpu.Tensor.device_empty((2,), np.int32)
+    dev.range_init(ranges.data_ptr, 1, stream)
+    before = ranges.numpy()
+    dx, dn = d(x), d(np.full((rows, hidden), np.nan, np.float32))
+    dev.layernorm(dn.data_ptr, None, rows, hidden, gamma.data_ptr, beta.data_ptr, 1e-5,
+                  y.data_ptr, ranges.data_ptr, stream)
+    assert np.array_equal(ranges.numpy(), before)
+    dev.layernorm(dx.data_ptr, None, rows, hidden, gamma.data_ptr, beta.data_ptr, 1e-5,
+                  y.data_ptr, ranges.data_ptr, stream)
+    out = y.numpy()
+    assert tuple(_range(ranges)) == (np.nanmin(out), np.nanmax(out))
+    assert np.nanargmax(out) == r * hidden + 5
+
+
+@pytest.mark.parametrize("B,S,heads", [(1, 128, 1), (3, 256, 12), (26, 128, 12), (16, 384, 12)])
+def test_running_range_of_attention(gpu, B, S, heads):
+    from omcuda import dev
+    H = 64 * heads
+    rng = np.random.default_rng(B + S)
+    x = rng.normal(size=(B * S, 3 * H)).astype(np.float32)
+    x[B * S // 2, 2 * H + 1] = 300.0
+    stream = gpu.lib().omcudaGetStream()
+    planes = gpu.Tensor.device_empty((2, B * S, 3 * H), np.uint16)
+    out = gpu.Tensor.device_empty((B * S, H), np.float32)
+    ranges = gpu.Tensor.device_empty((2,), np.int32)
+    lo = planes.data_ptr + 2 * B * S * 3 * H
+    dx = gpu.Tensor.from_numpy(x).to_device()
+    dev.split_bf16(dx.data_ptr, B * S, 3 * H, 3 * H, planes.data_ptr, lo, 3 * H, 0, stream)
+    dev.range_init(ranges.data_ptr, 1, stream)
+    dev.attention_bf16(planes.data_ptr, lo, 3 * H, 0, H, 2 * H, B, S, heads, 64, 0.125,
+                       out.data_ptr, H, ranges.data_ptr, stream)
+    o = out.numpy()
+    assert tuple(_range(ranges)) == (o.min(), o.max())
