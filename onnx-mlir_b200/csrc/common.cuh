@@ -74,6 +74,12 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, unsigned block,
   }
   return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
+
+// Shared memory that a kernel does not use, but that keeps more than per_sm of its blocks
+// off an SM (of 228 KiB, 1 KiB of which is taken per block).  Set up behind a kernel that
+// fills the SMs it runs on, blocks go to the first that are left, as many as fit, and half of
+// the machine may then have none.
+inline size_t spread_bytes(int64_t per_sm) { return (size_t)(228 * 1024 / (per_sm + 1) - 896); }
 #endif
 
 // ---- device side -----------------------------------------------------------

@@ -802,12 +802,30 @@ int launch_quantize_pass(const float *x, int64_t n, uint8_t *y, const QuantSourc
   // and of more blocks some start a round late (3.6 M values 9.3 us with four, 7.7 with two, 5 M
   // 9.7 and 12.5; between the kernels of an encoder four are better at any size).
   const int resident = folds && n <= 4800000 ? 2 : folds || in_l2 ? kWideBlocksPerSm : 0;
-  if (quant_wide(x, n, y, src.range != nullptr))
-    OMCUDA_CHECK(launch_pdl(!kSigned && once ? quantize_wide_kernel<kSigned, !kSigned>
-                                             : quantize_wide_kernel<kSigned, false>,
-        pass_grid(n, kWideGroups * 8 * kDqlThreads, resident), kDqlThreads, 0, st, 0,
-        overlap, x, n, y, src, outs, quant_mode()));
-  else if (((uintptr_t)x & 15u) == 0 && ((uintptr_t)y & 3u) == 0)
+  if (quant_wide(x, n, y, src.range != nullptr)) {
+    const auto kernel =
+        !kSigned && once ? quantize_wide_kernel<kSigned, !kSigned> : quantize_wide_kernel<kSigned, false>;
+    const int grid = pass_grid(n, kWideGroups * 8 * kDqlThreads, resident);
+    // Two or three blocks per SM, kept apart (encoder base 8 x 128 716 -> 708 us, 3 x 500 1122 ->
+    // 1107, large 2 x 512 1850 -> 1823; one per SM is better left to the GEMM behind it, 2 x 128 515
+    // and 518).
+    const int64_t per_sm = ceil_div((int64_t)grid, (int64_t)sm_count());
+    size_t spread = 0;
+    if (src.range && overlap && per_sm > 1 && per_sm < kWideBlocksPerSm) {
+      static PerDeviceInt can[2]; // 1: yes, 2: no
+      PerDeviceInt &c = can[once];
+      if (!c.get()) {
+        c.set(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                  (int)spread_bytes(2)) == cudaSuccess
+                  ? 1
+                  : 2);
+        (void)cudaGetLastError();
+      }
+      spread = c.get() == 1 ? spread_bytes(per_sm) : 0;
+    }
+    OMCUDA_CHECK(launch_pdl(kernel, (unsigned)grid, kDqlThreads, spread, st, 0, overlap, x, n, y,
+        src, outs, quant_mode()));
+  } else if (((uintptr_t)x & 15u) == 0 && ((uintptr_t)y & 3u) == 0)
     OMCUDA_CHECK(launch_pdl(quantize_kernel<kSigned>,
         pass_grid(n, kDqlThreads * 4 * unroll, folds || in_l2 ? 8 : 0), kDqlThreads, 0, st, 0,
         overlap, x, n, y, src, outs, quant_mode(), unroll));

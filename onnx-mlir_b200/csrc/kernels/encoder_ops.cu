@@ -451,6 +451,36 @@ extern "C" int omcudaDevSoftmax(
   return OMCUDA_OK;
 }
 
+namespace {
+
+// Overlapped, its blocks are kept apart: behind a GEMM whose CTAs fill their SMs, 512 blocks of
+// 8 rows of 768 took 9.5 us (in a row of their own 6.9), so 8.2; encoder base 32 x 128 1350 -> 1315
+// us, large 4 x 512 2439 -> 2323; of few rows base 2 x 128 517 -> 515.
+template <int NV, bool kFew>
+int launch_layernorm_vec(const float *x, const float *residual, int64_t rows, const float *gamma,
+    const float *beta, float eps, float *y, uint32_t *range, unsigned warps, cudaStream_t st) {
+  const auto kernel = layernorm_rows_vec_kernel<NV, kFew>;
+  const bool overlap = pdl_pays(rows * NV * 128);
+  const int64_t blocks = ceil_div(rows, warps), per_sm = ceil_div(blocks, (int64_t)sm_count());
+  size_t spread = 0;
+  if (overlap && per_sm < 8) { // (eight fit without it)
+    static PerDeviceInt can; // 1: yes, 2: no
+    if (!can.get()) {
+      can.set(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                  (int)spread_bytes(1)) == cudaSuccess
+                  ? 1
+                  : 2);
+      (void)cudaGetLastError();
+    }
+    spread = can.get() == 1 ? spread_bytes(per_sm) : 0;
+  }
+  OMCUDA_CHECK(launch_pdl(kernel, (unsigned)blocks, 32 * warps, spread, st, 0, overlap, x,
+      residual, rows, gamma, beta, eps, y, range));
+  return OMCUDA_OK;
+}
+
+} // namespace
+
 extern "C" int omcudaDevLayerNorm(const float *x, const float *residual,
     int64_t rows, int64_t cols, const float *gamma, const float *beta,
     float eps, float *y, void *out_minmax, void *stream) {
@@ -467,16 +497,17 @@ extern "C" int omcudaDevLayerNorm(const float *x, const float *residual,
   // and gamma and beta ahead.
   const bool few = rows <= 8 * (int64_t)sm_count();
   const unsigned warps = few && rows > 0 ? (unsigned)ceil_div(rows, (int64_t)sm_count()) : 8;
-  if (vec_ok && (cols == 768 || cols == 1024))
-    OMCUDA_CHECK(launch_pdl(cols == 768 ? (few ? layernorm_rows_vec_kernel<6, true>
-                                               : layernorm_rows_vec_kernel<6, false>)
-                                        : (few ? layernorm_rows_vec_kernel<8, true>
-                                               : layernorm_rows_vec_kernel<8, false>),
-        (unsigned)ceil_div(rows, warps), 32 * warps, 0, st, 0, pdl_pays(rows * cols), x, residual,
-        rows, gamma, beta, eps, y, rng));
-  else
+  if (vec_ok && (cols == 768 || cols == 1024)) {
+    const auto launch = cols == 768
+                            ? (few ? launch_layernorm_vec<6, true> : launch_layernorm_vec<6, false>)
+                            : (few ? launch_layernorm_vec<8, true> : launch_layernorm_vec<8, false>);
+    const int rc = launch(x, residual, rows, gamma, beta, eps, y, rng, warps, st);
+    if (rc != OMCUDA_OK)
+      return rc;
+  } else {
     layernorm_rows_kernel<<<grid, 256, 0, st>>>(
         x, residual, rows, cols, gamma, beta, eps, y, rng);
+  }
   OMCUDA_CHECK_LAUNCH("layernorm_rows_kernel");
   return OMCUDA_OK;
 }
