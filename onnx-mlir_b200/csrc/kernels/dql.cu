@@ -64,10 +64,14 @@ __device__ __forceinline__ void block_range(float &lo, float &hi) {
 // Bound by the read of x: 64 Mi values in 39 us (6.9 TB/s), 16 Mi that lie in L2 in
 // 6 (11 TB/s).  Plain loads and not streaming ones: the quantize pass finds in
 // L2 what still fits there.  kFull: the run is kRangeUnroll float4 a thread, known to
-// the compiler (64 Mi values 104 us the whole call without that, 101 with).  kZero: sets the `zeros` words of `sums` to zero as well,
-// for a pass behind it that adds to them.
-template <bool kFull, bool kZero, int kThreads>
-__global__ void __launch_bounds__(kThreads)
+// the compiler (64 Mi values 104 us the whole call without that, 101 with).  kZero: sets the
+// `zeros` words of `sums` to zero as well, for a pass behind it that adds to them.  kDeep:
+// registers for all loads of a run at once.  With the 32 of a full SM the compiler makes two or
+// three round trips of them, all that a few blocks have to do: linear 128 x 4096 x 4096 17.9 ->
+// 15.3 us, 64 x 8192 x 8192 24.3 -> 22.0, 700 x 768 x 768 11.3 -> 10.3, 777 x 1001 x 1537 17.3 -> 16.2;
+// DynamicQuantizeLinear of 600000 values 5.2 -> 4.6, 6 M 11.9 -> 10.8, 64 Mi 92.9 -> 90.8.
+template <bool kFull, bool kZero, int kThreads, bool kDeep>
+__global__ void __launch_bounds__(kThreads, kDeep ? 1024 / kThreads : 2048 / kThreads)
     dql_minmax_kernel(const float *__restrict__ x, int64_t n, float2 *__restrict__ part,
         int unroll, int32_t *__restrict__ sums, int zeros) {
   pdl_sync();
@@ -861,21 +865,24 @@ int launch_range_parts(const float *x, int64_t n, void *scratch, RangeParts *par
   // 70000 values 4.21 -> 3.96 us, 100000 4.23 -> 4.06, linear 128 x 768 x 768 8.71 -> 8.59, 35 x
   // 2500 x 640 9.42 -> 9.08, but 100 x 1024 x 1024 9.16 and 9.25; 150000 4.32 and 4.49.
   const int64_t small_blocks = ceil_div(n, (int64_t)kRangeFewThreads * 4);
-  if (aligned && 2 * small_blocks <= 3 * sm_count()) {
+  const bool few = aligned && 2 * small_blocks <= 3 * sm_count();
+  if (few)
     grid = small_blocks < 1 ? 1 : small_blocks;
-    OMCUDA_CHECK(launch_pdl(sums ? dql_minmax_kernel<false, true, kRangeFewThreads>
-                                 : dql_minmax_kernel<false, false, kRangeFewThreads>,
-        (unsigned)grid, kRangeFewThreads, 0, st, 0, overlap, x, n, part, 1, sums, zeros));
-    OMCUDA_CHECK_LAUNCH("dql_minmax_kernel");
-    parts->part = part;
-    parts->count = (int)grid;
-    return OMCUDA_OK;
-  }
-  OMCUDA_CHECK(launch_pdl(full ? (sums ? dql_minmax_kernel<true, true, kRangeThreads>
-                                       : dql_minmax_kernel<true, false, kRangeThreads>)
-                               : (sums ? dql_minmax_kernel<false, true, kRangeThreads>
-                                       : dql_minmax_kernel<false, false, kRangeThreads>),
-      (unsigned)grid, kRangeThreads, 0, st, 0, overlap, x, n, part, unroll, sums, zeros));
+  // All loads of a run in flight, except where the blocks are one to two per SM: more of
+  // them than fit with those registers beside what else is resident (3.1 M values 6.8 us
+  // without, 8.3 with; 6 M 11.9 and 10.8).
+  const bool deep = grid <= sm_count() || grid > 2 * sm_count();
+  const auto kernel =
+      few     ? (sums ? dql_minmax_kernel<false, true, kRangeFewThreads, true>
+                      : dql_minmax_kernel<false, false, kRangeFewThreads, true>)
+      : !full ? (sums ? dql_minmax_kernel<false, true, kRangeThreads, true>
+                      : dql_minmax_kernel<false, false, kRangeThreads, true>)
+      : deep  ? (sums ? dql_minmax_kernel<true, true, kRangeThreads, true>
+                      : dql_minmax_kernel<true, false, kRangeThreads, true>)
+              : (sums ? dql_minmax_kernel<true, true, kRangeThreads, false>
+                      : dql_minmax_kernel<true, false, kRangeThreads, false>);
+  OMCUDA_CHECK(launch_pdl(kernel, (unsigned)grid, few ? kRangeFewThreads : kRangeThreads, 0, st, 0,
+      overlap, x, n, part, few ? 1 : unroll, sums, zeros));
   OMCUDA_CHECK_LAUNCH("dql_minmax_kernel");
   parts->part = part;
   parts->count = (int)grid;

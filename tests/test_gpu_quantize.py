@@ -413,6 +413,18 @@ def test_quantize_alignments(gpu, orc, n, xs, ys):
     assert s.item() == want_s and z.item() == want_z
 
 
+@pytest.mark.parametrize("n", [113700, 802815, 802821, 2424830, 2424833, 4849663, 4849668, 9699333])
+@pytest.mark.parametrize("at", [0.0, 0.37, 1.0])
+def test_dynamic_quantize_extremes_of_deep_and_full_blocks(gpu, orc, n, at):
+    """The reduction's forms (runs of one to eight groups; up to one, one to two and more
+    blocks of 16384 values per SM; single values): an extreme anywhere is found."""
+    x = np.random.default_rng(n).normal(size=4096).astype(np.float32)
+    x = np.resize(x, n)
+    i = min(int(at * n), n - 2)
+    x[i], x[i + 1] = 77.0, -55.0
+    check_dql(gpu, orc, x, device=True)
+
+
 @pytest.mark.parametrize("n", [199999, 200000, 200007, 204800, 204801, 208897, 3031041, 39010313])
 @pytest.mark.parametrize("xs,ys", [(0, 0), (8, 8), (4, 0), (0, 4)])
 def test_wide_pass(gpu, orc, n, xs, ys):
