@@ -595,7 +595,10 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
       }
       // The row pitch of Y is not a multiple of 16 bytes (a ragged N), so no TMA
       // store: a 32 x 32 block passes through the slab and every row leaves as
-      // one coalesced warp-wide store, instead of 32 rows in 32 sectors each.
+      // one coalesced warp-wide store, instead of 32 rows in 32 sectors each.  Eight rows
+      // together, their words asked for before the first leaves (before, row after row:
+      // QLinearMatMul 16384 x 768 x 3001 99.7 -> 84.0 us, 2000 x 1024 x 1537 18.9 -> 17.5, linear
+      // 16384 x 768 x 1537 79.6 -> 75.1; sixteen gain no more).
       if (kSplit) {
         if (lane >= rows)
           continue;
@@ -619,22 +622,33 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
       __syncwarp();
       const int piece = kBytesOut ? lane >> 4 : lane >> 2;
       const uint32_t in_piece = kBytesOut ? (uint32_t)(lane & 15) & ~3u : (uint32_t)(lane & 3) * 4u;
-      for (int r = 0; r < rows; ++r) {
-        const uint32_t w = ld_shared_u32(
-            slab0 + (uint32_t)r * 128u + (uint32_t)((piece ^ (r & 7)) * 16) + in_piece);
-        if (lane < valid) {
-          const int64_t y_at = (m_warp + r) * p.N + nc + lane;
-          if (kRes) {
-            const float f = __fadd_rn(__uint_as_float(w), __ldg(p.residual + y_at));
-            lo = fminf(lo, f);
-            hi = fmaxf(hi, f);
-            reinterpret_cast<float *>(p.Y)[y_at] = f;
-          } else if (!kBytesOut) {
-            reinterpret_cast<uint32_t *>(p.Y)[y_at] = w;
-          } else {
-            reinterpret_cast<uint8_t *>(p.Y)[y_at] = (uint8_t)(w >> (8 * (lane & 3)));
-          }
+#pragma unroll 1
+      for (int r0 = 0; r0 < rows; r0 += 8) {
+        uint32_t w[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+          w[r] = ld_shared_u32(
+              slab0 + (uint32_t)(r0 + r) * 128u + (uint32_t)((piece ^ r) * 16) + in_piece);
+        const int64_t y0 = (m_warp + r0) * p.N + nc + lane;
+        if (kRes && lane < valid) {
+#pragma unroll
+          for (int r = 0; r < 8; ++r)
+            if (r0 + r < rows) {
+              const float f =
+                  __fadd_rn(__uint_as_float(w[r]), __ldg(p.residual + y0 + r * p.N));
+              lo = fminf(lo, f);
+              hi = fmaxf(hi, f);
+              w[r] = __float_as_uint(f);
+            }
         }
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+          if (lane < valid && r0 + r < rows) {
+            if (!kBytesOut)
+              reinterpret_cast<uint32_t *>(p.Y)[y0 + r * p.N] = w[r];
+            else
+              reinterpret_cast<uint8_t *>(p.Y)[y0 + r * p.N] = (uint8_t)(w[r] >> (8 * (lane & 3)));
+          }
       }
     }
   }

@@ -931,6 +931,41 @@ def test_ragged_k_and_n(gpu, orc, M, K, N, wdt):
         assert np.array_equal(gpu.qlinear_matmul(*args), orc.qlinear_matmul(*args))
 
 
+@pytest.mark.parametrize("rest", [1, 7, 8, 9, 24, 25, 31])
+@pytest.mark.parametrize("N", [259, 1537])
+@pytest.mark.parametrize("tail", ["i32", "dequant", "requant"])
+def test_ragged_rows_leave_eight_together(gpu, rest, N, tail):
+    # The last 32-row block of a tile has `rest` rows, the last 32 columns 3 or 1: whole
+    # results, and nothing before or behind them.
+    M, K, pad = 672 + rest, 64, 64
+    rng = np.random.default_rng(rest + N)
+    A, B = rand8(rng, (M, K), np.uint8), rand8(rng, (K, N), np.int8)
+    dg = DevGemm(gpu)
+    D = dg.dev
+    pb, keep = dg.prepare(B)
+    dA = dg.dtensor(A)
+    esize = 1 if tail == "requant" else 4
+    Y = dg.dtensor(np.full((M * N + 2 * pad) * esize, 0x5a, np.uint8))
+    S = dg.dtensor(np.full(1, 0.03125, np.float32))
+    g = D.GemmArgs()
+    g.M, g.N, g.K, g.A, g.a_signed, g.B = M, N, K, dA.data_ptr, 0, pb
+    g.Y = Y.data_ptr + pad * esize
+    g.sa = g.sb = S.data_ptr
+    g.sb_len = 1
+    g.kernel_choice = D.KERNEL_TENSOR_CORE
+    g.epilogue = {"i32": D.EPI_I32, "dequant": D.EPI_DEQUANT, "requant": D.EPI_REQUANT}[tail]
+    if tail == "requant":
+        g.sa = None
+    D.gemm_i8(g, dg.stream)
+    out = Y.numpy()
+    gpu.synchronize()
+    acc = A.astype(np.int64) @ B.astype(np.int64)
+    want = {"i32": acc.astype(np.int32), "dequant": (acc * 2.0 ** -10).astype(np.float32),
+            "requant": np.rint(acc * 2.0 ** -5).astype(np.int64).astype(np.uint8)}[tail]
+    assert out[pad * esize:-pad * esize].tobytes() == want.tobytes()
+    assert (out[:pad * esize] == 0x5a).all() and (out[-pad * esize:] == 0x5a).all()
+
+
 @pytest.mark.parametrize("ydt", [np.uint8, np.int8])
 @pytest.mark.parametrize("M,K,N,per_column", [(1, 64, 40, False), (9, 48, 33, True),
                                               (40, 100, 300, True), (300, 64, 512, False)])
