@@ -1323,10 +1323,20 @@ struct SplitPlan {
   int32_t *ws = nullptr; // [split][ws_rows][N]
 };
 
-// One thread per four adjacent outputs of a row.
+// One thread per four adjacent outputs of a row, the loads of four slices together.  Set up
+// behind the pass that writes them, its own successor only when its blocks leave: with the
+// operator's next reduction set up while it runs, 256 x 14336 x 4096 took 35.6 us instead of 33.5
+// (36.4 without any overlap; 128 x 14336 x 2400 26.8 -> 24.5, 512 x 12000 x 4096 46.2 -> 44.7).
 __global__ void __launch_bounds__(256)
     splitk_reduce_kernel(const int32_t *__restrict__ ws, int split, int64_t ws_rows,
-        EpiParams p) {
+        EpiParams args) {
+  __shared__ RangeBlock range;
+  if (threadIdx.x == 0)
+    range_block_init(range, blockDim.x >> 5);
+  __syncthreads();
+  pdl_wait();
+  ws = after_pdl(ws);
+  const EpiParams p = epi_after_pdl(args);
   const int64_t n4 = p.N >> 2; // the split path requires N % 4 == 0
   const int64_t total = p.M * n4;
   const EpiScalars sc = epi_scalars(p);
@@ -1336,13 +1346,21 @@ __global__ void __launch_bounds__(256)
        i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t m = i / n4, n = (i - m * n4) << 2;
     int4 acc = make_int4(0, 0, 0, 0);
-    for (int k = 0; k < split; ++k) {
-      const int4 v = __ldcs(reinterpret_cast<const int4 *>(
-          ws + ((int64_t)k * ws_rows + m) * p.N + n));
-      acc.x += v.x;
-      acc.y += v.y;
-      acc.z += v.z;
-      acc.w += v.w;
+    const int32_t *src = ws + m * p.N + n;
+    const int64_t slice = ws_rows * p.N;
+    for (int k0 = 0; k0 < split; k0 += 4) {
+      int4 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        v[k] = k0 + k < split ? __ldcs(reinterpret_cast<const int4 *>(src + (k0 + k) * slice))
+                              : make_int4(0, 0, 0, 0);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        acc.x += v[k].x;
+        acc.y += v[k].y;
+        acc.z += v[k].z;
+        acc.w += v[k].w;
+      }
     }
     const EpiRow row = epi_row(p, m);
     const int32_t v[4] = {epi_int(p, row, acc.x, n), epi_int(p, row, acc.y, n + 1),
@@ -1384,7 +1402,7 @@ __global__ void __launch_bounds__(256)
     }
   }
   if (p.out_range && p.kind == OMCUDA_EPI_DEQUANT)
-    range_commit_warp(p.out_range, lo, hi);
+    range_commit_block(range, p.out_range, lo, hi, blockIdx.x);
 }
 
 // The arguments of the pass that produces the raw partial sums.
@@ -1693,9 +1711,10 @@ int launch_split_k(const GemmCall &a, cudaStream_t st, int split) {
     const int64_t total = a.M * (a.N >> 2);
     const int64_t blocks = ceil_div(total, 256);
     const int64_t cap = (int64_t)sm_count() * 8;
-    splitk_reduce_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(
-        plan.ws, split, plan.ws_rows, p);
-    cudaError_t ce = cudaGetLastError();
+    cudaError_t ce = launch_pdl(splitk_reduce_kernel, (unsigned)(blocks < cap ? blocks : cap), 256,
+        0, st, 0, true, plan.ws, split, plan.ws_rows, p);
+    if (ce == cudaSuccess)
+      ce = cudaGetLastError();
     if (ce != cudaSuccess)
       rc = fail(OMCUDA_ECUDA, "splitk_reduce_kernel: %s", cudaGetErrorString(ce));
     else
