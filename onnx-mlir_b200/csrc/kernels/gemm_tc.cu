@@ -1334,7 +1334,10 @@ __global__ void __launch_bounds__(256)
   if (threadIdx.x == 0)
     range_block_init(range, blockDim.x >> 5);
   __syncthreads();
-  pdl_wait();
+  if (args.early_next)
+    pdl_sync();
+  else
+    pdl_wait();
   ws = after_pdl(ws);
   const EpiParams p = epi_after_pdl(args);
   const int64_t n4 = p.N >> 2; // the split path requires N % 4 == 0
