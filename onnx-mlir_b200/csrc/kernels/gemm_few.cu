@@ -303,7 +303,10 @@ __global__ void __launch_bounds__(kFewThreads, 3)
   const uint32_t tmem_base = tmem_base_slot;
   if (split > 1)
     cluster_arrive(); // "has started": waited for before the first copy
-  pdl_sync();
+  if (p.early_next)
+    pdl_sync();
+  else
+    pdl_wait();
   const EpiParams e = epi_after_pdl(p);
 
   if (warp == kFewWarps) {

@@ -315,7 +315,10 @@ __global__ void __launch_bounds__(32 * kWarps)
   const int64_t groups = ceil_div(p.N, CB);
   for (int64_t g = blockIdx.x; g < groups; g += gridDim.x)
     prefetch_weight(Bt, kp, g * CB, CB, p.N);
-  pdl_sync();
+  if (p.early_next)
+    pdl_sync();
+  else
+    pdl_wait();
   // (opaque: with after_pdl the compiler overlaps trips and takes 94 registers
   // instead of 64, and 1 x 4096 x 14336 went from 17.7 to 18.5 us in blocks of four warps)
   A = after_pdl_opaque(A);
@@ -463,7 +466,10 @@ __global__ void __launch_bounds__(32 * kGemvMmaWarps)
   if (blockIdx.y == 0)
     for (int64_t grp = blockIdx.x; grp < groups; grp += gridDim.x)
       prefetch_weight(Bt, kp, grp * kCols, kCols, p.N);
-  pdl_sync();
+  if (p.early_next)
+    pdl_sync();
+  else
+    pdl_wait();
   A = after_pdl(A);
   Bt = after_pdl(Bt);
   const EpiScalars sc = epi_scalars(p);

@@ -88,7 +88,7 @@ struct GemmCall : omcudaGemmArgs {
   // The host has seen the preparation of B finish: no kernel that may still be running when
   // this GEMM is set up writes it.
   bool b_settled;
-  // The kernel behind may be set up while this product runs (gemm_tc.cu).  Not for the
+  // The kernel behind may be set up while this product runs.  Not for the
   // operators, whose successor may be anything: the blocks of a pass that come early find
   // the SMs of this kernel's last tiles taken and stay together on those that were free.  us
   // of a chain of calls, set up early / at the end (and before dequantize and the passes of
@@ -99,6 +99,8 @@ struct GemmCall : omcudaGemmArgs {
   //   4096 x 4096 x 4096   linear after linear                           168 / 159 (180)
   //   777 x 1001 x 1537                                                  35.7 / 33.1 (37.2)
   //   700 x 768 x 768                                                    23.5 / 22.9 (25.0)
+  // One linear of few rows after another, the same way: 128 x 768 x 768 8.5 / 8.1, 64 x 8192 x 8192
+  // 21.6 / 21.1, 61 x 768 x 768 8.0 / 7.7; of one row 768 x 3072 5.8 / 5.6, 4096 x 14336 14.9 / 14.9.
   // For the encoder's, behind which LayerNorm, attention and the quantize pass that folds
   // nothing wait: base 32 x 128 tokens 1400 / 1479, large 32 x 128 3384 / 3527, base 8 x 128 787 /
   // 802 us.
