@@ -929,7 +929,10 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
   g.K = d.K;
   g.lda = (d.K + 15) & ~int64_t(15);
   // (one launch writes parts of Y while others still read X, so not onto X)
+  // More than one group of columns per cluster: quantize and product are faster (the figures are
+  // at linear_rows_wanted), but take scratch, which a captured call must not.
   if (d.K > 0 && linear_rows_wanted(d.M, d.N, g.lda) &&
+      !(wzn <= 1 && linear_rows_groups(d.N) > 1 && !is_capturing(st)) &&
       !ranges_overlap(dX, d.M * d.K * 4, dY, d.M * d.N * 4)) {
     if (wzn) {
       g.b_zp = dWz;

@@ -68,7 +68,12 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
   const int len = (int)(kp - k0 < slice ? (kp > k0 ? kp - k0 : 0) : slice); // of Bt
   uint8_t *a_rows = rows_mem; // [16][pitch]
   int32_t *part = reinterpret_cast<int32_t *>(rows_mem + kRowsMax * pitch); // [rounds][16][64]
-  pdl_sync();
+  // (the successor at the end, see GemmCall::early_next: 16 x 768 x 768 5.9 -> 5.7 us; not where
+  // it may prefetch a weight meanwhile, 2 x 8192 x 8192 16.7 and 18.0)
+  if (rounds > 1)
+    pdl_sync();
+  else
+    pdl_wait();
   x = after_pdl(x);
   Bt = after_pdl(Bt);
   const EpiParams e = epi_after_pdl(p);
@@ -285,6 +290,8 @@ int rows_rounds(int64_t N) {
 
 } // namespace
 
+int linear_rows_groups(int64_t N) { return rows_rounds(N); }
+
 bool linear_rows_wanted(int64_t M, int64_t N, int64_t kp) {
   // Every cluster reads all of x, so x has to be small next to the weight a cluster
   // reads: 16 x 256 x 256 5.8 us here and 7.0 as quantize and product, 16 x 768 x 768 5.8
@@ -294,9 +301,11 @@ bool linear_rows_wanted(int64_t M, int64_t N, int64_t kp) {
   // was more than 2 % faster as two kernels.  Against the few-rows kernel, which now makes
   // the product of large weights, that holds for one column group per cluster (0.55 to
   // 0.94 of the two kernels' time on 39 sizes), not for more (1.02 to 1.8 on 19): 2 x
-  // 8192 x 8192 16.6 and 12.0 with the weight in L2, 19.4 and 16.9 beyond, 2 x 4096 x 14336
-  // 15.5 and 11.1, 18.0 and 15.4, 15 x 2176 x 15360 17.2 and 9.5, 19.7 and 12.1, 5 x 1650 x 5419
-  // 8.7 and 8.4, 9.4 and 8.8.
+  // 8192 x 8192 16.8 and 11.6 with the weight in L2, 19.5 and 16.7 beyond, 2 x 4096 x 14336
+  // 15.4 and 11.0, 18.1 and 15.7, 15 x 2176 x 15360 17.4 and 9.7, 19.7 and 12.1, 5 x 1650 x 5419
+  // 9.0 and 8.2, 9.3 and 8.2.  Calls with more that may take scratch are therefore two
+  // kernels, but for zero points per column (2 x 8192 x 8192 17.1 and 12.4, 19.7 and 17.2: one
+  // launch is what their callers have counted on).
   if (M < 2 || M > kRowsMax || N > (int64_t)1 << 24)
     return false;
   if (M * kp > 16384 && (M * kp > 32768 || N < 1024 * M))
@@ -306,7 +315,7 @@ bool linear_rows_wanted(int64_t M, int64_t N, int64_t kp) {
   if (M * (rows_slice(kp) / 4) > kRowsHeld * kRowsThreads)
     return false;
   // More than one column group per cluster: not for weights of a few MB (4 x 768 x 3072:
-  // 7.1 us here, 6.9 as two kernels).  (Nor, by the times above, for larger ones.)
+  // 7.1 us here, 6.9 as two kernels).
   const int rounds = rows_rounds(N);
   if (rounds > 1 && N * kp < (int64_t)8 << 20)
     return false;

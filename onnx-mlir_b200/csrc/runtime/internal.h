@@ -140,6 +140,7 @@ int launch_repitch(const void *A, int a_signed, int64_t M, int64_t K, int64_t pi
 // linear_rows.cu: DynamicQuantizeLinear, product and DEQUANT tail of up to 16 f32 rows
 // in one launch (a: as for gemm_i8, but for its A and what describes it).
 bool linear_rows_wanted(int64_t M, int64_t N, int64_t kp);
+int linear_rows_groups(int64_t N); // groups of columns per cluster
 int launch_linear_rows(const float *x, const GemmCall &a, cudaStream_t st);
 
 // gemm_batched.cu: every product of a MatMulInteger whose B is an activation in

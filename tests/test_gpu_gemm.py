@@ -931,6 +931,49 @@ def test_ragged_k_and_n(gpu, orc, M, K, N, wdt):
         assert np.array_equal(gpu.qlinear_matmul(*args), orc.qlinear_matmul(*args))
 
 
+@pytest.mark.parametrize("wdt,zp", [(np.int8, None), (np.uint8, 131)])
+@pytest.mark.parametrize("M,K,N", [(2, 8192, 9000), (15, 2176, 15400), (4, 4096, 14337), (3, 5000, 10000)])
+def test_few_rows_of_many_column_groups(gpu, M, K, N, wdt, zp):
+    # Sizes that a cluster would take in several column groups: quantize and product by
+    # themselves, one launch (no scratch) while the stream is being captured, and the same
+    # bits: the zero point of the weight is one value here.
+    import torch
+    rng = np.random.default_rng(M + N)
+    x = torch.from_numpy(rng.normal(0.1, 1, size=(M, K)).astype(np.float32)).cuda()
+    w = torch.from_numpy(rand8(rng, (K, N), wdt)).cuda()
+    ws, y = torch.tensor(0.0157, device="cuda"), torch.zeros((2, M, N), device="cuda")
+    z = torch.tensor(zp, dtype=torch.uint8, device="cuda") if zp else None
+    T = gpu.Tensor.from_cuda_array
+    t = [T(x), T(w), T(ws)] + ([T(z)] if zp else [])
+    ys = [T(y[0]), T(y[1])]
+    L = gpu.lib()
+    L.omcudaRegisterConstant(t[1].handle)
+    args = [a.handle for a in t] + ([] if zp else [None]) + [None, 0]
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    try:
+        L.omcudaSetStream(stream.cuda_stream)
+        for _ in range(2):
+            before = gpu.launch_count()
+            L.omcudaDynQuantLinear(ys[0].handle, *args)
+            assert gpu.launch_count() - before >= 2
+        gpu.check()
+        gpu.synchronize()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            before = gpu.launch_count()
+            L.omcudaDynQuantLinear(ys[1].handle, *args)
+            assert gpu.launch_count() - before == 1
+        gpu.check()
+        graph.replay()
+        torch.cuda.synchronize()
+        got = y.cpu().numpy()
+        assert got[0].tobytes() == got[1].tobytes() and np.abs(got[0]).max() > 0
+    finally:
+        L.omcudaSetStream(None)
+        torch.cuda.synchronize()
+        L.omcudaForgetConstants()
+
+
 @pytest.mark.parametrize("rest", [1, 7, 8, 9, 24, 25, 31])
 @pytest.mark.parametrize("N", [259, 1537])
 @pytest.mark.parametrize("tail", ["i32", "dequant", "requant"])
