@@ -294,10 +294,20 @@ __device__ __forceinline__ Eight load_eight(const float *p) {
 // zeros, say).  Out of line, as the kernel below is short of registers.
 template <bool kSigned>
 __device__ __noinline__ void quantize_pass_exact(
-    const float *x, int64_t n, uint8_t *y, float scale, float zp_f, bool use_rcp) {
+    const float *x, int64_t n, uint8_t *y, float scale, float zp_f, bool use_rcp, bool zeros) {
   const int64_t step = (int64_t)gridDim.x * kDqlThreads, n4 = n >> 2;
   const int64_t tid = (int64_t)blockIdx.x * kDqlThreads + threadIdx.x;
   const float4 *x4 = reinterpret_cast<const float4 *>(x);
+  if (zeros) { // one quotient, 0 / 0, for all
+    const uint32_t w = quantize_four_exact<kSigned>(
+        make_float4(0.0f, 0.0f, 0.0f, 0.0f), scale, zp_f, use_rcp);
+#pragma unroll 1
+    for (int64_t i = tid; i < n4; i += step)
+      reinterpret_cast<uint32_t *>(y)[i] = w;
+    if (tid < (n & 3))
+      y[(n4 << 2) + tid] = (uint8_t)w;
+    return;
+  }
 #pragma unroll 1
   for (int64_t i = tid; i < n4; i += 2 * step) {
     const bool two = i + step < n4;
@@ -344,7 +354,9 @@ __global__ void __launch_bounds__(kDqlThreads, kWideBlocksPerSm)
       v[u] = load_eight<kOnce>(xr + u * (kDqlThreads * 8));
   const QuantConsts qc = quant_scalars<kSigned>(src, outs, mode);
   if (!qc.fast) {
-    quantize_pass_exact<kSigned>(x, n, y, qc.scale, qc.zp_f, qc.use_rcp);
+    // (a range of nothing but zero: x holds zeros, and NaNs, whose quotient is the same)
+    quantize_pass_exact<kSigned>(
+        x, n, y, qc.scale, qc.zp_f, qc.use_rcp, !src.scale && qc.scale == 0.0f);
     return;
   }
   uint2 *yr = reinterpret_cast<uint2 *>(y) + ((int64_t)r * kRun + threadIdx.x);

@@ -425,6 +425,16 @@ def test_dynamic_quantize_extremes_of_deep_and_full_blocks(gpu, orc, n, at):
     check_dql(gpu, orc, x, device=True)
 
 
+@pytest.mark.parametrize("n", [200000, 262147, 4000003])
+def test_wide_pass_of_zeros(gpu, orc, n):
+    x = np.zeros(n, np.float32)
+    x[::3] = -0.0
+    check_dql(gpu, orc, x, device=True)
+    x[5::7] = np.nan
+    with np.errstate(all="ignore"):
+        check_dql(gpu, orc, x, device=True)
+
+
 @pytest.mark.parametrize("n", [199999, 200000, 200007, 204800, 204801, 208897, 3031041, 39010313])
 @pytest.mark.parametrize("xs,ys", [(0, 0), (8, 8), (4, 0), (0, 4)])
 def test_wide_pass(gpu, orc, n, xs, ys):
