@@ -590,7 +590,6 @@ EpiParams make_epi_params(const GemmCall &a) {
   const uintptr_t sb_vec = a.sb_len > 1 ? (uintptr_t)a.sb : 0;
   p.vec_ok = ((((uintptr_t)a.B.colsum | (uintptr_t)a.bias | sb_vec) & 15u) == 0) &&
              (a.N % 4 == 0);
-  p.line_store = 0;
   p.l2_hints = 0;
   p.early_next = a.early_next;
   p.quant_mode = quant_mode();

@@ -434,10 +434,15 @@ __device__ __forceinline__ void prefetch_residual(const EpiParams &p, int64_t m,
 // A residual is added to the values where they lie in the slab, by lanes that
 // stand on neighbouring columns: whole 128-byte lines of it per load.  (One row per
 // thread, as the accumulator comes, touched 32 lines per load.)
-template <int BN, int EPI, int EW, typename Release>
+//
+// kLines: Y takes the TMA stores.  Kernels of their own, although the code differs only behind
+// the arithmetic: with that for other pitches beside it a launch took up to 4 % longer
+// (QLinearMatMul 4096 x 480 x 3072 19.5 us, 18.6 apart, 2378 x 480 x 3072 15.0 and 14.5; the
+// others gain too: 16384 x 768 x 3001 130 with the rows one by one, 109 now).
+template <int BN, int EPI, int EW, bool kLines, typename Release>
 __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
     const EpiScalars &sc, const QuantConsts &qc, uint32_t taddr, const WarpPlace &at,
-    const EpiRow &row, uint32_t slab0, int lane, bool use_slab, float &lo, float &hi,
+    const EpiRow &row, uint32_t slab0, int lane, float &lo, float &hi,
     const CUtensorMap *map_y, const CUtensorMap *map_y2, Release &&release) {
   const int64_t m_warp = at.m, n0 = at.n;
   const bool hint_store = (p.l2_hints & 1) != 0;
@@ -511,7 +516,7 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
             __float_as_uint(f.w));
       }
     };
-    if (kRes && use_slab)
+    if (kRes && kLines)
       load_res(g, 0);
     uint32_t v[kStep / 32][32];
     __syncwarp(); // tcgen05.ld is warp-collective: enter it converged
@@ -541,7 +546,7 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
         continue;
       if (kSplit)
         split_words_bf16(v[h]);
-      if (use_slab) {
+      if (kLines) {
         if (c % kSlabCols == 0) {
           // The previous store must have read the slab before it is rewritten.
           if (elect_one())
@@ -658,7 +663,7 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
 
 // ---- the kernel -------------------------------------------------------------------
 
-template <int BN, int EPI, int EW>
+template <int BN, int EPI, int EW, bool kLines>
 __global__ void __launch_bounds__(tc_threads(EW), 1)
     gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a,
         const __grid_constant__ CUtensorMap map_b,
@@ -696,7 +701,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   if (threadIdx.x == 32) { // (a thread that has nothing else to set up)
     prefetch_tensormap(&map_a);
     prefetch_tensormap(&map_b);
-    if (p.line_store) {
+    if (kLines) {
       prefetch_tensormap(&map_y);
       if (EPI == OMCUDA_EPI_DEQUANT_SPLIT)
         prefetch_tensormap(&map_y2);
@@ -817,7 +822,6 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
     const int c_lo = (ew >> 2) * kHalfCols; // this warp's share of the columns
     const EpiScalars sc = epi_scalars(p);
     const QuantConsts qc = epi_quant_consts<EPI>(p, warp == 2 && lane == 0 && blockIdx.x == 0);
-    const bool use_slab = p.line_store != 0;
     const uint32_t slab0 = staging_base + (uint32_t)ew * Cfg::kSlabBytes;
     const EpiParams ahead = epi_after_pdl(p); // (its loads are not behind an mbarrier)
     bool ok = true;
@@ -851,7 +855,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
           tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN + c_lo);
       // The accumulator buffer may be overwritten once every warp has read
       // its share of it.
-      epilogue_tile<BN, EPI, EW>(p, sc, qc, taddr, at, row, slab0, lane, use_slab, lo, hi,
+      epilogue_tile<BN, EPI, EW, kLines>(p, sc, qc, taddr, at, row, slab0, lane, lo, hi,
           &map_y, &map_y2, [&] {
             tcgen05_fence_before();
             __syncwarp();
@@ -920,7 +924,7 @@ __device__ __forceinline__ PairUnit pair_unit(int64_t u, int64_t full_units) {
   return r;
 }
 
-template <int EPI, int EW>
+template <int EPI, int EW, bool kLines>
 __global__ void __launch_bounds__(tc_threads(EW), 1)
     gemm_i8_tc2_kernel(const __grid_constant__ CUtensorMap map_a,
         const __grid_constant__ CUtensorMap map_b,
@@ -964,7 +968,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   if (threadIdx.x == 32) { // (a thread that has nothing else to set up)
     prefetch_tensormap(&map_a);
     prefetch_tensormap(&map_b);
-    if (p.line_store) {
+    if (kLines) {
       prefetch_tensormap(&map_y);
       if (EPI == OMCUDA_EPI_DEQUANT_SPLIT)
         prefetch_tensormap(&map_y2);
@@ -1091,7 +1095,6 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
     const int c_lo = (ew >> 2) * kHalfCols;
     const EpiScalars sc = epi_scalars(p);
     const QuantConsts qc = epi_quant_consts<EPI>(p, warp == 2 && lane == 0 && blockIdx.x == 0);
-    const bool use_slab = p.line_store != 0;
     const uint32_t slab0 = staging_base + (uint32_t)ew * kSlabBytes;
     const EpiParams ahead = epi_after_pdl(p); // (its loads are not behind an mbarrier)
     bool ok = true;
@@ -1133,7 +1136,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
           mbar_arrive_cluster(mapa_shared(smem_u32(&bar_acc_empty[buf]), 0));
       };
       if (mine)
-        epilogue_tile<BN, EPI, EW>(p, sc, qc, taddr, at, row, slab0, lane, use_slab, lo, hi,
+        epilogue_tile<BN, EPI, EW, kLines>(p, sc, qc, taddr, at, row, slab0, lane, lo, hi,
             &map_y, &map_y2, release);
       else
         release();
@@ -1430,12 +1433,12 @@ GemmCall split_pass_args(const GemmCall &a, const SplitPlan &plan) {
   return r;
 }
 
-template <int BN, int EPI, int EW>
-int launch_bn_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan = SplitPlan()) {
+template <int BN, int EPI, int EW, bool kLines>
+int launch_bn_lines(const GemmCall &a, cudaStream_t st, const SplitPlan &plan) {
   using Cfg = TcConfig<BN, EW>;
   static PerDeviceInt attr_set;
   if (!attr_set.get()) {
-    OMCUDA_CHECK(cudaFuncSetAttribute(gemm_i8_tc_kernel<BN, EPI, EW>,
+    OMCUDA_CHECK(cudaFuncSetAttribute(gemm_i8_tc_kernel<BN, EPI, EW, kLines>,
         cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
     attr_set.set(1);
   }
@@ -1447,7 +1450,6 @@ int launch_bn_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan =
   if (rc != OMCUDA_OK)
     return rc;
   EpiParams p = make_epi_params(a);
-  p.line_store = y_takes_line_stores<EPI>(a);
   p.l2_hints = l2_hints_wanted();
   p.split_k = plan.split;
   p.ws_rows = plan.ws_rows;
@@ -1458,17 +1460,25 @@ int launch_bn_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan =
   GemmCall ya = a; // the matrix the stores see: all slices of the workspace
   if (plan.split > 1)
     ya.M = plan.split * plan.ws_rows;
-  rc = make_y_maps<EPI>(ya, epi_cols_per_warp(BN, EW), p.line_store != 0, &map_y, &map_y2);
+  rc = make_y_maps<EPI>(ya, epi_cols_per_warp(BN, EW), kLines, &map_y, &map_y2);
   if (rc != OMCUDA_OK)
     return rc;
   int64_t tiles = ceil_div(a.M, kBM) * ceil_div(a.N, BN) * plan.split;
   int grid = (int)(tiles < sm_count() ? tiles : sm_count());
   uint32_t idesc = make_idesc(a.a_signed, a.B.b_signed, BN);
-  OMCUDA_CHECK(launch_pdl(gemm_i8_tc_kernel<BN, EPI, EW>, (unsigned)grid, tc_threads(EW),
+  OMCUDA_CHECK(launch_pdl(gemm_i8_tc_kernel<BN, EPI, EW, kLines>, (unsigned)grid, tc_threads(EW),
       Cfg::kSmemBytes, st, 0, tc_overlap(a), map_a, map_b, map_y, map_y2, p, idesc, status,
       tc_wait_limit_ns()));
   OMCUDA_CHECK_LAUNCH("gemm_i8_tc_kernel");
   return OMCUDA_OK;
+}
+
+template <int BN, int EPI, int EW>
+int launch_bn_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan = SplitPlan()) {
+  if constexpr (EPI != OMCUDA_EPI_DEQUANT_RANGE) // (which stores nothing)
+    if (!y_takes_line_stores<EPI>(a))
+      return launch_bn_lines<BN, EPI, EW, false>(a, st, plan);
+  return launch_bn_lines<BN, EPI, EW, true>(a, st, plan);
 }
 
 // OMCUDA_GEMM_EW=8|16 overrides the choice below, for experiments; else 0.
@@ -1540,8 +1550,8 @@ inline bool pair_half_tiles_wanted() {
 }
 
 // The 2-CTA kernel: 256 x 256 tiles on clusters of two CTAs.
-template <int EPI, int EW>
-int launch_pair_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan = SplitPlan()) {
+template <int EPI, int EW, bool kLines>
+int launch_pair_lines(const GemmCall &a, cudaStream_t st, const SplitPlan &plan) {
   constexpr int kThreads = tc_threads(EW);
   constexpr int kPairSmemBytes =
       tc_stages(kBM * kBK + 128 * kBK, EW) * (kBM * kBK + 128 * kBK) +
@@ -1549,7 +1559,7 @@ int launch_pair_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan
   static PerDeviceInt max_clusters_dev;
   int max_clusters = max_clusters_dev.get();
   if (max_clusters == 0) {
-    OMCUDA_CHECK(cudaFuncSetAttribute(gemm_i8_tc2_kernel<EPI, EW>,
+    OMCUDA_CHECK(cudaFuncSetAttribute(gemm_i8_tc2_kernel<EPI, EW, kLines>,
         cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes));
     cudaLaunchConfig_t q = {};
     q.gridDim = dim3((unsigned)sm_count() & ~1u, 1, 1);
@@ -1563,7 +1573,7 @@ int launch_pair_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan
     q.attrs = qa;
     q.numAttrs = 1;
     int n = 0;
-    OMCUDA_CHECK(cudaOccupancyMaxActiveClusters(&n, gemm_i8_tc2_kernel<EPI, EW>, &q));
+    OMCUDA_CHECK(cudaOccupancyMaxActiveClusters(&n, gemm_i8_tc2_kernel<EPI, EW, kLines>, &q));
     max_clusters = n > 0 ? n : 1;
     max_clusters_dev.set(max_clusters);
   }
@@ -1579,7 +1589,6 @@ int launch_pair_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan
   if (rc != OMCUDA_OK)
     return rc;
   EpiParams p = make_epi_params(a);
-  p.line_store = y_takes_line_stores<EPI>(a);
   p.l2_hints = l2_hints_wanted();
   p.split_k = plan.split;
   p.ws_rows = plan.ws_rows;
@@ -1606,14 +1615,22 @@ int launch_pair_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan
   GemmCall ya = a; // the matrix the stores see: all slices of the workspace
   if (plan.split > 1)
     ya.M = plan.split * plan.ws_rows;
-  rc = make_y_maps<EPI>(ya, epi_cols_per_warp(256, EW), p.line_store != 0, &map_y, &map_y2);
+  rc = make_y_maps<EPI>(ya, epi_cols_per_warp(256, EW), kLines, &map_y, &map_y2);
   if (rc != OMCUDA_OK)
     return rc;
-  OMCUDA_CHECK(launch_pdl(gemm_i8_tc2_kernel<EPI, EW>, (unsigned)(2 * clusters), kThreads,
+  OMCUDA_CHECK(launch_pdl(gemm_i8_tc2_kernel<EPI, EW, kLines>, (unsigned)(2 * clusters), kThreads,
       kPairSmemBytes, st, 2, tc_overlap(a), map_a, map_b, map_b_half, map_y, map_y2,
       p, idesc, idesc_half, full_units, num_units, status, tc_wait_limit_ns()));
   count_launch();
   return OMCUDA_OK;
+}
+
+template <int EPI, int EW>
+int launch_pair_epi_ew(const GemmCall &a, cudaStream_t st, const SplitPlan &plan = SplitPlan()) {
+  if constexpr (EPI != OMCUDA_EPI_DEQUANT_RANGE) // (which stores nothing)
+    if (!y_takes_line_stores<EPI>(a))
+      return launch_pair_lines<EPI, EW, false>(a, st, plan);
+  return launch_pair_lines<EPI, EW, true>(a, st, plan);
 }
 
 template <int EPI>
