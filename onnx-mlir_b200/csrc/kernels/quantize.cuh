@@ -31,9 +31,15 @@ __device__ __forceinline__ void dql_params_from_range(
 // (QuantizeLinear.cpp:124-145): IEEE divide, round half even, add the zero
 // point, clip, convert.
 template <bool kSigned>
+__device__ __forceinline__ uint32_t quantize_quotient(float q, float zp_f);
+template <bool kSigned>
 __device__ __forceinline__ uint32_t quantize_one_exact(
     float x, float scale, float zp_f, bool use_rcp = false) {
-  float q = use_rcp ? __fmul_rn(x, __fdiv_rn(1.0f, scale)) : __fdiv_rn(x, scale);
+  return quantize_quotient<kSigned>(
+      use_rcp ? __fmul_rn(x, __fdiv_rn(1.0f, scale)) : __fdiv_rn(x, scale), zp_f);
+}
+template <bool kSigned>
+__device__ __forceinline__ uint32_t quantize_quotient(float q, float zp_f) {
   float r = round_even(q);
   float a = __fadd_rn(r, zp_f);
   if (kSigned) {

@@ -435,6 +435,72 @@ def test_wide_pass_of_zeros(gpu, orc, n):
         check_dql(gpu, orc, x, device=True)
 
 
+# Ranges whose 255th part is no longer a positive fp32 number although not all values are zero
+# (127 steps of the least denormal and fewer), the first ranges above, denormal and least scales.
+TINY = {"positive": (1e-44, 2e-44, 1e-43, 0.0, -0.0), "both": (1e-44, -2e-44, 1e-43, 0.0),
+        "least": (1.4e-45, 0.0, 0.0), "negative": (-7e-44, 0.0, np.nan),
+        "mostly zeros": (0.0,) * 4099 + (7e-44,), "step of scale": (1.79e-43, 0.0, 1e-44),
+        "denormal scale": (1e-40, -3e-39, 0.0), "least normal": (1.2e-38, -2.3e-38, 1e-44)}
+
+
+@pytest.mark.parametrize("n", [199999, 200000, 4000003])
+@pytest.mark.parametrize("xs", [0, 4])
+@pytest.mark.parametrize("values", sorted(TINY))
+def test_wide_pass_of_denormals(gpu, orc, n, xs, values):
+    import torch
+    v = np.resize(np.array(TINY[values], np.float32), n)
+    xt = torch.zeros(n + 4, device="cuda")
+    xt[xs:xs + n] = torch.from_numpy(v).cuda()
+    y = torch.full((n + 8,), 99, dtype=torch.uint8, device="cuda")
+    s, z = torch.zeros((), device="cuda"), torch.zeros((), dtype=torch.uint8, device="cuda")
+    t = [gpu.Tensor.from_cuda_array(a) for a in (y[:n], s, z, xt[xs:xs + n])]
+    torch.cuda.synchronize()
+    gpu.lib().omcudaDynamicQuantizeLinear(*[a.handle for a in t])
+    gpu.synchronize()
+    with np.errstate(all="ignore"):
+        want_y, want_s, want_z = orc.dynamic_quantize_linear(v)
+    assert s.cpu().numpy().tobytes() == want_s.tobytes() and z.item() == want_z
+    got = y.cpu().numpy()
+    assert np.array_equal(got[:n], want_y) and (got[n:] == 99).all()
+
+
+# (from 606209 values the blocks are two per SM, from 1212417 three, then four)
+@pytest.mark.parametrize("n", [23999, 24000, 24007, 606208, 606209, 700001, 1212417, 1500003, 2000000])
+@pytest.mark.parametrize("values", ["normal", "zeros", "no range"] + sorted(TINY))
+def test_quantize_from_range(gpu, orc, n, values):
+    """What an encoder's linears do to a tensor whose range its producer has kept.  "no range":
+    a range of nothing but zero beside values that are not; they are quantized with it."""
+    import ctypes
+
+    import torch
+    rng = np.random.default_rng(n)
+    v = np.resize(np.zeros(1, np.float32) if values == "zeros" else
+                  np.array(TINY[values], np.float32) if values in TINY else
+                  rng.normal(0, 3, size=65537).astype(np.float32), n)
+    of = np.zeros(1, np.float32) if values == "no range" else v
+    x, f = torch.from_numpy(v).cuda(), torch.from_numpy(of).cuda()
+    y = torch.full((n + 8,), 99, dtype=torch.uint8, device="cuda")
+    par = torch.zeros(4, device="cuda")
+    ranges = torch.zeros(2, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    L, st = gpu.lib(), ctypes.c_void_p(gpu.lib().omcudaGetStream())
+    from omcuda import dev
+    dev.range_init(ranges.data_ptr(), 1, st)
+    assert L.omcudaDevRangeFold(ctypes.c_void_p(f.data_ptr()), ctypes.c_int64(of.size),
+                                ctypes.c_void_p(ranges.data_ptr()), st) == 0
+    dev.quantize_from_range(x.data_ptr(), n, ranges.data_ptr(), y.data_ptr(), par.data_ptr(),
+                            par.data_ptr() + 8, par.data_ptr() + 12, st)
+    gpu.synchronize()
+    with np.errstate(all="ignore"):
+        want_y, want_s, want_z = orc.dynamic_quantize_linear(of)
+        if values == "no range":
+            want_y = orc.quantize(v, want_s, float(want_z), False)
+    p, got = par.cpu().numpy(), y.cpu().numpy()
+    assert p[0].tobytes() == want_s.tobytes() == p[2].tobytes() and p[1] == want_z
+    assert p[3:].view(np.uint8)[0] == want_z
+    assert np.array_equal(got[:n], want_y) and (got[n:] == 99).all()
+
+
 @pytest.mark.parametrize("n", [199999, 200000, 200007, 204800, 204801, 208897, 3031041, 39010313])
 @pytest.mark.parametrize("xs,ys", [(0, 0), (8, 8), (4, 0), (0, 4)])
 def test_wide_pass(gpu, orc, n, xs, ys):
