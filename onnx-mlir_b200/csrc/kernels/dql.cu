@@ -330,6 +330,25 @@ __device__ __noinline__ void quantize_pass_exact(
       y[j] = (uint8_t)one(__ldg(x + j));
     return;
   }
+  if (!use_rcp && scale > 0.0f && scale < INFINITY) {
+    // A power of two that goes into x as well leaves the quotients as they are (what of x it takes
+    // below 2^-126 has a quotient below 2^-160) and makes the scale one of quantize_four_fast's.
+    // (Values of 1e-30, DynamicQuantizeLinear: 300000 in the 16-byte pass 5.6 us, here divided one
+    // by one 8.6, so 5.0; 64 Mi 229, 248 and 103; 24000 from a range 2.8, 6.1 and 2.6.)
+    const float f = scale < 1.0f ? 0x1p64f : 0x1p-64f;
+    const QuantConsts qc = make_quant_consts<kSigned>(__fmul_rn(scale, f), zp_f);
+#pragma unroll 2
+    for (int64_t i = tid; i < n4; i += step) {
+      const float4 v = __ldg(x4 + i);
+      y4[i] = quantize_four_fast<kSigned>(
+          make_float4(__fmul_rn(v.x, f), __fmul_rn(v.y, f), __fmul_rn(v.z, f), __fmul_rn(v.w, f)), qc);
+    }
+    if (j < n) {
+      const float e = __fmul_rn(__ldg(x + j), f);
+      y[j] = (uint8_t)quantize_four_fast<kSigned>(make_float4(e, e, e, e), qc);
+    }
+    return;
+  }
 #pragma unroll 1
   for (int64_t i = tid; i < n4; i += 2 * step) {
     const bool two = i + step < n4;

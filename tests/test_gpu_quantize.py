@@ -464,6 +464,34 @@ def test_wide_pass_of_denormals(gpu, orc, n, xs, values):
     assert np.array_equal(got[:n], want_y) and (got[n:] == 99).all()
 
 
+@pytest.mark.parametrize("n", [200000, 212999])
+@pytest.mark.parametrize("scale", [1.4e-45, 7e-45, 5e-40, 1.1754944e-38, 9.9e-31, 1e-30, 1.0000001e-30,
+                                   0.99e30, 1e30, 3e32, 1.3e38, 3.4e38, np.inf, np.nan, -0.0, -0.5, -1e-40])
+def test_wide_pass_of_scales_that_are_not_ordinary(gpu, orc, n, scale):
+    """Ties, their neighbours and all that saturates, under scales whose reciprocal or
+    residuals fp32 does not hold (those between are divided by with multiplications alone)."""
+    import torch
+    rng = np.random.default_rng(n)
+    s = np.float32(scale)
+    with np.errstate(all="ignore"):
+        k = rng.integers(-600, 600, size=n) * 0.5 + rng.choice([0.0, 1e-6, -1e-6, 0.2], size=n)
+        v = (k * (np.float64(s) if np.isfinite(s) else 1.0)).astype(np.float32)
+    v[::3] = np.nextafter(v[::3], np.float32(0))
+    v[1::501] = rng.normal(0, 1, size=v[1::501].size)
+    v[:8] = (np.inf, -np.inf, np.nan, 3.4e38, -3.4e38, 1.4e-45, -1.4e-45, -0.0)
+    v[-3:] = v[2:5]
+    x, st = torch.from_numpy(v).cuda(), torch.tensor(scale, device="cuda")
+    for zp in (np.array(131, np.uint8), np.array(-7, np.int8), np.array(0, np.uint8)):
+        y, z = torch.empty(n, dtype=getattr(torch, zp.dtype.name), device="cuda"), torch.tensor(zp).cuda()
+        t = [gpu.Tensor.from_cuda_array(a) for a in (y, x, st, z)]
+        torch.cuda.synchronize()
+        gpu.lib().omcudaQuantizeLinear(*[a.handle for a in t])
+        gpu.synchronize()
+        with np.errstate(all="ignore"):
+            want = orc.quantize(v, s, float(zp), zp.dtype == np.int8)
+        assert np.array_equal(y.cpu().numpy(), want)
+
+
 # (from 606209 values the blocks are two per SM, from 1212417 three, then four)
 @pytest.mark.parametrize("n", [23999, 24000, 24007, 606208, 606209, 700001, 1212417, 1500003, 2000000])
 @pytest.mark.parametrize("values", ["normal", "zeros", "no range"] + sorted(TINY))
