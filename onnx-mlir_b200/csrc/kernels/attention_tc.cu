@@ -31,11 +31,11 @@
 //              maximum (exchanged through shared memory), p = 2^(s*c - m),
 //              running sum, p split into bf16 hi/lo and stored back over the
 //              scores in tensor memory;
-//   the product warp issues O_j = P V as 16 MMAs with P read from tensor memory
-//              and V (keys x 64, MN-major) from shared memory: P_hi against
-//              [V_hi | V_lo] as one N = 128 product per 16-key slice (into
-//              128 columns of tensor memory), P_lo V_hi on top of the first
-//              64 columns; and right behind them the next block's S;
+//   the product warp issues O_j = P V as 24 MMAs with P read from tensor memory
+//              and V (keys x 64, MN-major) from shared memory: per 16-key
+//              slice P_hi V_hi and P_lo V_hi into 64 columns of tensor memory,
+//              P_hi V_lo into 64 others; and once they are done the next
+//              block's S;
 //   the load warp (att_loads) refills each buffer (TMA, 128-byte swizzle) once
 //              the products that read it are done, and sends results off.
 // O accumulates in tensor memory over the key blocks of an item (the P V MMAs
@@ -50,12 +50,11 @@
 // What bounds it: the chain of a CTA (scores -> softmax -> P V -> scores), two of
 // which share an SM.  One warp used to issue products and copies beside its rows,
 // with a CTA barrier between any two phases: of some 5100 clocks per block 1180 were
-// spent issuing copies and waking up, and 2600 more per item on its results.  With warps
-// of their own for products and copies, mbarriers between the phases, S queued behind
-// P V and the results out of V's way, a block takes some 4400 and an item 500 more (two
-// CTAs share the SM meanwhile: 1536 clocks of MMAs per block each).  Batch x sequence x
-// heads, us: 256 x 512 x 16 835 -> 750, 64 x 384 x 16 138 -> 112, 1 x 512 x 16 16.5 ->
-// 13.1, 32 x 128 x 12 11.3 -> 11.0, 1024 x 128 x 16 338 -> 326 (HBM).  The largest runs
+// spent issuing copies and waking up, and 2600 more per item on its results.  Now warps
+// of their own issue products and copies, mbarriers stand between the phases and the
+// results are out of V's way (two CTAs share the SM: 1536 clocks of MMAs per block each).
+// Batch x sequence x heads, us: 256 x 512 x 16 829 -> 741, 64 x 384 x 16 124 -> 113, 1 x 512 x
+// 16 13.8 -> 12.4, 32 x 128 x 12 11.6 -> 11.5, 1024 x 128 x 16 336 -> 325 (HBM).  The largest runs
 // at the power limit, clocks at 1.35 GHz.  Every sum is in the order it was in.
 // Every wait on an mbarrier is bounded (tc_ptx.cuh); a timeout raises the
 // CTA's abort flag, the CTA frees its tensor memory, writes the status word
@@ -117,18 +116,23 @@ __device__ __forceinline__ void umma_scores(uint32_t d_tmem, uint64_t ql, uint64
                : "memory");
 }
 
-// O += P V of a block, sixteen MMAs of 16 keys: A (P) from tensor memory, eight columns per
-// slice, hi parts of 32 keys at column 0 and lo parts at 16 of every 32; B (V, MN-major)
-// advances 16 keys = 2048 bytes (descriptor + 128).  P_hi [V_hi | V_lo] into columns
-// 0..127, then P_lo V_hi on top of columns 0..63.
-__device__ __forceinline__ void umma_values(uint32_t d_tmem, uint32_t p_tmem, uint64_t v2,
-    uint64_t vh, uint32_t idesc2, uint32_t idesc, uint32_t accumulate_first) {
+// O += P V of a block, 24 MMAs of 16 keys: A (P) from tensor memory, eight columns per slice,
+// hi parts of 32 keys at column 0 and lo parts at 16 of every 32; B (V, MN-major) advances 16
+// keys = 2048 bytes (descriptor + 128).  P_hi V_hi, then P_lo V_hi into columns 0..63, P_hi V_lo
+// into 64..127.  All of one shape, for only products of one accumulator and one shape are promised
+// to run in the order of issue (PTX ISA, pipelined tcgen05 instructions).  P_hi [V_hi | V_lo] as
+// eight products of N = 128 with P_lo V_hi on top takes the tensor pipe as long (32 clocks per
+// product of N = 64, 64 per one of N = 128) and was no faster: 64 x 384 x 16 114.2 and so 112.9 us,
+// 16 x 512 x 16 54.7 and 53.1, 32 x 128 x 12 11.5 and 11.4, 1 x 512 x 16 11.9 and 11.9.
+__device__ __forceinline__ void umma_values(uint32_t d_tmem, uint32_t p_tmem, uint64_t vl,
+    uint64_t vh, uint32_t idesc, uint32_t accumulate_first) {
   asm volatile("{\n\t"
                ".reg .pred p, t;\n\t"
-               ".reg .b32 a1, a2, a3, a4, a5, a6, a7, c0, c1, c2, c3, c4, c5, c6, c7;\n\t"
+               ".reg .b32 a1, a2, a3, a4, a5, a6, a7, c0, c1, c2, c3, c4, c5, c6, c7, d1;\n\t"
                ".reg .b64 v1, v2, v3, v4, v5, v6, v7, w1, w2, w3, w4, w5, w6, w7;\n\t"
-               "setp.ne.b32 p, %6, 0;\n\t"
+               "setp.ne.b32 p, %5, 0;\n\t"
                "setp.eq.b32 t, 0, 0;\n\t"
+               "add.u32 d1, %0, 64;\n\t"
                "add.u32 a1, %1, 8; add.u32 a2, %1, 32; add.u32 a3, %1, 40; add.u32 a4, %1, 64;\n\t"
                "add.u32 a5, %1, 72; add.u32 a6, %1, 96; add.u32 a7, %1, 104;\n\t"
                "add.u32 c0, %1, 16; add.u32 c1, %1, 24; add.u32 c2, %1, 48; add.u32 c3, %1, 56;\n\t"
@@ -137,24 +141,32 @@ __device__ __forceinline__ void umma_values(uint32_t d_tmem, uint32_t p_tmem, ui
                "add.u64 v5, %2, 640; add.u64 v6, %2, 768; add.u64 v7, %2, 896;\n\t"
                "add.u64 w1, %3, 128; add.u64 w2, %3, 256; add.u64 w3, %3, 384; add.u64 w4, %3, 512;\n\t"
                "add.u64 w5, %3, 640; add.u64 w6, %3, 768; add.u64 w7, %3, 896;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %4, p;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], v1, %4, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], v2, %4, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], v3, %4, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a4], v4, %4, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a5], v5, %4, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a6], v6, %4, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a7], v7, %4, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c0], %3, %5, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c1], w1, %5, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c2], w2, %5, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c3], w3, %5, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c4], w4, %5, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c5], w5, %5, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c6], w6, %5, t;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c7], w7, %5, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %3, %4, p;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], w1, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], w2, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], w3, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a4], w4, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a5], w5, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a6], w6, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [a7], w7, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c0], %3, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c1], w1, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c2], w2, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c3], w3, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c4], w4, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c5], w5, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c6], w6, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [c7], w7, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [d1], [%1], %2, %4, p;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [d1], [a1], v1, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [d1], [a2], v2, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [d1], [a3], v3, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [d1], [a4], v4, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [d1], [a5], v5, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [d1], [a6], v6, %4, t;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [d1], [a7], v7, %4, t;\n\t"
                "}" ::"r"(d_tmem),
-               "r"(p_tmem), "l"(v2), "l"(vh), "r"(idesc2), "r"(idesc), "r"(accumulate_first)
+               "r"(p_tmem), "l"(vl), "l"(vh), "r"(idesc), "r"(accumulate_first)
                : "memory");
 }
 
@@ -269,27 +281,23 @@ __device__ __forceinline__ bool mbar_spin(
 // The tensor pipe's part, by one elected thread of a warp that does nothing else.  Returns
 // false when a wait ran out (or the CTA is aborting).
 //
-// Products of one thread run in the order of issue, so the next block's S = Q K^T is queued
-// right behind P V, which still reads P from the columns that it overwrites: no wait between
-// the two, and the first block of the next item runs while the softmax warps are still busy
-// with the results of the one before.
+// The next block's S = Q K^T overwrites the columns that P V reads P from, and the two have
+// different accumulators, whose order nothing promises (see umma_values): it waits for P V.
+// (Queued right behind it, some 130 clocks a block less where a CTA has the SM for itself: 1 x
+// 2048 x 9 heads 37.5 and so 39.6 us, 1 x 512 x 16 11.9 and 12.4; nothing measurable where two share
+// it.)  With that, whoever has seen scores ready has seen every P V before them done as well.  The
+// first block of the next item runs while the softmax warps are still busy with the results of the
+// one before.
 __device__ __forceinline__ bool att_products(const AttTiles &s, const AttBars &bar,
     uint32_t tmem, int nkb, int64_t n_items, volatile int *abortp, uint64_t wait_ns) {
   constexpr uint32_t kIdescQK = att_idesc(kTK, 0);
   constexpr uint32_t kIdescPV = att_idesc(kTDh, 1);
-  // P_hi against V_hi and V_lo in one MMA of N = 128: the B descriptor's
-  // leading-dimension offset (stride between 64-element groups along N) is
-  // the distance from the V_hi tile to the V_lo tile, so output columns
-  // 0..63 hold P_hi V_hi and 64..127 hold P_hi V_lo.
-  constexpr uint32_t kIdescPV2 = att_idesc(2 * kTDh, 1);
-  constexpr uint64_t kLboField = (uint64_t)0x3fff << 16;
   static_assert(kTDh == 64, "four K slices per operand row");
   static_assert(kTK == 128, "eight 16-key slices per block");
   const uint32_t t_s = tmem, t_o = tmem + 128u;
   const uint64_t dqh = make_smem_desc(s.qh), dql = make_smem_desc(s.ql),
                  dkh = make_smem_desc(s.kh), dkl = make_smem_desc(s.kl),
-                 dvh = make_smem_desc(s.vh);
-  const uint64_t dv2 = (dvh & ~kLboField) | ((uint64_t)((s.vl - s.vh) >> 4) << 16);
+                 dvh = make_smem_desc(s.vh), dvl = make_smem_desc(s.vl);
   auto wait = [&](uint32_t b, uint32_t parity) {
     return mbar_spin(b, parity & 1u, abortp, wait_ns);
   };
@@ -307,11 +315,12 @@ __device__ __forceinline__ bool att_products(const AttTiles &s, const AttBars &b
       if (!wait(bar.v, n) || !wait(bar.p, n))
         return false;
       tcgen05_fence_after();
-      umma_values(t_o, t_s, dv2, dvh, kIdescPV2, kIdescPV, j != 0 ? 1u : 0u);
+      umma_values(t_o, t_s, dvl, dvh, kIdescPV, j != 0 ? 1u : 0u);
       umma_commit(bar.o);
       if (!last || has_next) {
-        if ((last && !wait(bar.q, nitem + 1)) || !wait(bar.k, n + 1))
+        if (!wait(bar.o, n) || (last && !wait(bar.q, nitem + 1)) || !wait(bar.k, n + 1))
           return false;
+        tcgen05_fence_after();
         umma_scores(t_s, dql, dqh, dkh, dkl, kIdescQK);
         umma_commit(bar.s);
       }
@@ -509,7 +518,8 @@ __global__ void __launch_bounds__(kTcAttThreads, 2)
       float l_run = 0.0f;      // running sum of p
 
       for (int j = 0; j < nkb; ++j, ++n) {
-        // (the scores come behind P V of the block before on the tensor pipe, so that is done too)
+        // (S is issued once P V of the block before is done, so bar.o is at most one phase behind
+        // here and the wait for it at the end of the item may skip the phases between)
         ok = mbar_wait(bar.s, n & 1u, abortp, wait_ns) && ok;
         tcgen05_fence_after();
 
