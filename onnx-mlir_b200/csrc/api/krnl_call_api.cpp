@@ -106,10 +106,12 @@ public:
       rc_ = rc;
   }
 
-  void *scratch(size_t bytes) {
-    void *p = pool_alloc_on(bytes ? bytes : 1, st_);
+  // optional: lack of memory is no error, the call can do without.
+  void *scratch(size_t bytes, bool optional = false) {
+    void *p = pool_alloc_on(bytes ? bytes : 1, st_, optional);
     if (!p) {
-      set(OMCUDA_ENOMEM);
+      if (!optional)
+        set(OMCUDA_ENOMEM);
       return nullptr;
     }
     temps_.push_back(p);
@@ -196,7 +198,9 @@ bool is_capturing(cudaStream_t st) {
   return cs != cudaStreamCaptureStatusNone;
 }
 
-void *dql_scratch_for(Stage &sg) { return sg.scratch((size_t)omcudaDevDqlScratchBytes(0)); }
+void *dql_scratch_for(Stage &sg, bool optional = false) {
+  return sg.scratch((size_t)omcudaDevDqlScratchBytes(0), optional);
+}
 
 // ---- constants: prepared B operands cached by buffer ----------------------------------
 
@@ -929,11 +933,26 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
   g.K = d.K;
   g.lda = (d.K + 15) & ~int64_t(15);
   // (one launch writes parts of Y while others still read X, so not onto X)
+  const bool one_launch = d.K > 0 && linear_rows_wanted(d.M, d.N, g.lda) &&
+                          !ranges_overlap(dX, d.M * d.K * 4, dY, d.M * d.N * 4);
   // More than one group of columns per cluster: quantize and product are faster (the figures are
-  // at linear_rows_wanted), but take scratch, which a captured call must not.
-  if (d.K > 0 && linear_rows_wanted(d.M, d.N, g.lda) &&
-      !(wzn <= 1 && linear_rows_groups(d.N) > 1 && !is_capturing(st)) &&
-      !ranges_overlap(dX, d.M * d.K * 4, dY, d.M * d.N * 4)) {
+  // at linear_rows_wanted), but take scratch, which a captured call must not.  Where there is none
+  // left, the one launch does it.
+  const bool small = dql_small_wanted(d.M, g.lda);
+  uint8_t *xq = nullptr;
+  float *xs = nullptr;
+  void *scr = nullptr;
+  bool have_scratch = false;
+  if (!one_launch || (wzn <= 1 && linear_rows_groups(d.N) > 1 && !is_capturing(st))) {
+    xq = (uint8_t *)sg.scratch((size_t)(d.M * g.lda), one_launch);
+    xs = (float *)sg.scratch(16, one_launch);
+    scr = small ? nullptr : dql_scratch_for(sg, one_launch);
+    if (wzn)
+      g.a_rowsum = (int32_t *)sg.scratch((size_t)d.M * sizeof(int32_t), one_launch);
+    have_scratch = xq && xs && (small || scr) && (!wzn || g.a_rowsum);
+  }
+  if (one_launch && !have_scratch) {
+    g.a_rowsum = nullptr; // (it makes its own)
     if (wzn) {
       g.b_zp = dWz;
       g.b_zp_len = wzn;
@@ -951,19 +970,12 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
     sg.finish(false);
     return;
   }
-  uint8_t *xq = (uint8_t *)sg.scratch((size_t)(d.M * g.lda));
-  float *xs = (float *)sg.scratch(16);
-  const bool small = dql_small_wanted(d.M, g.lda);
-  void *scr = small ? nullptr : dql_scratch_for(sg);
-  if (!sg.ok() || (!small && !scr))
+  if (!sg.ok() || !have_scratch)
     return;
   uint8_t *xz = (uint8_t *)(xs + 1);
   if (wzn) {
     g.b_zp = dWz;
     g.b_zp_len = wzn;
-    g.a_rowsum = (int32_t *)sg.scratch((size_t)d.M * sizeof(int32_t));
-    if (!sg.ok())
-      return;
   }
   if (small) {
     sg.set(launch_dql_small(

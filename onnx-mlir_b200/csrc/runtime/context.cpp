@@ -206,7 +206,7 @@ cudaStream_t current_stream() {
   return g_stream;
 }
 
-void *pool_alloc_on(size_t bytes, cudaStream_t st) {
+void *pool_alloc_on(size_t bytes, cudaStream_t st, bool optional) {
   if (ensure_init() != OMCUDA_OK)
     return nullptr;
   size_t sz = round_size(bytes);
@@ -249,7 +249,10 @@ void *pool_alloc_on(size_t bytes, cudaStream_t st) {
     pool_release_all();
     e = cudaMalloc(&p, sz);
     if (e != cudaSuccess) {
-      check_cuda(e, "cudaMalloc");
+      if (optional)
+        (void)cudaGetLastError();
+      else
+        check_cuda(e, "cudaMalloc");
       return nullptr;
     }
   }

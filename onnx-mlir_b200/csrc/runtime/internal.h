@@ -14,10 +14,10 @@ bool sticky_error();
 cudaStream_t current_stream();
 // Device-memory pool with stream-ordered reuse.  The plain forms use the
 // calling thread's stream (omcudaGetStream); the _on forms name the stream the
-// block will be / was last used on.
+// block will be / was last used on.  optional: lack of memory is not recorded as an error.
 void *pool_alloc(size_t bytes);
 void pool_free(void *p);
-void *pool_alloc_on(size_t bytes, cudaStream_t st);
+void *pool_alloc_on(size_t bytes, cudaStream_t st, bool optional = false);
 void pool_free_on(void *p, cudaStream_t st);
 bool pool_owns(const void *p);
 

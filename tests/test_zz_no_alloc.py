@@ -74,3 +74,60 @@ def test_no_alloc_entry_rejects_oversized_input(gpu):
     assert rc == gpu.EINVAL
     assert b"exceed the limit" in L.omcudaGetLastErrorString()
     L.omcudaClearError()
+
+
+def test_linear_of_few_rows_when_no_memory_is_left(gpu):
+    """Two kernels and their scratch where there is memory for it; the one launch that needs
+    none, with the same bits, where every byte of the device is taken."""
+    import torch
+    L, T = gpu.lib(), gpu.Tensor.from_cuda_array
+    M, K, N = 3, 5000, 10000
+    rng = np.random.default_rng(7)
+    x = torch.from_numpy(rng.normal(0, 1, size=(M, K)).astype(np.float32)).cuda()
+    w = torch.from_numpy(rng.integers(-127, 128, size=(K, N)).astype(np.int8)).cuda()
+    ws, y = torch.tensor(0.0157, device="cuda"), torch.zeros((3, M, N), device="cuda")
+    t = [T(x), T(w), T(ws)]
+    ys = [T(y[i]) for i in range(3)]
+    L.omcudaRegisterConstant(t[1].handle)
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    driver, taken = ctypes.CDLL("libcuda.so.1"), []
+
+    def call(out):
+        before = gpu.launch_count()
+        L.omcudaDynQuantLinear(ys[out].handle, *[a.handle for a in t], None, None, 0)
+        gpu.check()
+        return gpu.launch_count() - before
+
+    torch.cuda.synchronize()
+    try:
+        L.omcudaSetStream(stream.cuda_stream)
+        assert call(0) >= 2
+        gpu.synchronize()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            call(1)
+        graph.replay()  # (the kernel of the one launch is on the device now)
+        torch.cuda.synchronize()
+        assert L.omcudaDeviceAlloc(ctypes.c_int64(1 << 50)) in (None, 0)  # the pool lets go of its blocks
+        L.omcudaClearError()
+        size, ptr = 1 << 38, ctypes.c_uint64()
+        while size >= 256:
+            if driver.cuMemAlloc_v2(ctypes.byref(ptr), ctypes.c_size_t(size)) == 0:
+                taken.append(ptr.value)
+            else:
+                size //= 2
+        assert call(2) == 1
+        gpu.synchronize()
+        for p in taken:
+            driver.cuMemFree_v2(ctypes.c_uint64(p))
+        taken = []
+        assert call(0) >= 2
+        gpu.synchronize()
+        got = y.cpu().numpy()
+        assert np.abs(got[0]).max() > 0
+        assert got[0].tobytes() == got[1].tobytes() == got[2].tobytes()
+    finally:
+        for p in taken:
+            driver.cuMemFree_v2(ctypes.c_uint64(p))
+        L.omcudaSetStream(None)
+        torch.cuda.synchronize()
+        L.omcudaForgetConstants()
