@@ -663,6 +663,15 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
 
 // ---- the kernel -------------------------------------------------------------------
 
+// Whether split-K passes are made with a kernel (launch_split_k): raw sums, the widest tiles,
+// eight warps on the epilogue.  In the others the count of slices is 1 for the compiler, which
+// takes the divisions by it out of what every warp does before its first tile, 0.2 to 0.4 us of a
+// launch: QLinearMatMul 2000 x 1024 x 2048 12.4 -> 12.1 us, 1100 x 480 x 1536 7.2 -> 6.9, 16384 x 1024 x
+// 4096 62.3 -> 61.6, linear 777 x 1001 x 1537 15.2 -> 14.9, 4096 x 4096 x 4096 73.6 -> 72.9.
+__host__ __device__ constexpr bool tc_splits_k(int bn, int epi, int ew) {
+  return bn == 256 && epi == OMCUDA_EPI_I32 && ew == 8;
+}
+
 template <int BN, int EPI, int EW, bool kLines>
 __global__ void __launch_bounds__(tc_threads(EW), 1)
     gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a,
@@ -695,7 +704,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   const int num_kb = (int)ceil_div(p.K, kBK);
   // Work units: tiles, or (split-K pass) the split_k K slices of every tile,
   // slices of one tile next to each other.
-  const int split = p.split_k;
+  const int split = tc_splits_k(BN, EPI, EW) ? p.split_k : 1;
   const int64_t num_units = tiles_m * tiles_n * split;
 
   if (threadIdx.x == 32) { // (a thread that has nothing else to set up)
@@ -964,7 +973,7 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   const int num_kb = (int)ceil_div(p.K, kBK);
   // Split-K pass: unit u is K slice u % split of tile u / split (all units
   // whole tiles then).
-  const int split = p.split_k;
+  const int split = tc_splits_k(BN, EPI, EW) ? p.split_k : 1;
   if (threadIdx.x == 32) { // (a thread that has nothing else to set up)
     prefetch_tensormap(&map_a);
     prefetch_tensormap(&map_b);
@@ -1728,6 +1737,7 @@ int launch_split_k(const GemmCall &a, cudaStream_t st, int split) {
   if (!plan.ws)
     return fail(OMCUDA_ENOMEM, "GemmI8: cannot allocate the split-K workspace");
   const GemmCall part = split_pass_args(a, plan);
+  static_assert(tc_splits_k(256, OMCUDA_EPI_I32, 8), "the kernels of both launches");
   int rc;
   if (a.M > kBM)
     rc = launch_pair_epi_ew<OMCUDA_EPI_I32, 8>(part, st, plan);
