@@ -891,9 +891,9 @@ int launch_quantize_pass(const float *x, int64_t n, uint8_t *y, const QuantSourc
   return OMCUDA_OK;
 }
 
-// DynamicQuantizeLinear's reduction alone.
+// DynamicQuantizeLinear's reduction alone.  deep_blocks: see `deep`.
 int launch_range_parts(const float *x, int64_t n, void *scratch, RangeParts *parts,
-    cudaStream_t st, bool overlap, int32_t *sums = nullptr, int zeros = 0) {
+    cudaStream_t st, bool overlap, int64_t deep_blocks, int32_t *sums = nullptr, int zeros = 0) {
   float2 *part = scratch_parts(scratch);
   // Runs of one to eight float4 a thread, so that about a third of the SMs has a
   // block until those are full: no block without work, whose empty partial every
@@ -921,8 +921,9 @@ int launch_range_parts(const float *x, int64_t n, void *scratch, RangeParts *par
     grid = small_blocks < 1 ? 1 : small_blocks;
   // All loads of a run in flight, except where the blocks are one to two per SM: more of
   // them than fit with those registers beside what else is resident (3.1 M values 6.8 us
-  // without, 8.3 with; 6 M 11.9 and 10.8).
-  const bool deep = grid <= sm_count() || grid > 2 * sm_count();
+  // without, 8.3 with; 6 M 11.9 and 10.8).  Full runs of fewer blocks too leave the pass
+  // that is set up meanwhile too little room, from as many as the caller says.
+  const bool deep = grid <= deep_blocks || grid > 2 * sm_count();
   const auto kernel =
       few     ? (sums ? dql_minmax_kernel<false, true, kRangeFewThreads, true>
                       : dql_minmax_kernel<false, false, kRangeFewThreads, true>)
@@ -955,11 +956,14 @@ int launch_dql_rows(const float *x, int64_t rows, int64_t cols, int64_t pitch, u
     split = split < most ? split : most > 0 ? most : 1;
   }
   RangeParts parts;
+  const int64_t blocks = warps ? ceil_div(rows, kDqlThreads / 32) : rows * split;
+  // The reduction's blocks take half the registers of an SM if deep: as long as the pass finds
+  // SMs without one (linears, deep and not: 900 x 1001 x 768 13.8 and 13.1 us, 777 x 1385 x 2048
+  // 17.2 and 16.4, 1544 x 1385 x 768 18.2 and 17.4, but 777 x 1001 x 2048 14.4 and 14.5).
   int rc = launch_range_parts(x, rows * cols, scratch, &parts, st, pdl_pays(rows * cols),
-      split > 1 ? rowsum : nullptr, (int)rows);
+      sm_count() - blocks, split > 1 ? rowsum : nullptr, (int)rows);
   if (rc != OMCUDA_OK)
     return rc;
-  const int64_t blocks = warps ? ceil_div(rows, kDqlThreads / 32) : rows * split;
   const int64_t cap = (int64_t)sm_count() * 8;
   const int vec_in = ((uintptr_t)x & 15u) == 0 && cols % 4 == 0;
   OMCUDA_CHECK(launch_pdl(warps       ? quantize_rows_kernel<1, false>
@@ -1063,7 +1067,7 @@ extern "C" int64_t omcudaDevDqlScratchBytes(int64_t) {
 }
 
 int omcuda::launch_dql(const float *x, int64_t n, uint8_t *y, float *y_scale, uint8_t *y_zp,
-    void *scratch, cudaStream_t st, bool alone) {
+    void *scratch, cudaStream_t st, int64_t rows) {
   if (n < 0 || (n > 0 && (!x || !y)) || !scratch)
     return fail(OMCUDA_EINVAL, "DynamicQuantizeLinear: bad argument");
   if (dql_small_wanted(1, n) ||
@@ -1073,7 +1077,13 @@ int omcuda::launch_dql(const float *x, int64_t n, uint8_t *y, float *y_scale, ui
   // Set up early whatever the size where what runs before is as a rule a pass like this
   // (64 Mi values 100.7 -> 99.0 us), but not behind a GEMM of a long linear, whose SMs its
   // blocks would take (8192 x 4096 x 4096 149 and 155).
-  int rc = launch_range_parts(x, n, scratch, &parts, st, alone || pdl_pays(n));
+  // Deep blocks of the reduction beside those of the pass, two per SM: by itself and in front of
+  // a product of tiles up to some 60 (DynamicQuantizeLinear, deep and not: 900000 values 4.8 and
+  // 5.1 us, 1.2 M 5.4 and 5.3, 2 M 6.0 and 5.6; linear 1024 x 768 x 768 10.4 and 10.5, 1100 x 1384 x
+  // 768 14.5 and 14.2, 2000 x 1024 x 768 12.8 and 12.4); in front of one of few rows, which is next
+  // to be set up, one per SM (200 x 8192 x 4096 23.5 and 23.9, 128 x 14336 x 768 13.7 and 13.9).
+  const int64_t deep = rows > 0 && rows <= 256 ? sm_count() : sm_count() * 2 / 5;
+  int rc = launch_range_parts(x, n, scratch, &parts, st, rows == 0 || pdl_pays(n), deep);
   if (rc != OMCUDA_OK)
     return rc;
   return launch_quantize_pass<false>(x, n, y, QuantSource{parts, nullptr, nullptr, nullptr},
@@ -1082,7 +1092,7 @@ int omcuda::launch_dql(const float *x, int64_t n, uint8_t *y, float *y_scale, ui
 
 extern "C" int omcudaDevDynamicQuantizeLinear(const float *x, int64_t n,
     uint8_t *y, float *y_scale, uint8_t *y_zp, void *scratch, void *stream) {
-  return launch_dql(x, n, y, y_scale, y_zp, scratch, (cudaStream_t)stream, false);
+  return launch_dql(x, n, y, y_scale, y_zp, scratch, (cudaStream_t)stream, 1);
 }
 
 extern "C" int omcudaDevRangeFold(const float *x, int64_t n, void *range, void *stream) {
