@@ -330,13 +330,20 @@ __device__ __noinline__ void quantize_pass_exact(
       y[j] = (uint8_t)one(__ldg(x + j));
     return;
   }
-  if (!use_rcp && scale > 0.0f && scale < INFINITY) {
-    // A power of two that goes into x as well leaves the quotients as they are (what of x it takes
-    // below 2^-126 has a quotient below 2^-160) and makes the scale one of quantize_four_fast's.
+  const float rcp = __fdiv_rn(1.0f, scale);
+  if (fabsf(scale) < INFINITY && (!use_rcp || fabsf(rcp) < INFINITY)) {
+    // The sign and a power of two that go into x as well leave the quotients as they are (what of x
+    // it takes below 2^-126 has a quotient below 2^-62) and make the scale one of quantize_four_fast's.
+    // Fast-math mode's reciprocal is that of the scale as it is, rounded where it is a denormal.
     // (Values of 1e-30, DynamicQuantizeLinear: 300000 in the 16-byte pass 5.6 us, here divided one
-    // by one 8.6, so 5.0; 64 Mi 229, 248 and 103; 24000 from a range 2.8, 6.1 and 2.6.)
-    const float f = scale < 1.0f ? 0x1p64f : 0x1p-64f;
-    const QuantConsts qc = make_quant_consts<kSigned>(__fmul_rn(scale, f), zp_f);
+    // by one 8.6, so 5.0; 64 Mi 229, 248 and 103; 24000 from a range 2.8, 6.1 and 2.6.  A given scale
+    // of -0.05, the same three: 300000 2.5, 4.4 and 2.5, 64 Mi 91, 146 and 80; in fast-math mode 2.2, 3.7
+    // and 2.5, 84, 135 and 80.)
+    const float f = copysignf(fabsf(scale) < 1.0f ? 0x1p64f : 0x1p-64f, scale);
+    QuantConsts qc = make_quant_consts<kSigned>(
+        __fmul_rn(scale, f), zp_f, use_rcp ? OMCUDA_MODE_FAST_MATH : 0);
+    if (use_rcp)
+      qc.rcp = __fmul_rn(rcp, copysignf(fabsf(scale) < 1.0f ? 0x1p-64f : 0x1p64f, scale));
 #pragma unroll 2
     for (int64_t i = tid; i < n4; i += step) {
       const float4 v = __ldg(x4 + i);
@@ -349,18 +356,16 @@ __device__ __noinline__ void quantize_pass_exact(
     }
     return;
   }
-#pragma unroll 1
-  for (int64_t i = tid; i < n4; i += 2 * step) {
-    const bool two = i + step < n4;
-    const float4 v = __ldg(x4 + i), w = two ? __ldg(x4 + i + step) : v;
-    const uint32_t a = quantize_four_exact<kSigned>(v, scale, zp_f, use_rcp);
-    const uint32_t b = quantize_four_exact<kSigned>(w, scale, zp_f, use_rcp);
-    y4[i] = a;
-    if (two)
-      y4[i + step] = b;
+  // What is left are products by 0 (an infinite scale, also by definition), an infinity or a NaN.
+  // (An infinite scale: 64 Mi in the 16-byte pass 143 us, divided one by one 202, so 83.)
+  const auto one = [&](float f) { return quantize_quotient<kSigned>(__fmul_rn(f, rcp), zp_f); };
+#pragma unroll 4
+  for (int64_t i = tid; i < n4; i += step) {
+    const float4 v = __ldg(x4 + i);
+    y4[i] = one(v.x) | one(v.y) << 8 | one(v.z) << 16 | one(v.w) << 24;
   }
   if (j < n)
-    y[j] = (uint8_t)quantize_one_exact<kSigned>(__ldg(x + j), scale, zp_f, use_rcp);
+    y[j] = (uint8_t)one(__ldg(x + j));
 }
 
 // The pass above for many values, x 32-byte and y 8-byte aligned.  That kernel takes what

@@ -492,6 +492,41 @@ def test_wide_pass_of_scales_that_are_not_ordinary(gpu, orc, n, scale):
         assert np.array_equal(y.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("n", [199999, 200000, 212999])
+@pytest.mark.parametrize("flags", [0, 2])  # 2: OMCUDA_MODE_FAST_MATH, x times the rounded reciprocal
+@pytest.mark.parametrize("scale", [1.4e-45, 3e-39, 1e-32, 0.05, 3e32, 3.4e38, np.inf, np.nan])
+def test_wide_pass_of_scales_of_either_sign_in_both_modes(gpu, orc, n, flags, scale):
+    import torch
+    rng = np.random.default_rng(n + flags)
+    for s in (np.float32(scale), -np.float32(scale)):
+        with np.errstate(all="ignore"):
+            k = rng.integers(-600, 600, size=n) * 0.5 + rng.choice([0.0, 1e-6, -1e-6, 0.2], size=n)
+            v = (k * (np.float64(s) if np.isfinite(s) else 1.0)).astype(np.float32)
+        v[::3] = np.nextafter(v[::3], np.float32(0))
+        v[1::501] = rng.normal(0, 1, size=v[1::501].size)
+        v[:8] = (np.inf, -np.inf, np.nan, 3.4e38, -3.4e38, 1.4e-45, -1.4e-45, -0.0)
+        v[-3:] = v[:3]
+        x, st = torch.from_numpy(v).cuda(), torch.tensor(float(s), device="cuda")
+        for zp in (np.array(131, np.uint8), np.array(-7, np.int8)):
+            y, z = torch.empty(n, dtype=getattr(torch, zp.dtype.name), device="cuda"), torch.tensor(zp).cuda()
+            t = [gpu.Tensor.from_cuda_array(a) for a in (y, x, st, z)]
+            torch.cuda.synchronize()
+            try:
+                gpu.lib().omcudaSetQuantizationMode(flags)
+                gpu.lib().omcudaQuantizeLinear(*[a.handle for a in t])
+                gpu.synchronize()
+            finally:
+                gpu.lib().omcudaSetQuantizationMode(0)
+            with np.errstate(all="ignore"):
+                if flags:
+                    q = np.rint(v * (np.float32(1) / s)) + np.float32(zp)
+                    lim = np.iinfo(zp.dtype)
+                    want = np.fmin(np.fmax(q, np.float32(lim.min)), np.float32(lim.max)).astype(zp.dtype)
+                else:
+                    want = orc.quantize(v, s, float(zp), zp.dtype == np.int8)
+            assert np.array_equal(y.cpu().numpy(), want)
+
+
 # (from 606209 values the blocks are two per SM, from 1212417 three, then four)
 @pytest.mark.parametrize("n", [23999, 24000, 24007, 606208, 606209, 700001, 1212417, 1500003, 2000000])
 @pytest.mark.parametrize("values", ["normal", "zeros", "no range"] + sorted(TINY))
