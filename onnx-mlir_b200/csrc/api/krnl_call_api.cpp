@@ -598,7 +598,7 @@ void omcudaDynamicQuantizeLinear(
   void *scr = dql_scratch_for(sg);
   if (!sg.ok() || !scr)
     return;
-  sg.set(launch_dql(dx, n, dy, ds, dz, scr, st, 0));
+  sg.set(launch_dql(dx, n, dy, ds, dz, scr, st, true));
   sg.finish(false);
 }
 
@@ -981,7 +981,7 @@ void omcudaDynQuantLinear(OMTensor *Y, const OMTensor *X, const OMTensor *Wq,
     sg.set(launch_dql_small(
         dX, d.M, d.K, g.lda, xq, (int32_t *)g.a_rowsum, xs, xz, st));
   } else if (g.lda == d.K && !wzn) {
-    sg.set(launch_dql(dX, d.M * d.K, xq, xs, xz, scr, st, d.M));
+    sg.set(omcudaDevDynamicQuantizeLinear(dX, d.M * d.K, xq, xs, xz, scr, st));
   } else {
     sg.set(launch_dql_rows(
         dX, d.M, d.K, g.lda, xq, (int32_t *)g.a_rowsum, xs, xz, scr, st));

@@ -69,7 +69,8 @@ __device__ __forceinline__ void block_range(float &lo, float &hi) {
 // registers for all loads of a run at once.  With the 32 of a full SM the compiler makes two or
 // three round trips of them, all that a few blocks have to do: linear 128 x 4096 x 4096 17.9 ->
 // 15.3 us, 64 x 8192 x 8192 24.3 -> 22.0, 700 x 768 x 768 11.3 -> 10.3, 777 x 1001 x 1537 17.3 -> 16.2;
-// DynamicQuantizeLinear of 600000 values 5.2 -> 4.6, 6 M 11.9 -> 10.8, 64 Mi 92.9 -> 90.8.
+// DynamicQuantizeLinear of 600000 values 5.2 -> 4.6, 6 M 11.9 -> 10.8, 64 Mi 92.9 -> 90.8 (all on the
+// same values call after call, of which L2 keeps some).
 template <bool kFull, bool kZero, int kThreads, bool kDeep>
 __global__ void __launch_bounds__(kThreads, kDeep ? 1024 / kThreads : 2048 / kThreads)
     dql_minmax_kernel(const float *__restrict__ x, int64_t n, float2 *__restrict__ part,
@@ -368,18 +369,19 @@ __device__ __noinline__ void quantize_pass_exact(
     y[j] = (uint8_t)one(__ldg(x + j));
 }
 
-// The pass above for many values, x 32-byte and y 8-byte aligned.  That kernel takes what
+// quantize_kernel's pass for many values, x 32-byte and y 8-byte aligned.  That kernel takes what
 // lies in L2 hardly faster than what comes from HBM (16 Mi values 11.5 us, 7.4 without its
 // arithmetic): it executes 72 instructions per float4, half of them predicates and 64-bit
 // addresses.  Here runs are whole (what is left goes group by group), the addresses of a
 // run are one pointer and constants, a load is 32 bytes a lane and a store 8.  Two groups a
-// thread: four take 79 registers, three blocks per SM and no less time.  Whole calls,
-// before and now: DynamicQuantizeLinear of 1 Mi values 5.2 -> 4.9 us, 6 M 13.2 -> 11.9,
-// 16 Mi 28.6 -> 24.5, 64 Mi 99.1 -> 91.3, 128 Mi 201 -> 184; a given scale 2 M 3.7 -> 2.9,
-// 64 Mi 52.6 -> 50.0 (6.7 TB/s).
+// thread: four take 79 registers, three blocks per SM and no less time.  Whole calls
+// on values that change from call to call, before this pass and the deeper loads of the reduction
+// and now: DynamicQuantizeLinear of 1 Mi values 6.0 -> 5.7 us, 6 M 13.1 -> 10.7, 16 Mi 28.8 -> 23.6,
+// 64 Mi 102.5 -> 93.7 (9 bytes a value: 6.4 TB/s), 128 Mi 208 -> 183; a given scale 2 M 3.5 -> 3.0,
+// 64 Mi 58.1 -> 53.3.
 constexpr int kWideGroups = 2;
 // Resident at once.  (Five leave 51 registers, and what then goes to memory costs
-// DynamicQuantizeLinear of 64 Mi 102 us instead of 92.)
+// DynamicQuantizeLinear of 64 Mi 102 us instead of 92, the same values call after call.)
 constexpr int kWideBlocksPerSm = 4;
 template <bool kSigned, bool kOnce>
 __global__ void __launch_bounds__(kDqlThreads, kWideBlocksPerSm)
@@ -896,9 +898,10 @@ int launch_quantize_pass(const float *x, int64_t n, uint8_t *y, const QuantSourc
   return OMCUDA_OK;
 }
 
-// DynamicQuantizeLinear's reduction alone.  deep_blocks: see `deep`.
+// DynamicQuantizeLinear's reduction alone.  roomy: the pass behind can wait for the registers of
+// deep blocks (see `deep`).
 int launch_range_parts(const float *x, int64_t n, void *scratch, RangeParts *parts,
-    cudaStream_t st, bool overlap, int64_t deep_blocks, int32_t *sums = nullptr, int zeros = 0) {
+    cudaStream_t st, bool overlap, bool roomy = true, int32_t *sums = nullptr, int zeros = 0) {
   float2 *part = scratch_parts(scratch);
   // Runs of one to eight float4 a thread, so that about a third of the SMs has a
   // block until those are full: no block without work, whose empty partial every
@@ -926,9 +929,8 @@ int launch_range_parts(const float *x, int64_t n, void *scratch, RangeParts *par
     grid = small_blocks < 1 ? 1 : small_blocks;
   // All loads of a run in flight, except where the blocks are one to two per SM: more of
   // them than fit with those registers beside what else is resident (3.1 M values 6.8 us
-  // without, 8.3 with; 6 M 11.9 and 10.8).  Full runs of fewer blocks too leave the pass
-  // that is set up meanwhile too little room, from as many as the caller says.
-  const bool deep = grid <= deep_blocks || grid > 2 * sm_count();
+  // without, 8.3 with; 6 M 11.9 and 10.8).
+  const bool deep = (roomy && grid <= sm_count()) || grid > 2 * sm_count();
   const auto kernel =
       few     ? (sums ? dql_minmax_kernel<false, true, kRangeFewThreads, true>
                       : dql_minmax_kernel<false, false, kRangeFewThreads, true>)
@@ -962,15 +964,19 @@ int launch_dql_rows(const float *x, int64_t rows, int64_t cols, int64_t pitch, u
   }
   RangeParts parts;
   const int64_t blocks = warps ? ceil_div(rows, kDqlThreads / 32) : rows * split;
-  // The reduction's blocks take half the registers of an SM if deep: as long as the pass finds
-  // SMs without one (linears, deep and not: 900 x 1001 x 768 13.8 and 13.1 us, 777 x 1385 x 2048
-  // 17.2 and 16.4, 1544 x 1385 x 768 18.2 and 17.4, but 777 x 1001 x 2048 14.4 and 14.5).
+  const int vec_in = ((uintptr_t)x & 15u) == 0 && cols % 4 == 0;
+  // The reduction's blocks take half the registers of an SM if deep, which pays but in front of
+  // long rows that a warp each takes value by value: those take longest and want to be in
+  // place.  Linears, deep and not: 900 x 1001 x 768 13.0 and 12.4 us, 777 x 1385 x 1024 14.6 and 13.9, 650 x
+  // 3001 x 1024 20.0 and 18.6, 1544 x 1385 x 768 17.5 and 16.6, but of shorter rows 1500 x 501 x 3072 14.5
+  // and 15.5, 1200 x 801 x 1024 13.8 and 14.1, with four values a load 1544 x 768 x 3072 18.4 and 19.6, 700 x
+  // 1536 x 1024 13.8 and 14.2, a block per row 147 x 9001 x 2048 21.6 and 23.0, 300 x 4800 x 1600 16.5 and 17.1.
+  const bool roomy = !(warps && !vec_in && cols >= 1000);
   int rc = launch_range_parts(x, rows * cols, scratch, &parts, st, pdl_pays(rows * cols),
-      sm_count() - blocks, split > 1 ? rowsum : nullptr, (int)rows);
+      roomy, split > 1 ? rowsum : nullptr, (int)rows);
   if (rc != OMCUDA_OK)
     return rc;
   const int64_t cap = (int64_t)sm_count() * 8;
-  const int vec_in = ((uintptr_t)x & 15u) == 0 && cols % 4 == 0;
   OMCUDA_CHECK(launch_pdl(warps       ? quantize_rows_kernel<1, false>
                           : split > 1 ? quantize_rows_kernel<8, true>
                                       : quantize_rows_kernel<8, false>,
@@ -1072,7 +1078,7 @@ extern "C" int64_t omcudaDevDqlScratchBytes(int64_t) {
 }
 
 int omcuda::launch_dql(const float *x, int64_t n, uint8_t *y, float *y_scale, uint8_t *y_zp,
-    void *scratch, cudaStream_t st, int64_t rows) {
+    void *scratch, cudaStream_t st, bool alone) {
   if (n < 0 || (n > 0 && (!x || !y)) || !scratch)
     return fail(OMCUDA_EINVAL, "DynamicQuantizeLinear: bad argument");
   if (dql_small_wanted(1, n) ||
@@ -1082,13 +1088,7 @@ int omcuda::launch_dql(const float *x, int64_t n, uint8_t *y, float *y_scale, ui
   // Set up early whatever the size where what runs before is as a rule a pass like this
   // (64 Mi values 100.7 -> 99.0 us), but not behind a GEMM of a long linear, whose SMs its
   // blocks would take (8192 x 4096 x 4096 149 and 155).
-  // Deep blocks of the reduction beside those of the pass, two per SM: by itself and in front of
-  // a product of tiles up to some 60 (DynamicQuantizeLinear, deep and not: 900000 values 4.8 and
-  // 5.1 us, 1.2 M 5.4 and 5.3, 2 M 6.0 and 5.6; linear 1024 x 768 x 768 10.4 and 10.5, 1100 x 1384 x
-  // 768 14.5 and 14.2, 2000 x 1024 x 768 12.8 and 12.4); in front of one of few rows, which is next
-  // to be set up, one per SM (200 x 8192 x 4096 23.5 and 23.9, 128 x 14336 x 768 13.7 and 13.9).
-  const int64_t deep = rows > 0 && rows <= 256 ? sm_count() : sm_count() * 2 / 5;
-  int rc = launch_range_parts(x, n, scratch, &parts, st, rows == 0 || pdl_pays(n), deep);
+  int rc = launch_range_parts(x, n, scratch, &parts, st, alone || pdl_pays(n));
   if (rc != OMCUDA_OK)
     return rc;
   return launch_quantize_pass<false>(x, n, y, QuantSource{parts, nullptr, nullptr, nullptr},
@@ -1097,7 +1097,7 @@ int omcuda::launch_dql(const float *x, int64_t n, uint8_t *y, float *y_scale, ui
 
 extern "C" int omcudaDevDynamicQuantizeLinear(const float *x, int64_t n,
     uint8_t *y, float *y_scale, uint8_t *y_zp, void *scratch, void *stream) {
-  return launch_dql(x, n, y, y_scale, y_zp, scratch, (cudaStream_t)stream, 1);
+  return launch_dql(x, n, y, y_scale, y_zp, scratch, (cudaStream_t)stream, false);
 }
 
 extern "C" int omcudaDevRangeFold(const float *x, int64_t n, void *range, void *stream) {

@@ -55,9 +55,9 @@ inline bool ranges_overlap(const void *a, int64_t a_bytes, const void *b, int64_
 int launch_dql_rows(const float *x, int64_t rows, int64_t cols, int64_t pitch, uint8_t *y,
     int32_t *rowsum, float *y_scale, uint8_t *y_zp, void *scratch, cudaStream_t st);
 
-// omcudaDevDynamicQuantizeLinear; rows: of the product behind, 0: an operator by itself.
+// omcudaDevDynamicQuantizeLinear; alone: as an operator by itself.
 int launch_dql(const float *x, int64_t n, uint8_t *y, float *y_scale, uint8_t *y_zp,
-    void *scratch, cudaStream_t st, int64_t rows);
+    void *scratch, cudaStream_t st, bool alone);
 
 // The same in one launch, without scratch, for a tensor that one cluster holds in
 // its registers.  [rows, cols] into rows of `pitch` bytes as above, or one row
