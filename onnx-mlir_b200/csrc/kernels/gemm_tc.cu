@@ -437,8 +437,7 @@ __device__ __forceinline__ void prefetch_residual(const EpiParams &p, int64_t m,
 //
 // kLines: Y takes the TMA stores.  Kernels of their own, although the code differs only behind
 // the arithmetic: with that for other pitches beside it a launch took up to 4 % longer
-// (QLinearMatMul 4096 x 480 x 3072 19.5 us, 18.6 apart, 2378 x 480 x 3072 15.0 and 14.5; the
-// others gain too: 16384 x 768 x 3001 130 with the rows one by one, 109 now).
+// (QLinearMatMul 4096 x 480 x 3072 19.5 us, 18.6 apart, 2378 x 480 x 3072 15.0 and 14.5).
 template <int BN, int EPI, int EW, bool kLines, typename Release>
 __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
     const EpiScalars &sc, const QuantConsts &qc, uint32_t taddr, const WarpPlace &at,
@@ -601,9 +600,10 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
       // The row pitch of Y is not a multiple of 16 bytes (a ragged N), so no TMA
       // store: a 32 x 32 block passes through the slab and every row leaves as
       // one coalesced warp-wide store, instead of 32 rows in 32 sectors each.  Eight rows
-      // together, their words asked for before the first leaves (before, row after row:
-      // QLinearMatMul 16384 x 768 x 3001 99.7 -> 84.0 us, 2000 x 1024 x 1537 18.9 -> 17.5, linear
-      // 16384 x 768 x 1537 79.6 -> 75.1; sixteen gain no more).
+      // together, their words asked for before the first leaves (row after row in the kernel of
+      // both ways out, and so; inputs that change from call to call: QLinearMatMul 16384 x 768 x 3001
+      // 131.9 -> 110.8 us, 2000 x 1024 x 1537 18.4 -> 16.5, linear 16384 x 768 x 1537 82.3 -> 74.9;
+      // sixteen gain no more).
       if (kSplit) {
         if (lane >= rows)
           continue;
@@ -973,7 +973,11 @@ __global__ void __launch_bounds__(tc_threads(EW), 1)
   const int num_kb = (int)ceil_div(p.K, kBK);
   // Split-K pass: unit u is K slice u % split of tile u / split (all units
   // whole tiles then).
-  const int split = tc_splits_k(BN, EPI, EW) ? p.split_k : 1;
+  // (To bytes of a ragged N the division stays: without it the compiler lays the same epilogue out
+  // differently, QLinearMatMul 16384 x 768 x 3001 108.8 -> 110.8 us, 14615 x 303 x 947 45.4 -> 46.0, 9000 x
+  // 2000 x 777 32.9 -> 33.4, and the first tile gains nothing: 2000 x 1024 x 1537 16.5 either way.)
+  constexpr bool kDivides = tc_splits_k(BN, EPI, EW) || (EPI == OMCUDA_EPI_REQUANT && !kLines);
+  const int split = kDivides ? p.split_k : 1;
   if (threadIdx.x == 32) { // (a thread that has nothing else to set up)
     prefetch_tensormap(&map_a);
     prefetch_tensormap(&map_b);
