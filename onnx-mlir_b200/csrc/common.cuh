@@ -364,7 +364,9 @@ __device__ __forceinline__ void range_block_init(RangeBlock &b, int warps) { // 
   b.hi = 0;
   b.left = warps;
 }
-constexpr unsigned kRangeFirstBlocks = 4 * 148; // about as many as start together
+// About as many as start together on the 148 SMs of a B200.  It decides on speed alone, so what
+// the device really has is not handed to every kernel.
+constexpr unsigned kRangeFirstBlocks = 4 * 148;
 // Behind a barrier of the block that follows range_block_init.  block: this one's number.
 __device__ __forceinline__ void range_commit_block(
     RangeBlock &b, uint32_t *range, float lo, float hi, unsigned block) {

@@ -52,7 +52,7 @@
 // with a CTA barrier between any two phases: of some 5100 clocks per block 1180 were
 // spent issuing copies and waking up, and 2600 more per item on its results.  Now warps
 // of their own issue products and copies, mbarriers stand between the phases and the
-// results are out of V's way (two CTAs share the SM: 1536 clocks of MMAs per block each).
+// results are out of V's way (two CTAs share the SM: the tensor pipe counts 1536 clocks per block and CTA).
 // Batch x sequence x heads, us: 256 x 512 x 16 829 -> 741, 64 x 384 x 16 124 -> 113, 1 x 512 x
 // 16 13.8 -> 12.4, 32 x 128 x 12 11.6 -> 11.5, 1024 x 128 x 16 336 -> 325 (HBM).  The largest runs
 // at the power limit, clocks at 1.35 GHz.  Every sum is in the order it was in.

@@ -455,7 +455,10 @@ namespace {
 
 // Overlapped, its blocks are kept apart: behind a GEMM whose CTAs fill their SMs, 512 blocks of
 // 8 rows of 768 took 9.5 us (in a row of their own 6.9), so 8.2; encoder base 32 x 128 1350 -> 1315
-// us, large 4 x 512 2439 -> 2323; of few rows base 2 x 128 517 -> 515.
+// us, large 4 x 512 2439 -> 2323; of few rows base 2 x 128 517 -> 515.  Also where its registers let in
+// no more than the grid comes to (five per SM of 768 columns, four of 1024): the memory keeps blocks
+// off SMs that a CTA of the GEMM still holds, too (base 50 x 128 tokens, six per SM, 1819 us without and
+// 1790, large 13 x 384, five, 4235 and 4197, base 40 x 128, five, 1428 and 1425).
 template <int NV, bool kFew>
 int launch_layernorm_vec(const float *x, const float *residual, int64_t rows, const float *gamma,
     const float *beta, float eps, float *y, uint32_t *range, unsigned warps, cudaStream_t st) {
@@ -463,7 +466,7 @@ int launch_layernorm_vec(const float *x, const float *residual, int64_t rows, co
   const bool overlap = pdl_pays(rows * NV * 128);
   const int64_t blocks = ceil_div(rows, warps), per_sm = ceil_div(blocks, (int64_t)sm_count());
   size_t spread = 0;
-  if (overlap && per_sm < 8) { // (eight fit without it)
+  if (overlap && per_sm < 8) { // (up to about two rounds of blocks)
     static PerDeviceInt can; // 1: yes, 2: no
     if (!can.get()) {
       can.set(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -602,7 +602,7 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
       // one coalesced warp-wide store, instead of 32 rows in 32 sectors each.  Eight rows
       // together, their words asked for before the first leaves (row after row in the kernel of
       // both ways out, and so; inputs that change from call to call: QLinearMatMul 16384 x 768 x 3001
-      // 131.9 -> 110.8 us, 2000 x 1024 x 1537 18.4 -> 16.5, linear 16384 x 768 x 1537 82.3 -> 74.9;
+      // 131.9 -> 108.8 us, 2000 x 1024 x 1537 18.4 -> 16.4, linear 16384 x 768 x 1537 82.3 -> 74.5;
       // sixteen gain no more).
       if (kSplit) {
         if (lane >= rows)
@@ -664,9 +664,9 @@ __device__ __forceinline__ void epilogue_tile(const EpiParams &p,
 // ---- the kernel -------------------------------------------------------------------
 
 // Whether split-K passes are made with a kernel (launch_split_k): raw sums, the widest tiles,
-// eight warps on the epilogue.  In the others the count of slices is 1 for the compiler, which
-// takes the divisions by it out of what every warp does before its first tile, 0.2 to 0.4 us of a
-// launch: QLinearMatMul 2000 x 1024 x 2048 12.4 -> 12.1 us, 1100 x 480 x 1536 7.2 -> 6.9, 16384 x 1024 x
+// eight warps on the epilogue.  In the others, one kind of pair kernel aside, the count of slices
+// is 1 for the compiler, which takes the divisions by it out of what every warp does before its first
+// tile, 0.2 to 0.4 us of a launch: QLinearMatMul 2000 x 1024 x 2048 12.4 -> 12.1 us, 1100 x 480 x 1536 7.2 -> 6.9, 16384 x 1024 x
 // 4096 62.3 -> 61.6, linear 777 x 1001 x 1537 15.2 -> 14.9, 4096 x 4096 x 4096 73.6 -> 72.9.
 __host__ __device__ constexpr bool tc_splits_k(int bn, int epi, int ew) {
   return bn == 256 && epi == OMCUDA_EPI_I32 && ew == 8;

@@ -304,8 +304,9 @@ bool linear_rows_wanted(int64_t M, int64_t N, int64_t kp) {
   // 8192 x 8192 16.8 and 11.6 with the weight in L2, 19.5 and 16.7 beyond, 2 x 4096 x 14336
   // 15.4 and 11.0, 18.1 and 15.7, 15 x 2176 x 15360 17.4 and 9.7, 19.7 and 12.1, 5 x 1650 x 5419
   // 9.0 and 8.2, 9.3 and 8.2.  Calls with more that may take scratch are therefore two
-  // kernels, but for zero points per column (2 x 8192 x 8192 17.1 and 12.4, 19.7 and 17.2: one
-  // launch is what their callers have counted on).
+  // kernels.  With zero points per column two would be faster as well (2 x 8192 x 8192 17.1 and 12.4,
+  // 19.7 and 17.2), but such a call has always been one launch and is held to that by the test
+  // that counts them (test_linear_of_few_rows_values).
   if (M < 2 || M > kRowsMax || N > (int64_t)1 << 24)
     return false;
   if (M * kp > 16384 && (M * kp > 32768 || N < 1024 * M))

@@ -82,7 +82,7 @@ __device__ __forceinline__ QuantConsts make_quant_consts(
   c.x_hi = __fmul_rn(QuantBounds<kSigned>::hi - c.zp_f + 0.25f, scale);
   // The shortcut needs a normal, finite reciprocal and residuals that do not
   // underflow; anything else (scale 0 from an all-zero tensor, negative,
-  // denormal or huge scales) takes the exact path.
+  // denormal or huge scales) takes another path to the same results.
   c.fast = (scale > 1e-30f) && (scale < 1e30f);
   return c;
 }
@@ -127,8 +127,8 @@ __device__ __noinline__ uint32_t quantize_four_exact(
 // above, rounded half-even by adding kQuantMagic, the zero point added to that,
 // and the result is the low byte (two's complement for the signed type) of the
 // mantissa.  About six arithmetic instructions an element; with the moves in and out of
-// packed pairs, predicates, addresses and the fold of the partials quantize_kernel executes 18
-// (4096 x 4096 values).  (An approximate quotient with
+// packed pairs, predicates, addresses and the fold of the partials quantize_kernel executed 18 on
+// 16 Mi values, which are quantize_wide_kernel's now: 8.5.  (An approximate quotient with
 // the exact divide for elements near a tie costs less on paper, but with a test
 // at 0.499 a fifth of the warps had such an element among their 128 and took the
 // divide: 16 Mi values 16.4 us, 7.3 without any arithmetic.)
